@@ -17,8 +17,8 @@
 // reference.
 //
 // Accumulation of S_D:
-//   INT mode  (weights and offset integral, |w - offset| <= 2^22): exact
-//             integer sums, so any order gives the reference's doubles.
+//   INT mode  (SumMode::exact, engine.cuh): exact integer sums of fixed-point
+//             units, so any order gives the reference's doubles.
 //   FP64 mode: degree <= 1000 adds in adjacency order (the reference's
 //             sequential flat_hash_map path, bit-exact); hubs add in any
 //             order, as the reference's concurrent map does.
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(256) BestMoveGroupKernel(BMArgs a, const uint3
     double S;
     if (kInt) {
       const int xi = cand ? (WeightToInt(wt) - a.ioffset) : 0;
-      S = static_cast<double>(GroupSumInt(peers, xi, a.w == nullptr, leader, reinterpret_cast<int*>(stage[warp])));
+      S = static_cast<double>(GroupSumInt<int>(peers, xi, a.w == nullptr, leader, reinterpret_cast<int*>(stage[warp])));
     } else {
       stage[warp][lane] = cand ? Dsub(static_cast<double>(wt), a.offset) : 0.0;
       __syncwarp();
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) BestMoveWarpKernel(BMAr
       }
       if (kInt) {
         const int xi = cand ? (WeightToInt(wt) - a.ioffset) : 0;
-        const int S = GroupSumInt(peers, xi, a.w == nullptr, leader, reinterpret_cast<int*>(stage));
+        const int S = GroupSumInt<int>(peers, xi, a.w == nullptr, leader, reinterpret_cast<int*>(stage));
         if (slot != kNone) vals[slot] += static_cast<unsigned long long>(static_cast<long long>(S));
       } else {
         stage[lane] = cand ? Dsub(static_cast<double>(wt), a.offset) : 0.0;
@@ -301,16 +301,16 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) BestMoveWarpKernel(BMAr
 // arithmetic onto the certified path (an FP64 warp instruction costs ~19
 // SM cycles on this GPU).  Both return whether the vertex must be appended
 // to the movers list; in replay mode they also run the self-check.
-template <int G>
+template <int G, typename V>
 __device__ __noinline__ bool GroupExact(const BMArgs& a, const VertexCtx& x, bool fp64, bool contender, unsigned gl,
-                                        int T, int S, double KD, uint32_t cu, bool replay, int cres,
+                                        V T, V S, double KD, uint32_t cu, bool replay, int cres,
                                         uint32_t cmove) {
   double change = 0.0, val = -CUDART_INF;
   uint32_t id = kNone;
   if (fp64) {
-    change = ChangeOf(a, x, static_cast<double>(T));
+    change = ChangeOf(a, x, UnitsToDouble<V>(a, T));
     if (contender) {
-      val = ValOf(a, x, change, static_cast<double>(S), KD);
+      val = ValOf(a, x, change, UnitsToDouble<V>(a, S), KD);
       id = cu;
     }
   }
@@ -337,14 +337,14 @@ __device__ __noinline__ bool WarpExact(const BMArgs& a, const VertexCtx& x, V T,
                                        const V* vals, const uint16_t* used, uint32_t nused, bool replay, int cres,
                                        uint32_t cmove) {
   const unsigned lane = LaneId();
-  const double change = ChangeOf(a, x, static_cast<double>(T));
+  const double change = ChangeOf(a, x, UnitsToDouble<V>(a, T));
   double best = -CUDART_INF;
   uint32_t bid = kNone;
   for (uint32_t i = lane; i < nused; i += 32) {
     const uint32_t slot = used[i];
     if (slot == 0xFFFFu) continue;
     const uint32_t key = keys[slot];
-    const double val = ValOf(a, x, change, static_cast<double>(vals[slot]), a.K[key]);
+    const double val = ValOf(a, x, change, UnitsToDouble<V>(a, vals[slot]), a.K[key]);
     if (Better(val, key, best, bid)) {
       best = val;
       bid = key;
@@ -368,11 +368,18 @@ __device__ __noinline__ bool WarpExact(const BMArgs& a, const VertexCtx& x, V T,
   return append;
 }
 
-template <int G>
+template <typename V>
+__device__ __forceinline__ V WarpMaxV(V x) {
+  if constexpr (sizeof(V) == 4) return __reduce_max_sync(kFull, x);
+  else return WarpMaxLL(x);
+}
+
+// V: int when every sum of a row fits in 32 bits, else long long.
+template <int G, typename V>
 __global__ void __launch_bounds__(256) CertGroupKernel(BMArgs a, const uint32_t* __restrict__ list,
                                                       const uint32_t* __restrict__ bin_counts,
                                                       const uint32_t* __restrict__ bin_starts, int bin) {
-  __shared__ int stage[8][32];
+  __shared__ V stage[8][32];
   __shared__ uint32_t mover_buf[8][64];
   WarpMoverBuffer mb{mover_buf[threadIdx.x >> 5]};
   const uint32_t count = bin_counts[bin];
@@ -414,21 +421,21 @@ __global__ void __launch_bounds__(256) CertGroupKernel(BMArgs a, const uint32_t*
     const uint32_t cu = cand ? __ldg(a.C + u) : kNone;
     const unsigned peers = __match_any_sync(kFull, cand ? cu : LaneSentinel(lane)) & gmask;
     const bool leader = cand && int(lane) == __ffs(peers) - 1;
-    const int xi = cand ? (WeightToInt(wt) - a.ioffset) : 0;
-    const int S = GroupSumInt(peers, xi, unit, leader, stage[warp]);
+    const V xi = cand ? EntryUnits<V, true>(a, wt) : V(0);
+    const V S = GroupSumInt<V>(peers, xi, unit, leader, stage[warp]);
     const unsigned tmask = __ballot_sync(kFull, leader && cu == x.c) & gmask;
-    const int Tsh = __shfl_sync(kFull, S, tmask ? __ffs(tmask) - 1 : int(lane));
-    const int T = tmask ? Tsh : 0;  // group sums stay below 2^29 in INT mode
-    int smax = leader ? S : INT_MIN;
+    const V Tsh = __shfl_sync(kFull, S, tmask ? __ffs(tmask) - 1 : int(lane));
+    const V T = tmask ? Tsh : V(0);
+    V smax = leader ? S : (sizeof(V) == 4 ? V(INT_MIN) : V(LLONG_MIN));
     if constexpr (G == 32) {
-      smax = __reduce_max_sync(kFull, smax);
+      smax = WarpMaxV<V>(smax);
     } else {
 #pragma unroll
       for (int o = G / 2; o >= 1; o >>= 1) smax = max(smax, __shfl_xor_sync(kFull, smax, o));
     }
     const float k32 = vvalid ? a.kf[x.v] : 0.f;
     const float Kc32 = vvalid ? a.Kf[x.c] : 0.f;
-    const ChangeApproxT<int> ca = ApproxChange<int>(Res32Of(a, x.v), a.int_nw != 0, k32, Kc32, T);
+    const ChangeApproxT<V> ca = ApproxChange<V>(Res32Of(a, x.v), a.int_nw != 0, k32, Kc32, T);
     const float cabs = ChangeAbsBound(ca);
     // FP32 pre-filter over the group's leaders.
     FilterVal f{0.f, 0.f, false};
@@ -436,7 +443,7 @@ __global__ void __launch_bounds__(256) CertGroupKernel(BMArgs a, const uint32_t*
     float lo = -CUDART_INF_F;
     if (leader) {
       KfD = a.Kf[cu];
-      f = FilterOf<int>(Res32Of(a, x.v), k32, KfD, S, smax, cabs);
+      f = FilterOf<V>(Res32Of(a, x.v), k32, KfD, S, smax, cabs);
       if (f.sane) lo = __fsub_rn(f.Y, f.e);
     }
     float U = lo;
@@ -448,7 +455,7 @@ __global__ void __launch_bounds__(256) CertGroupKernel(BMArgs a, const uint32_t*
     }
     const bool contender = leader && (!f.sane || __fadd_rn(f.Y, f.e) >= U);
     // The leading (S, K) class of the contenders and the trailing one.
-    LexKeyT<int> lead, tail;
+    LexKeyT<V> lead, tail;
     double KD = 0.0;
     if (contender) {
       KD = a.K[cu];
@@ -458,7 +465,7 @@ __global__ void __launch_bounds__(256) CertGroupKernel(BMArgs a, const uint32_t*
     }
     bool single;
     if constexpr (G == 32) {
-      single = LexWarpLeadInt(lead, tail);
+      single = LexWarpLead<V>(lead, tail);
     } else {
       LexGroupReduce<G>(lead);
       LexGroupReduce<G>(tail);
@@ -468,14 +475,14 @@ __global__ void __launch_bounds__(256) CertGroupKernel(BMArgs a, const uint32_t*
     uint32_t ctarget = kNone;
     if (vvalid && single) {
       const float KfA = lead.id != kNone ? a.Kf[lead.id] : 0.f;
-      cres = CertifyDecision<int>(ca, Res32Of(a, x.v), k32, lead.id != kNone, lead.S, KfA, lead.id, a.n, &ctarget);
+      cres = CertifyDecision<V>(ca, Res32Of(a, x.v), k32, lead.id != kNone, lead.S, KfA, lead.id, a.n, &ctarget);
     }
     const uint32_t cmove = cres == kUncertain ? kNone : CertifiedMove(a, x, ctarget, cres == kCertMove);
     const bool fp64 = vvalid && (replay || cres == kUncertain);
     bool append = false;
     if (vvalid && !fp64 && gl == 0) append = ApplyCertified(a, x, cmove);
     if (__ballot_sync(kFull, fp64)) {
-      const bool app = GroupExact<G>(a, x, fp64, contender, gl, T, S, KD, cu, replay, cres, cmove);
+      const bool app = GroupExact<G, V>(a, x, fp64, contender, gl, T, S, KD, cu, replay, cres, cmove);
       append = append || app;
     }
     mb.Add(&a.ctr->movers, a.movers, append, x.v);
@@ -500,7 +507,7 @@ constexpr size_t CertWarpSmem() {
 // its integer weight with a shared-memory atomic: INT-mode sums are exact in
 // any order, and grouping equal clusters first with match.any cost more than
 // the atomics it saves.
-template <int HC, typename V>
+template <int HC, typename V, bool kConv = sizeof(V) == 8>
 __global__ void __launch_bounds__(kWarpKernelWarps * 32) CertWarpKernel(BMArgs a, const uint32_t* __restrict__ list,
                                                                        const uint32_t* __restrict__ bin_counts,
                                                                        const uint32_t* __restrict__ bin_starts,
@@ -543,7 +550,7 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) CertWarpKernel(BMArgs a
       fam_v += 1;
     }
     uint32_t nused = 0;  // used[] entries (warp-uniform)
-    int tpart = 0;       // this lane's part of T (entries in the vertex's own cluster)
+    V tpart = 0;         // this lane's part of T (entries in the vertex's own cluster)
     for (uint32_t e0 = 0; e0 < x.d; e0 += 32 * kCertUnroll) {
       uint32_t uu[kCertUnroll], cc[kCertUnroll];
       float ww[kCertUnroll];
@@ -576,17 +583,16 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) CertWarpKernel(BMArgs a
         if (ins) used[nused + __popc(im & LaneMaskLt())] = static_cast<uint16_t>(slot);
         nused += __popc(im);
       }
-      const int xi = cand ? (WeightToInt(wt) - a.ioffset) : 0;
+      const V xi = cand ? EntryUnits<V, kConv>(a, wt) : V(0);
       if (cand && cu == x.c) tpart += xi;
       if (slot != kNone) {
         if constexpr (sizeof(V) == 4) atomicAdd(reinterpret_cast<int*>(&vals[slot]), xi);
-        else atomicAdd(reinterpret_cast<unsigned long long*>(&vals[slot]), static_cast<unsigned long long>(static_cast<long long>(xi)));
+        else atomicAdd(reinterpret_cast<unsigned long long*>(&vals[slot]), static_cast<unsigned long long>(xi));
       }
       __syncwarp();
       }
     }
-    // T: the lanes' own-cluster parts (a lane's part is at most
-    // ceil(1000 / 32) weights of |w - offset| <= 2^22, so it fits an int).
+    // T: the lanes' own-cluster parts.
     V T;
     if constexpr (sizeof(V) == 4) {
       T = __reduce_add_sync(kFull, tpart);
@@ -620,13 +626,7 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) CertWarpKernel(BMArgs a
       }
     }
     for (uint32_t i = lane + 32 * kCertRegRounds; i < nused; i += 32) vmax = max(vmax, vals[used[i]]);
-    if constexpr (sizeof(V) == 4) {
-      vmax = __reduce_max_sync(kFull, vmax);
-    } else {
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) vmax = max(vmax, __shfl_xor_sync(kFull, vmax, o));
-    }
-    const V smax = vmax;
+    const V smax = WarpMaxV<V>(vmax);
     float U = -CUDART_INF_F;
     // The two largest upper ends (Y + e; +inf outside the error model) of
     // this lane's candidates and the index of the largest: when the second
@@ -706,14 +706,7 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) CertWarpKernel(BMArgs a
       lead.Keep(S, ko, key);
       tail.Keep(-S, ~ko, key);
     }
-    bool single;
-    if constexpr (sizeof(V) == 4) {
-      single = LexWarpLeadInt(lead, tail);
-    } else {
-      LexGroupReduce<32>(lead);
-      LexGroupReduce<32>(tail);
-      single = lead.id == kNone || (-tail.S == lead.S && ~tail.K == lead.K);
-    }
+    const bool single = LexWarpLead<V>(lead, tail);
     int cres = kUncertain;
     uint32_t ctarget = kNone;
     if (single) {
@@ -762,18 +755,7 @@ constexpr size_t CertCtaSmem() {
   return size_t(HC) * (sizeof(V) + 4 + 2);  // vals, keys, used
 }
 
-template <typename V>
-__device__ __forceinline__ V WarpMaxV(V x) {
-  if constexpr (sizeof(V) == 4) {
-    return __reduce_max_sync(kFull, x);
-  } else {
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) x = max(x, __shfl_xor_sync(kFull, x, o));
-    return x;
-  }
-}
-
-template <int HC, typename V>
+template <int HC, typename V, bool kConv = sizeof(V) == 8>
 __global__ void __launch_bounds__(kCtaWarps * 32) CertCtaKernel(BMArgs a, const uint32_t* __restrict__ list,
                                                                const uint32_t* __restrict__ bin_counts,
                                                                const uint32_t* __restrict__ bin_starts, int bin) {
@@ -849,13 +831,13 @@ __global__ void __launch_bounds__(kCtaWarps * 32) CertCtaKernel(BMArgs a, const 
           base = __shfl_sync(kFull, base, first);
           if (ins) used[base + __popc(im & LaneMaskLt())] = static_cast<uint16_t>(slot);
         }
-        const int xi = cand ? (WeightToInt(ww[k]) - a.ioffset) : 0;
+        const V xi = cand ? EntryUnits<V, kConv>(a, ww[k]) : V(0);
         if (slot != kNone) {
           if constexpr (sizeof(V) == 4)
             atomicAdd(reinterpret_cast<int*>(&vals[slot]), xi);
           else
             atomicAdd(reinterpret_cast<unsigned long long*>(&vals[slot]),
-                      static_cast<unsigned long long>(static_cast<long long>(xi)));
+                      static_cast<unsigned long long>(xi));
         }
       }
     }
@@ -929,13 +911,8 @@ __global__ void __launch_bounds__(kCtaWarps * 32) CertCtaKernel(BMArgs a, const 
       lead.Keep(S, ko, key);
       tail.Keep(-S, ~ko, key);
     }
-    if constexpr (sizeof(V) == 4) {
-      LexWarpLeaderInt(lead);
-      LexWarpLeaderInt(tail);
-    } else {
-      LexGroupReduce<32>(lead);
-      LexGroupReduce<32>(tail);
-    }
+    LexWarpLeader<V>(lead);
+    LexWarpLeader<V>(tail);
     if (lane == 0) {
       s_ls[warp] = lead.S;
       s_lk[warp] = lead.K;
@@ -1080,10 +1057,17 @@ Status LaunchAll(Context* ctx, const BMArgs& a, const uint32_t* list, const uint
       PCC_COUNT(1);
       return Status::Ok();
     };
-    PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<4>, kBinG4, 64));
-    PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<8>, kBinG8, 32));
-    PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<16>, kBinG16, 16));
-    PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<32>, kBinG32, 8));
+    if (a.narrow || !a.conv) {  // 32 entries of at most 2^22 always fit
+      PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<4, int>, kBinG4, 64));
+      PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<8, int>, kBinG8, 32));
+      PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<16, int>, kBinG16, 16));
+      PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<32, int>, kBinG32, 8));
+    } else {
+      PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<4, long long>, kBinG4, 64));
+      PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<8, long long>, kBinG8, 32));
+      PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<16, long long>, kBinG16, 16));
+      PCC_RETURN_IF_ERROR(group_bin(CertGroupKernel<32, long long>, kBinG32, 8));
+    }
   } else {
     if (want(kBinG4) && !routed(kBinG4)) {
       BestMoveGroupKernel<4, kInt, kAsync><<<grid(kBinG4, 64, waves(sms * 8)), 256, 0, st>>>(a, list, counts, starts,
@@ -1111,30 +1095,27 @@ Status LaunchAll(Context* ctx, const BMArgs& a, const uint32_t* list, const uint
   for (int b = kBinG4; b <= kBinW1000; ++b) nw += want(b) && (b > kBinG32 || routed(b)) ? 1 : 0;
   if (families & kLaunchWarps) FamBegin(ctx, kFamWarp);
   if constexpr (kCert) {
-    if (a.narrow) {
-      PCC_RETURN_IF_ERROR(routed_bins(CertWarpKernel<256, int>, CertWarpSmem<256, int>(), sms * 16));
-      PCC_RETURN_IF_ERROR(cert_bin(CertWarpKernel<256, int>, CertWarpSmem<256, int>(), CertCtaKernel<256, int>,
-                   CertCtaSmem<256, int>(), kBinW128, sms * 16));
-      PCC_RETURN_IF_ERROR(cert_bin(CertWarpKernel<512, int>, CertWarpSmem<512, int>(), CertCtaKernel<512, int>,
-                   CertCtaSmem<512, int>(), kBinW256, sms * 8));
-      PCC_RETURN_IF_ERROR(cert_bin(CertWarpKernel<1024, int>, CertWarpSmem<1024, int>(), CertCtaKernel<1024, int>,
-                   CertCtaSmem<1024, int>(), kBinW512, sms * 6));
-      PCC_RETURN_IF_ERROR(cert_bin(CertWarpKernel<2048, int>, CertWarpSmem<2048, int>(), CertCtaKernel<2048, int>,
-                   CertCtaSmem<2048, int>(), kBinW1000, sms * 3));
+    // The certified warp bins for one sum type: int or long long sums, with
+    // (kConv) or without the general weight conversion.
+    auto cert_bins = [&](auto sum, auto conv) -> Status {
+      using V = decltype(sum);
+      constexpr bool kC = decltype(conv)::value;
+      PCC_RETURN_IF_ERROR(routed_bins(CertWarpKernel<256, V, kC>, CertWarpSmem<256, V>(), sms * 16));
+      PCC_RETURN_IF_ERROR(cert_bin(CertWarpKernel<256, V, kC>, CertWarpSmem<256, V>(), CertCtaKernel<256, V, kC>,
+                                   CertCtaSmem<256, V>(), kBinW128, sms * 16));
+      PCC_RETURN_IF_ERROR(cert_bin(CertWarpKernel<512, V, kC>, CertWarpSmem<512, V>(), CertCtaKernel<512, V, kC>,
+                                   CertCtaSmem<512, V>(), kBinW256, sms * 8));
+      PCC_RETURN_IF_ERROR(cert_bin(CertWarpKernel<1024, V, kC>, CertWarpSmem<1024, V>(), CertCtaKernel<1024, V, kC>,
+                                   CertCtaSmem<1024, V>(), kBinW512, sms * 4));
+      return cert_bin(CertWarpKernel<2048, V, kC>, CertWarpSmem<2048, V>(), CertCtaKernel<2048, V, kC>,
+                      CertCtaSmem<2048, V>(), kBinW1000, sms * 2);
+    };
+    if (!a.narrow) {
+      PCC_RETURN_IF_ERROR(cert_bins(0ll, std::true_type{}));
+    } else if (a.conv) {
+      PCC_RETURN_IF_ERROR(cert_bins(0, std::true_type{}));
     } else {
-      PCC_RETURN_IF_ERROR(routed_bins(CertWarpKernel<256, long long>, CertWarpSmem<256, long long>(), sms * 16));
-      PCC_RETURN_IF_ERROR(
-          cert_bin(CertWarpKernel<256, long long>, CertWarpSmem<256, long long>(), CertCtaKernel<256, long long>,
-                   CertCtaSmem<256, long long>(), kBinW128, sms * 16));
-      PCC_RETURN_IF_ERROR(
-          cert_bin(CertWarpKernel<512, long long>, CertWarpSmem<512, long long>(), CertCtaKernel<512, long long>,
-                   CertCtaSmem<512, long long>(), kBinW256, sms * 8));
-      PCC_RETURN_IF_ERROR(
-          cert_bin(CertWarpKernel<1024, long long>, CertWarpSmem<1024, long long>(), CertCtaKernel<1024, long long>,
-                   CertCtaSmem<1024, long long>(), kBinW512, sms * 4));
-      PCC_RETURN_IF_ERROR(
-          cert_bin(CertWarpKernel<2048, long long>, CertWarpSmem<2048, long long>(), CertCtaKernel<2048, long long>,
-                   CertCtaSmem<2048, long long>(), kBinW1000, sms * 2));
+      PCC_RETURN_IF_ERROR(cert_bins(0, std::false_type{}));
     }
   } else {
     PCC_RETURN_IF_ERROR(routed_bins(BestMoveWarpKernel<256, kInt, kAsync>, WarpKernelSmem<256>(), sms * 16));
@@ -1160,24 +1141,36 @@ Status PrepareBestMoveKernels() {
   static bool done = false;
   std::lock_guard<std::mutex> lk(mu);
   if (done) return Status::Ok();
-  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<4>, 0, 256));
-  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<8>, 0, 256));
-  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<16>, 0, 256));
-  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<32>, 0, 256));
+  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<4, int>, 0, 256));
+  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<8, int>, 0, 256));
+  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<16, int>, 0, 256));
+  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<32, int>, 0, 256));
+  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<4, long long>, 0, 256));
+  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<8, long long>, 0, 256));
+  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<16, long long>, 0, 256));
+  PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<32, long long>, 0, 256));
   constexpr int kW = kWarpKernelWarps * 32;
-  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<256, int>, CertWarpSmem<256, int>(), kW));
-  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<512, int>, CertWarpSmem<512, int>(), kW));
-  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<1024, int>, CertWarpSmem<1024, int>(), kW));
-  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<2048, int>, CertWarpSmem<2048, int>(), kW));
+  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<256, int, false>, CertWarpSmem<256, int>(), kW));
+  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<256, int, true>, CertWarpSmem<256, int>(), kW));
+  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<512, int, false>, CertWarpSmem<512, int>(), kW));
+  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<512, int, true>, CertWarpSmem<512, int>(), kW));
+  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<1024, int, false>, CertWarpSmem<1024, int>(), kW));
+  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<1024, int, true>, CertWarpSmem<1024, int>(), kW));
+  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<2048, int, false>, CertWarpSmem<2048, int>(), kW));
+  PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<2048, int, true>, CertWarpSmem<2048, int>(), kW));
   PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<256, long long>, CertWarpSmem<256, long long>(), kW));
   PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<512, long long>, CertWarpSmem<512, long long>(), kW));
   PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<1024, long long>, CertWarpSmem<1024, long long>(), kW));
   PCC_RETURN_IF_ERROR(Prep(CertWarpKernel<2048, long long>, CertWarpSmem<2048, long long>(), kW));
   constexpr int kC = kCtaWarps * 32;
-  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<256, int>, CertCtaSmem<256, int>(), kC));
-  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<512, int>, CertCtaSmem<512, int>(), kC));
-  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<1024, int>, CertCtaSmem<1024, int>(), kC));
-  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<2048, int>, CertCtaSmem<2048, int>(), kC));
+  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<256, int, false>, CertCtaSmem<256, int>(), kC));
+  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<256, int, true>, CertCtaSmem<256, int>(), kC));
+  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<512, int, false>, CertCtaSmem<512, int>(), kC));
+  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<512, int, true>, CertCtaSmem<512, int>(), kC));
+  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<1024, int, false>, CertCtaSmem<1024, int>(), kC));
+  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<1024, int, true>, CertCtaSmem<1024, int>(), kC));
+  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<2048, int, false>, CertCtaSmem<2048, int>(), kC));
+  PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<2048, int, true>, CertCtaSmem<2048, int>(), kC));
   PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<256, long long>, CertCtaSmem<256, long long>(), kC));
   PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<512, long long>, CertCtaSmem<512, long long>(), kC));
   PCC_RETURN_IF_ERROR(Prep(CertCtaKernel<1024, long long>, CertCtaSmem<1024, long long>(), kC));

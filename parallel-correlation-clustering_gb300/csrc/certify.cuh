@@ -63,7 +63,16 @@ __device__ __forceinline__ float I2F(int x) {
   const float fl = SmallIntToFloat(x & 0xFFFF);
   return __fadd_rn(__fmul_rn(fh, 65536.0f), fl);
 }
-__device__ __forceinline__ float I2F(long long x) { return __ll2float_rn(x); }
+// 64-bit sums: the leading 31 bits of |x| through the 32-bit form, then a
+// power-of-two scaling.  Truncating the rest and the one rounding stay
+// within 2^-24 + 2^-30 of x, inside the 2^-23 |x| that the bounds below
+// allow for the conversion of sums above 2^24 (smaller ones are exact).
+__device__ __forceinline__ float I2F(long long x) {
+  const unsigned long long m = static_cast<unsigned long long>(x < 0 ? -x : x);
+  const int k = max(0, 33 - __clzll(static_cast<long long>(m)));
+  const float f = __fmul_rn(I2F(int(m >> k)), __int_as_float((k + 127) << 23));
+  return x < 0 ? -f : f;
+}
 
 __device__ __forceinline__ bool SaneF(float z) {
   const float m = fabsf(z);
@@ -132,11 +141,41 @@ __device__ __forceinline__ void LexWarpLeaderInt(LexKeyT<int>& lead) {
   lead.id = id;
 }
 
+// The same for 64-bit sums: S by its high (signed) and low words.
+__device__ __forceinline__ long long WarpMaxLL(long long x) {
+  const int hi = __reduce_max_sync(kFull, int(x >> 32));
+  const unsigned lo = __reduce_max_sync(kFull, int(x >> 32) == hi ? unsigned(x) : 0u);
+  return static_cast<long long>((static_cast<unsigned long long>(static_cast<unsigned>(hi)) << 32) | lo);
+}
+__device__ __forceinline__ void LexWarpLeaderLL(LexKeyT<long long>& lead) {
+  const bool has = lead.id != kNone;
+  const long long sm = WarpMaxLL(has ? lead.S : LLONG_MIN);
+  const bool m1 = has && lead.S == sm;
+  const unsigned hi = static_cast<unsigned>(lead.K >> 32), lo = static_cast<unsigned>(lead.K);
+  const unsigned khi = __reduce_min_sync(kFull, m1 ? hi : 0xFFFFFFFFu);
+  const bool m2 = m1 && hi == khi;
+  const unsigned klo = __reduce_min_sync(kFull, m2 ? lo : 0xFFFFFFFFu);
+  const unsigned id = __reduce_min_sync(kFull, m2 && lo == klo ? lead.id : kNone);
+  if (id == kNone) {
+    lead = LexKeyT<long long>{};
+    return;
+  }
+  lead.S = sm;
+  lead.K = (static_cast<unsigned long long>(khi) << 32) | klo;
+  lead.id = id;
+}
+template <typename V>
+__device__ __forceinline__ void LexWarpLeader(LexKeyT<V>& lead) {
+  if constexpr (sizeof(V) == 4) LexWarpLeaderInt(lead);
+  else LexWarpLeaderLL(lead);
+}
+
 // The warp leader, and whether every lane's trailing contender (`tail`,
 // kept with (-S, ~K)) lies in the leader's (S, K) class, i.e. the test the
 // butterfly over `tail` decided.
-__device__ __forceinline__ bool LexWarpLeadInt(LexKeyT<int>& lead, const LexKeyT<int>& tail) {
-  LexWarpLeaderInt(lead);
+template <typename V>
+__device__ __forceinline__ bool LexWarpLead(LexKeyT<V>& lead, const LexKeyT<V>& tail) {
+  LexWarpLeader<V>(lead);
   if (lead.id == kNone) return true;
   const bool diff = tail.id != kNone && (-tail.S != lead.S || ~tail.K != lead.K);
   return !__any_sync(kFull, diff);

@@ -637,26 +637,57 @@ __global__ void RowCountKernel(uint32_t R, const uint32_t* __restrict__ ids, con
     row_count[ids[r]] = ucount[r];
 }
 
+// Adds a block's per-thread weight statistics to *out (every thread of the
+// block calls; blocks of at most 1024 threads).
+__device__ __forceinline__ void FlushWeightStats(WeightStats ws, WeightStats* out) {
+  __shared__ WeightStats sh[32];
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    WeightStats y;
+    y.sumabs = __shfl_xor_sync(kFull, ws.sumabs, o);
+    y.maxabs = __shfl_xor_sync(kFull, ws.maxabs, o);
+    y.frac = __shfl_xor_sync(kFull, ws.frac, o);
+    ws = Combine(ws, y);
+  }
+  if (LaneId() == 0) sh[threadIdx.x >> 5] = ws;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (unsigned w = 1; w < blockDim.x / 32; ++w) ws = Combine(ws, sh[w]);
+  if (ws.sumabs) atomicAdd(&out->sumabs, ws.sumabs);
+  if (ws.maxabs > 0.f) atomicMax(reinterpret_cast<int*>(&out->maxabs), __float_as_int(ws.maxabs));
+  if (ws.frac) atomicMax(&out->frac, ws.frac);
+}
+
 // The unique pairs of each segment (at its start) into the new CSR; one
-// warp per cluster.
+// warp per cluster.  The weights' statistics, self-loops left out, are taken
+// on the way: a contracted graph's self-loops hold the clusters' inner
+// weight, which grows far beyond every other weight while no best move ever
+// reads it.
 __global__ void __launch_bounds__(256) GatherRowsKernel(uint32_t R, const uint32_t* __restrict__ ids,
                                                         const uint32_t* __restrict__ ucount,
                                                         const uint64_t* __restrict__ segbase,
                                                         const uint64_t* __restrict__ off2,
                                                         const uint32_t* __restrict__ akey,
                                                         const uint32_t* __restrict__ aval,
-                                                        uint32_t* __restrict__ nbr2, float* __restrict__ w2) {
+                                                        uint32_t* __restrict__ nbr2, float* __restrict__ w2,
+                                                        WeightStats* __restrict__ stats) {
   const unsigned lane = LaneId(), warp = threadIdx.x >> 5;
+  WeightStats ws{0, 0.f, 0};
   for (uint64_t r = uint64_t(blockIdx.x) * 8 + warp; r < R; r += uint64_t(gridDim.x) * 8) {
     const uint32_t cnt = ucount[r];
     const uint64_t src = segbase[r];
     if (cnt == 0 || segbase[r + 1] - src > kSegCtaMax) continue;  // global-path rows: BigPlaceKernel
-    const uint64_t dst = off2[ids[r]];
+    const uint32_t id = ids[r];
+    const uint64_t dst = off2[id];
     for (uint32_t t = lane; t < cnt; t += 32) {
-      nbr2[dst + t] = akey[src + t];
-      w2[dst + t] = __uint_as_float(aval[src + t]);
+      const uint32_t u = akey[src + t];
+      const float x = __uint_as_float(aval[src + t]);
+      nbr2[dst + t] = u;
+      w2[dst + t] = x;
+      if (u != id) ws = Combine(ws, WeightStatsOf(x));
     }
   }
+  FlushWeightStats(ws, stats);
 }
 
 // Global-path rows into the new CSR, one thread per kept run.
@@ -665,16 +696,21 @@ __global__ void BigPlaceKernel(uint32_t S, const uint32_t* __restrict__ seg_star
                                const uint32_t* __restrict__ big_list, const uint32_t* __restrict__ ids,
                                const uint64_t* __restrict__ off2, const uint32_t* __restrict__ bkey,
                                const uint32_t* __restrict__ bval, uint32_t* __restrict__ nbr2,
-                               float* __restrict__ w2) {
+                               float* __restrict__ w2, WeightStats* __restrict__ stats) {
   const uint64_t low_mask = (uint64_t(1) << kbits) - 1;
+  WeightStats ws{0, 0.f, 0};
   for (uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; s < S; s += uint64_t(gridDim.x) * blockDim.x) {
     const uint64_t key = keys[seg_start[s]];
     if (static_cast<uint32_t>(key & low_mask) >= drop) continue;
     const uint32_t g = static_cast<uint32_t>(key >> kbits);
-    const uint64_t pos = off2[ids[big_list[g]]] + (static_cast<uint32_t>(s) - grun[g]);
+    const uint32_t id = ids[big_list[g]];
+    const uint64_t pos = off2[id] + (static_cast<uint32_t>(s) - grun[g]);
+    const float x = __uint_as_float(bval[s]);
     nbr2[pos] = bkey[s];
-    w2[pos] = __uint_as_float(bval[s]);
+    w2[pos] = x;
+    if (bkey[s] != id) ws = Combine(ws, WeightStatsOf(x));
   }
+  FlushWeightStats(ws, stats);
 }
 
 __global__ void NodeWeightKernel(uint32_t n, const uint32_t* __restrict__ C, const double* __restrict__ k,
@@ -895,14 +931,17 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
   res->m = m2;
   PCC_RETURN_IF_ERROR(res->nbr.Alloc(ctx, m2 ? m2 : 1));
   PCC_RETURN_IF_ERROR(res->w.Alloc(ctx, m2 ? m2 : 1));
+  DBuf<WeightStats> stats;
+  PCC_RETURN_IF_ERROR(stats.Alloc(ctx, 1));
+  PCC_RETURN_IF_ERROR(stats.Zero());
   if (m2) {
     GatherRowsKernel<<<Blocks(R, 8, ctx->num_sms * 16), 256, 0, st>>>(R, ids.p, ucount.p, segbase.p, res->off.p,
-                                                                      akey.p, aval.p, res->nbr.p, res->w.p);
+                                                                      akey.p, aval.p, res->nbr.p, res->w.p, stats.p);
     PCC_COUNT(1);
     if (S) {
       BigPlaceKernel<<<Blocks(S, 256, ctx->num_sms * 16), 256, 0, st>>>(
           S, seg_start.p, bkeys.p, place_kbits, drop, grun.p, lists.p + 3 * uint64_t(R), ids.p, res->off.p, bkey.p,
-          bval.p, res->nbr.p, res->w.p);
+          bval.p, res->nbr.p, res->w.p, stats.p);
       PCC_COUNT(1);
     }
   }
@@ -919,7 +958,7 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
   PCC_RETURN_IF_ERROR(res->node_w.Zero());
   NodeWeightKernel<<<Blocks(n, 256, ctx->num_sms * 8), 256, 0, st>>>(n, C, k, res->node_w.p); PCC_COUNT(1);
   PCC_RETURN_IF_ERROR(LaunchCheck());
-  PCC_RETURN_IF_ERROR(ComputeGraphProperties(ctx, res.get()));
+  PCC_RETURN_IF_ERROR(ComputeGraphProperties(ctx, res.get(), stats.p));
   *out = std::move(res);
   return Status::Ok();
 }

@@ -71,15 +71,84 @@ struct DevGraph {
   mutable BinSet bins_all;  // all vertices (built on first use)
   mutable std::shared_ptr<HubPlan> hub_plan;  // degree > 1000 (built on first use)
   uint32_t max_deg = 0;
+  // Of the weights that a best move reads: in compressed graphs the
+  // self-loops are left out (a vertex's own entry is never a candidate).
   bool integral = true;   // every weight is an integer value
   double max_abs_w = 1.0; // max |w| (1 for unit weights)
   double row_abs_bound = 0; // upper bound of any row's sum of |w|
+  int frac_bits = 0;      // every weight is a multiple of 2^-frac_bits (kNoFrac: inf or NaN among them)
   const float* wp() const { return w.p; }
 };
 
+// Weight statistics: the sum of |w| (rounded up per weight; it bounds every
+// row's sum when every |w| < 2^32), max |w| and the fractional bits the
+// weights need.  Zero-initialised, it is the identity of both reductions.
+constexpr int kNoFrac = 1000;
+struct WeightStats {
+  unsigned long long sumabs;
+  float maxabs;  // >= 0: atomicMax on its bits orders it
+  int frac;
+};
+
+__device__ __forceinline__ WeightStats WeightStatsOf(float x) {
+  WeightStats r;
+  r.maxabs = fabsf(x);
+  r.sumabs = __float2uint_ru(r.maxabs);  // saturates
+  // Exponent of the lowest set bit: mantissa m * 2^(e - 150) (e >= 1).
+  const uint32_t bits = __float_as_uint(r.maxabs);
+  const int e = int(bits >> 23);
+  const uint32_t m = e ? (bits & 0x7FFFFFu) | 0x800000u : bits;
+  r.frac = e == 255 ? kNoFrac : m == 0u ? 0 : max(0, 151 - max(e, 1) - __ffs(int(m)));
+  return r;
+}
+// (m < 2^32 weights of at most 2^32 each: the sum cannot wrap.)
+__device__ __forceinline__ WeightStats Combine(WeightStats a, WeightStats b) {
+  return WeightStats{a.sumabs + b.sumabs, fmaxf(a.maxabs, b.maxabs), max(a.frac, b.frac)};
+}
+
+// How a level's synchronous best moves sum the weights.
+//   exact = false: FP64, in the reference's order (below degree 1000).
+//   exact: every cluster sum is held as an integer multiple of 2^-shift, so
+//     any order of additions gives the reference's doubles.  conv = false:
+//     integer weights and offset, |w - offset| <= 2^22.  conv = true: offset
+//     0 and weights that are multiples of 2^-shift whose sums over any row
+//     stay below 2^52 units: the reference's partial sums are then exact
+//     doubles as well, whatever their order, and an FP32 image of w - offset
+//     (its hub path) is w itself.
+//   narrow: every sum is below 2^30 units and held in 32 bits, else in 64.
+// Why: GB300 runs FP64 at 1/64 of FP32, so ordered FP64 sums bound every
+// real-weighted level (an LFR graph of 1M vertices: 189.6 ms a clustering in
+// FP64, 152.2 ms in 64-bit units; its warp kernels 365 -> 344 us a round and
+// its hubs 409 -> 321).  Weights spread too widely for 52 bits keep FP64.
+struct SumMode {
+  bool exact = false;
+  bool conv = false;
+  bool narrow = false;
+  int shift = 0;
+};
+
+inline SumMode SumModeFor(const DevGraph& g, double offset) {
+  SumMode r;
+  const double off = offset < 0 ? -offset : offset;
+  if (g.integral && off <= 4194304.0 && offset == static_cast<double>(static_cast<int64_t>(offset)) &&
+      g.max_abs_w + off <= 4194304.0) {
+    r.exact = true;
+    r.narrow = g.row_abs_bound + off * static_cast<double>(g.max_deg) < 1073741824.0;
+  } else if (offset == 0.0 && g.frac_bits <= 60) {
+    const double units = g.row_abs_bound * static_cast<double>(1ull << g.frac_bits);
+    if (units < 4503599627370496.0) {  // 2^52 (false for an infinite bound)
+      r.exact = r.conv = true;
+      r.narrow = units < 1073741824.0;
+      r.shift = g.frac_bits;
+    }
+  }
+  return r;
+}
+
 // Computes max degree / weight properties and the static degree bins on
-// the device (one sync).
-Status ComputeGraphProperties(Context* ctx, DevGraph* g);
+// the device.  d_stats: the weights' statistics, already on the device (null:
+// reduced here).
+Status ComputeGraphProperties(Context* ctx, DevGraph* g, const WeightStats* d_stats = nullptr);
 // Builds g->bins_all (degree bins including isolated vertices) if absent.
 Status EnsureAllBins(Context* ctx, const DevGraph* g);
 
@@ -196,6 +265,11 @@ struct BMArgs {
   float res32;              // FilterF32(res)
   int int_nw;               // all node weights are integers (certified decisions)
   int narrow;               // INT mode and every cluster sum fits in 32 bits
+  // SumMode::conv: sums in units of 2^-shift; wscale = 2^shift, winv =
+  // 2^-shift (1 otherwise).  res32 is scaled by wscale as well.
+  int conv;
+  float wscale;
+  double winv;
   double offset;
   int32_t ioffset;          // integer offset (INT mode)
   uint32_t stamp;
@@ -238,7 +312,23 @@ struct BMArgs {
 };
 
 __device__ __forceinline__ double ResOf(const BMArgs& a, uint32_t v) { return a.vres ? a.vres[v] : a.res; }
-__device__ __forceinline__ float Res32Of(const BMArgs& a, uint32_t v) { return a.vres32 ? a.vres32[v] : a.res32; }
+// The FP32 resolution in the units of the sums (SumMode::shift).
+__device__ __forceinline__ float Res32Of(const BMArgs& a, uint32_t v) {
+  return a.vres32 ? __fmul_rn(a.vres32[v], a.wscale) : a.res32;
+}
+
+// The sum mode's fields of the arguments (res set before).
+inline void SetSumMode(BMArgs* a, const SumMode& m) {
+  a->narrow = m.exact && m.narrow ? 1 : 0;
+  a->conv = m.conv ? 1 : 0;
+  a->wscale = 1.0f;
+  a->winv = 1.0;
+  if (m.conv) {
+    a->wscale = static_cast<float>(1ull << m.shift);
+    a->winv = 1.0 / static_cast<double>(1ull << m.shift);
+  }
+  a->res32 = FilterF32(a->res * static_cast<double>(a->wscale));
+}
 
 // Asynchronous whole-cluster moves (AsyncSetMoves, clustermoves.cu).
 struct SetMoveArgs {

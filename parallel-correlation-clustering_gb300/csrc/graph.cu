@@ -19,34 +19,12 @@ struct DegreeInput {
   __device__ uint32_t operator()(uint64_t i) const { return static_cast<uint32_t>(off[i + 1] - off[i]); }
 };
 
-// Non-integral weight count and max |w| (as float bits of the magnitude).
-// Weight statistics: non-integral count, max |w| and the sum of |w| over
-// integral weights below 2^32 (saturating; it bounds every row's sum).
-struct WeightStats {
-  unsigned long long nonint;
-  float maxabs;
-  unsigned long long sumabs;
-};
 struct WeightInput {
   const float* w;
-  __device__ WeightStats operator()(uint64_t i) const {
-    const float x = w[i];
-    WeightStats r;
-    r.nonint = (x != truncf(x) || isnan(x) || isinf(x)) ? 1ull : 0ull;
-    r.maxabs = fabsf(x);
-    r.sumabs = r.maxabs < 4294967296.0f ? __float2uint_rz(r.maxabs) : 0xFFFFFFFFull;
-    return r;
-  }
+  __device__ WeightStats operator()(uint64_t i) const { return WeightStatsOf(w[i]); }
 };
 struct WeightOp {
-  __device__ WeightStats operator()(WeightStats a, WeightStats b) const {
-    WeightStats r;
-    r.nonint = a.nonint + b.nonint;
-    r.maxabs = fmaxf(a.maxabs, b.maxabs);
-    r.sumabs = a.sumabs + b.sumabs;
-    if (r.sumabs < a.sumabs) r.sumabs = ~0ull;
-    return r;
-  }
+  __device__ WeightStats operator()(WeightStats a, WeightStats b) const { return Combine(a, b); }
 };
 
 __global__ void CheckCsrKernel(uint32_t n, uint64_t m, const uint64_t* __restrict__ off,
@@ -116,7 +94,7 @@ __global__ void BinStartsKernel(const uint32_t* counts, uint32_t* starts, uint32
   starts[kNumBins] = acc;
 }
 
-Status ComputeGraphProperties(Context* ctx, DevGraph* g) {
+Status ComputeGraphProperties(Context* ctx, DevGraph* g, const WeightStats* d_stats) {
   DBuf<uint32_t> part, out;
   PCC_RETURN_IF_ERROR(out.Alloc(ctx, 1));
   uint32_t maxd = 0;
@@ -124,8 +102,10 @@ Status ComputeGraphProperties(Context* ctx, DevGraph* g) {
     PCC_RETURN_IF_ERROR(Reduce<uint32_t>(ctx, g->n, DegreeInput{g->off.p}, OpMax{}, 0u, out.p, part));
     PCC_RETURN_IF_ERROR(out.ToHost(&maxd, 1));
   }
-  WeightStats ws{0, 1.0f, g->m};
-  if (g->w.p && g->m) {
+  WeightStats ws{g->m, 1.0f, 0};
+  if (d_stats) {
+    PCC_CUDA(cudaMemcpyAsync(&ws, d_stats, sizeof(ws), cudaMemcpyDeviceToHost, ctx->stream));
+  } else if (g->w.p && g->m) {
     DBuf<WeightStats> wpart, wout;
     PCC_RETURN_IF_ERROR(wout.Alloc(ctx, 1));
     PCC_RETURN_IF_ERROR(Reduce<WeightStats>(ctx, g->m, WeightInput{g->w.p}, WeightOp{}, WeightStats{0, 0.0f, 0},
@@ -135,11 +115,12 @@ Status ComputeGraphProperties(Context* ctx, DevGraph* g) {
   }
   PCC_RETURN_IF_ERROR(BuildBins(ctx, g, &g->bins, false));
   g->max_deg = maxd;
-  g->integral = ws.nonint == 0;
+  g->integral = ws.frac == 0;
   g->max_abs_w = ws.maxabs;
+  g->frac_bits = ws.frac;
   // A row's sum of |w| is at most max|w| * degree and at most the total.
-  g->row_abs_bound = std::min(static_cast<double>(ws.maxabs) * static_cast<double>(maxd),
-                              static_cast<double>(ws.sumabs));
+  g->row_abs_bound = static_cast<double>(ws.maxabs) * static_cast<double>(maxd);
+  if (ws.maxabs < 4294967296.0f) g->row_abs_bound = std::min(g->row_abs_bound, static_cast<double>(ws.sumabs));
   return Status::Ok();
 }
 

@@ -123,7 +123,6 @@ struct HubShared {
   double red_d[kW];
   float red_f[kW + 1];
   uint32_t red_i[kW + 1];
-  int stage_i[kW][32];
   double stage_d[kW][32];
   uint32_t cont_key[kMaxCont];
   long long cont_S[kMaxCont];
@@ -382,36 +381,32 @@ __device__ __forceinline__ uint32_t HubInsert(uint32_t* keys, uint32_t cap, uint
 
 // Entry contribution w - offset: integer in INT mode, the reference hub
 // path's float-rounded value in FP64 mode.
-template <bool kInt>
-__device__ __forceinline__ void EntryWeight(const BMArgs& a, float wt, int* xi, double* xd) {
-  if (kInt) {
-    *xi = WeightToInt(wt) - a.ioffset;
+template <bool kInt, typename V>
+__device__ __forceinline__ void EntryWeight(const BMArgs& a, float wt, V* xi, double* xd) {
+  if constexpr (kInt) {
+    *xi = EntryUnits<V, true>(a, wt);
   } else {
     *xd = static_cast<double>(static_cast<float>(Dsub(static_cast<double>(wt), a.offset)));
   }
 }
 
-// Warp-aggregated sum of the entry weights of each match group.
-template <int BT, bool kInt>
-__device__ __forceinline__ void GroupWeights(const BMArgs& a, unsigned peers, bool leader, int xi, double xd,
-                                             HubShared<BT>& sh, int* Si, double* Sd) {
+// Warp-aggregated FP64 sum of the entry weights of each match group, in lane
+// order (for the group's leader).
+template <int BT>
+__device__ __forceinline__ double GroupWeights(unsigned peers, bool leader, double xd, HubShared<BT>& sh) {
   const unsigned warp = threadIdx.x >> 5, lane = LaneId();
-  if (kInt) {
-    *Si = GroupSumInt(peers, xi, a.w == nullptr, leader, sh.stage_i[warp]);
-  } else {
-    sh.stage_d[warp][lane] = xd;
-    __syncwarp();
-    double acc = 0.0;
-    if (leader) {
-      unsigned mm = peers;
-      while (mm) {
-        acc = Dadd(acc, sh.stage_d[warp][__ffs(mm) - 1]);
-        mm &= mm - 1;
-      }
+  sh.stage_d[warp][lane] = xd;
+  __syncwarp();
+  double acc = 0.0;
+  if (leader) {
+    unsigned mm = peers;
+    while (mm) {
+      acc = Dadd(acc, sh.stage_d[warp][__ffs(mm) - 1]);
+      mm &= mm - 1;
     }
-    __syncwarp();
-    *Sd = acc;
   }
+  __syncwarp();
+  return acc;
 }
 
 // Evaluates the CTA's table: returns (to every thread) the best (exact FP64
@@ -433,7 +428,7 @@ __device__ void EvalTable(const BMArgs& a, const VertexCtx& x, float k32, double
   constexpr int kB = kEvalBatch;
   if (kFilter) {
     const I smax = static_cast<I>(smax_ll);
-    const float c32 = sh.change32;
+    const float c32 = __fmul_rn(sh.change32, a.wscale);  // in the units of the sums
     const float r32 = Res32Of(a, x.v);
     float U = -CUDART_INF_F;
     // The two largest upper ends (Y + e; +inf for a candidate outside the
@@ -481,7 +476,7 @@ __device__ void EvalTable(const BMArgs& a, const VertexCtx& x, float k32, double
           sh.cont_key[pos] = key;
           sh.cont_S[pos] = S;
         } else {
-          KeepBest(lv, lid, ValOf(a, x, change, static_cast<double>(S), KD), key);  // list full: now
+          KeepBest(lv, lid, ValOf(a, x, change, UnitsToDouble<I>(a, S), KD), key);  // list full: now
         }
       }
       for (uint32_t s = tid; s < cap; s += BT) {
@@ -527,7 +522,7 @@ __device__ void EvalTable(const BMArgs& a, const VertexCtx& x, float k32, double
           sh.cont_key[pos] = key;
           sh.cont_S[pos] = S;
         } else {
-          KeepBest(lv, lid, ValOf(a, x, change, static_cast<double>(S), KD), key);  // list full: now
+          KeepBest(lv, lid, ValOf(a, x, change, UnitsToDouble<I>(a, S), KD), key);  // list full: now
         }
       }
     }
@@ -546,11 +541,11 @@ __device__ void EvalTable(const BMArgs& a, const VertexCtx& x, float k32, double
         const I S = static_cast<I>(sh.cont_S[i]);
         const double KD = a.K[key];
         if (S == lead.S && KOrder(KD) == lead.K) continue;  // the leading class
-        KeepBest(lv, lid, ValOf(a, x, change, static_cast<double>(S), KD), key);
+        KeepBest(lv, lid, ValOf(a, x, change, UnitsToDouble<I>(a, S), KD), key);
       }
     }
     if (tid == 0 && lead.id != kNone)
-      KeepBest(lv, lid, ValOf(a, x, change, static_cast<double>(lead.S), a.K[lead.id]), lead.id);
+      KeepBest(lv, lid, ValOf(a, x, change, UnitsToDouble<I>(a, lead.S), a.K[lead.id]), lead.id);
   } else {
     for (uint32_t s0 = tid; s0 < cap; s0 += BT * kB) {
       uint32_t kk[kB];
@@ -574,7 +569,8 @@ __device__ void EvalTable(const BMArgs& a, const VertexCtx& x, float k32, double
       for (int j = 0; j < kB; ++j) kd[j] = kk[j] != kNone ? LdK<kAsync>(a.K + kk[j]) : 0.0;
 #pragma unroll
       for (int j = 0; j < kB; ++j)
-        if (kk[j] != kNone) KeepBest(lv, lid, ValOf(a, x, change, static_cast<double>(sv[j]), kd[j]), kk[j]);
+        if (kk[j] != kNone) KeepBest(lv, lid, ValOf(a, x, change, kInt ? UnitsToDouble<I>(a, static_cast<I>(sv[j])) : static_cast<double>(sv[j]), kd[j]),
+                   kk[j]);
     }
   }
   BlockArgmax<BT>(lv, lid, sh.red_k, sh.red_i);
@@ -624,9 +620,9 @@ __device__ __forceinline__ void ScanRow(const BMArgs& a, const VertexCtx& x, uin
       if (e0 + k * BT >= x.d) break;  // uniform over the CTA
       const bool cand = uu[k] != v;
       const uint32_t cu = cc[k];
-      int xi = 0;
+      V xi = 0;
       double xd = 0.0;
-      if (cand) EntryWeight<kInt>(a, ww[k], &xi, &xd);
+      if (cand) EntryWeight<kInt, V>(a, ww[k], &xi, &xd);
       if (want_T && cand && cu == x.c) {
         if (kInt)
           *t_int += xi;
@@ -643,12 +639,11 @@ __device__ __forceinline__ void ScanRow(const BMArgs& a, const VertexCtx& x, uin
       // order first, one atomic per cluster.
       unsigned peers = 0;
       bool leader = mine;
-      int Si = xi;
       double Sd = 0.0;
       if (!kInt) {
         peers = __match_any_sync(kFull, mine ? cu : LaneSentinel(lane));
         leader = mine && int(lane) == __ffs(peers) - 1;
-        GroupWeights<BT, kInt>(a, peers, leader, xi, xd, sh, &Si, &Sd);
+        Sd = GroupWeights<BT>(peers, leader, xd, sh);
       }
       if (leader && *reinterpret_cast<volatile uint32_t*>(&sh.overflow) == 0) {
         bool ins;
@@ -658,8 +653,8 @@ __device__ __forceinline__ void ScanRow(const BMArgs& a, const VertexCtx& x, uin
         } else {
           if (ins && atomicAdd(&sh.nkeys, 1u) + 1 > maxkeys) sh.overflow = 1;
           if (kInt) {
-            const V old = AtomicAddV<V>(svals + slot, static_cast<V>(Si));
-            *smax = max(*smax, static_cast<long long>(old) + Si);
+            const V old = AtomicAddV<V>(svals + slot, xi);
+            *smax = max(*smax, static_cast<long long>(old) + static_cast<long long>(xi));
           } else {
             AtomicAddV<V>(svals + slot, static_cast<V>(Sd));
           }
@@ -675,7 +670,7 @@ __device__ __forceinline__ double HubChange(const BMArgs& a, const VertexCtx& x,
                                             HubShared<BT>& sh) {
   double T;
   if (kInt)
-    T = static_cast<double>(BlockSum<BT, long long>(t_int, sh.red_ll));
+    T = UnitsToDouble<long long>(a, BlockSum<BT, long long>(t_int, sh.red_ll));
   else
     T = BlockSum<BT, double>(t_dbl, sh.red_d);
   if (threadIdx.x == 0) {
@@ -722,7 +717,7 @@ __device__ __forceinline__ double HubChangeSmax(const BMArgs& a, const VertexCtx
         wm = max(wm, __shfl_xor_sync(kFull, wm, o));
       }
       if (threadIdx.x == 0) {
-        sh.change = ChangeOf(a, x, static_cast<double>(wt));
+        sh.change = ChangeOf(a, x, UnitsToDouble<long long>(a, wt));
         sh.change32 = static_cast<float>(sh.change);
         sh.red_mx[kW] = wm;
       }
@@ -939,9 +934,9 @@ __global__ void __launch_bounds__(kGlobThreads) HubGlobalAccumKernel(HubArgs h) 
         if (e0 + k * BT >= e_end) break;  // uniform over the CTA
         const bool cand = uu[k] != v;
         const uint32_t cu = cc[k];
-        int xi = 0;
+        V xi = 0;
         double xd = 0.0;
-        if (cand) EntryWeight<kInt>(a, ww[k], &xi, &xd);
+        if (cand) EntryWeight<kInt, V>(a, ww[k], &xi, &xd);
         if (cand && cu == x.c) {
           if (kInt)
             t_int += xi;
@@ -950,12 +945,11 @@ __global__ void __launch_bounds__(kGlobThreads) HubGlobalAccumKernel(HubArgs h) 
         }
         unsigned peers = 0;
         bool leader = cand;
-        int Si = xi;
         double Sd = 0.0;
         if (!kInt) {
           peers = __match_any_sync(kFull, cand ? cu : LaneSentinel(lane));
           leader = cand && int(lane) == __ffs(peers) - 1;
-          GroupWeights<BT, kInt>(a, peers, leader, xi, xd, sh, &Si, &Sd);
+          Sd = GroupWeights<BT>(peers, leader, xd, sh);
         }
         if (leader) {
           bool ins;
@@ -963,8 +957,8 @@ __global__ void __launch_bounds__(kGlobThreads) HubGlobalAccumKernel(HubArgs h) 
           if (slot == kNone) {
             atomicExch(&a.ctr->error, kErrHashFull);  // cannot happen: 2 * degree + 2 slots
           } else if (kInt) {
-            const V old = AtomicAddV<V>(vals + slot, static_cast<V>(Si));
-            smax = max(smax, static_cast<long long>(old) + Si);
+            const V old = AtomicAddV<V>(vals + slot, xi);
+            smax = max(smax, static_cast<long long>(old) + static_cast<long long>(xi));
           } else {
             AtomicAddV<V>(vals + slot, static_cast<V>(Sd));
           }
@@ -1010,7 +1004,7 @@ __global__ void __launch_bounds__(kGlobThreads) HubGlobalEvalKernel(HubArgs h) {
         fam_e += x.d;
         fam_v += 1;
       }
-      const double T = kInt ? static_cast<double>(__ldcg(h.gt_int + gi)) : __ldcg(h.gt_dbl + gi);
+      const double T = kInt ? UnitsToDouble<long long>(a, __ldcg(h.gt_int + gi)) : __ldcg(h.gt_dbl + gi);
       sh.change = ChangeOf(a, x, T);
       sh.change32 = static_cast<float>(sh.change);
     }

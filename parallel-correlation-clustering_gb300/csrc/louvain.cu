@@ -642,7 +642,9 @@ struct Level {
   // from given labels).  From singletons an isolated vertex never moves:
   // its value is 0 and no vertex can join it.
   const BinSet* bins = nullptr;
-  bool int_mode = false;
+  // Integer sums in synchronous rounds; asynchronous ones take them for
+  // integer weights only (no SumMode::conv).
+  SumMode mode;
   // Subclustering: the vertex of the next level every vertex became (its
   // subcluster id); empty when the level was compressed by cluster id.
   DBuf<uint32_t> sub;
@@ -663,13 +665,6 @@ struct RunResult {
   uint64_t algo_bytes_compress = 0;
 };
 
-// INT mode with every neighbour-cluster sum below 2^30 in magnitude (so
-// sums and their differences fit in int): a cluster sum is at most the
-// row's sum of |w| plus degree * |offset|.
-bool NarrowSums(const DevGraph& g, double offset) {
-  return g.row_abs_bound + std::fabs(offset) * static_cast<double>(g.max_deg) < 1073741824.0;
-}
-
 // Sequential waves of an async round (see Round); 16 keeps the mean quality
 // over seeds within 0.15% of the reference restatement on SBM, RMAT and
 // LFR-like graphs, where one wave loses up to 1.6%.
@@ -681,12 +676,6 @@ constexpr uint32_t kAsyncWaves = 16;
 // and k' (16 B per new vertex).
 uint64_t CompressBytes(const DevGraph& in, const DevGraph& out) {
   return (in.w.p ? 12ull : 8ull) * in.m + 8ull * out.m + 20ull * in.n + 16ull * out.n;
-}
-
-bool IntModeFor(const DevGraph& g, double offset) {
-  if (!g.integral) return false;
-  if (offset != std::floor(offset) || std::fabs(offset) > 4194304.0) return false;
-  return g.max_abs_w + std::fabs(offset) <= 4194304.0;  // 2^22
 }
 
 class Engine {
@@ -781,7 +770,8 @@ class Engine {
       NodeKfKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, L->k.p, L->kf.p); PCC_COUNT(1);
       PCC_RETURN_IF_ERROR(LaunchCheck());
     }
-    L->int_mode = IntModeFor(*g, cfg_.edge_weight_offset);
+    L->mode = SumModeFor(*g, cfg_.edge_weight_offset);
+    if (cfg_.async && L->mode.conv) L->mode = SumMode{};
     PCC_RETURN_IF_ERROR(SeedFreeIds(n, L->s.p));
     if (un_ && un_->d_res.p && n) {
       PCC_RETURN_IF_ERROR(L->vres.Alloc(ctx_, n));
@@ -827,9 +817,8 @@ class Engine {
     a.Kf = L->Kf.p;
     a.kf = L->kf.p;
     a.int_nw = int_nw_ ? 1 : 0;
-    a.narrow = (L->int_mode && NarrowSums(g, cfg_.edge_weight_offset)) ? 1 : 0;
     a.res = cfg_.resolution;
-    a.res32 = FilterF32(cfg_.resolution);
+    SetSumMode(&a, L->mode);
     a.offset = cfg_.edge_weight_offset;
     a.ioffset = static_cast<int32_t>(cfg_.edge_weight_offset);
     a.stamp = stamp_;
@@ -868,8 +857,8 @@ class Engine {
       for (uint32_t w = 0; w < a.waves; ++w) {
         a.wave = w;
         PCC_RETURN_IF_ERROR(LaunchBestMoves(ctx_, a, bins.list.p, bins.counts.p, bins.counts.p + kNumBins,
-                                            bins.host_counts, L->int_mode, g.max_deg));
-        PCC_RETURN_IF_ERROR(LaunchHubBestMoves(ctx_, a, *g.hub_plan, hub_state_, L->int_mode, a.narrow != 0));
+                                            bins.host_counts, L->mode.exact, g.max_deg));
+        PCC_RETURN_IF_ERROR(LaunchHubBestMoves(ctx_, a, *g.hub_plan, hub_state_, L->mode.exact, a.narrow != 0));
       }
     }
     timer_.End(kPhaseBestMoves);
@@ -962,20 +951,20 @@ class Engine {
     Status st;
     {
       OnSideStream on(ctx_, 0);
-      st = LaunchHubBestMoves(ctx_, a, *g.hub_plan, hub_state_, L->int_mode, a.narrow != 0, kLaunchBigHubs);
+      st = LaunchHubBestMoves(ctx_, a, *g.hub_plan, hub_state_, L->mode.exact, a.narrow != 0, kLaunchBigHubs);
     }
     if (st.ok()) {
       OnSideStream on(ctx_, 1);
       st = LaunchBestMoves(ctx_, a, bins.list.p, bins.counts.p, bins.counts.p + kNumBins, bins.host_counts,
-                           L->int_mode, g.max_deg, kLaunchWarps);
+                           L->mode.exact, g.max_deg, kLaunchWarps);
     }
     if (st.ok()) {
       OnSideStream on(ctx_, 2);
-      st = LaunchHubBestMoves(ctx_, a, *g.hub_plan, hub_state_, L->int_mode, a.narrow != 0, kLaunchSmallHubs);
+      st = LaunchHubBestMoves(ctx_, a, *g.hub_plan, hub_state_, L->mode.exact, a.narrow != 0, kLaunchSmallHubs);
     }
     if (st.ok())
       st = LaunchBestMoves(ctx_, a, bins.list.p, bins.counts.p, bins.counts.p + kNumBins, bins.host_counts,
-                           L->int_mode, g.max_deg, kLaunchGroups);
+                           L->mode.exact, g.max_deg, kLaunchGroups);
     for (int i = 0; i < Context::kSideStreams; ++i) {
       PCC_CUDA(cudaEventRecord(ctx_->join_ev[i], ctx_->side[i]));
       PCC_CUDA(cudaStreamWaitEvent(ctx_->stream, ctx_->join_ev[i], 0));
@@ -1002,7 +991,7 @@ class Engine {
     PCC_CUDA(cudaMemsetAsync(new_stamp_.p, 0, sizeof(uint32_t) * n, ctx_->stream));
     // Integral entry values whose every partial sum stays below 2^53 sum
     // exactly in any order.
-    const bool exact = L->int_mode && static_cast<double>(g.m) * (g.max_abs_w + std::fabs(cfg_.edge_weight_offset)) <
+    const bool exact = L->mode.exact && !L->mode.conv && static_cast<double>(g.m) * (g.max_abs_w + std::fabs(cfg_.edge_weight_offset)) <
                                           9007199254740992.0;
     PCC_RETURN_IF_ERROR(FindClusterMoves(ctx_, g, L->C.p, L->k.p, L->K.p, cfg_.resolution, cfg_.edge_weight_offset,
                                          exact, moves_.p, movers_.p, ctr_.p));
@@ -1030,7 +1019,7 @@ class Engine {
   Status AsyncWholeClusterMoves(Level* L, const BMArgs& round_args) {
     const DevGraph& g = *L->g;
     const BinSet& bins = *L->bins;
-    const bool exact = L->int_mode && static_cast<double>(g.m) * (g.max_abs_w + std::fabs(cfg_.edge_weight_offset)) <
+    const bool exact = L->mode.exact && !L->mode.conv && static_cast<double>(g.m) * (g.max_abs_w + std::fabs(cfg_.edge_weight_offset)) <
                                           9007199254740992.0;
     SetMoveArgs sm{};
     sm.g = &g;
@@ -1064,8 +1053,8 @@ class Engine {
       b.moved_stamp = sm_moved_.p;
       b.moved_cluster_stamp = sm_dummy_.p;
       PCC_RETURN_IF_ERROR(LaunchBestMoves(ctx_, b, bins.list.p, bins.counts.p, bins.counts.p + kNumBins,
-                                          bins.host_counts, L->int_mode, g.max_deg));
-      return LaunchHubBestMoves(ctx_, b, *g.hub_plan, hub_state_, L->int_mode, b.narrow != 0);
+                                          bins.host_counts, L->mode.exact, g.max_deg));
+      return LaunchHubBestMoves(ctx_, b, *g.hub_plan, hub_state_, L->mode.exact, b.narrow != 0);
     };
     return AsyncSetMoves(ctx_, sm, vertex_moves);
   }
@@ -2361,9 +2350,9 @@ Status BestMovesImpl(pcc_context* pctx, const pcc_graph* graph, const pcc_config
   a.Kf = dKf.p;
   a.kf = dkf.p;
   a.int_nw = IntegralWeights(k, n) ? 1 : 0;
-  a.narrow = (IntModeFor(g, config->edge_weight_offset) && NarrowSums(g, config->edge_weight_offset)) ? 1 : 0;
   a.res = config->resolution;
-  a.res32 = FilterF32(config->resolution);
+  const SumMode mode = SumModeFor(g, config->edge_weight_offset);
+  SetSumMode(&a, mode);
   a.offset = config->edge_weight_offset;
   a.ioffset = static_cast<int32_t>(config->edge_weight_offset);
   a.stamp = 1;
@@ -2378,9 +2367,8 @@ Status BestMovesImpl(pcc_context* pctx, const pcc_graph* graph, const pcc_config
   PCC_RETURN_IF_ERROR(EnsureAllBins(ctx, &g));
   const BinSet& ab = g.bins_all;
   PCC_RETURN_IF_ERROR(LaunchBestMoves(ctx, a, ab.list.p, ab.counts.p, ab.counts.p + kNumBins, ab.host_counts,
-                                      IntModeFor(g, config->edge_weight_offset), g.max_deg));
-  const bool im = IntModeFor(g, config->edge_weight_offset);
-  PCC_RETURN_IF_ERROR(LaunchHubBestMoves(ctx, a, *g.hub_plan, hs, im, im && NarrowSums(g, config->edge_weight_offset)));
+                                      mode.exact, g.max_deg));
+  PCC_RETURN_IF_ERROR(LaunchHubBestMoves(ctx, a, *g.hub_plan, hs, mode.exact, mode.narrow));
   PCC_RETURN_IF_ERROR(dt.ToHost(out_t, n));
   PCC_RETURN_IF_ERROR(dv.ToHost(out_v, n));
   if (out_moves) PCC_RETURN_IF_ERROR(dm.ToHost(out_moves, n));

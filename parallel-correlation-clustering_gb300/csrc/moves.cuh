@@ -326,17 +326,59 @@ __device__ __forceinline__ int WeightToInt(float w) {
   return __float_as_int(__fadd_rn(w, 12582912.0f)) - 0x4B400000;
 }
 
+// An integral weight |x| < 2^30 as an int, likewise: x = h * 2^16 + l with h
+// the nearest integer to x / 2^16 (|h| <= 2^14) and |l| <= 2^15, both exact.
+__device__ __forceinline__ int BigWeightToInt(float x) {
+  const float t = __fadd_rn(__fmul_rn(x, 1.52587890625e-05f /* 2^-16 */), 12582912.0f);
+  const float h = __fsub_rn(t, 12582912.0f);
+  const float l = __fsub_rn(x, __fmul_rn(h, 65536.0f));
+  return (__float_as_int(t) - 0x4B400000) * 65536 + WeightToInt(l);
+}
+
+// A finite weight w, a multiple of 2^-shift with |w| * 2^shift < 2^52, in
+// units of 2^-shift (wscale = 2^shift), from its bits: no conversion
+// instruction.  (The product is a power-of-two scaling: exact.)
+__device__ __forceinline__ long long WeightToUnits(float w, float wscale) {
+  const uint32_t bits = __float_as_uint(__fmul_rn(w, wscale));
+  const int e = int((bits >> 23) & 255u) - 150;
+  const long long m = e > -150 ? static_cast<long long>((bits & 0x7FFFFFu) | 0x800000u) : 0ll;
+  const long long x = e >= 0 ? m << e : m >> min(-e, 24);
+  return (bits >> 31) ? -x : x;
+}
+
+// w - offset in the units of the sums.  kConv: weights of either form (by
+// a.conv); else integers of at most 2^22 only, which saves the warp kernels
+// the general conversion's registers (6% of their time on block models).
+template <typename V, bool kConv>
+__device__ __forceinline__ V EntryUnits(const BMArgs& a, float w) {
+  if constexpr (sizeof(V) == 8) {
+    return WeightToUnits(w, a.wscale) - a.ioffset;  // ioffset is 0 when conv
+  } else if constexpr (kConv) {
+    return a.conv ? BigWeightToInt(__fmul_rn(w, a.wscale)) : WeightToInt(w) - a.ioffset;
+  } else {
+    return WeightToInt(w) - a.ioffset;
+  }
+}
+
+// A sum in the weights' own units (exact: below 2^53 units).
+template <typename V>
+__device__ __forceinline__ double UnitsToDouble(const BMArgs& a, V s) {
+  const double d = static_cast<double>(s);
+  return a.conv ? Dmul(d, a.winv) : d;
+}
+
 // Sum of the integer weights x over the calling lane's match_any group
 // `peers`; every lane of the warp calls it.  (__reduce_add_sync with a
 // different mask per group executes once per distinct group -- up to 32
 // passes per instruction.)  Unit weights: every lane's x is the same, so the
 // sum is x * |group|.  Other weights: the group's leader adds its peers'
-// values from the warp's 32-int stage row (passes = the largest group).
-__device__ __forceinline__ int GroupSumInt(unsigned peers, int x, bool unit, bool leader, int* stage) {
+// values from the warp's 32-value stage row (passes = the largest group).
+template <typename V>
+__device__ __forceinline__ V GroupSumInt(unsigned peers, V x, bool unit, bool leader, V* stage) {
   if (unit) return x * __popc(peers);
   stage[LaneId()] = x;
   __syncwarp();
-  int s = 0;
+  V s = 0;
   if (leader) {
     unsigned mm = peers;
     while (mm) {

@@ -1,0 +1,112 @@
+"""Which kernels a call takes must not show in its result: graphs at the
+edges of the rules that choose between the integer and the FP64 sums and
+between launch shapes, against the oracle (bit for bit: every sum here is
+exact in any order)."""
+
+import numpy as np
+import pytest
+
+import oracle as O
+import pcc_gb300 as P
+import pcc_graphs as G
+
+pytestmark = pytest.mark.gpu
+
+
+def _weighted(g, w_of):
+    """g with symmetric weights w_of(min id, max id)."""
+    src = np.repeat(np.arange(g.n), np.diff(g.offsets).astype(np.int64))
+    a, b = np.minimum(src, g.neighbors), np.maximum(src, g.neighbors)
+    return P.CsrGraph(g.offsets, g.neighbors, w_of(a, b).astype(np.float32))
+
+
+def _same(ctx, g, cfg, modularity=False):
+    dg, og = ctx.upload(g), O.OracleGraph(g)
+    run = (P.modularity_cluster, O.modularity_cluster) if modularity else (P.correlation_cluster, O.correlation_cluster)
+    lab, st = run[0](dg, cfg)
+    want, sto = run[1](og, cfg)
+    np.testing.assert_array_equal(lab, want)
+    for key in ("edge_visits", "rounds", "levels", "refine_passes"):
+        assert st[key] == sto[key], key
+    dg.free()
+    return st
+
+
+@pytest.mark.parametrize("scale,move,res", [
+    (1, P.NBHR_CLUSTER_MOVE, 0.3), (1, P.NBHR_MOVE, 0.3),
+    (30000, P.ALL_MOVE, 0.3), (4000000, P.ALL_MOVE, 0.3),                   # self-loops alone above 2^22
+    (4000000, P.NBHR_CLUSTER_MOVE, 1.2e6), (4000000, P.NBHR_MOVE, 1.2e6)])  # other weights too
+def test_heavy_self_loops(ctx, scale, move, res):
+    """Contracted levels whose self-loops exceed 2^22 while the other weights
+    may not: the self-loops must not decide the arithmetic, nor the result."""
+    g, block = G.sbm(1500, 12, 0.2, 0.01, 5)
+    gw = _weighted(g, lambda a, b: np.where(block[a] == block[b], scale, 1) + (a + b) % 3)
+    st = _same(ctx, gw, P.make_config(resolution=res, refine=True, move_method=move))
+    assert st["levels"] >= 2
+
+
+def _hubby(n=6000, seed=3):
+    """A block model with vertices of degree 700, 1500, 3000 and 5000, so that
+    every kernel shape below the split rows takes part."""
+    g, _ = G.sbm(n, 30, 0.05, 0.002, seed)
+    src = np.repeat(np.arange(n), np.diff(g.offsets).astype(np.int64))
+    keep = src < g.neighbors
+    s, d = [src[keep]], [g.neighbors[keep].astype(np.int64)]
+    for hub, deg in ((0, 700), (1, 1500), (2, 3000), (3, 5000)):
+        s.append(np.full(deg, hub)), d.append(np.arange(10, 10 + deg))
+    return P.CsrGraph.from_edges(n, np.concatenate(s), np.concatenate(d))
+
+
+def _unit_hash(a, b):
+    h = (a.astype(np.uint64) * np.uint64(0x9E3779B97F4A7C15) + b.astype(np.uint64) * np.uint64(0xD6E8FEB86659FD93))
+    return ((h ^ (h >> np.uint64(29))) * np.uint64(0xBF58476D1CE4E5B9) >> np.uint64(40)).astype(np.float64) / 2.0 ** 24
+
+
+# Weights by what the fixed-point rule has to say of them, and whether sums of
+# any order are exact (then hubs equal the oracle's bits as well).
+WEIGHTS = {
+    "quarters": (lambda a, b: np.floor(_unit_hash(a, b) * 16) / 4, True),                  # 32-bit sums of 2^-2
+    "negative": (lambda a, b: np.floor(_unit_hash(a, b) * 64) / 8 - 3, True),              # 32 bits, both signs, zeros
+    "big_ints": (lambda a, b: np.floor(_unit_hash(a, b) * 9e4) + 4.3e6 * ((a + b) % 97 == 0), True),  # above 2^22
+    "wide_ints": (lambda a, b: np.floor(_unit_hash(a, b) * 2 ** 20) * 2.0 ** 16, True),     # 64-bit sums
+    "uniform": (lambda a, b: 0.5 + _unit_hash(a, b), True),                                # 64-bit sums of 2^-24
+    "signed": (lambda a, b: _unit_hash(a, b) * 2 - 0.75, True),                            # 64 bits, both signs
+    "spread": (lambda a, b: 10.0 ** (_unit_hash(a, b) * 12 - 9), False),                   # too wide: FP64
+}
+
+
+@pytest.mark.parametrize("kind", list(WEIGHTS))
+def test_fixed_point_best_moves(ctx, kind):
+    """One best-move pass per weight kind: targets, values and moves are the
+    oracle's bits; certified and exact decisions are checked against each
+    other on the device."""
+    w_of, exact = WEIGHTS[kind]
+    g = _weighted(_hubby(), w_of)
+    dg, og = ctx.upload(g), O.OracleGraph(g)
+    scale = max(float(np.abs(g.weights).mean()), 1e-6)
+    low = np.diff(g.offsets) <= 1000
+    for clusters, res, off in ((6000, 0.3, 0.0), (40, 0.002, 0.0), (40, 0.05, 0.0), (3, 0.001, 0.5)):
+        rng = np.random.default_rng(clusters)
+        C = rng.integers(0, clusters, g.n).astype(np.uint32)
+        k = rng.integers(1, 5, g.n).astype(np.float64)
+        s = np.bincount(C, minlength=g.n).astype(np.uint32)
+        K = np.bincount(C, weights=k, minlength=g.n)
+        cfg = P.make_config(resolution=res * scale, edge_weight_offset=off * scale)
+        t, v, m = P.best_moves(dg, cfg, C, s, k, K)
+        to, vo, mo = O.best_moves(og, cfg, C, s, k, K)
+        part = slice(None) if exact and off == 0.0 else low
+        np.testing.assert_array_equal(t[part], to[part])
+        np.testing.assert_array_equal(v[part].view(np.uint64), vo[part].view(np.uint64))
+        np.testing.assert_array_equal(m[part], mo[part])
+    dg.free()
+
+
+@pytest.mark.parametrize("kind", [k for k in WEIGHTS if WEIGHTS[k][1]])
+@pytest.mark.parametrize("modularity", [False, True])
+def test_fixed_point_clusterings(ctx, kind, modularity):
+    """Whole clusterings on the weights whose sums are exact: every label."""
+    g = _weighted(_hubby(seed=4), WEIGHTS[kind][0])
+    scale = max(float(np.abs(g.weights).mean()), 1e-6)
+    for move, res in ((P.NBHR_CLUSTER_MOVE, 0.02), (P.NBHR_MOVE, 0.2)):
+        cfg = P.make_config(resolution=1.0 if modularity else res * scale, refine=True, move_method=move)
+        _same(ctx, g, cfg, modularity)
