@@ -22,8 +22,7 @@
 //   FP64 mode: degree <= 1000 adds in adjacency order (the reference's
 //             sequential flat_hash_map path, bit-exact); hubs add in any
 //             order, as the reference's concurrent map does.
-#include "certify.cuh"
-#include "moves.cuh"
+#include "certmoves.cuh"
 
 namespace pcc {
 
@@ -116,7 +115,7 @@ __global__ void __launch_bounds__(256) BestMoveGroupKernel(BMArgs a, const uint3
       }
     }
     bool append = false;
-    if (vvalid && gl == 0) append = Decide<kAsync>(a, x, val, id, change);
+    if (vvalid && gl == 0) append = Decide<kAsync>(a, x, val, id, change, StampIn(a.rs, a.stamp));
     if (!kAsync) mb.Add(&a.ctr->movers, a.movers, append, x.v);
   }
   if (!kAsync) mb.Flush(&a.ctr->movers, a.movers);
@@ -130,8 +129,6 @@ __global__ void __launch_bounds__(256) BestMoveGroupKernel(BMArgs a, const uint3
 // which keeps the reference's adjacency-order summation exactly.
 // ---------------------------------------------------------------------------
 constexpr int kWarpKernelWarps = 4;
-constexpr int kCertUnroll = 4;  // chunks of 32 entries loaded together
-constexpr int kCertRegRounds = 1;  // candidates per lane held in registers
 
 template <int HC>
 constexpr size_t WarpKernelSmem() {
@@ -278,7 +275,7 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) BestMoveWarpKernel(BMAr
       vals[slot] = 0ull;
     }
     bool append = false;
-    if (lane == 0) append = Decide<kAsync>(a, x, best, bid, change);
+    if (lane == 0) append = Decide<kAsync>(a, x, best, bid, change, StampIn(a.rs, a.stamp));
     if (!kAsync) mb.Add(&a.ctr->movers, a.movers, append, x.v);
     __syncwarp();
     if (lane == 0) *used_count = 0;
@@ -289,92 +286,9 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) BestMoveWarpKernel(BMAr
 }
 
 // ---------------------------------------------------------------------------
-// INT-mode synchronous rounds: certified decisions (certify.cuh).  The FP32
-// pre-filter selects the survivors; when they form one (S, K) class and the
-// FP32 bounds decide the move, no FP64 instruction runs for the vertex.
-// Otherwise -- and always in replay mode, where the exact values are outputs
-// -- the exact FP64 values decide; in replay mode a certified decision that
-// differs from the FP64 one raises kErrCertMismatch (a self-check).
+// INT-mode synchronous rounds: the certified bodies of certmoves.cuh over one
+// degree bin each.
 // ---------------------------------------------------------------------------
-// Exact FP64 fallbacks of the certified kernels.  They are separate
-// non-inlined functions so that the compiler cannot hoist their FP64
-// arithmetic onto the certified path (an FP64 warp instruction costs ~19
-// SM cycles on this GPU).  Both return whether the vertex must be appended
-// to the movers list; in replay mode they also run the self-check.
-template <int G, typename V>
-__device__ __noinline__ bool GroupExact(const BMArgs& a, const VertexCtx& x, bool fp64, bool contender, unsigned gl,
-                                        V T, V S, double KD, uint32_t cu, bool replay, int cres,
-                                        uint32_t cmove) {
-  double change = 0.0, val = -CUDART_INF;
-  uint32_t id = kNone;
-  if (fp64) {
-    change = ChangeOf(a, x, UnitsToDouble<V>(a, T));
-    if (contender) {
-      val = ValOf(a, x, change, UnitsToDouble<V>(a, S), KD);
-      id = cu;
-    }
-  }
-#pragma unroll
-  for (int o = G / 2; o >= 1; o >>= 1) {
-    const double ov = __shfl_xor_sync(kFull, val, o);
-    const uint32_t oid = __shfl_xor_sync(kFull, id, o);
-    if (Better(ov, oid, val, id)) {
-      val = ov;
-      id = oid;
-    }
-  }
-  bool append = false;
-  if (fp64 && gl == 0) {
-    append = Decide<false>(a, x, val, id, change);
-    if (replay && cres != kUncertain && a.out_moves && a.out_moves[x.v] != cmove)
-      atomicExch(&a.ctr->error, kErrCertMismatch);
-  }
-  return append;
-}
-
-template <int HC, typename V>
-__device__ __noinline__ bool WarpExact(const BMArgs& a, const VertexCtx& x, V T, const uint32_t* keys,
-                                       const V* vals, const uint16_t* used, uint32_t nused, bool replay, int cres,
-                                       uint32_t cmove) {
-  const unsigned lane = LaneId();
-  const double change = ChangeOf(a, x, UnitsToDouble<V>(a, T));
-  double best = -CUDART_INF;
-  uint32_t bid = kNone;
-  for (uint32_t i = lane; i < nused; i += 32) {
-    const uint32_t slot = used[i];
-    if (slot == 0xFFFFu) continue;
-    const uint32_t key = keys[slot];
-    const double val = ValOf(a, x, change, UnitsToDouble<V>(a, vals[slot]), a.K[key]);
-    if (Better(val, key, best, bid)) {
-      best = val;
-      bid = key;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-    const double ov = __shfl_xor_sync(kFull, best, o);
-    const uint32_t oid = __shfl_xor_sync(kFull, bid, o);
-    if (Better(ov, oid, best, bid)) {
-      best = ov;
-      bid = oid;
-    }
-  }
-  bool append = false;
-  if (lane == 0) {
-    append = Decide<false>(a, x, best, bid, change);
-    if (replay && cres != kUncertain && a.out_moves && a.out_moves[x.v] != cmove)
-      atomicExch(&a.ctr->error, kErrCertMismatch);
-  }
-  return append;
-}
-
-template <typename V>
-__device__ __forceinline__ V WarpMaxV(V x) {
-  if constexpr (sizeof(V) == 4) return __reduce_max_sync(kFull, x);
-  else return WarpMaxLL(x);
-}
-
-// V: int when every sum of a row fits in 32 bits, else long long.
 template <int G, typename V>
 __global__ void __launch_bounds__(256) CertGroupKernel(BMArgs a, const uint32_t* __restrict__ list,
                                                       const uint32_t* __restrict__ bin_counts,
@@ -384,108 +298,21 @@ __global__ void __launch_bounds__(256) CertGroupKernel(BMArgs a, const uint32_t*
   WarpMoverBuffer mb{mover_buf[threadIdx.x >> 5]};
   const uint32_t count = bin_counts[bin];
   const uint32_t start = bin_starts[bin];
-  const unsigned lane = LaneId(), warp = threadIdx.x >> 5;
+  const unsigned warp = threadIdx.x >> 5;
   constexpr unsigned kVpw = 32 / G;
-  const unsigned g = lane / G, gl = lane % G;
-  const unsigned gmask = G == 32 ? kFull : (((1u << G) - 1u) << (g * G));
+  const unsigned g = LaneId() / G;
   unsigned long long fam_e = 0, fam_v = 0;
   const bool replay = a.out_target != nullptr;
-  const bool unit = a.w == nullptr;
+  const RoundView rv = RoundOf(a);
   const uint64_t stride = uint64_t(gridDim.x) * 8 * kVpw;
   // Vertex ids are loaded one iteration ahead (latency-bound kernel).
   uint64_t base = (uint64_t(blockIdx.x) * 8 + warp) * kVpw;
   uint32_t vid = base + g < count ? list[start + base + g] : 0u;
   for (; base < count; base += stride) {
-    const uint64_t idx = base + g;
     const uint32_t nvid = base + stride + g < count ? list[start + base + stride + g] : 0u;
-    bool vvalid = idx < count;
-    VertexCtx x{};
-    if (vvalid) {
-      vvalid = InFront(a, vid);
-      if (vvalid) x = LoadVertex<false>(a, vid);
-    }
+    const bool append = GroupStep<G, V, ConstLoads>(a, rv, base + g < count, vid, stage[warp], replay, fam_e, fam_v);
+    mb.Add(&a.ctr->movers, a.movers, append, vid);
     vid = nvid;
-    if (__ballot_sync(kFull, vvalid) == 0) continue;
-    if (vvalid && gl == 0) {
-      fam_e += x.d;
-      fam_v += 1;
-    }
-    const bool has = vvalid && gl < x.d;
-    uint32_t u = x.v;
-    float wt = 0.f;
-    if (has) {
-      u = a.nbr[x.b + gl];
-      wt = a.w ? a.w[x.b + gl] : 1.0f;
-    }
-    const bool cand = has && u != x.v;
-    const uint32_t cu = cand ? __ldg(a.C + u) : kNone;
-    const unsigned peers = __match_any_sync(kFull, cand ? cu : LaneSentinel(lane)) & gmask;
-    const bool leader = cand && int(lane) == __ffs(peers) - 1;
-    const V xi = cand ? EntryUnits<V, true>(a, wt) : V(0);
-    const V S = GroupSumInt<V>(peers, xi, unit, leader, stage[warp]);
-    const unsigned tmask = __ballot_sync(kFull, leader && cu == x.c) & gmask;
-    const V Tsh = __shfl_sync(kFull, S, tmask ? __ffs(tmask) - 1 : int(lane));
-    const V T = tmask ? Tsh : V(0);
-    V smax = leader ? S : (sizeof(V) == 4 ? V(INT_MIN) : V(LLONG_MIN));
-    if constexpr (G == 32) {
-      smax = WarpMaxV<V>(smax);
-    } else {
-#pragma unroll
-      for (int o = G / 2; o >= 1; o >>= 1) smax = max(smax, __shfl_xor_sync(kFull, smax, o));
-    }
-    const float k32 = vvalid ? a.kf[x.v] : 0.f;
-    const float Kc32 = vvalid ? a.Kf[x.c] : 0.f;
-    const ChangeApproxT<V> ca = ApproxChange<V>(Res32Of(a, x.v), a.int_nw != 0, k32, Kc32, T);
-    const float cabs = ChangeAbsBound(ca);
-    // FP32 pre-filter over the group's leaders.
-    FilterVal f{0.f, 0.f, false};
-    float KfD = 0.f;
-    float lo = -CUDART_INF_F;
-    if (leader) {
-      KfD = a.Kf[cu];
-      f = FilterOf<V>(Res32Of(a, x.v), k32, KfD, S, smax, cabs);
-      if (f.sane) lo = __fsub_rn(f.Y, f.e);
-    }
-    float U = lo;
-    if constexpr (G == 32) {
-      U = WarpMaxFinite(U);
-    } else {
-#pragma unroll
-      for (int o = G / 2; o >= 1; o >>= 1) U = fmaxf(U, __shfl_xor_sync(kFull, U, o));
-    }
-    const bool contender = leader && (!f.sane || __fadd_rn(f.Y, f.e) >= U);
-    // The leading (S, K) class of the contenders and the trailing one.
-    LexKeyT<V> lead, tail;
-    double KD = 0.0;
-    if (contender) {
-      KD = a.K[cu];
-      const unsigned long long ko = KOrder(KD);
-      lead.Keep(S, ko, cu);
-      tail.Keep(-S, ~ko, cu);
-    }
-    bool single;
-    if constexpr (G == 32) {
-      single = LexWarpLead<V>(lead, tail);
-    } else {
-      LexGroupReduce<G>(lead);
-      LexGroupReduce<G>(tail);
-      single = lead.id == kNone || (-tail.S == lead.S && ~tail.K == lead.K);
-    }
-    int cres = kUncertain;
-    uint32_t ctarget = kNone;
-    if (vvalid && single) {
-      const float KfA = lead.id != kNone ? a.Kf[lead.id] : 0.f;
-      cres = CertifyDecision<V>(ca, Res32Of(a, x.v), k32, lead.id != kNone, lead.S, KfA, lead.id, a.n, &ctarget);
-    }
-    const uint32_t cmove = cres == kUncertain ? kNone : CertifiedMove(a, x, ctarget, cres == kCertMove);
-    const bool fp64 = vvalid && (replay || cres == kUncertain);
-    bool append = false;
-    if (vvalid && !fp64 && gl == 0) append = ApplyCertified(a, x, cmove);
-    if (__ballot_sync(kFull, fp64)) {
-      const bool app = GroupExact<G, V>(a, x, fp64, contender, gl, T, S, KD, cu, replay, cres, cmove);
-      append = append || app;
-    }
-    mb.Add(&a.ctr->movers, a.movers, append, x.v);
   }
   mb.Flush(&a.ctr->movers, a.movers);
   FlushFamily(a, kFamGroup, fam_e, fam_v);
@@ -502,11 +329,6 @@ constexpr size_t CertWarpSmem() {
   return size_t(kWarpKernelWarps) * CertWarpStride<HC, V>();
 }
 
-// V: int when every cluster sum fits in 32 bits (narrow), else long long.
-// Every entry inserts its cluster itself (atomicCAS claims a slot) and adds
-// its integer weight with a shared-memory atomic: INT-mode sums are exact in
-// any order, and grouping equal clusters first with match.any cost more than
-// the atomics it saves.
 template <int HC, typename V, bool kConv = sizeof(V) == 8>
 __global__ void __launch_bounds__(kWarpKernelWarps * 32) CertWarpKernel(BMArgs a, const uint32_t* __restrict__ list,
                                                                        const uint32_t* __restrict__ bin_counts,
@@ -524,6 +346,7 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) CertWarpKernel(BMArgs a
   uint16_t* used = reinterpret_cast<uint16_t*>(base + size_t(HC) * (sizeof(V) + 4) + 32 * 4);
   unsigned long long fam_e = 0, fam_v = 0;
   const bool replay = a.out_target != nullptr;
+  const RoundView rv = RoundOf(a);
   for (int i = lane; i < HC; i += 32) {
     keys[i] = kNone;
     vals[i] = 0;
@@ -539,196 +362,17 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) CertWarpKernel(BMArgs a
   for (; idx < count; idx += wstride) {
     const uint64_t nidx = idx + wstride;
     const uint32_t nvid = nidx < count ? list[start + nidx] : 0u;
-    if (!InFront(a, vid)) {
+    if (!InFront(a, rv, vid)) {
       vid = nvid;
       continue;
     }
-    const VertexCtx x = LoadVertex<false>(a, vid);
+    const VertexCtx x = LoadVertexAs<ConstLoads>(a, vid);
     vid = nvid;
     if (lane == 0) {
       fam_e += x.d;
       fam_v += 1;
     }
-    uint32_t nused = 0;  // used[] entries (warp-uniform)
-    V tpart = 0;         // this lane's part of T (entries in the vertex's own cluster)
-    for (uint32_t e0 = 0; e0 < x.d; e0 += 32 * kCertUnroll) {
-      uint32_t uu[kCertUnroll], cc[kCertUnroll];
-      float ww[kCertUnroll];
-#pragma unroll
-      for (int k = 0; k < kCertUnroll; ++k) {
-        const uint32_t e = e0 + 32 * k + lane;
-        uu[k] = x.v;
-        ww[k] = 0.f;
-        if (e < x.d) {
-          uu[k] = a.nbr[x.b + e];
-          ww[k] = a.w ? a.w[x.b + e] : 1.0f;
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < kCertUnroll; ++k) cc[k] = uu[k] != x.v ? __ldg(a.C + uu[k]) : kNone;
-#pragma unroll
-      for (int k = 0; k < kCertUnroll; ++k) {
-      if (e0 + 32 * k >= x.d) break;  // warp-uniform
-      const float wt = ww[k];
-      const bool cand = uu[k] != x.v;
-      const uint32_t cu = cc[k];
-      uint32_t slot = kNone;
-      bool ins = false;
-      if (cand) {
-        slot = FindOrInsertT<false>(keys, HC, cu, &ins);
-        if (slot == kNone) atomicExch(&a.ctr->error, kErrHashFull);
-      }
-      const unsigned im = __ballot_sync(kFull, ins);
-      if (im) {
-        if (ins) used[nused + __popc(im & LaneMaskLt())] = static_cast<uint16_t>(slot);
-        nused += __popc(im);
-      }
-      const V xi = cand ? EntryUnits<V, kConv>(a, wt) : V(0);
-      if (cand && cu == x.c) tpart += xi;
-      if (slot != kNone) {
-        if constexpr (sizeof(V) == 4) atomicAdd(reinterpret_cast<int*>(&vals[slot]), xi);
-        else atomicAdd(reinterpret_cast<unsigned long long*>(&vals[slot]), static_cast<unsigned long long>(xi));
-      }
-      __syncwarp();
-      }
-    }
-    // T: the lanes' own-cluster parts.
-    V T;
-    if constexpr (sizeof(V) == 4) {
-      T = __reduce_add_sync(kFull, tpart);
-    } else {
-      T = tpart;
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) T += __shfl_xor_sync(kFull, T, o);
-    }
-    const float r32 = Res32Of(a, x.v);
-    const float k32 = a.kf[x.v];
-    const ChangeApproxT<V> ca = ApproxChange<V>(r32, a.int_nw != 0, k32, a.Kf[x.c], T);
-    const float cabs = ChangeAbsBound(ca);
-    // The first kCertRegRounds candidates of each lane (i = lane + 32 r) keep
-    // their slot, sum, Kf and filter value in registers across the passes;
-    // any further ones are read again.
-    uint32_t rslot[kCertRegRounds];
-    V rS[kCertRegRounds];
-    float rKf[kCertRegRounds];
-    V vmax = sizeof(V) == 4 ? V(INT_MIN) : V(LLONG_MIN);
-#pragma unroll
-    for (int r = 0; r < kCertRegRounds; ++r) {
-      const uint32_t i = lane + 32 * r;
-      rslot[r] = 0xFFFFu;
-      rS[r] = 0;
-      rKf[r] = 0.f;
-      if (i < nused) {
-        rslot[r] = used[i];
-        rS[r] = vals[rslot[r]];
-        rKf[r] = a.Kf[keys[rslot[r]]];
-        vmax = max(vmax, rS[r]);
-      }
-    }
-    for (uint32_t i = lane + 32 * kCertRegRounds; i < nused; i += 32) vmax = max(vmax, vals[used[i]]);
-    const V smax = WarpMaxV<V>(vmax);
-    float U = -CUDART_INF_F;
-    // The two largest upper ends (Y + e; +inf outside the error model) of
-    // this lane's candidates and the index of the largest: when the second
-    // is below U, only that one can be a contender.  Kept for the bins of
-    // more than 128 entries, where lanes hold several candidates (in the
-    // 33-128 bin it costs about what it saves).
-    constexpr bool kTop2 = HC >= 512;
-    float hi1 = -CUDART_INF_F, hi2 = -CUDART_INF_F;
-    uint32_t i1 = kNone;
-    FilterVal rf[kCertRegRounds];
-#pragma unroll
-    for (int r = 0; r < kCertRegRounds; ++r) {
-      rf[r].sane = false;
-      if (lane + 32 * r < nused) {
-        rf[r] = FilterOf<V>(r32, k32, rKf[r], rS[r], smax, cabs);
-        if (rf[r].sane) U = fmaxf(U, __fsub_rn(rf[r].Y, rf[r].e));
-        if (kTop2) KeepTop2(hi1, hi2, i1, rf[r].sane ? __fadd_rn(rf[r].Y, rf[r].e) : CUDART_INF_F, lane + 32 * r);
-      }
-    }
-    for (uint32_t i = lane + 32 * kCertRegRounds; i < nused; i += 32) {
-      const uint32_t slot = used[i];
-      const FilterVal f = FilterOf<V>(r32, k32, a.Kf[keys[slot]], vals[slot], smax, cabs);
-      if (f.sane) U = fmaxf(U, __fsub_rn(f.Y, f.e));
-      if (kTop2) KeepTop2(hi1, hi2, i1, f.sane ? __fadd_rn(f.Y, f.e) : CUDART_INF_F, i);
-    }
-    U = WarpMaxFinite(U);
-    LexKeyT<V> lead, tail;
-    // The contenders are the candidates with Y + e >= U (all when U = -inf).
-    const bool skip = kTop2 && hi2 < U;
-    if (skip) {
-      // At most candidate i1 is a contender: the others are cleared and
-      // marked without evaluating them again.
-      for (uint32_t i = lane; i < nused; i += 32) {
-        const uint32_t slot = used[i];
-        if (i == i1 && !(hi1 < U)) {
-          const uint32_t key = keys[slot];
-          const V S = vals[slot];
-          const unsigned long long ko = KOrder(a.K[key]);
-          lead.Keep(S, ko, key);
-          tail.Keep(-S, ~ko, key);
-          continue;
-        }
-        keys[slot] = kNone;
-        vals[slot] = 0;
-        used[i] = 0xFFFFu;
-      }
-    }
-    const uint32_t rescan_end = skip ? 0u : nused;
-#pragma unroll
-    for (int r = 0; r < kCertRegRounds; ++r) {
-      const uint32_t i = lane + 32 * r;
-      if (i >= rescan_end) continue;
-      const uint32_t slot = rslot[r];
-      if (rf[r].sane && __fadd_rn(rf[r].Y, rf[r].e) < U) {
-        keys[slot] = kNone;  // not a contender: cleared now, skipped later
-        vals[slot] = 0;
-        used[i] = 0xFFFFu;
-        continue;
-      }
-      const uint32_t key = keys[slot];
-      const unsigned long long ko = KOrder(a.K[key]);
-      lead.Keep(rS[r], ko, key);
-      tail.Keep(-rS[r], ~ko, key);
-    }
-    for (uint32_t i = lane + 32 * kCertRegRounds; i < rescan_end; i += 32) {
-      const uint32_t slot = used[i];
-      const uint32_t key = keys[slot];
-      const FilterVal f = FilterOf<V>(r32, k32, a.Kf[key], vals[slot], smax, cabs);
-      if (f.sane && __fadd_rn(f.Y, f.e) < U) {
-        keys[slot] = kNone;  // not a contender: cleared now, skipped later
-        vals[slot] = 0;
-        used[i] = 0xFFFFu;
-        continue;
-      }
-      const unsigned long long ko = KOrder(a.K[key]);
-      const V S = vals[slot];
-      lead.Keep(S, ko, key);
-      tail.Keep(-S, ~ko, key);
-    }
-    const bool single = LexWarpLead<V>(lead, tail);
-    int cres = kUncertain;
-    uint32_t ctarget = kNone;
-    if (single) {
-      const float KfA = lead.id != kNone ? a.Kf[lead.id] : 0.f;
-      cres = CertifyDecision<V>(ca, r32, k32, lead.id != kNone, lead.S, KfA, lead.id, a.n, &ctarget);
-    }
-    const uint32_t cmove = cres == kUncertain ? kNone : CertifiedMove(a, x, ctarget, cres == kCertMove);
-    bool append = false;
-    if (replay || cres == kUncertain) {
-      append = WarpExact<HC, V>(a, x, T, keys, vals, used, nused, replay, cres, cmove);
-    } else if (lane == 0) {
-      append = ApplyCertified(a, x, cmove);
-    }
-    __syncwarp();
-    // Clear the table through the key list (used[] may hold 0xFFFF marks).
-    for (uint32_t i = lane; i < nused; i += 32) {
-      const uint32_t slot = used[i];
-      if (slot != 0xFFFFu) {
-        keys[slot] = kNone;
-        vals[slot] = 0;
-      }
-    }
+    const bool append = WarpStep<HC, V, kConv, ConstLoads>(a, rv, x, vals, keys, used, replay);
     mb.Add(&a.ctr->movers, a.movers, append, x.v);
     __syncwarp();
   }
@@ -748,8 +392,6 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) CertWarpKernel(BMArgs a
 // shared memory.  An uncertain (or replayed) vertex takes WarpExact on warp 0
 // over the whole table, exactly as in the warp kernel.
 // ---------------------------------------------------------------------------
-constexpr int kCtaWarps = 4;
-
 template <int HC, typename V>
 constexpr size_t CertCtaSmem() {
   return size_t(HC) * (sizeof(V) + 4 + 2);  // vals, keys, used
@@ -764,199 +406,37 @@ __global__ void __launch_bounds__(kCtaWarps * 32) CertCtaKernel(BMArgs a, const 
   V* vals = reinterpret_cast<V*>(smem);
   uint32_t* keys = reinterpret_cast<uint32_t*>(smem + size_t(HC) * sizeof(V));
   uint16_t* used = reinterpret_cast<uint16_t*>(smem + size_t(HC) * (sizeof(V) + 4));
-  __shared__ uint32_t s_nused;
-  __shared__ V s_max[kCtaWarps];
-  __shared__ float s_u[kCtaWarps];
-  __shared__ V s_ls[kCtaWarps], s_ts[kCtaWarps];
-  __shared__ unsigned long long s_lk[kCtaWarps], s_tk[kCtaWarps];
-  __shared__ uint32_t s_li[kCtaWarps], s_ti[kCtaWarps];
+  __shared__ CtaShared<V> sh;
   __shared__ uint32_t mover_buf[64];  // warp 0's
   WarpMoverBuffer mb{mover_buf};
   const uint32_t count = bin_counts[bin];
   const uint32_t start = bin_starts[bin];
-  const unsigned tid = threadIdx.x, lane = LaneId(), warp = tid >> 5;
+  const unsigned tid = threadIdx.x, warp = tid >> 5;
   unsigned long long fam_e = 0, fam_v = 0;
   const bool replay = a.out_target != nullptr;
+  const RoundView rv = RoundOf(a);
   for (int i = tid; i < HC; i += BT) {
     keys[i] = kNone;
     vals[i] = 0;
   }
-  if (tid == 0) s_nused = 0;
+  if (tid == 0) sh.nused = 0;
   __syncthreads();
   uint32_t vid = blockIdx.x < count ? list[start + blockIdx.x] : 0u;
   for (uint64_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
     const uint64_t nidx = idx + gridDim.x;
     const uint32_t nvid = nidx < count ? list[start + nidx] : 0u;
-    if (!InFront(a, vid)) {  // uniform over the CTA
+    if (!InFront(a, rv, vid)) {  // uniform over the CTA
       vid = nvid;
       continue;
     }
-    const VertexCtx x = LoadVertex<false>(a, vid);
+    const VertexCtx x = LoadVertexAs<ConstLoads>(a, vid);
     vid = nvid;
     if (tid == 0) {
       fam_e += x.d;
       fam_v += 1;
     }
-    for (uint32_t e0 = 0; e0 < x.d; e0 += BT * kCertUnroll) {
-      uint32_t uu[kCertUnroll], cc[kCertUnroll];
-      float ww[kCertUnroll];
-#pragma unroll
-      for (int k = 0; k < kCertUnroll; ++k) {
-        const uint32_t e = e0 + BT * k + tid;
-        uu[k] = x.v;
-        ww[k] = 0.f;
-        if (e < x.d) {
-          uu[k] = a.nbr[x.b + e];
-          ww[k] = a.w ? a.w[x.b + e] : 1.0f;
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < kCertUnroll; ++k) cc[k] = uu[k] != x.v ? __ldg(a.C + uu[k]) : kNone;
-#pragma unroll
-      for (int k = 0; k < kCertUnroll; ++k) {
-        if (e0 + BT * k + 32 * warp >= x.d) break;  // uniform over the warp
-        const bool cand = uu[k] != x.v;
-        const uint32_t cu = cc[k];
-        uint32_t slot = kNone;
-        bool ins = false;
-        if (cand) {
-          slot = FindOrInsertT<false>(keys, HC, cu, &ins);
-          if (slot == kNone) atomicExch(&a.ctr->error, kErrHashFull);
-        }
-        const unsigned im = __ballot_sync(kFull, ins);
-        if (im) {
-          const int first = __ffs(im) - 1;
-          uint32_t base = 0;
-          if (int(lane) == first) base = atomicAdd(&s_nused, uint32_t(__popc(im)));
-          base = __shfl_sync(kFull, base, first);
-          if (ins) used[base + __popc(im & LaneMaskLt())] = static_cast<uint16_t>(slot);
-        }
-        const V xi = cand ? EntryUnits<V, kConv>(a, ww[k]) : V(0);
-        if (slot != kNone) {
-          if constexpr (sizeof(V) == 4)
-            atomicAdd(reinterpret_cast<int*>(&vals[slot]), xi);
-          else
-            atomicAdd(reinterpret_cast<unsigned long long*>(&vals[slot]),
-                      static_cast<unsigned long long>(xi));
-        }
-      }
-    }
-    __syncthreads();  // table complete
-    const uint32_t nused = s_nused;
-    V T = 0;
-    {
-      const uint32_t slot = FindT<false>(keys, HC, x.c);
-      if (slot != kNone) T = vals[slot];
-    }
-    const float k32 = a.kf[x.v];
-    const ChangeApproxT<V> ca = ApproxChange<V>(Res32Of(a, x.v), a.int_nw != 0, k32, a.Kf[x.c], T);
-    const float cabs = ChangeAbsBound(ca);
-    V vmax = sizeof(V) == 4 ? V(INT_MIN) : V(LLONG_MIN);
-    for (uint32_t i = tid; i < nused; i += BT) vmax = max(vmax, vals[used[i]]);
-    vmax = WarpMaxV<V>(vmax);
-    if (lane == 0) s_max[warp] = vmax;
-    __syncthreads();
-    V smax = s_max[0];
-#pragma unroll
-    for (int w = 1; w < kCtaWarps; ++w) smax = max(smax, s_max[w]);
-    float U = -CUDART_INF_F;
-    float hi1 = -CUDART_INF_F, hi2 = -CUDART_INF_F;  // KeepTop2 of this thread's candidates
-    uint32_t i1 = kNone;
-    for (uint32_t i = tid; i < nused; i += BT) {
-      const uint32_t slot = used[i];
-      const FilterVal f = FilterOf<V>(Res32Of(a, x.v), k32, a.Kf[keys[slot]], vals[slot], smax, cabs);
-      if (f.sane) U = fmaxf(U, __fsub_rn(f.Y, f.e));
-      KeepTop2(hi1, hi2, i1, f.sane ? __fadd_rn(f.Y, f.e) : CUDART_INF_F, i);
-    }
-    U = WarpMaxFinite(U);
-    if (lane == 0) s_u[warp] = U;
-    __syncthreads();
-    U = s_u[0];
-#pragma unroll
-    for (int w = 1; w < kCtaWarps; ++w) U = fmaxf(U, s_u[w]);
-    LexKeyT<V> lead, tail;
-    // The contenders are the candidates with Y + e >= U (all when U = -inf);
-    // when this thread's runner-up is below U, at most its candidate i1 is
-    // one, and the others are cleared and marked without a second
-    // evaluation.
-    const bool rescan = !(hi2 < U);
-    if (!rescan) {
-      for (uint32_t i = tid; i < nused; i += BT) {
-        const uint32_t slot = used[i];
-        if (i == i1 && !(hi1 < U)) {
-          const uint32_t key = keys[slot];
-          const V S = vals[slot];
-          const unsigned long long ko = KOrder(a.K[key]);
-          lead.Keep(S, ko, key);
-          tail.Keep(-S, ~ko, key);
-          continue;
-        }
-        keys[slot] = kNone;
-        vals[slot] = 0;
-        used[i] = 0xFFFFu;
-      }
-    }
-    for (uint32_t i = tid; i < (rescan ? nused : 0u); i += BT) {
-      const uint32_t slot = used[i];
-      const uint32_t key = keys[slot];
-      const FilterVal f = FilterOf<V>(Res32Of(a, x.v), k32, a.Kf[key], vals[slot], smax, cabs);
-      if (f.sane && __fadd_rn(f.Y, f.e) < U) {
-        keys[slot] = kNone;  // not a contender: cleared now, skipped later
-        vals[slot] = 0;
-        used[i] = 0xFFFFu;
-        continue;
-      }
-      const unsigned long long ko = KOrder(a.K[key]);
-      const V S = vals[slot];
-      lead.Keep(S, ko, key);
-      tail.Keep(-S, ~ko, key);
-    }
-    LexWarpLeader<V>(lead);
-    LexWarpLeader<V>(tail);
-    if (lane == 0) {
-      s_ls[warp] = lead.S;
-      s_lk[warp] = lead.K;
-      s_li[warp] = lead.id;
-      s_ts[warp] = tail.S;
-      s_tk[warp] = tail.K;
-      s_ti[warp] = tail.id;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      LexKeyT<V> L, Tl;
-#pragma unroll
-      for (int w = 0; w < kCtaWarps; ++w) {
-        L.Keep(s_ls[w], s_lk[w], s_li[w]);
-        Tl.Keep(s_ts[w], s_tk[w], s_ti[w]);
-      }
-      // One (S, K) class among the contenders iff the lowest-ranked one
-      // (Tl: smallest S, then largest K) is in the leader's class.
-      const bool single = L.id == kNone || (-Tl.S == L.S && ~Tl.K == L.K);
-      int cres = kUncertain;
-      uint32_t ctarget = kNone;
-      if (single) {
-        const float KfA = L.id != kNone ? a.Kf[L.id] : 0.f;
-        cres = CertifyDecision<V>(ca, Res32Of(a, x.v), k32, L.id != kNone, L.S, KfA, L.id, a.n, &ctarget);
-      }
-      const uint32_t cmove = cres == kUncertain ? kNone : CertifiedMove(a, x, ctarget, cres == kCertMove);
-      bool append = false;
-      if (replay || cres == kUncertain) {
-        append = WarpExact<HC, V>(a, x, T, keys, vals, used, nused, replay, cres, cmove);
-      } else if (lane == 0) {
-        append = ApplyCertified(a, x, cmove);
-      }
-      mb.Add(&a.ctr->movers, a.movers, append, x.v);
-    }
-    __syncthreads();  // the table is read by WarpExact up to here
-    for (uint32_t i = tid; i < nused; i += BT) {
-      const uint32_t slot = used[i];
-      if (slot != 0xFFFFu) {
-        keys[slot] = kNone;
-        vals[slot] = 0;
-      }
-    }
-    if (tid == 0) s_nused = 0;
-    __syncthreads();
+    const bool append = CtaStep<HC, V, kConv, ConstLoads>(a, rv, x, vals, keys, used, sh, tid, 0, replay);
+    if (warp == 0) mb.Add(&a.ctr->movers, a.movers, append, x.v);
   }
   if (warp == 0) {
     mb.Flush(&a.ctr->movers, a.movers);

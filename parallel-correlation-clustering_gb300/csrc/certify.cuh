@@ -323,9 +323,9 @@ __device__ __forceinline__ uint32_t CertifiedMove(const BMArgs& a, const VertexC
 
 // Effects of a certified sync decision (moved flag, mover list): returns
 // true when the vertex must be appended to the movers list.
-__device__ __forceinline__ bool ApplyCertified(const BMArgs& a, const VertexCtx& x, uint32_t move) {
+__device__ __forceinline__ bool ApplyCertified(const BMArgs& a, const VertexCtx& x, uint32_t move, uint32_t stamp) {
   if (move == kNone) return false;
-  a.moved_stamp[x.v] = StampIn(a.rs, a.stamp);
+  a.moved_stamp[x.v] = stamp;
   if (move == x.c) return false;
   a.moves[x.v] = move;
   return true;

@@ -226,6 +226,7 @@ struct DevCounters {
 constexpr int kErrProbeLimit = 1;   // async new-cluster probe exceeded its bound
 constexpr int kErrHashFull = 2;     // a best-move hash table filled up
 constexpr int kErrCertMismatch = 3; // a certified decision differed from FP64 (replay self-check)
+constexpr int kErrBarrier = 5;      // a grid barrier's bounded wait gave up
 constexpr int kErrUnionRange = 4;   // a union graph's new-cluster id fell outside its range
 
 // Round state in device memory for rounds that run inside a device-side
@@ -399,6 +400,14 @@ inline LaunchTuning TuningFor(const Context* ctx, uint32_t n) {
 Status LaunchBestMoves(Context* ctx, const BMArgs& a, const uint32_t* list, const uint32_t* bin_counts,
                        const uint32_t* bin_starts, const uint32_t* host_counts, bool int_mode,
                        uint32_t max_deg, int families = kLaunchGroups | kLaunchWarps);
+
+// Level graphs of at most this many entries run their rounds in one kernel
+// (roundloop.cu).  Ten rounds, degree-binned kernels in a graph loop against
+// one kernel: 5.7M entries 4.3 -> 2.8 ms, 9.7M 6.5 -> 5.1 ms, 13.3M with 64-bit
+// sums 6.6 -> 6.5 ms, 20M with 64-bit sums 10.2 -> 12.4 ms, 31.4M 11.9 ->
+// 12.7 ms: above it the tails and launches that the one kernel saves are
+// small, and the binned kernels' higher occupancy wins.
+constexpr uint64_t kLoopMaxEntries = 12ull << 20;
 
 // The hub plan of a graph (built on first use).
 Status EnsureHubPlan(Context* ctx, const DevGraph* g);

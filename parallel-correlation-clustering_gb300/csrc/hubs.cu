@@ -8,20 +8,12 @@
 #include <mutex>
 #include <numeric>
 #include <unordered_map>
-#include <type_traits>
 #include <vector>
 
-#include "certify.cuh"
-#include "hubs.cuh"
-#include "moves.cuh"
+#include "hubeval.cuh"
 
 namespace pcc {
 namespace {
-
-constexpr int kHubUnroll = 4;              // entries per thread in flight
-constexpr uint32_t kHubMaxSub = 1u << 12;  // sub-partitions before giving up
-constexpr uint32_t kMaxCont = 256;         // contender list per CTA
-constexpr int kEvalBatch = 4;              // table slots per thread in flight (EvalTable)
 
 constexpr int kSmallThreads = 256;         // small hubs: CTA size, table slots
 constexpr uint32_t kSmallSlots = 2 * kHubSmallMax;
@@ -71,663 +63,6 @@ struct HubArgs {
   uint32_t* gdone;
 };
 
-// MurmurHash3's 32-bit finalizer (a bijection; every output bit depends on
-// every input bit).  The product with the capacity's high half picks the
-// slot, bits 8..19 the sub-partition, the top bits (again through a
-// product) the partition.
-__device__ __forceinline__ uint32_t Mix32(uint32_t x) {
-  x ^= x >> 16;
-  x *= 0x85EBCA6Bu;
-  x ^= x >> 13;
-  x *= 0xC2B2AE35u;
-  x ^= x >> 16;
-  return x;
-}
-
-__device__ __forceinline__ uint32_t SlotHash(uint32_t cu) {
-  // A second mix so that the slot is independent of the partition bits.
-  return Mix32(cu ^ 0x9E3779B9u);
-}
-
-__device__ __forceinline__ void KeepBest(double& bv, uint32_t& bi, double v, uint32_t i) {
-  if (i == kNone) return;
-  if (bi == kNone || v > bv || (v == bv && i < bi)) {
-    bv = v;
-    bi = i;
-  }
-}
-
-// Value types of the tables: int (narrow INT sums), long long (INT sums),
-// double (FP64 sums).
-template <typename V>
-__device__ __forceinline__ V AtomicAddV(V* p, V x) {
-  if constexpr (std::is_same<V, int>::value) {
-    return atomicAdd(p, x);
-  } else if constexpr (std::is_same<V, long long>::value) {
-    return static_cast<long long>(atomicAdd(reinterpret_cast<unsigned long long*>(p),
-                                            static_cast<unsigned long long>(x)));
-  } else {
-    return atomicAdd(p, x);
-  }
-}
-
-// Shared scratch of a hub CTA of BT threads besides its table.  The
-// reduction arrays hold one partial per warp; their last element carries a
-// result that warp 0 publishes (wide CTAs, HubChangeSmax).
-template <int BT>
-struct HubShared {
-  static constexpr int kW = BT / 32;
-  long long red_ll[kW + 1];
-  long long red_mx[kW + 1];
-  unsigned long long red_k[kW + 1];
-  double red_d[kW];
-  float red_f[kW + 1];
-  uint32_t red_i[kW + 1];
-  double stage_d[kW][32];
-  uint32_t cont_key[kMaxCont];
-  long long cont_S[kMaxCont];
-  uint32_t ncont;
-  uint32_t overflow;
-  uint32_t nkeys;
-  uint32_t last;  // global path: this CTA evaluated the hub's last slice
-  double change;
-  float change32;
-};
-
-// Block reductions; every thread receives the result.  In wide CTAs (512
-// threads and more) warp 0 combines the warps' partials and publishes the
-// result in red[BT / 32], so that the other threads read one value instead
-// of BT / 32; the combines here (max, integer sum, lexicographic and
-// (value, id) selections) give the same result in any order.
-template <int BT>
-constexpr bool kWideBlock = BT >= 512;
-
-template <int BT>
-__device__ __forceinline__ long long BlockMaxLL(long long x, long long* red) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) x = max(x, __shfl_xor_sync(kFull, x, o));
-  if (LaneId() == 0) red[threadIdx.x >> 5] = x;
-  __syncthreads();
-  if constexpr (kWideBlock<BT>) {
-    if (threadIdx.x < 32) {
-      long long r = threadIdx.x < BT / 32 ? red[threadIdx.x] : LLONG_MIN;
-#pragma unroll
-      for (int o = 16; o; o >>= 1) r = max(r, __shfl_xor_sync(kFull, r, o));
-      if (threadIdx.x == 0) red[BT / 32] = r;
-    }
-    __syncthreads();
-    return red[BT / 32];
-  }
-  long long r = red[0];
-#pragma unroll
-  for (int w = 1; w < BT / 32; ++w) r = max(r, red[w]);
-  __syncthreads();
-  return r;
-}
-
-template <int BT>
-__device__ __forceinline__ float BlockMaxF(float x, float* red) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) x = fmaxf(x, __shfl_xor_sync(kFull, x, o));
-  if (LaneId() == 0) red[threadIdx.x >> 5] = x;
-  __syncthreads();
-  if constexpr (kWideBlock<BT>) {
-    if (threadIdx.x < 32) {
-      float r = threadIdx.x < BT / 32 ? red[threadIdx.x] : -CUDART_INF_F;
-#pragma unroll
-      for (int o = 16; o; o >>= 1) r = fmaxf(r, __shfl_xor_sync(kFull, r, o));
-      if (threadIdx.x == 0) red[BT / 32] = r;
-    }
-    __syncthreads();
-    return red[BT / 32];
-  }
-  float r = red[0];
-#pragma unroll
-  for (int w = 1; w < BT / 32; ++w) r = fmaxf(r, red[w]);
-  __syncthreads();
-  return r;
-}
-
-// Deterministic sum: butterfly inside warps, then the warps in order.
-template <int BT, class T>
-__device__ __forceinline__ T BlockSum(T x, T* red) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    if constexpr (std::is_floating_point<T>::value) {
-      x = Dadd(x, __shfl_xor_sync(kFull, x, o));
-    } else {
-      x += __shfl_xor_sync(kFull, x, o);
-    }
-  }
-  if (LaneId() == 0) red[threadIdx.x >> 5] = x;
-  __syncthreads();
-  if constexpr (kWideBlock<BT> && std::is_integral<T>::value) {
-    if (threadIdx.x < 32) {
-      T r = threadIdx.x < BT / 32 ? red[threadIdx.x] : T(0);
-#pragma unroll
-      for (int o = 16; o; o >>= 1) r += __shfl_xor_sync(kFull, r, o);
-      if (threadIdx.x == 0) red[BT / 32] = r;
-    }
-    __syncthreads();
-    return red[BT / 32];
-  }
-  T r = red[0];
-#pragma unroll
-  for (int w = 1; w < BT / 32; ++w) {
-    if constexpr (std::is_floating_point<T>::value) {
-      r = Dadd(r, red[w]);
-    } else {
-      r += red[w];
-    }
-  }
-  __syncthreads();
-  return r;
-}
-
-// Argmax over (value desc, id asc) with integer compares: the values are
-// mapped to order-preserving 64-bit images (no FP64 instruction; the values
-// here are never -0, the only case where the image order and IEEE equality
-// differ).
-__device__ __forceinline__ unsigned long long ValBits(double d) {
-  const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(d));
-  return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
-}
-__device__ __forceinline__ double BitsVal(unsigned long long k) {
-  const unsigned long long b = (k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k;
-  return __longlong_as_double(static_cast<long long>(b));
-}
-__device__ __forceinline__ void KeepBits(unsigned long long& bo, uint32_t& bi, unsigned long long o, uint32_t i) {
-  if (i == kNone) return;
-  if (bi == kNone || o > bo || (o == bo && i < bi)) {
-    bo = o;
-    bi = i;
-  }
-}
-
-template <int BT>
-__device__ __forceinline__ void BlockArgmax(double& v, uint32_t& id, unsigned long long* redv, uint32_t* redi) {
-  unsigned long long o = ValBits(v);
-#pragma unroll
-  for (int off = 16; off; off >>= 1) {
-    const unsigned long long oo = __shfl_xor_sync(kFull, o, off);
-    const uint32_t oi = __shfl_xor_sync(kFull, id, off);
-    KeepBits(o, id, oo, oi);
-  }
-  if (LaneId() == 0) {
-    redv[threadIdx.x >> 5] = o;
-    redi[threadIdx.x >> 5] = id;
-  }
-  __syncthreads();
-  if constexpr (kWideBlock<BT>) {
-    if (threadIdx.x < 32) {
-      const bool in = threadIdx.x < BT / 32;
-      unsigned long long wo = redv[in ? threadIdx.x : 0];
-      uint32_t wi = in ? redi[threadIdx.x] : kNone;
-#pragma unroll
-      for (int off = 16; off; off >>= 1) {
-        const unsigned long long oo = __shfl_xor_sync(kFull, wo, off);
-        const uint32_t oi = __shfl_xor_sync(kFull, wi, off);
-        KeepBits(wo, wi, oo, oi);
-      }
-      if (threadIdx.x == 0) {
-        redv[BT / 32] = wo;
-        redi[BT / 32] = wi;
-      }
-    }
-    __syncthreads();
-    v = BitsVal(redv[BT / 32]);
-    id = redi[BT / 32];
-    return;
-  }
-  unsigned long long ro = redv[0];
-  uint32_t ri = redi[0];
-#pragma unroll
-  for (int w = 1; w < BT / 32; ++w) KeepBits(ro, ri, redv[w], redi[w]);
-  __syncthreads();
-  v = BitsVal(ro);
-  id = ri;
-}
-
-template <int BT, typename I>
-__device__ __forceinline__ LexKeyT<I> BlockLex(LexKeyT<I> x, long long* rs, unsigned long long* rk, uint32_t* ri) {
-  LexGroupReduce<32, I>(x);
-  if (LaneId() == 0) {
-    rs[threadIdx.x >> 5] = x.S;
-    rk[threadIdx.x >> 5] = x.K;
-    ri[threadIdx.x >> 5] = x.id;
-  }
-  __syncthreads();
-  if constexpr (kWideBlock<BT>) {
-    if (threadIdx.x < 32) {
-      LexKeyT<I> w;
-      if (threadIdx.x < BT / 32) w.Keep(static_cast<I>(rs[threadIdx.x]), rk[threadIdx.x], ri[threadIdx.x]);
-      LexGroupReduce<32, I>(w);
-      if (threadIdx.x == 0) {
-        rs[BT / 32] = w.S;
-        rk[BT / 32] = w.K;
-        ri[BT / 32] = w.id;
-      }
-    }
-    __syncthreads();
-    LexKeyT<I> r;
-    r.Keep(static_cast<I>(rs[BT / 32]), rk[BT / 32], ri[BT / 32]);
-    return r;
-  }
-  LexKeyT<I> r;
-#pragma unroll
-  for (int w = 0; w < BT / 32; ++w) r.Keep(static_cast<I>(rs[w]), rk[w], ri[w]);
-  __syncthreads();
-  return r;
-}
-
-// Block leader of `lead` and the class test over `tail` (the two BlockLex
-// calls and the (S, K) comparison) with 32-bit sums: warp leaders by REDUX,
-// the warps' leaders combined by every thread, the test by one barrier with
-// a predicate.
-template <int BT>
-__device__ __forceinline__ bool BlockLexLeadInt(LexKeyT<int>& lead, const LexKeyT<int>& tail, long long* rs,
-                                                unsigned long long* rk, uint32_t* ri) {
-  LexWarpLeaderInt(lead);
-  if (LaneId() == 0) {
-    rs[threadIdx.x >> 5] = lead.S;
-    rk[threadIdx.x >> 5] = lead.K;
-    ri[threadIdx.x >> 5] = lead.id;
-  }
-  __syncthreads();
-  LexKeyT<int> r;
-  if constexpr (kWideBlock<BT>) {
-    if (threadIdx.x < 32) {
-      LexKeyT<int> w;
-      if (threadIdx.x < BT / 32) w.Keep(static_cast<int>(rs[threadIdx.x]), rk[threadIdx.x], ri[threadIdx.x]);
-      LexWarpLeaderInt(w);
-      if (threadIdx.x == 0) {
-        rs[BT / 32] = w.S;
-        rk[BT / 32] = w.K;
-        ri[BT / 32] = w.id;
-      }
-    }
-    __syncthreads();
-    r.Keep(static_cast<int>(rs[BT / 32]), rk[BT / 32], ri[BT / 32]);
-  } else {
-#pragma unroll
-    for (int w = 0; w < BT / 32; ++w) r.Keep(static_cast<int>(rs[w]), rk[w], ri[w]);
-  }
-  lead = r;
-  const bool diff = r.id != kNone && tail.id != kNone && (-tail.S != r.S || ~tail.K != r.K);
-  return !__syncthreads_or(diff);  // also orders the reads of rs/rk/ri before their next use
-}
-
-// Finds or inserts `key` in a table of `cap` slots (any capacity), probing
-// linearly from the slot the hash picks; kNone when the table is full.
-__device__ __forceinline__ uint32_t HubInsert(uint32_t* keys, uint32_t cap, uint32_t hsh, uint32_t key,
-                                              bool* ins) {
-  uint32_t s = __umulhi(hsh, cap);
-  *ins = false;
-  for (uint32_t pr = 0; pr < cap; ++pr) {
-    const uint32_t k = *reinterpret_cast<volatile uint32_t*>(keys + s);
-    if (k == key) return s;
-    if (k == kNone) {
-      const uint32_t old = atomicCAS(keys + s, kNone, key);
-      if (old == kNone) {
-        *ins = true;
-        return s;
-      }
-      if (old == key) return s;
-    }
-    s = s + 1 == cap ? 0 : s + 1;
-  }
-  return kNone;
-}
-
-// Entry contribution w - offset: integer in INT mode, the reference hub
-// path's float-rounded value in FP64 mode.
-template <bool kInt, typename V>
-__device__ __forceinline__ void EntryWeight(const BMArgs& a, float wt, V* xi, double* xd) {
-  if constexpr (kInt) {
-    *xi = EntryUnits<V, true>(a, wt);
-  } else {
-    *xd = static_cast<double>(static_cast<float>(Dsub(static_cast<double>(wt), a.offset)));
-  }
-}
-
-// Warp-aggregated FP64 sum of the entry weights of each match group, in lane
-// order (for the group's leader).
-template <int BT>
-__device__ __forceinline__ double GroupWeights(unsigned peers, bool leader, double xd, HubShared<BT>& sh) {
-  const unsigned warp = threadIdx.x >> 5, lane = LaneId();
-  sh.stage_d[warp][lane] = xd;
-  __syncwarp();
-  double acc = 0.0;
-  if (leader) {
-    unsigned mm = peers;
-    while (mm) {
-      acc = Dadd(acc, sh.stage_d[warp][__ffs(mm) - 1]);
-      mm &= mm - 1;
-    }
-  }
-  __syncwarp();
-  return acc;
-}
-
-// Evaluates the CTA's table: returns (to every thread) the best (exact FP64
-// value, id) of its keys and clears the table.  INT sync mode: FP32
-// pre-filter, then FP64 only for the survivors outside the leading (S, K)
-// class, whose members share one FP64 value (evaluated once).
-template <int BT, bool kInt, bool kAsync, typename V>
-__device__ void EvalTable(const BMArgs& a, const VertexCtx& x, float k32, double change, long long smax_ll,
-                          uint32_t* skeys, V* svals, uint32_t cap, HubShared<BT>& sh, double* out_v,
-                          uint32_t* out_id) {
-  // Integer type of the sums: int for narrow tables (32-bit conversions).
-  using I = typename std::conditional<std::is_same<V, int>::value, int, long long>::type;
-  const unsigned tid = threadIdx.x;
-  constexpr bool kFilter = kInt && !kAsync;
-  double lv = 0.0;
-  uint32_t lid = kNone;
-  // Slots are read kEvalBatch at a time per thread, so that the gathers of
-  // their cluster weights are in flight together.
-  constexpr int kB = kEvalBatch;
-  if (kFilter) {
-    const I smax = static_cast<I>(smax_ll);
-    const float c32 = __fmul_rn(sh.change32, a.wscale);  // in the units of the sums
-    const float r32 = Res32Of(a, x.v);
-    float U = -CUDART_INF_F;
-    // The two largest upper ends (Y + e; +inf for a candidate outside the
-    // error model) among this thread's slots, and the slot of the largest:
-    // when the second is below the block's U, no other slot of the thread
-    // can be a contender and the second pass need not re-evaluate them.
-    float hi1 = -CUDART_INF_F, hi2 = -CUDART_INF_F;
-    uint32_t slot1 = kNone;
-    for (uint32_t s0 = tid; s0 < cap; s0 += BT * kB) {
-      uint32_t kk[kB];
-      I ss[kB];
-      float kf[kB];
-#pragma unroll
-      for (int j = 0; j < kB; ++j) {
-        const uint32_t s = s0 + j * BT;
-        kk[j] = s < cap ? skeys[s] : kNone;
-        ss[j] = s < cap ? static_cast<I>(svals[s]) : I(0);
-      }
-#pragma unroll
-      for (int j = 0; j < kB; ++j) kf[j] = kk[j] != kNone ? a.Kf[kk[j]] : 0.f;
-#pragma unroll
-      for (int j = 0; j < kB; ++j) {
-        if (kk[j] == kNone) continue;
-        const FilterVal f = FilterOf<I>(r32, k32, kf[j], ss[j], smax, c32);
-        if (f.sane) U = fmaxf(U, __fsub_rn(f.Y, f.e));
-        KeepTop2(hi1, hi2, slot1, f.sane ? __fadd_rn(f.Y, f.e) : CUDART_INF_F, s0 + j * BT);
-      }
-    }
-    if (tid == 0) sh.ncont = 0;
-    U = BlockMaxF<BT>(U, sh.red_f);
-    LexKeyT<I> lead, tail;
-    // The contenders are the slots with hi >= U (every slot when U = -inf).
-    const bool rescan = !(hi2 < U);
-    if (!rescan) {
-      // At most slot1 is a contender; the thread's other slots are cleared.
-      if (slot1 != kNone && !(hi1 < U)) {
-        const uint32_t key = skeys[slot1];
-        const I S = static_cast<I>(svals[slot1]);
-        const double KD = a.K[key];
-        const unsigned long long ko = KOrder(KD);
-        lead.Keep(S, ko, key);
-        tail.Keep(-S, ~ko, key);
-        const uint32_t pos = atomicAdd(&sh.ncont, 1u);
-        if (pos < kMaxCont) {
-          sh.cont_key[pos] = key;
-          sh.cont_S[pos] = S;
-        } else {
-          KeepBest(lv, lid, ValOf(a, x, change, UnitsToDouble<I>(a, S), KD), key);  // list full: now
-        }
-      }
-      for (uint32_t s = tid; s < cap; s += BT) {
-        if (skeys[s] != kNone) {
-          skeys[s] = kNone;
-          svals[s] = V(0);
-        }
-      }
-    }
-    for (uint32_t s0 = rescan ? tid : cap; s0 < cap; s0 += BT * kB) {
-      uint32_t kk[kB];
-      I ss[kB];
-      float kf[kB];
-#pragma unroll
-      for (int j = 0; j < kB; ++j) {
-        const uint32_t s = s0 + j * BT;
-        kk[j] = kNone;
-        ss[j] = I(0);
-        if (s < cap) {
-          kk[j] = skeys[s];
-          if (kk[j] != kNone) {
-            ss[j] = static_cast<I>(svals[s]);
-            skeys[s] = kNone;
-            svals[s] = V(0);
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kB; ++j) kf[j] = kk[j] != kNone ? a.Kf[kk[j]] : 0.f;
-#pragma unroll
-      for (int j = 0; j < kB; ++j) {
-        const uint32_t key = kk[j];
-        if (key == kNone) continue;
-        const I S = ss[j];
-        const FilterVal f = FilterOf<I>(r32, k32, kf[j], S, smax, c32);
-        if (f.sane && __fadd_rn(f.Y, f.e) < U) continue;
-        const double KD = a.K[key];
-        const unsigned long long ko = KOrder(KD);
-        lead.Keep(S, ko, key);
-        tail.Keep(-S, ~ko, key);
-        const uint32_t pos = atomicAdd(&sh.ncont, 1u);
-        if (pos < kMaxCont) {
-          sh.cont_key[pos] = key;
-          sh.cont_S[pos] = S;
-        } else {
-          KeepBest(lv, lid, ValOf(a, x, change, UnitsToDouble<I>(a, S), KD), key);  // list full: now
-        }
-      }
-    }
-    bool single;
-    if constexpr (std::is_same<I, int>::value) {
-      single = BlockLexLeadInt<BT>(lead, tail, sh.red_ll, sh.red_k, sh.red_i);
-    } else {
-      lead = BlockLex<BT, I>(lead, sh.red_ll, sh.red_k, sh.red_i);
-      tail = BlockLex<BT, I>(tail, sh.red_ll, sh.red_k, sh.red_i);
-      single = lead.id == kNone || (-tail.S == lead.S && ~tail.K == lead.K);
-    }
-    const uint32_t nc = min(sh.ncont, kMaxCont);
-    if (!single) {
-      for (uint32_t i = tid; i < nc; i += BT) {
-        const uint32_t key = sh.cont_key[i];
-        const I S = static_cast<I>(sh.cont_S[i]);
-        const double KD = a.K[key];
-        if (S == lead.S && KOrder(KD) == lead.K) continue;  // the leading class
-        KeepBest(lv, lid, ValOf(a, x, change, UnitsToDouble<I>(a, S), KD), key);
-      }
-    }
-    if (tid == 0 && lead.id != kNone)
-      KeepBest(lv, lid, ValOf(a, x, change, UnitsToDouble<I>(a, lead.S), a.K[lead.id]), lead.id);
-  } else {
-    for (uint32_t s0 = tid; s0 < cap; s0 += BT * kB) {
-      uint32_t kk[kB];
-      V sv[kB];
-      double kd[kB];
-#pragma unroll
-      for (int j = 0; j < kB; ++j) {
-        const uint32_t s = s0 + j * BT;
-        kk[j] = kNone;
-        sv[j] = V(0);
-        if (s < cap) {
-          kk[j] = skeys[s];
-          if (kk[j] != kNone) {
-            sv[j] = svals[s];
-            skeys[s] = kNone;
-            svals[s] = V(0);
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kB; ++j) kd[j] = kk[j] != kNone ? LdK<kAsync>(a.K + kk[j]) : 0.0;
-#pragma unroll
-      for (int j = 0; j < kB; ++j)
-        if (kk[j] != kNone) KeepBest(lv, lid, ValOf(a, x, change, kInt ? UnitsToDouble<I>(a, static_cast<I>(sv[j])) : static_cast<double>(sv[j]), kd[j]),
-                   kk[j]);
-    }
-  }
-  BlockArgmax<BT>(lv, lid, sh.red_k, sh.red_i);
-  *out_v = lv;
-  *out_id = lid;
-}
-
-template <bool kAsync>
-__device__ __forceinline__ void HubDecide(const BMArgs& a, const VertexCtx& x, double bv, uint32_t bi,
-                                          double change) {
-  if (bi == kNone) {  // no entries: the reduce identity (0, 0.0)
-    bv = 0.0;
-    bi = 0;
-  }
-  const bool append = Decide<kAsync>(a, x, bv, bi, change);
-  if (!kAsync && append) a.movers[atomicAdd(&a.ctr->movers, 1u)] = x.v;
-}
-
-// One CTA's scan of a hub row: the entries whose cluster falls in partition
-// p / sub-partition q are added into the CTA's table; "together" (the hub's
-// own cluster) accumulates when want_T.  Returns the largest sum seen
-// (INT mode) through *smax.
-template <int BT, bool kInt, bool kAsync, typename V>
-__device__ __forceinline__ void ScanRow(const BMArgs& a, const VertexCtx& x, uint32_t P, uint32_t p, uint32_t Q,
-                                        uint32_t q, bool want_T, uint32_t* skeys, V* svals, uint32_t cap,
-                                        uint32_t maxkeys, HubShared<BT>& sh, long long* t_int, double* t_dbl,
-                                        long long* smax) {
-  const unsigned tid = threadIdx.x, lane = LaneId();
-  const uint32_t v = x.v;
-  for (uint32_t e0 = 0; e0 < x.d; e0 += BT * kHubUnroll) {
-    uint32_t uu[kHubUnroll], cc[kHubUnroll];
-    float ww[kHubUnroll];
-#pragma unroll
-    for (int k = 0; k < kHubUnroll; ++k) {
-      const uint32_t e = e0 + k * BT + tid;
-      uu[k] = v;
-      ww[k] = 0.f;
-      if (e < x.d) {
-        uu[k] = a.nbr[x.b + e];
-        ww[k] = a.w ? a.w[x.b + e] : 1.0f;
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < kHubUnroll; ++k) cc[k] = uu[k] != v ? LdC<kAsync>(a.C + uu[k]) : kNone;
-#pragma unroll
-    for (int k = 0; k < kHubUnroll; ++k) {
-      if (e0 + k * BT >= x.d) break;  // uniform over the CTA
-      const bool cand = uu[k] != v;
-      const uint32_t cu = cc[k];
-      V xi = 0;
-      double xd = 0.0;
-      if (cand) EntryWeight<kInt, V>(a, ww[k], &xi, &xd);
-      if (want_T && cand && cu == x.c) {
-        if (kInt)
-          *t_int += xi;
-        else
-          *t_dbl = Dadd(*t_dbl, xd);
-      }
-      bool mine = cand;
-      if (P > 1 || Q > 1) {
-        const uint32_t hp = Mix32(cu);
-        mine = mine && __umulhi(hp, P) == p && ((hp >> 8) & (Q - 1)) == q;
-      }
-      // INT mode: every entry adds its own integer weight (exact in any
-      // order); FP64 mode: equal clusters of the warp are summed in lane
-      // order first, one atomic per cluster.
-      unsigned peers = 0;
-      bool leader = mine;
-      double Sd = 0.0;
-      if (!kInt) {
-        peers = __match_any_sync(kFull, mine ? cu : LaneSentinel(lane));
-        leader = mine && int(lane) == __ffs(peers) - 1;
-        Sd = GroupWeights<BT>(peers, leader, xd, sh);
-      }
-      if (leader && *reinterpret_cast<volatile uint32_t*>(&sh.overflow) == 0) {
-        bool ins;
-        const uint32_t slot = HubInsert(skeys, cap, SlotHash(cu), cu, &ins);
-        if (slot == kNone) {
-          sh.overflow = 1;
-        } else {
-          if (ins && atomicAdd(&sh.nkeys, 1u) + 1 > maxkeys) sh.overflow = 1;
-          if (kInt) {
-            const V old = AtomicAddV<V>(svals + slot, xi);
-            *smax = max(*smax, static_cast<long long>(old) + static_cast<long long>(xi));
-          } else {
-            AtomicAddV<V>(svals + slot, static_cast<V>(Sd));
-          }
-        }
-      }
-    }
-  }
-}
-
-// The hub's "together" and change, once per item (FP64 by one thread).
-template <int BT, bool kInt>
-__device__ __forceinline__ double HubChange(const BMArgs& a, const VertexCtx& x, long long t_int, double t_dbl,
-                                            HubShared<BT>& sh) {
-  double T;
-  if (kInt)
-    T = UnitsToDouble<long long>(a, BlockSum<BT, long long>(t_int, sh.red_ll));
-  else
-    T = BlockSum<BT, double>(t_dbl, sh.red_d);
-  if (threadIdx.x == 0) {
-    sh.change = ChangeOf(a, x, T);
-    sh.change32 = static_cast<float>(sh.change);
-  }
-  __syncthreads();
-  return sh.change;
-}
-
-// HubChange and, in INT mode, the block maximum of the running sums.  Wide
-// CTAs take both in one reduction: warp 0 combines the warps' (sum, max)
-// partials and its lane 0 computes the change, so that the table scan's end
-// costs two barriers.
-template <int BT, bool kInt>
-__device__ __forceinline__ double HubChangeSmax(const BMArgs& a, const VertexCtx& x, long long t_int, double t_dbl,
-                                                long long* smax, HubShared<BT>& sh) {
-  if constexpr (!kWideBlock<BT>) {
-    __syncthreads();
-    const double change = HubChange<BT, kInt>(a, x, t_int, t_dbl, sh);
-    if (kInt) *smax = BlockMaxLL<BT>(*smax, sh.red_ll);
-    return change;
-  } else if constexpr (!kInt) {
-    return HubChange<BT, kInt>(a, x, t_int, t_dbl, sh);
-  } else {
-    constexpr int kW = BT / 32;
-    long long t = t_int, m = *smax;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      t += __shfl_xor_sync(kFull, t, o);
-      m = max(m, __shfl_xor_sync(kFull, m, o));
-    }
-    if (LaneId() == 0) {
-      sh.red_ll[threadIdx.x >> 5] = t;
-      sh.red_mx[threadIdx.x >> 5] = m;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      long long wt = threadIdx.x < kW ? sh.red_ll[threadIdx.x] : 0;
-      long long wm = threadIdx.x < kW ? sh.red_mx[threadIdx.x] : LLONG_MIN;
-#pragma unroll
-      for (int o = 16; o; o >>= 1) {
-        wt += __shfl_xor_sync(kFull, wt, o);
-        wm = max(wm, __shfl_xor_sync(kFull, wm, o));
-      }
-      if (threadIdx.x == 0) {
-        sh.change = ChangeOf(a, x, UnitsToDouble<long long>(a, wt));
-        sh.change32 = static_cast<float>(sh.change);
-        sh.red_mx[kW] = wm;
-      }
-    }
-    __syncthreads();
-    *smax = sh.red_mx[kW];
-    return sh.change;
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Small hubs: one CTA per hub, a table of 2 * degree slots (never full).
 // ---------------------------------------------------------------------------
@@ -771,7 +106,7 @@ __global__ void __launch_bounds__(kSmallThreads) HubSmallKernel(HubArgs h) {
     double bv;
     uint32_t bi;
     EvalTable<BT, kInt, kAsync, V>(a, x, a.kf[v], change, smax, skeys, svals, cap, sh, &bv, &bi);
-    if (tid == 0) HubDecide<kAsync>(a, x, bv, bi, change);
+    if (tid == 0) HubDecide<kAsync>(a, x, bv, bi, change, StampIn(a.rs, a.stamp), &a.ctr->movers);
     __syncthreads();
   }
   if (tid == 0 && fam_v) {
@@ -820,6 +155,7 @@ __global__ void __launch_bounds__(kBigThreads) HubBigKernel(HubArgs h) {
     uint32_t Q = 1, q = 0;
     bool have_T = false;
     double change = 0.0;
+    long long shift = 0;  // sub-passes of 64-bit sums: the first one's
     double bestv = 0.0;
     uint32_t bestid = kNone;
     while (true) {
@@ -830,10 +166,12 @@ __global__ void __launch_bounds__(kBigThreads) HubBigKernel(HubArgs h) {
       // The reductions' barriers also order the reads of sh.overflow.
       if (!have_T) {
         change = HubChangeSmax<BT, kInt>(a, x, t_int, t_dbl, &smax, sh);
+        shift = smax;
         have_T = true;
       } else {
         __syncthreads();
         if (kInt) smax = BlockMaxLL<BT>(smax, sh.red_ll);
+        if (kInt && smax == LLONG_MIN) smax = shift;
       }
       const bool overflow = sh.overflow != 0;
       __syncthreads();
@@ -877,7 +215,7 @@ __global__ void __launch_bounds__(kBigThreads) HubBigKernel(HubArgs h) {
         uint32_t bi = kNone;
         for (uint32_t j = 0; j < P; ++j) KeepBest(bv, bi, __ldcg(h.part_val + pb + j), __ldcg(h.part_id + pb + j));
         h.done[hb] = 0;
-        HubDecide<kAsync>(a, x, bv, bi, change);
+        HubDecide<kAsync>(a, x, bv, bi, change, StampIn(a.rs, a.stamp), &a.ctr->movers);
       }
     }
     __syncthreads();
@@ -946,10 +284,10 @@ __global__ void __launch_bounds__(kGlobThreads) HubGlobalAccumKernel(HubArgs h) 
         unsigned peers = 0;
         bool leader = cand;
         double Sd = 0.0;
-        if (!kInt) {
+        if constexpr (!kInt) {
           peers = __match_any_sync(kFull, cand ? cu : LaneSentinel(lane));
           leader = cand && int(lane) == __ffs(peers) - 1;
-          Sd = GroupWeights<BT>(peers, leader, xd, sh);
+          Sd = GroupWeights<BT>(peers, leader, xd);
         }
         if (leader) {
           bool ins;
@@ -1031,7 +369,7 @@ __global__ void __launch_bounds__(kGlobThreads) HubGlobalEvalKernel(HubArgs h) {
       for (uint32_t j = tid; j < ns; j += BT) KeepBest(cv, ci, __ldcg(h.gpart_val + sb + j), __ldcg(h.gpart_id + sb + j));
       BlockArgmax<BT>(cv, ci, sh.red_k, sh.red_i);
       if (tid == 0) {
-        HubDecide<false>(a, x, cv, ci, change);
+        HubDecide<false>(a, x, cv, ci, change, StampIn(a.rs, a.stamp), &a.ctr->movers);
         h.gdone[gi] = 0;
         h.gt_int[gi] = 0;
         h.gt_dbl[gi] = 0.0;
@@ -1169,7 +507,9 @@ Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan
   std::vector<uint32_t> small_v, big_v, parts, pbase, item_hub, item_part;
   std::vector<uint32_t> big_glob, glob_hub, glob_cap, glob_item, glob_item_start;
   std::vector<uint32_t> glob_nslices, glob_sbase, slice_hub, slice_start;
-  std::vector<unsigned long long> glob_base;
+  std::vector<uint32_t> loop_cap, loop_nslices, loop_sbase, loop_chunk_hub, loop_chunk_start, loop_slice_hub,
+      loop_slice_start;
+  std::vector<unsigned long long> glob_base, loop_base;
   uint64_t total = 0;
   for (uint32_t r = 0; r < count; ++r) {
     const uint32_t i = order[r];
@@ -1203,6 +543,22 @@ Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan
     } else {
       big_glob.push_back(kNone);
     }
+    if (g.m <= kLoopMaxEntries) {
+      const uint32_t cap = 2 * hd[i] + 2;
+      loop_base.push_back(plan->loop_slots);
+      plan->loop_slots += cap;
+      loop_cap.push_back(cap);
+      loop_nslices.push_back((cap + kLoopSlice - 1) / kLoopSlice);
+      loop_sbase.push_back(static_cast<uint32_t>(loop_slice_hub.size()));
+      for (uint32_t e = 0; e < hd[i]; e += kLoopChunk) {
+        loop_chunk_hub.push_back(hb);
+        loop_chunk_start.push_back(e);
+      }
+      for (uint32_t s0 = 0; s0 < cap; s0 += kLoopSlice) {
+        loop_slice_hub.push_back(hb);
+        loop_slice_start.push_back(s0);
+      }
+    }
     parts.push_back(P);
     pbase.push_back(static_cast<uint32_t>(total));
     total += P;
@@ -1216,32 +572,53 @@ Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan
   plan->num_big = static_cast<uint32_t>(big_v.size());
   plan->num_items = static_cast<uint32_t>(item_hub.size());
   plan->num_partials = total;
-  auto up = [&](DBuf<uint32_t>& d, const std::vector<uint32_t>& hvec) -> Status {
-    if (hvec.empty()) return Status::Ok();
-    PCC_RETURN_IF_ERROR(d.Alloc(ctx, hvec.size()));
-    return d.FromHost(hvec.data(), hvec.size());
+  // One upload for the 32-bit lists, one for the 64-bit ones.
+  std::vector<uint32_t> pack;
+  std::vector<std::pair<const uint32_t**, size_t>> at;
+  auto add = [&](const uint32_t** field, const std::vector<uint32_t>& x) {
+    at.emplace_back(field, pack.size());
+    pack.insert(pack.end(), x.begin(), x.end());
   };
-  PCC_RETURN_IF_ERROR(up(plan->small_v, small_v));
-  PCC_RETURN_IF_ERROR(up(plan->big_v, big_v));
-  PCC_RETURN_IF_ERROR(up(plan->big_parts, parts));
-  PCC_RETURN_IF_ERROR(up(plan->big_pbase, pbase));
-  PCC_RETURN_IF_ERROR(up(plan->item_hub, item_hub));
-  PCC_RETURN_IF_ERROR(up(plan->item_part, item_part));
+  add(&plan->small_v, small_v);
+  add(&plan->big_v, big_v);
+  add(&plan->big_parts, parts);
+  add(&plan->big_pbase, pbase);
+  add(&plan->item_hub, item_hub);
+  add(&plan->item_part, item_part);
   plan->num_glob = static_cast<uint32_t>(glob_hub.size());
   plan->num_glob_items = static_cast<uint32_t>(glob_item.size());
+  plan->num_glob_slices = static_cast<uint32_t>(slice_hub.size());
   if (plan->num_glob) {
-    PCC_RETURN_IF_ERROR(up(plan->big_glob, big_glob));
-    PCC_RETURN_IF_ERROR(up(plan->glob_hub, glob_hub));
-    PCC_RETURN_IF_ERROR(up(plan->glob_cap, glob_cap));
-    PCC_RETURN_IF_ERROR(up(plan->glob_item, glob_item));
-    PCC_RETURN_IF_ERROR(up(plan->glob_item_start, glob_item_start));
-    plan->num_glob_slices = static_cast<uint32_t>(slice_hub.size());
-    PCC_RETURN_IF_ERROR(up(plan->glob_nslices, glob_nslices));
-    PCC_RETURN_IF_ERROR(up(plan->glob_sbase, glob_sbase));
-    PCC_RETURN_IF_ERROR(up(plan->slice_hub, slice_hub));
-    PCC_RETURN_IF_ERROR(up(plan->slice_start, slice_start));
-    PCC_RETURN_IF_ERROR(plan->glob_base.Alloc(ctx, glob_base.size()));
-    PCC_RETURN_IF_ERROR(plan->glob_base.FromHost(glob_base.data(), glob_base.size()));
+    add(&plan->big_glob, big_glob);
+    add(&plan->glob_hub, glob_hub);
+    add(&plan->glob_cap, glob_cap);
+    add(&plan->glob_item, glob_item);
+    add(&plan->glob_item_start, glob_item_start);
+    add(&plan->glob_nslices, glob_nslices);
+    add(&plan->glob_sbase, glob_sbase);
+    add(&plan->slice_hub, slice_hub);
+    add(&plan->slice_start, slice_start);
+  }
+  std::vector<unsigned long long> pack64 = glob_base;
+  const size_t loop_base_at = pack64.size();
+  pack64.insert(pack64.end(), loop_base.begin(), loop_base.end());
+  plan->num_loop_chunks = static_cast<uint32_t>(loop_chunk_hub.size());
+  plan->num_loop_slices = static_cast<uint32_t>(loop_slice_hub.size());
+  add(&plan->loop_cap, loop_cap);
+  add(&plan->loop_nslices, loop_nslices);
+  add(&plan->loop_sbase, loop_sbase);
+  add(&plan->loop_chunk_hub, loop_chunk_hub);
+  add(&plan->loop_chunk_start, loop_chunk_start);
+  add(&plan->loop_slice_hub, loop_slice_hub);
+  add(&plan->loop_slice_start, loop_slice_start);
+  PCC_RETURN_IF_ERROR(plan->pack.Alloc(ctx, std::max<size_t>(pack.size(), 1)));
+  PCC_RETURN_IF_ERROR(plan->pack.FromHost(pack.data(), pack.size()));
+  for (const auto& f : at) *f.first = plan->pack.p + f.second;
+  if (!pack64.empty()) {
+    PCC_RETURN_IF_ERROR(plan->pack64.Alloc(ctx, pack64.size()));
+    PCC_RETURN_IF_ERROR(plan->pack64.FromHost(pack64.data(), pack64.size()));
+    plan->glob_base = plan->pack64.p;
+    plan->loop_base = plan->pack64.p + loop_base_at;
   }
   return Sync(ctx);  // host vectors go out of scope
 }
@@ -1254,27 +631,32 @@ Status AllocHubState(Context* ctx, const HubPlan& plan, HubState* st) {
   }
   const uint64_t nh = std::max<uint32_t>(plan.num_big, 1);
   if (st->done.count < nh) PCC_RETURN_IF_ERROR(st->done.Alloc(ctx, nh));
-  if (plan.num_glob) {
+  // Tables and accumulators of the global path or of the whole-level kernel
+  // (one of the two runs a level).
+  const uint64_t slots = std::max(plan.glob_slots, plan.loop_slots);
+  const uint32_t hubs = plan.loop_slots ? plan.num_big : plan.num_glob;
+  const uint32_t slices = std::max(plan.num_glob_slices, plan.num_loop_slices);
+  if (slots) {
     // The rounds leave the tables clean; they are reset here all the same,
     // at every level, so that a run cut short cannot leave keys behind.
-    if (st->gkeys.count < plan.glob_slots) {
-      PCC_RETURN_IF_ERROR(st->gkeys.Alloc(ctx, plan.glob_slots));
-      PCC_RETURN_IF_ERROR(st->gvals.Alloc(ctx, plan.glob_slots));
+    if (st->gkeys.count < slots) {
+      PCC_RETURN_IF_ERROR(st->gkeys.Alloc(ctx, slots));
+      PCC_RETURN_IF_ERROR(st->gvals.Alloc(ctx, slots));
     }
-    if (st->gt_int.count < plan.num_glob) {
-      PCC_RETURN_IF_ERROR(st->gt_int.Alloc(ctx, plan.num_glob));
-      PCC_RETURN_IF_ERROR(st->gt_dbl.Alloc(ctx, plan.num_glob));
-      PCC_RETURN_IF_ERROR(st->gsmax.Alloc(ctx, plan.num_glob));
-      PCC_RETURN_IF_ERROR(st->gdone.Alloc(ctx, plan.num_glob));
+    if (st->gt_int.count < hubs) {
+      PCC_RETURN_IF_ERROR(st->gt_int.Alloc(ctx, hubs));
+      PCC_RETURN_IF_ERROR(st->gt_dbl.Alloc(ctx, hubs));
+      PCC_RETURN_IF_ERROR(st->gsmax.Alloc(ctx, hubs));
+      PCC_RETURN_IF_ERROR(st->gdone.Alloc(ctx, hubs));
     }
-    if (st->gpart_val.count < plan.num_glob_slices) {
-      PCC_RETURN_IF_ERROR(st->gpart_val.Alloc(ctx, plan.num_glob_slices));
-      PCC_RETURN_IF_ERROR(st->gpart_id.Alloc(ctx, plan.num_glob_slices));
+    if (st->gpart_val.count < slices) {
+      PCC_RETURN_IF_ERROR(st->gpart_val.Alloc(ctx, slices));
+      PCC_RETURN_IF_ERROR(st->gpart_id.Alloc(ctx, slices));
     }
-    PCC_CUDA(cudaMemsetAsync(st->gkeys.p, 0xFF, plan.glob_slots * sizeof(uint32_t), ctx->stream));  // kNone
-    PCC_CUDA(cudaMemsetAsync(st->gvals.p, 0, plan.glob_slots * sizeof(unsigned long long), ctx->stream));
-    GlobalStateInitKernel<<<Blocks(plan.num_glob, 256, 1024), 256, 0, ctx->stream>>>(
-        plan.num_glob, st->gt_int.p, st->gt_dbl.p, st->gsmax.p, st->gdone.p);
+    PCC_CUDA(cudaMemsetAsync(st->gkeys.p, 0xFF, slots * sizeof(uint32_t), ctx->stream));  // kNone
+    PCC_CUDA(cudaMemsetAsync(st->gvals.p, 0, slots * sizeof(unsigned long long), ctx->stream));
+    GlobalStateInitKernel<<<Blocks(hubs, 256, 1024), 256, 0, ctx->stream>>>(hubs, st->gt_int.p, st->gt_dbl.p,
+                                                                            st->gsmax.p, st->gdone.p);
     PCC_COUNT(1);
   }
   return st->done.Zero();
@@ -1314,36 +696,36 @@ Status LaunchHubBestMoves(Context* ctx, const BMArgs& a, const HubPlan& plan, Hu
   if (plan.num_hubs == 0) return Status::Ok();
   HubArgs h;
   h.a = a;
-  h.small_v = plan.small_v.p;
+  h.small_v = plan.small_v;
   h.small_lo = 0;
   h.small_hi = plan.num_small;
-  h.big_v = plan.big_v.p;
-  h.big_parts = plan.big_parts.p;
-  h.big_pbase = plan.big_pbase.p;
-  h.item_hub = plan.item_hub.p;
-  h.item_part = plan.item_part.p;
+  h.big_v = plan.big_v;
+  h.big_parts = plan.big_parts;
+  h.big_pbase = plan.big_pbase;
+  h.item_hub = plan.item_hub;
+  h.item_part = plan.item_part;
   h.num_items = plan.num_items;
   h.part_val = st.part_val.p;
   h.part_id = st.part_id.p;
   h.done = st.done.p;
   h.num_glob = plan.num_glob;
   h.num_glob_items = plan.num_glob_items;
-  h.glob_hub = plan.glob_hub.p;
-  h.glob_base = plan.glob_base.p;
-  h.glob_cap = plan.glob_cap.p;
-  h.glob_item = plan.glob_item.p;
-  h.glob_item_start = plan.glob_item_start.p;
-  h.big_glob = plan.big_glob.p;
+  h.glob_hub = plan.glob_hub;
+  h.glob_base = plan.glob_base;
+  h.glob_cap = plan.glob_cap;
+  h.glob_item = plan.glob_item;
+  h.glob_item_start = plan.glob_item_start;
+  h.big_glob = plan.big_glob;
   h.gkeys = st.gkeys.p;
   h.gvals = st.gvals.p;
   h.gt_int = st.gt_int.p;
   h.gt_dbl = st.gt_dbl.p;
   h.gsmax = st.gsmax.p;
   h.num_glob_slices = plan.num_glob_slices;
-  h.glob_nslices = plan.glob_nslices.p;
-  h.glob_sbase = plan.glob_sbase.p;
-  h.slice_hub = plan.slice_hub.p;
-  h.slice_start = plan.slice_start.p;
+  h.glob_nslices = plan.glob_nslices;
+  h.glob_sbase = plan.glob_sbase;
+  h.slice_hub = plan.slice_hub;
+  h.slice_start = plan.slice_start;
   h.gpart_val = st.gpart_val.p;
   h.gpart_id = st.gpart_id.p;
   h.gdone = st.gdone.p;

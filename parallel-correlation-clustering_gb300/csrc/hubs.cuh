@@ -31,6 +31,8 @@ constexpr uint32_t kHubSmallMax = 4096;   // one-partition hubs
 constexpr uint32_t kHubBigKeys = 12288;   // expected distinct keys per big-hub partition
 constexpr uint32_t kHubGlobalParts = 4;    // big hubs with >= this many partitions take the global path
 constexpr uint32_t kHubGlobalSlice = 1024;   // table slots evaluated by one CTA
+constexpr uint32_t kLoopChunk = 2048;         // row entries per work item (roundloop.cu)
+constexpr uint32_t kLoopSlice = 2048;         // table slots per work item (roundloop.cu)
 
 // Static part (depends on the graph only).
 struct HubPlan {
@@ -41,12 +43,15 @@ struct HubPlan {
   uint32_t num_big = 0;
   uint32_t num_items = 0;      // big-hub work items (hub, partition)
   uint64_t num_partials = 0;   // one per big-hub item
-  DBuf<uint32_t> small_v;      // small hubs, largest first
-  DBuf<uint32_t> big_v;        // big hubs, largest first
-  DBuf<uint32_t> big_parts;    // P per big hub
-  DBuf<uint32_t> big_pbase;    // first partial of the big hub
-  DBuf<uint32_t> item_hub;     // work items, largest hubs first
-  DBuf<uint32_t> item_part;
+  // The lists below lie in one device buffer each (one upload per plan).
+  DBuf<uint32_t> pack;
+  DBuf<unsigned long long> pack64;
+  const uint32_t* small_v = nullptr;    // small hubs, largest first
+  const uint32_t* big_v = nullptr;      // big hubs, largest first
+  const uint32_t* big_parts = nullptr;  // P per big hub
+  const uint32_t* big_pbase = nullptr;  // first partial of the big hub
+  const uint32_t* item_hub = nullptr;   // work items, largest hubs first
+  const uint32_t* item_part = nullptr;
   // Big hubs with at least kHubGlobalParts partitions, synchronous rounds:
   // many CTAs accumulate a row's chunks into one per-hub table in HBM, then
   // one CTA per hub evaluates it (a row of millions of entries would
@@ -54,19 +59,33 @@ struct HubPlan {
   uint32_t num_glob = 0;
   uint32_t num_glob_items = 0;
   uint64_t glob_slots = 0;
-  DBuf<uint32_t> glob_hub;               // per global hub: its big-hub index
-  DBuf<unsigned long long> glob_base;    // first table slot
-  DBuf<uint32_t> glob_cap;               // table slots (2 * degree + 2: never full)
-  DBuf<uint32_t> glob_item;              // per work item: global hub index
-  DBuf<uint32_t> glob_item_start;        // first entry of the item's chunk
-  DBuf<uint32_t> big_glob;               // per big hub: global hub index or kNone
+  const uint32_t* glob_hub = nullptr;              // per global hub: its big-hub index
+  const unsigned long long* glob_base = nullptr;   // first table slot
+  const uint32_t* glob_cap = nullptr;              // table slots (2 * degree + 2: never full)
+  const uint32_t* glob_item = nullptr;             // per work item: global hub index
+  const uint32_t* glob_item_start = nullptr;       // first entry of the item's chunk
+  const uint32_t* big_glob = nullptr;              // per big hub: global hub index or kNone
   // Evaluation: the table is split into slices of kHubGlobalSlice slots, one
   // CTA each; the hub's last CTA combines the slices' bests.
   uint32_t num_glob_slices = 0;
-  DBuf<uint32_t> glob_nslices;           // per global hub
-  DBuf<uint32_t> glob_sbase;             // per global hub: first partial
-  DBuf<uint32_t> slice_hub;              // per slice: global hub index
-  DBuf<uint32_t> slice_start;            // per slice: first slot (within the hub's table)
+  const uint32_t* glob_nslices = nullptr;          // per global hub
+  const uint32_t* glob_sbase = nullptr;            // per global hub: first partial
+  const uint32_t* slice_hub = nullptr;             // per slice: global hub index
+  const uint32_t* slice_start = nullptr;           // per slice: first slot (within the hub's table)
+  // The same for every big hub, in rows of kLoopChunk entries and slices of
+  // kLoopSlice slots: the kernel that runs a whole level's rounds
+  // (roundloop.cu; graphs of at most kLoopMaxEntries entries).
+  uint32_t num_loop_chunks = 0;
+  uint32_t num_loop_slices = 0;
+  uint64_t loop_slots = 0;
+  const unsigned long long* loop_base = nullptr;   // per big hub: first table slot
+  const uint32_t* loop_cap = nullptr;              // per big hub: 2 * degree + 2
+  const uint32_t* loop_nslices = nullptr;          // per big hub
+  const uint32_t* loop_sbase = nullptr;            // per big hub: first partial
+  const uint32_t* loop_chunk_hub = nullptr;        // per chunk: big-hub index
+  const uint32_t* loop_chunk_start = nullptr;      // per chunk: first entry
+  const uint32_t* loop_slice_hub = nullptr;        // per slice: big-hub index
+  const uint32_t* loop_slice_start = nullptr;      // per slice: first slot
 };
 
 // Per-context mutable state; counters are zero between rounds.

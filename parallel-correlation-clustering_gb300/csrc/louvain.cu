@@ -20,6 +20,7 @@
 
 #include "graphops.cuh"
 #include "hubs.cuh"
+#include "roundloop.cuh"
 
 namespace pcc {
 
@@ -792,6 +793,45 @@ class Engine {
     return Status::Ok();
   }
 
+  // Best-move arguments of a level's rounds (frontier and round state unset).
+  BMArgs LevelArgs(const Level& L) {
+    const DevGraph& g = *L.g;
+    BMArgs a{};
+    a.n = g.n;
+    a.off = g.off.p;
+    a.nbr = g.nbr.p;
+    a.w = g.wp();
+    a.C = L.C.p;
+    a.s = L.s.p;
+    a.k = L.k.p;
+    a.K = L.K.p;
+    a.Kf = L.Kf.p;
+    a.kf = L.kf.p;
+    a.int_nw = int_nw_ ? 1 : 0;
+    a.res = cfg_.resolution;
+    SetSumMode(&a, L.mode);
+    a.offset = cfg_.edge_weight_offset;
+    a.ioffset = static_cast<int32_t>(cfg_.edge_weight_offset);
+    a.stamp = stamp_;
+    a.moves = moves_.p;
+    a.moved_stamp = moved_stamp_.p;
+    a.movers = movers_.p;
+    a.ctr = ctr_.p;
+    a.async = cfg_.async ? 1 : 0;
+    a.s_mut = L.s.p;
+    a.K_mut = L.K.p;
+    a.C_mut = L.C.p;
+    a.moved_cluster_stamp = mod_stamp_.p;
+    if (cfg_.async) {
+      a.free_ids = free_ids_.p;
+      a.free_ctr = free_ctr_.p;
+      a.free_cap = g.n;
+    }
+    a.vres = L.vres.p;
+    a.vres32 = L.vres32.p;
+    return a;
+  }
+
   // The work of one best-move round, enqueued on the context stream with no
   // host read: counter resets, the best-move kernels, the application of the
   // moves (sync) and, unless ALL_MOVE, the next frontier with its size and
@@ -805,40 +845,8 @@ class Engine {
     PCC_CUDA(cudaMemsetAsync(&ctr_.p->frontier, 0, sizeof(uint32_t) * 4, ctx_->stream));
     PCC_CUDA(cudaMemsetAsync(&ctr_.p->pend_edges, 0, sizeof(unsigned long long), ctx_->stream));
 
-    BMArgs a{};
-    a.n = n;
-    a.off = g.off.p;
-    a.nbr = g.nbr.p;
-    a.w = g.wp();
-    a.C = L->C.p;
-    a.s = L->s.p;
-    a.k = L->k.p;
-    a.K = L->K.p;
-    a.Kf = L->Kf.p;
-    a.kf = L->kf.p;
-    a.int_nw = int_nw_ ? 1 : 0;
-    a.res = cfg_.resolution;
-    SetSumMode(&a, L->mode);
-    a.offset = cfg_.edge_weight_offset;
-    a.ioffset = static_cast<int32_t>(cfg_.edge_weight_offset);
-    a.stamp = stamp_;
-    a.moves = moves_.p;
-    a.moved_stamp = moved_stamp_.p;
-    a.movers = movers_.p;
-    a.ctr = ctr_.p;
-    a.async = cfg_.async ? 1 : 0;
-    a.s_mut = L->s.p;
-    a.K_mut = L->K.p;
-    a.C_mut = L->C.p;
-    a.moved_cluster_stamp = mod_stamp_.p;
-    if (cfg_.async) {
-      a.free_ids = free_ids_.p;
-      a.free_ctr = free_ctr_.p;
-      a.free_cap = n;
-    }
+    BMArgs a = LevelArgs(*L);
     a.rs = rs;
-    a.vres = L->vres.p;
-    a.vres32 = L->vres32.p;
     a.front_stamp = (rs || front_stamp) ? next_stamp_.p : nullptr;
     a.front_val = front_stamp;
     const BinSet& bins = *L->bins;
@@ -1224,9 +1232,71 @@ class Engine {
     return Status::Ok();
   }
 
+  // IterateBestMoves in one cooperative kernel (roundloop.cu): levels of at
+  // most kLoopMaxEntries entries with exact sums.
+  Status IterateLoop(Level* L, int64_t num_inner, bool* moved_out) {
+    const DevGraph& g = *L->g;
+    RoundState h{};
+    h.front_all = 1;
+    h.front_edges = g.m;
+    h.front_size = g.n;
+    h.visited = L->bins->size;
+    h.stamp = stamp_;  // the first round's stamp is the next one
+    PCC_RETURN_IF_ERROR(rs_.FromHost(&h, 1));
+    PCC_CUDA(cudaMemsetAsync(&ctr_.p->level_moved, 0, sizeof(uint32_t) * 2, ctx_->stream));  // level_moved, rounds
+    PCC_CUDA(cudaMemsetAsync(&ctr_.p->edge_visits, 0, sizeof(unsigned long long) * 2, ctx_->stream));
+    PCC_CUDA(cudaMemsetAsync(&ctr_.p->sync_moves, 0, sizeof(unsigned long long) * 2, ctx_->stream));
+    if (!loop_state_.p) {
+      PCC_RETURN_IF_ERROR(loop_state_.Alloc(ctx_, 1));
+      PCC_RETURN_IF_ERROR(old_cluster_.Alloc(ctx_, std::max<uint64_t>(n_max_, 1)));
+    }
+    RoundLoopArgs l{};
+    l.a = LevelArgs(*L);
+    l.a.front_stamp = next_stamp_.p;
+    l.a.waves = 1;
+    l.list = L->bins->list.p;
+    l.starts = L->bins->counts.p + kNumBins;
+    l.push_list = g.bins.list.p;
+    l.push_starts = g.bins.counts.p + kNumBins;
+    l.m = g.m;
+    l.binned = L->bins->size;
+    l.num_inner = static_cast<uint32_t>(std::min<int64_t>(num_inner, 0xFFFFFFFF));
+    l.move_method = cfg_.move_method;
+    l.mod_stamp = mod_stamp_.p;
+    l.new_stamp = new_stamp_.p;
+    l.next_stamp = next_stamp_.p;
+    l.old_cluster = old_cluster_.p;
+    l.zero_ids = zero_ids_.p;
+    l.new_list = new_list_.p;
+    l.Kf_mut = L->Kf.p;
+    l.rs = rs_.p;
+    l.st = loop_state_.p;
+    SetLoopHubs(&l, *g.hub_plan, hub_state_);
+    PCC_RETURN_IF_ERROR(LaunchRoundLoop(ctx_, l, L->mode, L->bins->host_counts, g.max_deg));
+    DevCounters hc;
+    RoundState hr;
+    PCC_RETURN_IF_ERROR(ctr_.ToHost(&hc, 1));
+    PCC_RETURN_IF_ERROR(rs_.ToHost(&hr, 1));
+    PCC_RETURN_IF_ERROR(Sync(ctx_));
+    if (hc.error) return MakeError(PCC_INTERNAL, "device error flag " + std::to_string(hc.error));
+    stamp_ = hr.stamp;
+    res_.rounds += static_cast<int32_t>(hc.rounds);
+    res_.edge_visits += hc.edge_visits;
+    res_.vertex_visits += hc.vertex_visits;
+    res_.algo_bytes += (g.w.p ? 12ull : 8ull) * hc.edge_visits + 40ull * hc.visited;
+    res_.moves += hc.sync_moves;
+    *moved_out = hc.level_moved != 0;
+    return Status::Ok();
+  }
+
   // The round loop of one level: on the device when it can be (synchronous
-  // moves, one graph, no detailed timing), else driven from the host.
+  // moves, one graph, no detailed timing), else driven from the host.  The
+  // one-kernel loop takes the shapes it was built for: with launch shapes set
+  // by the caller, or serial families, the degree-binned kernels run.
   Status Iterate(Level* L, int64_t num_inner, bool* moved_out) {
+    if (!cfg_.async && !un_ && !ctx_->detailed_timing && !ctx_->tuned && ctx_->overlap_families && num_inner > 0 &&
+        cfg_.clustering_moves_method == PCC_LOUVAIN && RoundLoopFits(ctx_, *L->g, L->mode))
+      return IterateLoop(L, num_inner, moved_out);
     if (!cfg_.async && !un_ && !ctx_->detailed_timing && !ctx_->graphs_failed &&
         cfg_.clustering_moves_method == PCC_LOUVAIN && L->g->m >= ctx_->device_loop_min_entries)
       return IterateDevice(L, num_inner, moved_out);
@@ -1733,6 +1803,8 @@ class Engine {
   uint32_t sm_val_ = 0;
   DBuf<uint32_t> scan_tiles_;
   HubState hub_state_;
+  DBuf<LoopState> loop_state_;  // one-kernel round loop
+  DBuf<uint32_t> old_cluster_;
   DBuf<DevCounters> ctr_;
   RunResult res_;
   PhaseTimer timer_;

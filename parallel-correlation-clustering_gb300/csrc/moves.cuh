@@ -116,6 +116,24 @@ __device__ __forceinline__ uint32_t WaveOf(uint32_t v, uint32_t salt, uint32_t w
   return __umulhi(x, waves);
 }
 
+// The round a kernel works on: its stamp and its frontier (the vertices with
+// front_stamp == front_val, or every vertex).
+struct RoundView {
+  uint32_t stamp;
+  uint32_t front_val;
+  bool all;
+};
+__device__ __forceinline__ RoundView RoundOf(const BMArgs& a) {
+  RoundView r;
+  r.stamp = StampIn(a.rs, a.stamp);
+  r.front_val = a.rs ? a.rs->front_val : a.front_val;
+  r.all = a.rs ? a.rs->front_all != 0 : a.front_stamp == nullptr;
+  return r;
+}
+__device__ __forceinline__ bool InFront(const BMArgs& a, const RoundView& r, uint32_t v) {
+  return r.all || a.front_stamp[v] == r.front_val;
+}
+
 __device__ __forceinline__ bool InFront(const BMArgs& a, uint32_t v) {
   if (a.waves > 1 && WaveOf(v, a.wave_salt, a.waves) != a.wave) return false;
   if (a.rs) return a.rs->front_all || a.front_stamp[v] == a.rs->front_val;
@@ -130,6 +148,29 @@ struct VertexCtx {
   double kv;
   double Kc;
 };
+
+// The state as a kernel that also changes it between its own rounds reads
+// it: through L1, which the barrier between two phases invalidates, and not
+// through the read-only path.
+struct LiveLoads {
+  static __device__ __forceinline__ uint32_t C(const uint32_t* p) { return *p; }
+  static __device__ __forceinline__ double K(const double* p) { return *p; }
+};
+struct ConstLoads {
+  static __device__ __forceinline__ uint32_t C(const uint32_t* p) { return __ldg(p); }
+  static __device__ __forceinline__ double K(const double* p) { return __ldg(p); }
+};
+template <class L>
+__device__ __forceinline__ VertexCtx LoadVertexAs(const BMArgs& a, uint32_t v) {
+  VertexCtx x;
+  x.v = v;
+  x.b = a.off[v];
+  x.d = uint32_t(a.off[v + 1] - x.b);
+  x.c = L::C(a.C + v);
+  x.kv = a.k[v];
+  x.Kc = L::K(a.K + x.c);
+  return x;
+}
 
 template <bool kAsync>
 __device__ __forceinline__ VertexCtx LoadVertex(const BMArgs& a, uint32_t v) {
@@ -172,7 +213,7 @@ __device__ __forceinline__ float FilterBound(float R, float Y, float S, float ch
 // Returns true when the vertex must be appended to the movers list (sync).
 template <bool kAsync>
 __device__ __forceinline__ bool Decide(const BMArgs& a, const VertexCtx& x, double best, uint32_t bid,
-                                       double change) {
+                                       double change, uint32_t stamp) {
   uint32_t target;
   double value;
   if (bid == kNone || change >= best) {
@@ -245,8 +286,8 @@ __device__ __forceinline__ bool Decide(const BMArgs& a, const VertexCtx& x, doub
       dest = uint32_t(i);
     }
     __stcg(&a.C_mut[x.v], dest);
-    a.moved_cluster_stamp[dest] = StampIn(a.rs, a.stamp);
-    a.moved_stamp[x.v] = StampIn(a.rs, a.stamp);
+    a.moved_cluster_stamp[dest] = stamp;
+    a.moved_stamp[x.v] = stamp;
     atomicAdd(&a.ctr->moves, 1ull);
     return false;
   }
@@ -260,7 +301,7 @@ __device__ __forceinline__ bool Decide(const BMArgs& a, const VertexCtx& x, doub
   }
   if (a.out_moves) a.out_moves[x.v] = v2 > 0 ? t2 : kNone;
   if (v2 > 0) {
-    a.moved_stamp[x.v] = StampIn(a.rs, a.stamp);
+    a.moved_stamp[x.v] = stamp;
     if (t2 != x.c) {
       a.moves[x.v] = t2;
       return true;
@@ -358,6 +399,19 @@ __device__ __forceinline__ V EntryUnits(const BMArgs& a, float w) {
   } else {
     return WeightToInt(w) - a.ioffset;
   }
+}
+
+// Adds to a sum in shared memory.  64-bit sums take two 32-bit atomics, the
+// low word's carry going with the high one: each is one native instruction,
+// where a 64-bit shared-memory add is a compare-and-swap loop.  The sum is
+// whole once every add is done (a barrier).
+__device__ __forceinline__ void SharedAdd(int* p, int x) { atomicAdd(p, x); }
+__device__ __forceinline__ void SharedAdd(long long* p, long long x) {
+  unsigned* w = reinterpret_cast<unsigned*>(p);
+  const unsigned lo = static_cast<unsigned>(x);
+  const unsigned carry = atomicAdd(w, lo) > ~lo ? 1u : 0u;
+  const unsigned hi = static_cast<unsigned>(static_cast<unsigned long long>(x) >> 32) + carry;
+  if (hi) atomicAdd(w + 1, hi);
 }
 
 // A sum in the weights' own units (exact: below 2^53 units).

@@ -110,3 +110,73 @@ def test_fixed_point_clusterings(ctx, kind, modularity):
     for move, res in ((P.NBHR_CLUSTER_MOVE, 0.02), (P.NBHR_MOVE, 0.2)):
         cfg = P.make_config(resolution=1.0 if modularity else res * scale, refine=True, move_method=move)
         _same(ctx, g, cfg, modularity)
+
+
+def _ring_of_cliques(cliques, size, extra=0):
+    """cliques complete graphs of `size` vertices joined in a ring, and
+    `extra` isolated vertices at the end."""
+    s, d = [], []
+    for c in range(cliques):
+        i, j = np.triu_indices(size, 1)
+        s.append(c * size + i), d.append(c * size + j)
+    if cliques > 1:
+        s.append(np.arange(cliques) * size), d.append((np.arange(1, cliques + 1) % cliques) * size + 1)
+    return P.CsrGraph.from_edges(cliques * size + extra, np.concatenate(s), np.concatenate(d))
+
+
+# Sizes at the edges of the one-kernel round loop: one CTA and several, one
+# vertex, a last slice of ids that is not full, rows at the limits of the
+# lane groups, warps, teams and CTA tables, and rows above 4096.
+LOOP_GRAPHS = {
+    "two": lambda: P.CsrGraph.from_edges(2, [0], [1]),
+    "edgeless": lambda: P.CsrGraph.from_edges(37, [], []),
+    "cliques5": lambda: _ring_of_cliques(7, 5),
+    "cliques33": lambda: _ring_of_cliques(40, 33, extra=5),
+    "cliques130": lambda: _ring_of_cliques(9, 130, extra=70001),
+    "cliques258": lambda: _ring_of_cliques(6, 258),
+    "clique1002": lambda: _ring_of_cliques(3, 1002),
+    "hubby": lambda: _hubby(7001, 9),
+    "star9000": lambda: P.CsrGraph.from_edges(9001, np.zeros(9000, np.int64), np.arange(1, 9001)),
+    "rmat15": lambda: G.rmat(15, 12, seed=8),
+}
+
+
+@pytest.mark.parametrize("name", list(LOOP_GRAPHS))
+@pytest.mark.parametrize("move", [P.NBHR_CLUSTER_MOVE, P.NBHR_MOVE, P.ALL_MOVE])
+def test_one_kernel_rounds(ctx, name, move):
+    """A level's rounds in one kernel: labels and every counter equal the
+    oracle's, and the host-driven rounds'."""
+    g = LOOP_GRAPHS[name]()
+    for res, inner, modularity in ((0.02, 0, False), (0.7, 1, False), (1.0, 3, True)):
+        if modularity and g.m == 0:
+            continue
+        cfg = P.make_config(resolution=res, refine=True, move_method=move, louvain_num_inner_iterations=inner)
+        st = _same(ctx, g, cfg, modularity)
+        ctx.set_detailed_timing(True)
+        try:
+            host = _same(ctx, g, cfg, modularity)
+        finally:
+            ctx.set_detailed_timing(False)
+        for key in ("vertex_visits", "moves", "family_entries", "family_vertices", "objective"):
+            assert st[key] == host[key], key
+
+
+def test_one_kernel_rounds_given_labels(ctx):
+    """Rounds started from the caller's labels (isolated vertices included),
+    with node weights and with 64-bit sums."""
+    g, _ = G.sbm(3000, 20, 0.05, 0.002, 3)
+    g = P.CsrGraph.from_edges(3100, np.repeat(np.arange(3000), np.diff(g.offsets).astype(np.int64)),
+                              g.neighbors.astype(np.int64), symmetrize=False)
+    rng = np.random.default_rng(2)
+    init = rng.integers(0, 150, g.n).astype(np.uint32)
+    for kind in (None, "uniform"):
+        gw = g if kind is None else _weighted(g, WEIGHTS[kind][0])
+        dg, og = ctx.upload(gw), O.OracleGraph(gw)
+        for move in (P.NBHR_CLUSTER_MOVE, P.ALL_MOVE):
+            cfg = P.make_config(resolution=0.05, refine=True, move_method=move)
+            k = rng.integers(1, 4, g.n).astype(np.float64)
+            lab, st = P.correlation_cluster(dg, cfg, k, init)
+            want, so = O.correlation_cluster(og, cfg, k, init)
+            np.testing.assert_array_equal(lab, want)
+            assert (st["rounds"], st["edge_visits"]) == (so["rounds"], so["edge_visits"])
+        dg.free()
