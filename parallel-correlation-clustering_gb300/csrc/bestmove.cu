@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kWarpKernelWarps * 32) BestMoveWarpKernel(BMAr
 // degree bin each.
 // ---------------------------------------------------------------------------
 template <int G, typename V>
-__global__ void __launch_bounds__(256) CertGroupKernel(BMArgs a, const uint32_t* __restrict__ list,
+__global__ void __launch_bounds__(256, 4) CertGroupKernel(BMArgs a, const uint32_t* __restrict__ list,
                                                       const uint32_t* __restrict__ bin_counts,
                                                       const uint32_t* __restrict__ bin_starts, int bin) {
   __shared__ V stage[8][32];
@@ -301,18 +301,31 @@ __global__ void __launch_bounds__(256) CertGroupKernel(BMArgs a, const uint32_t*
   const unsigned warp = threadIdx.x >> 5;
   constexpr unsigned kVpw = 32 / G;
   const unsigned g = LaneId() / G;
-  unsigned long long fam_e = 0, fam_v = 0;
+  uint32_t fam_e = 0, fam_v = 0;
   const bool replay = a.out_target != nullptr;
   const RoundView rv = RoundOf(a);
+  Pending<V> pend;
+  auto exact = [&](uint32_t v, int cres, uint32_t cmove) {
+    return GroupExact<V, ConstLoads>(a, rv, v, cres, cmove);
+  };
   const uint64_t stride = uint64_t(gridDim.x) * 8 * kVpw;
-  // Vertex ids are loaded one iteration ahead (latency-bound kernel).
+  // The next step's rows are loaded during this one, their ids one step
+  // before that (latency-bound kernel).
   uint64_t base = (uint64_t(blockIdx.x) * 8 + warp) * kVpw;
-  uint32_t vid = base + g < count ? list[start + base + g] : 0u;
-  for (; base < count; base += stride) {
-    const uint32_t nvid = base + stride + g < count ? list[start + base + stride + g] : 0u;
-    const bool append = GroupStep<G, V, ConstLoads>(a, rv, base + g < count, vid, stage[warp], replay, fam_e, fam_v);
-    mb.Add(&a.ctr->movers, a.movers, append, vid);
-    vid = nvid;
+  auto id_at = [&](uint64_t i) { return i < count ? list[start + i] : 0u; };
+  GroupRow row, next;
+  GroupHead<ConstLoads>(a, rv, base + g < count, id_at(base + g), row);
+  GroupEntry<G>(a, row);
+  uint32_t vid = id_at(base + stride + g);
+  while (true) {
+    const bool more = base < count;
+    if (!more || pend.n + kVpw > 32) DecidePending<V, ConstLoads>(a, rv, pend, replay, mb, &a.ctr->movers, exact);
+    if (!more) break;
+    base += stride;
+    GroupHead<ConstLoads>(a, rv, base + g < count, vid, next);
+    vid = id_at(base + stride + g);
+    GroupScan<G, V, ConstLoads>(a, row, stage[warp], pend, fam_e, fam_v, [&] { GroupEntry<G>(a, next); });
+    row = next;
   }
   mb.Flush(&a.ctr->movers, a.movers);
   FlushFamily(a, kFamGroup, fam_e, fam_v);
@@ -330,7 +343,7 @@ constexpr size_t CertWarpSmem() {
 }
 
 template <int HC, typename V, bool kConv = sizeof(V) == 8>
-__global__ void __launch_bounds__(kWarpKernelWarps * 32) CertWarpKernel(BMArgs a, const uint32_t* __restrict__ list,
+__global__ void __launch_bounds__(kWarpKernelWarps * 32, 9) CertWarpKernel(BMArgs a, const uint32_t* __restrict__ list,
                                                                        const uint32_t* __restrict__ bin_counts,
                                                                        const uint32_t* __restrict__ bin_starts,
                                                                        int bin) {

@@ -1,8 +1,25 @@
-// certmoves.cuh -- the certified best move of one vertex (INT mode,
-// synchronous rounds), by a lane group, a warp or a team of warps: the bodies
-// shared by the degree-binned kernels (bestmove.cu) and the kernel that runs
-// a whole level's rounds (roundloop.cu).
+// certmoves.cuh -- the certified best move of a vertex (INT mode, synchronous
+// rounds), by a lane group, a warp or a team of warps: the bodies shared by
+// the degree-binned kernels (bestmove.cu) and the kernel that runs a whole
+// level's rounds (roundloop.cu).
+//
+// A lane-group vertex (degree <= 32) is handled in two parts.  The scan gathers
+// its entries, sums them per neighbour cluster and filters the candidates in
+// FP32; the next step's rows are loaded meanwhile.  What is left of it, the
+// together-sum and the leading class's sum and lowest id, waits in the lane of
+// a Pending record.  The decision (certify.cuh: change, bounds, singleton
+// rule, move) is then taken for up to 32 vertices at once, one per lane: taken
+// vertex by vertex by the whole warp, that scalar part was about half of the
+// 490 warp instructions that a vertex of degree 17-32 cost.  Lane-group kernels
+// of a clustering: RMAT-22 21.8 -> 16.2 ms, 128 block models 26.8 -> 18.9,
+// RMAT-20 correlation 19.0 -> 16.3.
+// Vertices that the bounds do not decide although their leading class is known
+// (5-10% of a correlation clustering's: moves of value 0) take their two FP64
+// values in their lane; those whose contenders are of several (S, K) classes
+// (below 1%) are scanned again and decided from every candidate's exact value.
 #pragma once
+
+#include <cmath>
 
 #include "certify.cuh"
 #include "moves.cuh"
@@ -14,50 +31,336 @@ constexpr int kCertUnroll = 4;  // chunks of 32 entries loaded together
 constexpr int kCertRegRounds = 1;  // candidates per lane held in registers
 constexpr int kCtaWarps = 4;  // warps of a team on a vertex of degree 257-1000
 
-// ---------------------------------------------------------------------------
-// INT-mode synchronous rounds: certified decisions (certify.cuh).  The FP32
-// pre-filter selects the survivors; when they form one (S, K) class and the
-// FP32 bounds decide the move, no FP64 instruction runs for the vertex.
-// Otherwise -- and always in replay mode, where the exact values are outputs
-// -- the exact FP64 values decide; in replay mode a certified decision that
-// differs from the FP64 one raises kErrCertMismatch (a self-check).
-// ---------------------------------------------------------------------------
-// Exact FP64 fallbacks of the certified kernels.  They are separate
-// non-inlined functions so that the compiler cannot hoist their FP64
-// arithmetic onto the certified path (an FP64 warp instruction costs ~19
-// SM cycles on this GPU).  Both return whether the vertex must be appended
-// to the movers list; in replay mode they also run the self-check.
-template <int G, typename V>
-__device__ __noinline__ bool GroupExact(const BMArgs& a, const VertexCtx& x, bool fp64, bool contender, unsigned gl,
-                                        V T, V S, double KD, uint32_t cu, bool replay, int cres,
-                                        uint32_t cmove, uint32_t stamp) {
-  double change = 0.0, val = -CUDART_INF;
-  uint32_t id = kNone;
-  if (fp64) {
-    change = ChangeOf(a, x, UnitsToDouble<V>(a, T));
-    if (contender) {
-      val = ValOf(a, x, change, UnitsToDouble<V>(a, S), KD);
-      id = cu;
-    }
-  }
+template <typename V>
+__device__ __forceinline__ V WarpAddV(V x) {
+  if constexpr (sizeof(V) == 4) {
+    return __reduce_add_sync(kFull, x);
+  } else {
 #pragma unroll
-  for (int o = G / 2; o >= 1; o >>= 1) {
-    const double ov = __shfl_xor_sync(kFull, val, o);
-    const uint32_t oid = __shfl_xor_sync(kFull, id, o);
-    if (Better(ov, oid, val, id)) {
-      val = ov;
-      id = oid;
+    for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
+    return x;
+  }
+}
+
+template <typename V>
+__host__ __device__ constexpr V LowestV() {
+  return sizeof(V) == 4 ? V(INT_MIN) : V(LLONG_MIN);
+}
+template <typename V>
+__device__ __forceinline__ V WarpMaxV(V x) {
+  if constexpr (sizeof(V) == 4) {
+    return __reduce_max_sync(kFull, x);
+  } else {
+    const int hi = __reduce_max_sync(kFull, int(x >> 32));
+    const unsigned lo = __reduce_max_sync(kFull, int(x >> 32) == hi ? unsigned(x) : 0u);
+    return static_cast<V>((static_cast<unsigned long long>(static_cast<unsigned>(hi)) << 32) | lo);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The filter.  A candidate's value is ordered by Y = (S - M) - R, R = res * kv
+// * K, with M the largest sum: an exact integer difference, so that candidates
+// of equal S are told apart by R alone (modularity's R is 1e-7 of S).  It is
+// known in FP32 within
+//   e = 2^-18 (|R| + |Y|) + base,  base = 2^-48 (|change| + |M|) and more:
+// FilterBound (moves.cuh) with |S| <= |Y| + |R| + |M|, whose first two terms
+// disappear in the margin of the first one.  Kf is FilterF32(K), so it is 0, in
+// [2^-100, 2^100] or NaN; R outside that range (or NaN) makes the candidate
+// a contender in any case.
+// ---------------------------------------------------------------------------
+struct VertexFilter {
+  float r32, k32, base;
+  bool ok;       // base is finite
+  bool int_nw;
+};
+
+template <typename V>
+__device__ __forceinline__ VertexFilter FilterFor(const BMArgs& a, uint32_t v, uint32_t c, V T, V M) {
+  VertexFilter f;
+  f.r32 = Res32Of(a, v);
+  f.k32 = a.kf[v];
+  const float kc = a.Kf[c];
+  const float m = __fmul_rn(fabsf(__fmul_rn(f.r32, f.k32)), __fadd_rn(fabsf(kc), fabsf(f.k32)));
+  f.base = __fmul_rn(3.6e-15f /* 1.01 * 2^-48 */, __fadd_rn(m, __fadd_rn(fabsf(I2F(T)), fabsf(I2F(M)))));
+  f.ok = f.base <= 3.0e38f;  // false for NaN
+  f.int_nw = a.int_nw != 0;
+  return f;
+}
+
+// Upper and lower end of a candidate's Y (+inf, -inf when unknown).
+template <typename V>
+__device__ __forceinline__ void FilterEnds(const VertexFilter& f, V S, V M, float Kf, float* hi, float* lo) {
+  const float R = __fmul_rn(f.r32, __fmul_rn(f.k32, Kf));
+  const float aR = fabsf(R);
+  const float Y = __fsub_rn(I2F(static_cast<V>(S - M)), R);
+  const float e = __fadd_rn(__fmul_rn(3.814697265625e-06f /* 2^-18 */, __fadd_rn(aR, fabsf(Y))), f.base);
+  const bool sane = f.ok && aR <= 1.2676506002282294e30f /* 2^100 */ &&
+                    (aR >= 7.888609052210118e-31f /* 2^-100 */ || aR == 0.0f);
+  *hi = sane ? __fadd_rn(Y, e) : CUDART_INF_F;
+  *lo = sane ? __fsub_rn(Y, e) : -CUDART_INF_F;
+}
+
+// Whether two clusters with equal FP32 weights have equal weights: integers
+// below 2^24 are exact in FP32, others are compared in FP64.
+template <class L>
+__device__ __forceinline__ bool SameK(const BMArgs& a, const VertexFilter& f, float Kf, uint32_t i, uint32_t j) {
+  return (f.int_nw && fabsf(Kf) < kTwo24) || L::K(a.K + i) == L::K(a.K + j);
+}
+
+// ---------------------------------------------------------------------------
+// Scanned vertices waiting for their decision, one per lane.
+// ---------------------------------------------------------------------------
+template <typename V>
+struct Pending {
+  uint32_t v = kNone;   // kNone: no vertex in this lane
+  uint32_t id = kNone;  // leading class: lowest id (kNone: no candidate) ...
+  V T = 0, S = 0;       // together-sum; the leading class's sum
+  bool single = false;  // every contender is of the leading class
+  uint32_t n = 0;       // lanes in use (warp-uniform)
+};
+
+// The decision from the exact values of the leading class (S, id) and of the
+// new cluster, each lane for itself.  (Not inlined, as every exact function.)
+template <typename V, class L>
+__device__ __noinline__ bool DecideClass(const BMArgs& a, uint32_t v, uint32_t id, V T, V S, uint32_t stamp) {
+  const VertexCtx x = LoadVertexAs<L>(a, v);
+  const double change = ChangeOf(a, x, UnitsToDouble<V>(a, T));
+  double val = -CUDART_INF;
+  if (id != kNone) val = ValOf(a, x, change, UnitsToDouble<V>(a, S), L::K(a.K + id));
+  return Decide<false>(a, x, val, id, change, stamp);
+}
+
+// The decision of the calling lane's vertex v (kNone: none) from its scan; the
+// certified ones are applied.  Not inlined: it runs once per 32 vertices, and
+// its bounds would otherwise hold registers in the scan loops.
+struct LaneDecision {
+  uint32_t cmove;   // certified move (kNone: none)
+  int cres;
+  bool append;      // to be appended to the movers list
+  bool redo;        // several classes, or replayed: decide from exact values
+};
+template <typename V, class L>
+__device__ __noinline__ LaneDecision DecideLane(const BMArgs& a, uint32_t stamp, uint32_t v, uint32_t id, V T, V S,
+                                                bool single, bool replay) {
+  LaneDecision d{kNone, kUncertain, false, false};
+  if (v == kNone) return d;
+  VertexCtx x{};
+  x.v = v;
+  x.c = L::C(a.C + v);
+  const float r32 = Res32Of(a, v), k32 = a.kf[v];
+  if (single) {
+    const ChangeApproxT<V> ca = ApproxChange<V>(r32, a.int_nw != 0, k32, a.Kf[x.c], T);
+    const float KfA = id != kNone ? a.Kf[id] : 0.f;
+    uint32_t target = kNone;
+    d.cres = CertifyDecision<V>(ca, r32, k32, id != kNone, S, KfA, id, a.n, &target);
+    if (d.cres != kUncertain) d.cmove = CertifiedMove(a, x, target, d.cres == kCertMove);
+  }
+  d.redo = replay || !single;
+  if (d.redo) return d;
+  d.append = d.cres == kUncertain ? DecideClass<V, L>(a, v, id, T, S, stamp) : ApplyCertified(a, x, d.cmove, stamp);
+  return d;
+}
+
+// Decides the pending vertices and empties the record (every lane of the warp
+// calls).  exact(v, cres, cmove): the whole warp decides v from exact values
+// and returns (lane 0) whether it must be appended to the movers list.
+// Replay decides every vertex exactly and checks the certified decision.
+template <typename V, class L, class F>
+__device__ __forceinline__ void DecidePending(const BMArgs& a, const RoundView& rv, Pending<V>& p, bool replay,
+                                              WarpMoverBuffer& mb, uint32_t* movers, F exact) {
+  if (p.n == 0) return;
+  const uint32_t pv = LaneId() < p.n ? p.v : kNone;
+  const LaneDecision d = DecideLane<V, L>(a, rv.stamp, pv, p.id, p.T, p.S, p.single, replay);
+  mb.Add(movers, a.movers, d.append, pv);
+  for (unsigned m = __ballot_sync(kFull, d.redo); m; m &= m - 1) {
+    const int j = __ffs(m) - 1;
+    const uint32_t v = __shfl_sync(kFull, pv, j);
+    const int cr = __shfl_sync(kFull, d.cres, j);
+    const uint32_t cm = __shfl_sync(kFull, d.cmove, j);
+    const bool app = exact(v, cr, cm);
+    mb.Add(movers, a.movers, app, v);
+  }
+  p.n = 0;
+}
+
+// The warp's best (value, id) and its decision; in replay also the check of
+// the certified decision.  Returns (lane 0) whether the vertex must be
+// appended to the movers list.
+__device__ __forceinline__ bool DecideExact(const BMArgs& a, const RoundView& rv, const VertexCtx& x, double best,
+                                            uint32_t bid, double change, int cres, uint32_t cmove) {
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    const double ov = __shfl_xor_sync(kFull, best, o);
+    const uint32_t oid = __shfl_xor_sync(kFull, bid, o);
+    if (Better(ov, oid, best, bid)) {
+      best = ov;
+      bid = oid;
     }
   }
   bool append = false;
-  if (fp64 && gl == 0) {
-    append = Decide<false>(a, x, val, id, change, stamp);
-    if (replay && cres != kUncertain && a.out_moves && a.out_moves[x.v] != cmove)
-      atomicExch(&a.ctr->error, kErrCertMismatch);
+  if (LaneId() == 0) {
+    append = Decide<false>(a, x, best, bid, change, rv.stamp);
+    if (cres != kUncertain && a.out_moves && a.out_moves[x.v] != cmove) atomicExch(&a.ctr->error, kErrCertMismatch);
   }
   return append;
 }
 
+// ---------------------------------------------------------------------------
+// Lane groups of G lanes, one vertex (degree <= G) per group.
+// ---------------------------------------------------------------------------
+// A vertex of degree <= 32 from exact FP64 values, by the warp.  A separate
+// non-inlined function (as the other exact ones), so that the compiler cannot
+// hoist its FP64 arithmetic onto the certified path: an FP64 warp instruction
+// costs ~19 SM cycles on this GPU.
+template <typename V, class L>
+__device__ __noinline__ bool GroupExact(const BMArgs& a, const RoundView& rv, uint32_t v, int cres, uint32_t cmove) {
+  const unsigned lane = LaneId();
+  const VertexCtx x = LoadVertexAs<L>(a, v);
+  const bool has = lane < x.d;
+  const uint32_t u = has ? a.nbr[x.b + lane] : v;
+  const bool cand = u != v;
+  const V xi = cand ? EntryUnits<V, true>(a, a.w ? a.w[x.b + lane] : 1.0f) : V(0);
+  const uint32_t cu = cand ? L::C(a.C + u) : kNone;
+  const unsigned peers = __match_any_sync(kFull, cand ? cu : LaneSentinel(lane));
+  V S = 0;
+  for (unsigned mm = peers; mm; mm &= mm - 1) S += __shfl_sync(peers, xi, __ffs(mm) - 1);
+  const bool leader = cand && int(lane) == __ffs(peers) - 1;
+  const V T = WarpAddV<V>(cand && cu == x.c ? xi : V(0));
+  const double change = ChangeOf(a, x, UnitsToDouble<V>(a, T));
+  double val = -CUDART_INF;
+  if (leader) val = ValOf(a, x, change, UnitsToDouble<V>(a, S), L::K(a.K + cu));
+  return DecideExact(a, rv, x, val, leader ? cu : kNone, change, cres, cmove);
+}
+
+// A lane's part of a group vertex, loaded ahead of its turn: first the row's
+// bounds, cluster and frontier mark, then the lane's entry.
+struct GroupRow {
+  uint32_t v = 0, d = 0, c = 0, u = 0;
+  uint64_t b = 0;
+  float w = 0.f;
+  bool in = false;
+};
+template <class L>
+__device__ __forceinline__ void GroupHead(const BMArgs& a, const RoundView& rv, bool in, uint32_t v, GroupRow& r) {
+  r.v = v;
+  r.d = 0;
+  r.in = in && InFront(a, rv, v);
+  if (in) {
+    r.b = a.off[v];
+    r.d = uint32_t(a.off[v + 1] - r.b);
+    r.c = L::C(a.C + v);
+  }
+}
+template <int G>
+__device__ __forceinline__ void GroupEntry(const BMArgs& a, GroupRow& r) {
+  const unsigned gl = LaneId() % G;
+  r.u = r.v;
+  if (r.in && gl < r.d) {
+    r.u = a.nbr[r.b + gl];
+    r.w = a.w ? a.w[r.b + gl] : 1.0f;
+  }
+}
+
+// Scans the groups' vertices r into p, which must have room for the warp's
+// 32 / G vertices.  stage: 32 values of the calling warp.  ahead() is called
+// while the scan waits for no load of its own: it loads the next row.  V: int
+// when every sum of a row fits in 32 bits, else long long.
+template <int G, typename V, class L, class F>
+__device__ __forceinline__ void GroupScan(const BMArgs& a, const GroupRow& r, V* stage, Pending<V>& p,
+                                          uint32_t& fam_e, uint32_t& fam_v, F ahead) {
+  constexpr unsigned kVpw = 32 / G;
+  const unsigned lane = LaneId();
+  const unsigned g = lane / G, gl = lane % G;
+  const unsigned gmask = G == 32 ? kFull : (((1u << G) - 1u) << (g * G));
+  const uint32_t vid = r.v, c = r.c;
+  const bool in = r.in;
+  if (__ballot_sync(kFull, in) == 0) {  // no frontier vertex in this warp
+    ahead();
+    return;
+  }
+  if (in && gl == 0) {
+    fam_e += r.d;
+    fam_v += 1;
+  }
+  const bool cand = r.u != vid;
+  const uint32_t cu = cand ? L::C(a.C + r.u) : kNone;
+  ahead();
+  float Kf = cand ? a.Kf[cu] : 0.f;  // (every entry's: the load overlaps the grouping)
+  const unsigned peers = __match_any_sync(kFull, cand ? cu : LaneSentinel(lane)) & gmask;
+  const bool leader = cand && int(lane) == __ffs(peers) - 1;
+  const V xi = cand ? EntryUnits<V, true>(a, r.w) : V(0);
+  const V S = GroupSumInt<V>(peers, xi, a.w == nullptr, leader, stage);
+  const unsigned tmask = __ballot_sync(kFull, leader && cu == c) & gmask;
+  const V Tsh = __shfl_sync(kFull, S, tmask ? __ffs(tmask) - 1 : int(lane));
+  const V T = tmask ? Tsh : V(0);
+  V M = leader ? S : LowestV<V>();
+  if constexpr (G == 32) {
+    M = WarpMaxV<V>(M);
+  } else {
+#pragma unroll
+    for (int o = G / 2; o >= 1; o >>= 1) M = max(M, __shfl_xor_sync(kFull, M, o));
+  }
+  float hi = -CUDART_INF_F, U = -CUDART_INF_F;
+  VertexFilter f{};
+  if (leader) {
+    f = FilterFor<V>(a, vid, c, T, M);
+    FilterEnds<V>(f, S, M, Kf, &hi, &U);
+  }
+  if constexpr (G == 32) {
+    U = WarpMaxFinite(U);
+  } else {
+#pragma unroll
+    for (int o = G / 2; o >= 1; o >>= 1) U = fmaxf(U, __shfl_xor_sync(kFull, U, o));
+  }
+  const bool cont = leader && hi >= U;
+  const unsigned m = __ballot_sync(kFull, cont) & gmask;
+  // The group's representative contender; with several, all must be of its
+  // (S, K) class and the lowest id leads.
+  const int j = m ? __ffs(m) - 1 : int(lane);
+  V lS = __shfl_sync(kFull, S, j);
+  uint32_t id = __shfl_sync(kFull, cu, j);
+  if (!m) id = kNone;
+  bool single = true;
+  if (__ballot_sync(kFull, (m & (m - 1)) != 0)) {
+    const float lK = __shfl_sync(kFull, Kf, j);
+    const bool diff = cont && (S != lS || !(Kf == lK) || !SameK<L>(a, f, Kf, cu, id));
+    single = (__ballot_sync(kFull, diff) & gmask) == 0;
+    uint32_t low = cont ? cu : kNone;
+    if constexpr (G == 32) {
+      low = __reduce_min_sync(kFull, low);
+    } else {
+#pragma unroll
+      for (int o = G / 2; o >= 1; o >>= 1) low = min(low, __shfl_xor_sync(kFull, low, o));
+    }
+    id = low;
+  }
+  // Lane p.n + i takes group i's result.
+  const unsigned slot = lane - p.n;
+  const int src = int((slot % kVpw) * G);
+  const uint32_t sv = __shfl_sync(kFull, in ? vid : kNone, src);
+  const uint32_t sid = __shfl_sync(kFull, id, src);
+  const V sT = __shfl_sync(kFull, T, src);
+  const V sS = __shfl_sync(kFull, lS, src);
+  const unsigned sing = __ballot_sync(kFull, single);
+  if (slot < kVpw) {
+    p.v = sv;
+    p.id = sid;
+    p.T = sT;
+    p.S = sS;
+    p.single = (sing >> src) & 1u;
+  }
+  p.n += kVpw;
+}
+
+// ---------------------------------------------------------------------------
+// One warp or one team of warps per vertex, decided at once.  (Deferring these
+// decisions as the lane groups do, with one pass over the candidates, measured
+// slower: RMAT-22's warps 33 -> 53 ms.  Their time is the table's and the
+// gathers' latency, and the pending record and the lanes' running classes cost
+// registers, so warps in flight.)
+// ---------------------------------------------------------------------------
+// Exact FP64 fallback.  Returns (lane 0) whether the vertex must be appended
+// to the movers list; in replay mode it also runs the self-check.
 template <int HC, typename V>
 __device__ __noinline__ bool WarpExact(const BMArgs& a, const VertexCtx& x, V T, const uint32_t* keys,
                                        const V* vals, const uint16_t* used, uint32_t nused, bool replay, int cres,
@@ -90,114 +393,6 @@ __device__ __noinline__ bool WarpExact(const BMArgs& a, const VertexCtx& x, V T,
     append = Decide<false>(a, x, best, bid, change, stamp);
     if (replay && cres != kUncertain && a.out_moves && a.out_moves[x.v] != cmove)
       atomicExch(&a.ctr->error, kErrCertMismatch);
-  }
-  return append;
-}
-
-template <typename V>
-__device__ __forceinline__ V WarpMaxV(V x) {
-  if constexpr (sizeof(V) == 4) return __reduce_max_sync(kFull, x);
-  else return WarpMaxLL(x);
-}
-
-// Lane groups of G lanes, one vertex (degree <= G) per group: vid is the
-// group's vertex when `in`.  Returns whether this lane's vertex must be
-// appended to the movers list (the group's first lane).  stage: 32 values of
-// the calling warp.  V: int when every sum of a row fits in 32 bits, else long
-// long.
-template <int G, typename V, class L>
-__device__ __forceinline__ bool GroupStep(const BMArgs& a, const RoundView& rv, bool in, uint32_t vid, V* stage,
-                                          bool replay, unsigned long long& fam_e, unsigned long long& fam_v) {
-  const unsigned lane = LaneId();
-  const unsigned g = lane / G, gl = lane % G;
-  const unsigned gmask = G == 32 ? kFull : (((1u << G) - 1u) << (g * G));
-  const bool unit = a.w == nullptr;
-  bool vvalid = in;
-  VertexCtx x{};
-  if (vvalid) {
-    vvalid = InFront(a, rv, vid);
-    if (vvalid) x = LoadVertexAs<L>(a, vid);
-  }
-  if (__ballot_sync(kFull, vvalid) == 0) return false;  // no frontier vertex in this warp
-  if (vvalid && gl == 0) {
-    fam_e += x.d;
-    fam_v += 1;
-  }
-  const bool has = vvalid && gl < x.d;
-  uint32_t u = x.v;
-  float wt = 0.f;
-  if (has) {
-    u = a.nbr[x.b + gl];
-    wt = a.w ? a.w[x.b + gl] : 1.0f;
-  }
-  const bool cand = has && u != x.v;
-  const uint32_t cu = cand ? L::C(a.C + u) : kNone;
-  const unsigned peers = __match_any_sync(kFull, cand ? cu : LaneSentinel(lane)) & gmask;
-  const bool leader = cand && int(lane) == __ffs(peers) - 1;
-  const V xi = cand ? EntryUnits<V, true>(a, wt) : V(0);
-  const V S = GroupSumInt<V>(peers, xi, unit, leader, stage);
-  const unsigned tmask = __ballot_sync(kFull, leader && cu == x.c) & gmask;
-  const V Tsh = __shfl_sync(kFull, S, tmask ? __ffs(tmask) - 1 : int(lane));
-  const V T = tmask ? Tsh : V(0);
-  V smax = leader ? S : (sizeof(V) == 4 ? V(INT_MIN) : V(LLONG_MIN));
-  if constexpr (G == 32) {
-    smax = WarpMaxV<V>(smax);
-  } else {
-#pragma unroll
-    for (int o = G / 2; o >= 1; o >>= 1) smax = max(smax, __shfl_xor_sync(kFull, smax, o));
-  }
-  const float k32 = vvalid ? a.kf[x.v] : 0.f;
-  const float Kc32 = vvalid ? a.Kf[x.c] : 0.f;
-  const ChangeApproxT<V> ca = ApproxChange<V>(Res32Of(a, x.v), a.int_nw != 0, k32, Kc32, T);
-  const float cabs = ChangeAbsBound(ca);
-  // FP32 pre-filter over the group's leaders.
-  FilterVal f{0.f, 0.f, false};
-  float KfD = 0.f;
-  float lo = -CUDART_INF_F;
-  if (leader) {
-    KfD = a.Kf[cu];
-    f = FilterOf<V>(Res32Of(a, x.v), k32, KfD, S, smax, cabs);
-    if (f.sane) lo = __fsub_rn(f.Y, f.e);
-  }
-  float U = lo;
-  if constexpr (G == 32) {
-    U = WarpMaxFinite(U);
-  } else {
-#pragma unroll
-    for (int o = G / 2; o >= 1; o >>= 1) U = fmaxf(U, __shfl_xor_sync(kFull, U, o));
-  }
-  const bool contender = leader && (!f.sane || __fadd_rn(f.Y, f.e) >= U);
-  // The leading (S, K) class of the contenders and the trailing one.
-  LexKeyT<V> lead, tail;
-  double KD = 0.0;
-  if (contender) {
-    KD = L::K(a.K + cu);
-    const unsigned long long ko = KOrder(KD);
-    lead.Keep(S, ko, cu);
-    tail.Keep(-S, ~ko, cu);
-  }
-  bool single;
-  if constexpr (G == 32) {
-    single = LexWarpLead<V>(lead, tail);
-  } else {
-    LexGroupReduce<G>(lead);
-    LexGroupReduce<G>(tail);
-    single = lead.id == kNone || (-tail.S == lead.S && ~tail.K == lead.K);
-  }
-  int cres = kUncertain;
-  uint32_t ctarget = kNone;
-  if (vvalid && single) {
-    const float KfA = lead.id != kNone ? a.Kf[lead.id] : 0.f;
-    cres = CertifyDecision<V>(ca, Res32Of(a, x.v), k32, lead.id != kNone, lead.S, KfA, lead.id, a.n, &ctarget);
-  }
-  const uint32_t cmove = cres == kUncertain ? kNone : CertifiedMove(a, x, ctarget, cres == kCertMove);
-  const bool fp64 = vvalid && (replay || cres == kUncertain);
-  bool append = false;
-  if (vvalid && !fp64 && gl == 0) append = ApplyCertified(a, x, cmove, rv.stamp);
-  if (__ballot_sync(kFull, fp64)) {
-    const bool app = GroupExact<G, V>(a, x, fp64, contender, gl, T, S, KD, cu, replay, cres, cmove,
-                                       rv.stamp);
-    append = append || app;
   }
   return append;
 }
@@ -377,10 +572,11 @@ __device__ __forceinline__ bool WarpStep(const BMArgs& a, const RoundView& rv, c
   }
   const uint32_t cmove = cres == kUncertain ? kNone : CertifiedMove(a, x, ctarget, cres == kCertMove);
   bool append = false;
-  if (replay || cres == kUncertain) {
+  if (replay || !single) {
     append = WarpExact<HC, V>(a, x, T, keys, vals, used, nused, replay, cres, cmove, rv.stamp);
   } else if (lane == 0) {
-    append = ApplyCertified(a, x, cmove, rv.stamp);
+    append = cres == kUncertain ? DecideClass<V, L>(a, x.v, lead.id, T, lead.S, rv.stamp)
+                                : ApplyCertified(a, x, cmove, rv.stamp);
   }
   __syncwarp();
   // Clear the table through the key list (used[] may hold 0xFFFF marks).
@@ -560,10 +756,11 @@ __device__ __forceinline__ bool CtaStep(const BMArgs& a, const RoundView& rv, co
     if (TW > kCtaWarps && nused == 0) {
       // A hub whose entries are all self-loops: the reduce identity (0, 0.0).
       if (lane == 0) append = Decide<false>(a, x, 0.0, 0, ChangeOf(a, x, 0.0), rv.stamp);
-    } else if (replay || cres == kUncertain) {
+    } else if (replay || !single) {
       append = WarpExact<HC, V>(a, x, T, keys, vals, used, nused, replay, cres, cmove, rv.stamp);
     } else if (lane == 0) {
-      append = ApplyCertified(a, x, cmove, rv.stamp);
+      append = cres == kUncertain ? DecideClass<V, L>(a, x.v, top.id, T, top.S, rv.stamp)
+                                  : ApplyCertified(a, x, cmove, rv.stamp);
     }
   }
   TeamSync<BT>(bar);  // the table is read by WarpExact up to here

@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
   // Degree bins of the teams: 257-1000, with 64-bit sums (two table words
   // more per entry) 129-1000.
   constexpr int kTeamLow = sizeof(V) == 4 ? kBinW512 : kBinW256;
+  Pending<V> pend;
 
   for (uint32_t round = 0; round < l.num_inner; ++round) {
     LoopCounters* ctr = &l.st->ctr[round % 3];
@@ -318,41 +319,83 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
     {
       const uint32_t s0 = sh.bin_start[kBinG4], s1 = sh.bin_start[kBinG8], s2 = sh.bin_start[kBinG16],
                      s3 = sh.bin_start[kBinG32], s4 = sh.bin_start[kBinW128];
+      auto exact = [&](uint32_t v, int cres, uint32_t cmove) {
+        return GroupExact<V, LiveLoads>(a, rv, v, cres, cmove);
+      };
       const uint32_t n32 = s4 - s3, n16 = (s3 - s2 + 1) / 2, n8 = (s2 - s1 + 3) / 4, n4 = (s1 - s0 + 7) / 8;
       const uint32_t steps = n32 + n16 + n8 + n4;
       const uint32_t run = min(8u, max(1u, steps / (G * kLW * 8)));
       const uint32_t runs = (steps + run - 1) / run;
-      uint32_t r = blockIdx.x * kLW + warp;
-      while (r < runs) {
-        uint32_t next = 0;
-        if (lane == 0) next = G * kLW + atomicAdd(&ctr->queue[3], 1u);
-        const uint32_t end = min(steps, (r + 1) * run);
-        for (uint32_t i = r * run; i < end; ++i) {
-          bool append;
-          uint32_t v;
-          if (i < n32) {
-            v = l.list[s3 + i];
-            append = GroupStep<32, V, LiveLoads>(a, rv, true, v, wstage, false, fam_e, fam_v);
-          } else if (i < n32 + n16) {
-            const uint32_t p = s2 + (i - n32) * 2 + lane / 16;
-            const bool in = p < s3;
-            v = in ? l.list[p] : 0u;
-            append = GroupStep<16, V, LiveLoads>(a, rv, in, v, wstage, false, fam_e, fam_v);
-          } else if (i < n32 + n16 + n8) {
-            const uint32_t p = s1 + (i - n32 - n16) * 4 + lane / 8;
-            const bool in = p < s2;
-            v = in ? l.list[p] : 0u;
-            append = GroupStep<8, V, LiveLoads>(a, rv, in, v, wstage, false, fam_e, fam_v);
-          } else {
-            const uint32_t p = s0 + (i - n32 - n16 - n8) * 8 + lane / 4;
-            const bool in = p < s1;
-            v = in ? l.list[p] : 0u;
-            append = GroupStep<4, V, LiveLoads>(a, rv, in, v, wstage, false, fam_e, fam_v);
-          }
-          mb.Add(movers, a.movers, append, v);
+      uint32_t r = blockIdx.x * kLW + warp, got = 0, i = 0, end = 0;
+      // The next step (kNone: none), as for the warps.
+      auto take = [&]() -> uint32_t {
+        if (i == end) {
+          if (end) r = __shfl_sync(kFull, got, 0);
+          if (r >= runs) return kNone;
+          if (lane == 0) got = G * kLW + atomicAdd(&ctr->queue[3], 1u);
+          i = r * run;
+          end = min(steps, i + run);
         }
-        r = __shfl_sync(kFull, next, 0);
+        return i++;
+      };
+      // Lanes per vertex of a step, and the vertex of the calling lane.
+      auto width = [&](uint32_t s) { return s < n32 ? 32u : s < n32 + n16 ? 16u : s < n32 + n16 + n8 ? 8u : 4u; };
+      auto head = [&](uint32_t s, GroupRow& row) {
+        uint32_t p, e;
+        if (s < n32) {
+          p = s3 + s;
+          e = s4;
+        } else if (s < n32 + n16) {
+          p = s2 + (s - n32) * 2 + lane / 16;
+          e = s3;
+        } else if (s < n32 + n16 + n8) {
+          p = s1 + (s - n32 - n16) * 4 + lane / 8;
+          e = s2;
+        } else {
+          p = s0 + (s - n32 - n16 - n8) * 8 + lane / 4;
+          e = s1;
+        }
+        const bool in = s != kNone && p < e;
+        GroupHead<LiveLoads>(a, rv, in, in ? l.list[p] : 0u, row);
+      };
+      auto entry = [&](unsigned g, GroupRow& row) {
+        const unsigned gl = lane & (g - 1);
+        row.u = row.v;
+        if (row.in && gl < row.d) {
+          row.u = a.nbr[row.b + gl];
+          row.w = a.w ? a.w[row.b + gl] : 1.0f;
+        }
+      };
+      uint32_t gf_e = 0, gf_v = 0;
+      GroupRow row, ahead;
+      uint32_t step = take();
+      if (step != kNone) {
+        unsigned g = width(step);
+        head(step, row);
+        entry(g, row);
+        while (true) {
+          step = take();
+          const bool more = step != kNone;
+          const unsigned gn = width(step);
+          head(step, ahead);
+          auto load = [&] { entry(gn, ahead); };
+          if (pend.n + 32 / g > 32) DecidePending<V, LiveLoads>(a, rv, pend, false, mb, movers, exact);
+          if (g == 32)
+            GroupScan<32, V, LiveLoads>(a, row, wstage, pend, gf_e, gf_v, load);
+          else if (g == 16)
+            GroupScan<16, V, LiveLoads>(a, row, wstage, pend, gf_e, gf_v, load);
+          else if (g == 8)
+            GroupScan<8, V, LiveLoads>(a, row, wstage, pend, gf_e, gf_v, load);
+          else
+            GroupScan<4, V, LiveLoads>(a, row, wstage, pend, gf_e, gf_v, load);
+          if (!more) break;
+          row = ahead;
+          g = gn;
+        }
+        DecidePending<V, LiveLoads>(a, rv, pend, false, mb, movers, exact);
       }
+      fam_e += gf_e;
+      fam_v += gf_v;
     }
     mb.Flush(movers, a.movers);
 #pragma unroll
