@@ -133,7 +133,20 @@ struct Context {
     PCC_CUDA(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
     return Status::Ok();
   }
+  // Page-locked staging for the small structs that a call sends to the device
+  // or reads back (at fixed offsets, each read after a Sync before its next
+  // use): copies from or to pageable memory make the host wait at the copy.
+  static constexpr size_t kPinnedBytes = 4096;
+  static constexpr size_t kPinCompress = 0, kPinBins = 512, kPinStats = 768, kPinLoop = 1024;
+  unsigned char* pinned = nullptr;
+  template <class T>
+  Status Pinned(size_t at, T** p) {
+    if (!pinned) PCC_CUDA(cudaMallocHost(&pinned, kPinnedBytes));
+    *p = reinterpret_cast<T*>(pinned + at);
+    return Status::Ok();
+  }
   ~Context() {
+    if (pinned) cudaFreeHost(pinned);
     for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
     for (int i = 0; i < kSideStreams; ++i) {
       if (side[i]) cudaStreamDestroy(side[i]);

@@ -42,14 +42,33 @@ constexpr int kSegCtaThreads = 256;
 constexpr int kSegCtaItems = kSegCtaMax / kSegCtaThreads;
 constexpr int kSegCtaWarps = kSegCtaThreads / 32;
 
-struct MaxOfU32 {
-  const uint32_t* a;
-  __device__ uint32_t operator()(uint64_t i) const { return a[i]; }
+// Counters of one contraction, read back together where they are needed.
+struct CompressHead {  // (at most 256 bytes: Context::kPinCompress)
+  uint32_t max_c;               // largest cluster id
+  uint32_t R;                   // clusters in use
+  uint32_t counts[4];           // segments per class
+  unsigned long long big_e;     // entries of the class-3 segments
+  unsigned long long m2;        // entries of the new graph
+  WeightStats stats;            // of its weights
 };
 
-__global__ void MarkPresentKernel(uint32_t n, const uint32_t* __restrict__ C, uint32_t* __restrict__ pres) {
-  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
-    pres[C[i]] = 1u;
+// pres[c] = 1 for every cluster id in use (< n), and the largest one.
+__global__ void __launch_bounds__(256) MarkPresentKernel(uint32_t n, const uint32_t* __restrict__ C,
+                                                         uint32_t* __restrict__ pres, uint32_t* __restrict__ max_c) {
+  __shared__ uint32_t sh[8];
+  uint32_t mx = 0;
+  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
+    const uint32_t c = C[i];
+    pres[c] = 1u;
+    mx = max(mx, c);
+  }
+  mx = __reduce_max_sync(kFull, mx);
+  if (LaneId() == 0) sh[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) mx = max(mx, sh[w]);
+    if (mx) atomicMax(max_c, mx);
+  }
 }
 
 struct PresInput {
@@ -84,21 +103,21 @@ struct SortedDegInput {
     return off[u + 1] - off[u];
   }
 };
+// Also segbase[r] = first slot of cluster rank r's segment (the first vertex of
+// the rank records it); segbase[R] = m.
 struct RowStartWriter {
+  const uint64_t* vkey;
   const uint32_t* vval;
   uint64_t* dstart;
-  __device__ void operator()(uint64_t p, uint64_t pre, uint64_t) const { dstart[vval[p]] = pre; }
-};
-
-// segbase[r] = first slot of cluster rank r's segment; segbase[R] = m.
-__global__ void SegBaseKernel(uint32_t n, const uint64_t* __restrict__ vkey, const uint32_t* __restrict__ vval,
-                              const uint64_t* __restrict__ dstart, uint64_t* __restrict__ segbase, uint32_t R,
-                              uint64_t m) {
-  for (uint64_t p = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n; p += uint64_t(gridDim.x) * blockDim.x) {
-    if (p == 0 || vkey[p] != vkey[p - 1]) segbase[vkey[p]] = dstart[vval[p]];
+  uint64_t* segbase;
+  uint32_t R;
+  uint64_t m;
+  __device__ void operator()(uint64_t p, uint64_t pre, uint64_t) const {
+    dstart[vval[p]] = pre;
+    if (p == 0 || vkey[p] != vkey[p - 1]) segbase[vkey[p]] = pre;
     if (p == 0) segbase[R] = m;
   }
-}
+};
 
 // Moves every entry to its row's place in the cluster-ordered array.
 struct MoveEntries {
@@ -156,7 +175,7 @@ __global__ void __launch_bounds__(256) SegWarpKernel(const uint32_t* __restrict_
                                                      const uint64_t* __restrict__ segbase,
                                                      const uint32_t* __restrict__ ids, uint32_t drop,
                                                      uint32_t* __restrict__ akey, uint32_t* __restrict__ aval,
-                                                     uint32_t* __restrict__ ucount) {
+                                                     uint32_t* __restrict__ ucount, uint32_t* __restrict__ row_count) {
   __shared__ uint32_t sk[8][kSegWarpMax], sv[8][kSegWarpMax];
   __shared__ uint8_t sf[8][kSegWarpMax];
   const unsigned lane = LaneId(), warp = threadIdx.x >> 5;
@@ -209,7 +228,7 @@ __global__ void __launch_bounds__(256) SegWarpKernel(const uint32_t* __restrict_
       aval[b + orank[h]] = __float_as_uint(sum[h]);
     }
     const uint32_t u = __popc(__ballot_sync(kFull, first[0])) + __popc(__ballot_sync(kFull, first[1]));
-    if (lane == 0) ucount[r] = u;
+    if (lane == 0) ucount[r] = row_count[ids[r]] = u;
     __syncwarp();
   }
 }
@@ -228,7 +247,7 @@ __global__ void __launch_bounds__(kSegMidWarps * 32) SegMidKernel(const uint32_t
                                                                  const uint32_t* __restrict__ ids, uint32_t drop,
                                                                  int passes, uint32_t* __restrict__ akey,
                                                                  uint32_t* __restrict__ aval,
-                                                                 uint32_t* __restrict__ ucount) {
+                                                                 uint32_t* __restrict__ ucount, uint32_t* __restrict__ row_count) {
   extern __shared__ __align__(16) unsigned char mid_smem[];
   const unsigned lane = LaneId(), warp = threadIdx.x >> 5;
   uint32_t* k0 = reinterpret_cast<uint32_t*>(mid_smem + size_t(warp) * (size_t(kSegMidMax) * 16 + 256 * 4));
@@ -322,7 +341,7 @@ __global__ void __launch_bounds__(kSegMidWarps * 32) SegMidKernel(const uint32_t
       }
       pre += __popc(hb);
     }
-    if (lane == 0) ucount[r] = pre;
+    if (lane == 0) ucount[r] = row_count[ids[r]] = pre;
     __syncwarp();
   }
 }
@@ -339,7 +358,7 @@ __global__ void __launch_bounds__(kSegCtaThreads) SegCtaKernel(const uint32_t* _
                                                               const uint32_t* __restrict__ ids, uint32_t drop,
                                                               int passes, uint32_t* __restrict__ akey,
                                                               uint32_t* __restrict__ aval,
-                                                              uint32_t* __restrict__ ucount) {
+                                                              uint32_t* __restrict__ ucount, uint32_t* __restrict__ row_count) {
   extern __shared__ __align__(16) unsigned char seg_smem[];
   uint32_t* k0 = reinterpret_cast<uint32_t*>(seg_smem);
   uint32_t* v0 = k0 + kSegCtaMax;
@@ -445,7 +464,7 @@ __global__ void __launch_bounds__(kSegCtaThreads) SegCtaKernel(const uint32_t* _
       aval[b + pre] = __float_as_uint(sum);
       ++pre;
     }
-    if (tid == 0) ucount[r] = s_total;
+    if (tid == 0) ucount[r] = row_count[ids[r]] = s_total;
     __syncthreads();
   }
 }
@@ -517,7 +536,7 @@ __global__ void BigRunKernel(uint32_t S, uint64_t E, const uint32_t* __restrict_
                              uint32_t drop, const uint32_t* __restrict__ grun, const uint32_t* __restrict__ big_list,
                              const uint32_t* __restrict__ ids, uint32_t* __restrict__ bkey,
                              uint32_t* __restrict__ bval, uint32_t* __restrict__ ucount,
-                             uint32_t* __restrict__ long_run, uint32_t* __restrict__ long_count) {
+                             uint32_t* __restrict__ row_count, uint32_t* __restrict__ long_run, uint32_t* __restrict__ long_count) {
   const uint64_t low_mask = (uint64_t(1) << kbits) - 1;
   for (uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; s < S; s += uint64_t(gridDim.x) * blockDim.x) {
     const uint64_t a = seg_start[s];
@@ -542,7 +561,7 @@ __global__ void BigRunKernel(uint32_t S, uint64_t E, const uint32_t* __restrict_
       const uint64_t kn = keys[seg_start[s + 1]];
       last = (kn >> kbits) != g || static_cast<uint32_t>(kn & low_mask) >= drop;
     }
-    if (last) ucount[r] = local + 1;
+    if (last) ucount[r] = row_count[ids[r]] = local + 1;
   }
 }
 
@@ -629,12 +648,6 @@ __global__ void __launch_bounds__(kLongThreads) BigLongKernel(const uint32_t* __
     }
     __syncthreads();
   }
-}
-
-__global__ void RowCountKernel(uint32_t R, const uint32_t* __restrict__ ids, const uint32_t* __restrict__ ucount,
-                               uint32_t* __restrict__ row_count) {
-  for (uint64_t r = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < R; r += uint64_t(gridDim.x) * blockDim.x)
-    row_count[ids[r]] = ucount[r];
 }
 
 // Adds a block's per-thread weight statistics to *out (every thread of the
@@ -731,40 +744,81 @@ int BitsFor(uint64_t count) {
   return b;
 }
 
+// Temporary arrays of a contraction: pieces of one allocation for the small
+// levels (whose 25 allocations and frees cost as much as their kernels),
+// separate ones, freed as soon as they are spent, for large graphs and under
+// an HBM budget.
+class Scratch {
+ public:
+  Scratch(Context* ctx, uint64_t n, uint64_t m) : ctx_(ctx) {
+    if (!ctx->budget && n <= (1u << 20) && m <= (16u << 20)) bytes_ = 80 * n + 8 * m + (n / kSortTile + 1) * 1024 + 16384;
+  }
+  template <class T>
+  Status Take(T** p, uint64_t count) {
+    const uint64_t need = (std::max<uint64_t>(count, 1) * sizeof(T) + 255) & ~uint64_t(255);
+    if (bytes_ && !arena_.p) PCC_RETURN_IF_ERROR(arena_.Alloc(ctx_, bytes_));
+    if (at_ + need <= bytes_) {
+      *p = reinterpret_cast<T*>(arena_.p + at_);
+      at_ += need;
+      return Status::Ok();
+    }
+    own_.emplace_back();
+    PCC_RETURN_IF_ERROR(own_.back().Alloc(ctx_, need));
+    *p = reinterpret_cast<T*>(own_.back().p);
+    return Status::Ok();
+  }
+  // The array is not used by work enqueued later.
+  void Done(const void* p) {
+    for (auto& b : own_)
+      if (b.p == p) b.Release();
+  }
+
+ private:
+  Context* ctx_;
+  uint64_t bytes_ = 0, at_ = 0;
+  DBuf<unsigned char> arena_;
+  std::vector<DBuf<unsigned char>> own_;
+};
+
 }  // namespace
 
-// Contracts g by C (device uint32[n]); k = node weights (device, or null for
-// 1).  The new graph carries its node weights in node_w.
+// Contracts g by C (device uint32[n], ids < n); k = node weights (device, or
+// null for 1).  The new graph carries its node weights in node_w.
+//
+// Host waits: the number of clusters; the segment classes, when a segment may
+// be longer than a CTA holds (the shorter ones are sorted meanwhile); the new
+// graph's size and properties together (above 16M entries its size alone
+// before, so that its arrays are not allocated at the old size).  A level of
+// 4,686 entries takes 3 waits and 18 kernels, 0.40 -> 0.2 ms.
 Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k,
                      std::unique_ptr<DevGraph>* out) {
   const uint32_t n = g.n;
   cudaStream_t st = ctx->stream;
-  DBuf<uint32_t> tmp32;
-  PCC_RETURN_IF_ERROR(tmp32.Alloc(ctx, 8));
-  DBuf<uint32_t> part32;
-  // n2 = 1 + max C
-  uint32_t maxc = 0;
-  if (n > 0) {
-    PCC_RETURN_IF_ERROR(Reduce<uint32_t>(ctx, n, MaxOfU32{C}, OpMax{}, 0u, tmp32.p, part32));
-    PCC_RETURN_IF_ERROR(tmp32.ToHost(&maxc, 1));
+  const unsigned sms = unsigned(ctx->num_sms);
+  Scratch sc(ctx, n, g.m);
+  CompressHead* head = nullptr;
+  CompressHead* hh;  // its copy on the host
+  PCC_RETURN_IF_ERROR(ctx->Pinned(Context::kPinCompress, &hh));
+  std::memset(hh, 0, sizeof(*hh));
+  uint32_t *pres, *rank, *ids;
+  PCC_RETURN_IF_ERROR(sc.Take(&head, 1));
+  PCC_CUDA(cudaMemsetAsync(head, 0, sizeof(CompressHead), st));
+  // Dense order-preserving rank of the cluster ids in use; n2 = 1 + max C.
+  PCC_RETURN_IF_ERROR(sc.Take(&pres, n));
+  PCC_RETURN_IF_ERROR(sc.Take(&rank, n));
+  PCC_RETURN_IF_ERROR(sc.Take(&ids, n));
+  DBuf<uint32_t> scan_tiles;
+  DBuf<uint64_t> scan64;
+  if (n) {
+    PCC_CUDA(cudaMemsetAsync(pres, 0, sizeof(uint32_t) * n, st));
+    MarkPresentKernel<<<Blocks(n, 256, sms * 8), 256, 0, st>>>(n, C, pres, &head->max_c); PCC_COUNT(1);
+    PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx, n, PresInput{pres}, RankWriter{rank, ids}, scan_tiles, &head->R));
+    PCC_CUDA(cudaMemcpyAsync(hh, head, sizeof(uint32_t) * 2, cudaMemcpyDeviceToHost, st));
     PCC_RETURN_IF_ERROR(Sync(ctx));
   }
-  const uint32_t n2 = maxc + 1;
-
-  // Dense order-preserving rank of the cluster ids in use.
-  DBuf<uint32_t> pres, rank, ids;
-  PCC_RETURN_IF_ERROR(pres.Alloc(ctx, n2));
-  PCC_RETURN_IF_ERROR(pres.Zero());
-  PCC_RETURN_IF_ERROR(rank.Alloc(ctx, n2));
-  PCC_RETURN_IF_ERROR(ids.Alloc(ctx, n2));
-  MarkPresentKernel<<<Blocks(n, 256, ctx->num_sms * 8), 256, 0, st>>>(n, C, pres.p); PCC_COUNT(1);
-  DBuf<uint32_t> scan_tiles;
-  PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx, n2, PresInput{pres.p}, RankWriter{rank.p, ids.p}, scan_tiles,
-                                          tmp32.p));
-  uint32_t R = 0;  // clusters in use
-  PCC_RETURN_IF_ERROR(tmp32.ToHost(&R, 1));
-  PCC_RETURN_IF_ERROR(Sync(ctx));
-  pres.Release();
+  sc.Done(pres);
+  const uint32_t n2 = hh->max_c + 1;
+  const uint32_t R = hh->R;  // clusters in use
   // Keys: a rank (< R) or the dropped-copy mark above every rank, in kbits
   // bits (32 when the ranks need 31 or more).
   const int bits = BitsFor(R);
@@ -774,68 +828,68 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
   auto res = std::make_unique<DevGraph>();
   res->n = n2;
   PCC_RETURN_IF_ERROR(res->off.Alloc(ctx, uint64_t(n2) + 1));
-  DBuf<uint32_t> row_count;
-  PCC_RETURN_IF_ERROR(row_count.Alloc(ctx, uint64_t(n2) + 1));
-  PCC_RETURN_IF_ERROR(row_count.Zero());
-  DBuf<uint32_t> akey, aval;
-  DBuf<uint64_t> segbase;
-  DBuf<uint32_t> ucount;
+  uint32_t* row_count;
+  PCC_RETURN_IF_ERROR(sc.Take(&row_count, uint64_t(n2) + 1));
+  PCC_CUDA(cudaMemsetAsync(row_count, 0, sizeof(uint32_t) * (uint64_t(n2) + 1), st));
+  uint32_t *akey = nullptr, *aval = nullptr, *ucount = nullptr, *lists = nullptr;
+  uint64_t* segbase = nullptr;
   // Global path, kept until its rows are placed: sorted keys, run starts,
   // first run per segment, and each kept run's neighbour id and sum.
   DBuf<uint64_t> bkeys;
-  DBuf<uint32_t> seg_start, grun, bkey, bval, lists;
+  DBuf<uint32_t> seg_start, grun, bkey, bval;
   uint32_t S = 0;
   int place_kbits = 0;
   if (g.m) {
     // Vertices in cluster order (stable: ascending id inside a cluster) and
     // where each row starts in the cluster-ordered entry array.
-    DBuf<uint64_t> vkey;
-    DBuf<uint32_t> vval;
-    PCC_RETURN_IF_ERROR(vkey.Alloc(ctx, n));
-    PCC_RETURN_IF_ERROR(vval.Alloc(ctx, n));
-    VertexKeysKernel<<<Blocks(n, 256, ctx->num_sms * 8), 256, 0, st>>>(n, C, rank.p, vkey.p, vval.p);
+    uint64_t *vkey, *dstart;
+    uint32_t* vval;
+    PCC_RETURN_IF_ERROR(sc.Take(&vkey, n));
+    PCC_RETURN_IF_ERROR(sc.Take(&vval, n));
+    VertexKeysKernel<<<Blocks(n, 256, sms * 8), 256, 0, st>>>(n, C, rank, vkey, vval);
     PCC_COUNT(1);
     {
-      SortScratch sc;
-      PCC_RETURN_IF_ERROR(RadixSortPairs(ctx, vkey.p, vval.p, n, bits, sc));
+      SortBuffers sb;
+      uint64_t* keys2;
+      uint32_t *vals2, *hist;
+      PCC_RETURN_IF_ERROR(sc.Take(&keys2, n));
+      PCC_RETURN_IF_ERROR(sc.Take(&vals2, n));
+      PCC_RETURN_IF_ERROR(sc.Take(&hist, SortHistWords(n)));
+      sb.keys = keys2;
+      sb.vals = vals2;
+      sb.hist = hist;
+      PCC_RETURN_IF_ERROR(RadixSortInto(ctx, &vkey, &vval, n, bits, sb, scan_tiles));
+      sc.Done(vkey == keys2 ? nullptr : keys2);
+      sc.Done(vval == vals2 ? nullptr : vals2);
+      sc.Done(hist);
     }
-    DBuf<uint64_t> dstart, scan64;
-    PCC_RETURN_IF_ERROR(dstart.Alloc(ctx, n));
-    PCC_RETURN_IF_ERROR(ScanApply<uint64_t>(ctx, n, SortedDegInput{g.off.p, vval.p}, RowStartWriter{vval.p, dstart.p},
-                                            scan64, static_cast<uint64_t*>(nullptr)));
-    PCC_RETURN_IF_ERROR(segbase.Alloc(ctx, uint64_t(R) + 1));
-    SegBaseKernel<<<Blocks(n, 256, ctx->num_sms * 8), 256, 0, st>>>(n, vkey.p, vval.p, dstart.p, segbase.p, R, g.m);
-    PCC_COUNT(1);
-    vkey.Release();
-    vval.Release();
+    PCC_RETURN_IF_ERROR(sc.Take(&dstart, n));
+    PCC_RETURN_IF_ERROR(sc.Take(&segbase, uint64_t(R) + 1));
+    PCC_RETURN_IF_ERROR(ScanApply<uint64_t>(ctx, n, SortedDegInput{g.off.p, vval},
+                                            RowStartWriter{vkey, vval, dstart, segbase, R, g.m}, scan64,
+                                            static_cast<uint64_t*>(nullptr)));
+    sc.Done(vkey);
+    sc.Done(vval);
     // Every row moved into its cluster's segment.
-    PCC_RETURN_IF_ERROR(akey.Alloc(ctx, g.m));
-    PCC_RETURN_IF_ERROR(aval.Alloc(ctx, g.m));
+    PCC_RETURN_IF_ERROR(sc.Take(&akey, g.m));
+    PCC_RETURN_IF_ERROR(sc.Take(&aval, g.m));
     LaunchEdgeIter(ctx, g.bins.list.p, g.bins.counts.p, g.bins.counts.p + kNumBins, g.bins.host_counts, g.off.p,
-                   MoveEntries{g.off.p, g.nbr.p, g.wp(), C, rank.p, dstart.p, drop, akey.p, aval.p});
+                   MoveEntries{g.off.p, g.nbr.p, g.wp(), C, rank, dstart, drop, akey, aval});
     PCC_RETURN_IF_ERROR(LaunchCheck());
-    dstart.Release();
+    sc.Done(dstart);
     // Segment classes.
-    DBuf<uint32_t> counts;
-    DBuf<unsigned long long> big_e;
-    PCC_RETURN_IF_ERROR(lists.Alloc(ctx, uint64_t(R) * 4));
-    const uint32_t* wlist = lists.p;
-    const uint32_t* mlist = lists.p + uint64_t(R);
-    const uint32_t* clist = lists.p + 2 * uint64_t(R);
-    const uint32_t* blist = lists.p + 3 * uint64_t(R);
-    PCC_RETURN_IF_ERROR(counts.Alloc(ctx, 4));
-    PCC_RETURN_IF_ERROR(counts.Zero());
-    PCC_RETURN_IF_ERROR(big_e.Alloc(ctx, 1));
-    PCC_RETURN_IF_ERROR(big_e.Zero());
-    PCC_RETURN_IF_ERROR(ucount.Alloc(ctx, R));
-    PCC_RETURN_IF_ERROR(ucount.Zero());
-    ClassifyKernel<<<Blocks(R, 256, ctx->num_sms * 8), 256, 0, st>>>(R, segbase.p, lists.p, counts.p, big_e.p);
+    PCC_RETURN_IF_ERROR(sc.Take(&lists, uint64_t(R) * 4));
+    const uint32_t* wlist = lists;
+    const uint32_t* mlist = lists + uint64_t(R);
+    const uint32_t* clist = lists + 2 * uint64_t(R);
+    const uint32_t* blist = lists + 3 * uint64_t(R);
+    PCC_RETURN_IF_ERROR(sc.Take(&ucount, R));
+    PCC_CUDA(cudaMemsetAsync(ucount, 0, sizeof(uint32_t) * R, st));
+    ClassifyKernel<<<Blocks(R, 256, sms * 8), 256, 0, st>>>(R, segbase, lists, head->counts, &head->big_e);
     PCC_COUNT(1);
-    uint32_t hc[4];
-    unsigned long long E = 0;
-    PCC_RETURN_IF_ERROR(counts.ToHost(hc, 4));
-    PCC_RETURN_IF_ERROR(big_e.ToHost(&E, 1));
-    PCC_RETURN_IF_ERROR(Sync(ctx));
+    const bool maybe_big = g.m > kSegCtaMax;
+    if (maybe_big)
+      PCC_CUDA(cudaMemcpyAsync(hh, head, offsetof(CompressHead, m2), cudaMemcpyDeviceToHost, st));
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [] {
@@ -845,37 +899,45 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
     });
     PCC_CUDA(attr);
     const int passes = (kbits + 7) / 8;
-    if (hc[0]) {
-      SegWarpKernel<<<Blocks(hc[0], 8, ctx->num_sms * 16), 256, 0, st>>>(wlist, counts.p, segbase.p, ids.p, drop,
-                                                                         akey.p, aval.p, ucount.p);
+    // The kernels read their class's length on the device; the grids follow
+    // bounds of it (a class-c segment has more than the class's entries).
+    const uint64_t max_mid = std::min<uint64_t>(R, g.m / (kSegWarpMax + 1));
+    const uint64_t max_cta = std::min<uint64_t>(R, g.m / (kSegMidMax + 1));
+    SegWarpKernel<<<Blocks(R, 8, sms * 16), 256, 0, st>>>(wlist, head->counts, segbase, ids, drop, akey, aval, ucount,
+                                                          row_count);
+    PCC_COUNT(1);
+    if (max_mid) {
+      SegMidKernel<<<Blocks(max_mid, kSegMidWarps, sms * 12), kSegMidWarps * 32, kSegMidSmem, st>>>(
+          mlist, head->counts, segbase, ids, drop, passes, akey, aval, ucount, row_count);
       PCC_COUNT(1);
     }
-    if (hc[1]) {
-      SegMidKernel<<<Blocks(hc[1], kSegMidWarps, ctx->num_sms * 12), kSegMidWarps * 32, kSegMidSmem, st>>>(
-          mlist, counts.p, segbase.p, ids.p, drop, passes, akey.p, aval.p, ucount.p);
+    if (max_cta) {
+      SegCtaKernel<<<Blocks(max_cta, 1, sms * 3), kSegCtaThreads, kSegCtaSmem, st>>>(
+          clist, head->counts, segbase, ids, drop, passes, akey, aval, ucount, row_count);
       PCC_COUNT(1);
     }
-    if (hc[2]) {
-      SegCtaKernel<<<Blocks(hc[2], 1, ctx->num_sms * 3), kSegCtaThreads, kSegCtaSmem, st>>>(
-          clist, counts.p, segbase.p, ids.p, drop, passes, akey.p, aval.p, ucount.p);
-      PCC_COUNT(1);
-    }
-    if (hc[3]) {
-      const uint32_t nbig = hc[3];
+    PCC_RETURN_IF_ERROR(LaunchCheck());
+    if (maybe_big) PCC_RETURN_IF_ERROR(Sync(ctx));
+    if (hh->counts[3]) {
+      const uint32_t nbig = hh->counts[3];
+      const uint64_t E = hh->big_e;
       place_kbits = kbits;
       DBuf<uint64_t> ebase;
-      DBuf<uint32_t> bvals, long_run, long_count;
+      DBuf<uint32_t> bvals, long_run, tmp32;
+      PCC_RETURN_IF_ERROR(tmp32.Alloc(ctx, 2));  // runs, long runs
+      PCC_RETURN_IF_ERROR(tmp32.Zero());
+      uint32_t* long_count = tmp32.p + 1;
       PCC_RETURN_IF_ERROR(ebase.Alloc(ctx, nbig));
-      PCC_RETURN_IF_ERROR(ScanApply<uint64_t>(ctx, nbig, BigLenInput{blist, segbase.p}, StorePrefix<uint64_t>{ebase.p},
+      PCC_RETURN_IF_ERROR(ScanApply<uint64_t>(ctx, nbig, BigLenInput{blist, segbase}, StorePrefix<uint64_t>{ebase.p},
                                               scan64, static_cast<uint64_t*>(nullptr)));
       PCC_RETURN_IF_ERROR(bkeys.Alloc(ctx, E));
       PCC_RETURN_IF_ERROR(bvals.Alloc(ctx, E));
-      BigGatherKernel<<<Blocks(E, kSegCtaMax, unsigned(ctx->num_sms) * 8), 256, 0, st>>>(
-          blist, nbig, E, segbase.p, ebase.p, akey.p, aval.p, kbits, bkeys.p, bvals.p);
+      BigGatherKernel<<<Blocks(E, kSegCtaMax, sms * 8), 256, 0, st>>>(blist, nbig, E, segbase, ebase.p, akey, aval,
+                                                                      kbits, bkeys.p, bvals.p);
       PCC_COUNT(1);
       {
-        SortScratch sc;
-        PCC_RETURN_IF_ERROR(RadixSortPairs(ctx, bkeys.p, bvals.p, E, kbits + BitsFor(nbig), sc));
+        SortScratch ss;
+        PCC_RETURN_IF_ERROR(RadixSortPairs(ctx, bkeys.p, bvals.p, E, kbits + BitsFor(nbig), ss));
       }
       PCC_RETURN_IF_ERROR(seg_start.Alloc(ctx, E));
       PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx, E, HeadInput{bkeys.p}, StoreIndexIfSet{seg_start.p}, scan_tiles,
@@ -886,16 +948,14 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
       PCC_RETURN_IF_ERROR(long_run.Alloc(ctx, S));
       PCC_RETURN_IF_ERROR(bkey.Alloc(ctx, S));
       PCC_RETURN_IF_ERROR(bval.Alloc(ctx, S));
-      PCC_RETURN_IF_ERROR(long_count.Alloc(ctx, 1));
-      PCC_RETURN_IF_ERROR(long_count.Zero());
-      BigGroupKernel<<<Blocks(S, 256, ctx->num_sms * 8), 256, 0, st>>>(S, seg_start.p, bkeys.p, kbits, grun.p);
+      BigGroupKernel<<<Blocks(S, 256, sms * 8), 256, 0, st>>>(S, seg_start.p, bkeys.p, kbits, grun.p);
       PCC_COUNT(1);
-      BigRunKernel<<<Blocks(S, 256, ctx->num_sms * 16), 256, 0, st>>>(
-          S, E, seg_start.p, bkeys.p, bvals.p, kbits, drop, grun.p, blist, ids.p, bkey.p, bval.p, ucount.p,
-          long_run.p, long_count.p);
+      BigRunKernel<<<Blocks(S, 256, sms * 16), 256, 0, st>>>(S, E, seg_start.p, bkeys.p, bvals.p, kbits, drop, grun.p,
+                                                             blist, ids, bkey.p, bval.p, ucount, row_count, long_run.p,
+                                                             long_count);
       PCC_COUNT(1);
       uint32_t nlong = 0;
-      PCC_RETURN_IF_ERROR(long_count.ToHost(&nlong, 1));
+      PCC_CUDA(cudaMemcpyAsync(&nlong, long_count, sizeof(nlong), cudaMemcpyDeviceToHost, st));
       PCC_RETURN_IF_ERROR(Sync(ctx));
       if (nlong) {
         DBuf<float> scratch;
@@ -908,40 +968,38 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
         uint64_t NB = 0;
         PCC_RETURN_IF_ERROR(nbtot.ToHost(&NB, 1));
         PCC_RETURN_IF_ERROR(Sync(ctx));
-        LongBlocksKernel<<<Blocks(NB, 256, unsigned(ctx->num_sms) * 16), 256, 0, st>>>(
-            nlong, NB, bbase.p, long_run.p, seg_start.p, S, E, bvals.p, scratch.p);
+        LongBlocksKernel<<<Blocks(NB, 256, sms * 16), 256, 0, st>>>(nlong, NB, bbase.p, long_run.p, seg_start.p, S, E,
+                                                                    bvals.p, scratch.p);
         PCC_COUNT(1);
-        BigLongKernel<<<unsigned(ctx->num_sms) * 2, kLongThreads, 0, st>>>(long_run.p, long_count.p, seg_start.p,
-                                                                           S, E, bvals.p, scratch.p, bval.p);
+        BigLongKernel<<<sms * 2, kLongThreads, 0, st>>>(long_run.p, long_count, seg_start.p, S, E, bvals.p, scratch.p,
+                                                        bval.p);
         PCC_COUNT(1);
       }
     }
     PCC_RETURN_IF_ERROR(LaunchCheck());
-    RowCountKernel<<<Blocks(R, 256, ctx->num_sms * 8), 256, 0, st>>>(R, ids.p, ucount.p, row_count.p);
-    PCC_COUNT(1);
   }
   // Offsets over the sparse id space [0, n2].
-  DBuf<uint64_t> scan64b, total;
-  PCC_RETURN_IF_ERROR(total.Alloc(ctx, 1));
-  PCC_RETURN_IF_ERROR(ScanApply<uint64_t>(ctx, uint64_t(n2) + 1, CountInput{row_count.p, n2},
-                                          StorePrefix<uint64_t>{res->off.p}, scan64b, total.p));
-  uint64_t m2 = 0;
-  PCC_RETURN_IF_ERROR(total.ToHost(&m2, 1));
-  PCC_RETURN_IF_ERROR(Sync(ctx));
-  res->m = m2;
-  PCC_RETURN_IF_ERROR(res->nbr.Alloc(ctx, m2 ? m2 : 1));
-  PCC_RETURN_IF_ERROR(res->w.Alloc(ctx, m2 ? m2 : 1));
-  DBuf<WeightStats> stats;
-  PCC_RETURN_IF_ERROR(stats.Alloc(ctx, 1));
-  PCC_RETURN_IF_ERROR(stats.Zero());
-  if (m2) {
-    GatherRowsKernel<<<Blocks(R, 8, ctx->num_sms * 16), 256, 0, st>>>(R, ids.p, ucount.p, segbase.p, res->off.p,
-                                                                      akey.p, aval.p, res->nbr.p, res->w.p, stats.p);
+  uint64_t* m2 = reinterpret_cast<uint64_t*>(&head->m2);
+  PCC_RETURN_IF_ERROR(ScanApply<uint64_t>(ctx, uint64_t(n2) + 1, CountInput{row_count, n2},
+                                          StorePrefix<uint64_t>{res->off.p}, scan64, m2));
+  uint64_t entries = g.m;  // at most
+  const bool wait = ctx->budget || g.m > (16u << 20);
+  if (wait) {
+    PCC_CUDA(cudaMemcpyAsync(&hh->m2, m2, sizeof(hh->m2), cudaMemcpyDeviceToHost, st));
+    PCC_RETURN_IF_ERROR(Sync(ctx));
+    entries = hh->m2;
+  }
+  res->m = entries;
+  PCC_RETURN_IF_ERROR(res->nbr.Alloc(ctx, entries ? entries : 1));
+  PCC_RETURN_IF_ERROR(res->w.Alloc(ctx, entries ? entries : 1));
+  if (entries) {
+    GatherRowsKernel<<<Blocks(R, 8, sms * 16), 256, 0, st>>>(R, ids, ucount, segbase, res->off.p, akey, aval,
+                                                             res->nbr.p, res->w.p, &head->stats);
     PCC_COUNT(1);
     if (S) {
-      BigPlaceKernel<<<Blocks(S, 256, ctx->num_sms * 16), 256, 0, st>>>(
-          S, seg_start.p, bkeys.p, place_kbits, drop, grun.p, lists.p + 3 * uint64_t(R), ids.p, res->off.p, bkey.p,
-          bval.p, res->nbr.p, res->w.p, stats.p);
+      BigPlaceKernel<<<Blocks(S, 256, sms * 16), 256, 0, st>>>(
+          S, seg_start.p, bkeys.p, place_kbits, drop, grun.p, lists + 3 * uint64_t(R), ids, res->off.p, bkey.p, bval.p,
+          res->nbr.p, res->w.p, &head->stats);
       PCC_COUNT(1);
     }
   }
@@ -950,15 +1008,15 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
   grun.Release();
   bkey.Release();
   bval.Release();
-  lists.Release();
-  akey.Release();
-  aval.Release();
+  sc.Done(lists);
+  sc.Done(akey);
+  sc.Done(aval);
   // Node weights.
   PCC_RETURN_IF_ERROR(res->node_w.Alloc(ctx, n2));
   PCC_RETURN_IF_ERROR(res->node_w.Zero());
-  NodeWeightKernel<<<Blocks(n, 256, ctx->num_sms * 8), 256, 0, st>>>(n, C, k, res->node_w.p); PCC_COUNT(1);
+  NodeWeightKernel<<<Blocks(n, 256, sms * 8), 256, 0, st>>>(n, C, k, res->node_w.p); PCC_COUNT(1);
   PCC_RETURN_IF_ERROR(LaunchCheck());
-  PCC_RETURN_IF_ERROR(ComputeGraphProperties(ctx, res.get(), stats.p));
+  PCC_RETURN_IF_ERROR(ComputeGraphProperties(ctx, res.get(), &head->stats, wait ? nullptr : m2));
   *out = std::move(res);
   return Status::Ok();
 }

@@ -49,7 +49,7 @@ __host__ __device__ inline int BinOf(uint64_t d) {
 // Degree-binned vertex list: bins are contiguous segments of `list`.
 struct BinSet {
   DBuf<uint32_t> list;       // n entries
-  DBuf<uint32_t> counts;     // [kNumBins] counts, then [kNumBins+1] starts
+  DBuf<uint32_t> counts;     // [kNumBins] counts, then [kNumBins+1] starts (graphops.cuh)
   uint64_t edges = 0;        // sum of degrees (host copy, static bins only)
   uint32_t size = 0;         // vertices (host copy, static bins only)
   uint32_t host_counts[kNumBins] = {0};
@@ -146,9 +146,11 @@ inline SumMode SumModeFor(const DevGraph& g, double offset) {
 }
 
 // Computes max degree / weight properties and the static degree bins on
-// the device.  d_stats: the weights' statistics, already on the device (null:
-// reduced here).
-Status ComputeGraphProperties(Context* ctx, DevGraph* g, const WeightStats* d_stats = nullptr);
+// the device (one sync).  d_stats: the weights' statistics, already on the
+// device (null: reduced here); d_m: the entries, read back with the rest (null:
+// g->m is set).
+Status ComputeGraphProperties(Context* ctx, DevGraph* g, const WeightStats* d_stats = nullptr,
+                              const uint64_t* d_m = nullptr);
 // Builds g->bins_all (degree bins including isolated vertices) if absent.
 Status EnsureAllBins(Context* ctx, const DevGraph* g);
 

@@ -14,11 +14,6 @@ namespace pcc {
 
 namespace {
 
-struct DegreeInput {
-  const uint64_t* off;
-  __device__ uint32_t operator()(uint64_t i) const { return static_cast<uint32_t>(off[i + 1] - off[i]); }
-};
-
 struct WeightInput {
   const float* w;
   __device__ WeightStats operator()(uint64_t i) const { return WeightStatsOf(w[i]); }
@@ -43,29 +38,23 @@ struct PredNonZeroDegree {
   __device__ bool operator()(uint32_t v) const { return off[v + 1] > off[v]; }
 };
 
-Status BuildBins(Context* ctx, const DevGraph* g, BinSet* b, bool include_isolated) {
-  PCC_RETURN_IF_ERROR(AllocBins(ctx, g->n, b));
-  DBuf<unsigned long long> sum;
-  DBuf<uint32_t> cnt;
-  PCC_RETURN_IF_ERROR(sum.Alloc(ctx, 1));
-  PCC_RETURN_IF_ERROR(cnt.Alloc(ctx, 1));
-  PCC_RETURN_IF_ERROR(sum.Zero());
-  PCC_RETURN_IF_ERROR(cnt.Zero());
+// Bins the vertices; waits for the stream (with whatever was queued before).
+Status BuildBins(Context* ctx, const DevGraph* g, BinSet* b, bool include_isolated, uint32_t* max_deg = nullptr) {
   if (include_isolated) {
-    PCC_RETURN_IF_ERROR(BinVertices(ctx, g->n, g->off.p, PredAll{}, b, sum.p, cnt.p));
+    PCC_RETURN_IF_ERROR(BinVertices(ctx, g->n, g->off.p, PredAll{}, b));
   } else {
-    PCC_RETURN_IF_ERROR(BinVertices(ctx, g->n, g->off.p, PredNonZeroDegree{g->off.p}, b, sum.p, cnt.p));
+    PCC_RETURN_IF_ERROR(BinVertices(ctx, g->n, g->off.p, PredNonZeroDegree{g->off.p}, b));
   }
-  uint32_t hc[kNumBins];
-  uint32_t hcnt = 0;
-  unsigned long long hsum = 0;
-  PCC_RETURN_IF_ERROR(b->counts.ToHost(hc, kNumBins));
-  PCC_RETURN_IF_ERROR(cnt.ToHost(&hcnt, 1));
-  PCC_RETURN_IF_ERROR(sum.ToHost(&hsum, 1));
+  uint32_t* h;
+  PCC_RETURN_IF_ERROR(ctx->Pinned(Context::kPinBins, &h));
+  PCC_RETURN_IF_ERROR(b->counts.ToHost(h, kBinWords));
   PCC_RETURN_IF_ERROR(Sync(ctx));
-  for (int i = 0; i < kNumBins; ++i) b->host_counts[i] = hc[i];
-  b->size = hcnt;
-  b->edges = hsum;
+  for (int i = 0; i < kNumBins; ++i) b->host_counts[i] = h[i];
+  b->size = h[kBinSize];
+  unsigned long long sum = 0;
+  std::memcpy(&sum, h + kBinDegSum, sizeof(sum));
+  b->edges = sum;
+  if (max_deg) *max_deg = h[kBinMaxDegAt];
   return Status::Ok();
 }
 
@@ -84,36 +73,29 @@ Status EnsureAllBins(Context* ctx, const DevGraph* g) {
   return BuildBins(ctx, g, &g->bins_all, true);
 }
 
-__global__ void BinStartsKernel(const uint32_t* counts, uint32_t* starts, uint32_t* cursor) {
-  uint32_t acc = 0;
-  for (int b = 0; b < kNumBins; ++b) {
-    starts[b] = acc;
-    acc += counts[b];
-    cursor[b] = 0;
-  }
-  starts[kNumBins] = acc;
-}
-
-Status ComputeGraphProperties(Context* ctx, DevGraph* g, const WeightStats* d_stats) {
-  DBuf<uint32_t> part, out;
-  PCC_RETURN_IF_ERROR(out.Alloc(ctx, 1));
-  uint32_t maxd = 0;
-  if (g->n) {
-    PCC_RETURN_IF_ERROR(Reduce<uint32_t>(ctx, g->n, DegreeInput{g->off.p}, OpMax{}, 0u, out.p, part));
-    PCC_RETURN_IF_ERROR(out.ToHost(&maxd, 1));
-  }
-  WeightStats ws{g->m, 1.0f, 0};
+Status ComputeGraphProperties(Context* ctx, DevGraph* g, const WeightStats* d_stats, const uint64_t* d_m) {
+  struct Read {
+    uint64_t m;
+    WeightStats ws;
+  };
+  Read* h;
+  PCC_RETURN_IF_ERROR(ctx->Pinned(Context::kPinStats, &h));
+  h->m = g->m;
+  h->ws = WeightStats{g->m, 1.0f, 0};
+  if (d_m) PCC_CUDA(cudaMemcpyAsync(&h->m, d_m, sizeof(h->m), cudaMemcpyDeviceToHost, ctx->stream));
+  DBuf<WeightStats> wpart, wout;
   if (d_stats) {
-    PCC_CUDA(cudaMemcpyAsync(&ws, d_stats, sizeof(ws), cudaMemcpyDeviceToHost, ctx->stream));
+    PCC_CUDA(cudaMemcpyAsync(&h->ws, d_stats, sizeof(h->ws), cudaMemcpyDeviceToHost, ctx->stream));
   } else if (g->w.p && g->m) {
-    DBuf<WeightStats> wpart, wout;
     PCC_RETURN_IF_ERROR(wout.Alloc(ctx, 1));
     PCC_RETURN_IF_ERROR(Reduce<WeightStats>(ctx, g->m, WeightInput{g->w.p}, WeightOp{}, WeightStats{0, 0.0f, 0},
                                             wout.p, wpart));
-    PCC_RETURN_IF_ERROR(wout.ToHost(&ws, 1));
-    PCC_RETURN_IF_ERROR(Sync(ctx));
+    PCC_RETURN_IF_ERROR(wout.ToHost(&h->ws, 1));
   }
-  PCC_RETURN_IF_ERROR(BuildBins(ctx, g, &g->bins, false));
+  uint32_t maxd = 0;
+  PCC_RETURN_IF_ERROR(BuildBins(ctx, g, &g->bins, false, &maxd));
+  g->m = h->m;
+  const WeightStats ws = h->ws;
   g->max_deg = maxd;
   g->integral = ws.frac == 0;
   g->max_abs_w = ws.maxabs;

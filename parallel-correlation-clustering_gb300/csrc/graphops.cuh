@@ -283,24 +283,34 @@ struct PredStamp {
   __device__ bool operator()(uint32_t v) const { return st[v] == StampIn(rs, stamp); }
 };
 
+// Layout of BinSet::counts: kNumBins counts, kNumBins + 1 starts, kNumBins
+// cursors, then the degree sum (64 bits), the vertices binned and the largest
+// degree.
+constexpr int kBinCursors = 2 * kNumBins + 1;
+constexpr int kBinDegSum = 32;
+constexpr int kBinSize = 34;
+constexpr int kBinMaxDegAt = 35;
+constexpr int kBinWords = 36;
+static_assert(kBinCursors + kNumBins <= kBinDegSum, "bin header");
+
 template <class P>
 __global__ void __launch_bounds__(256) BinCountKernel(uint32_t n, const uint64_t* __restrict__ off, P pred,
-                                                      uint32_t* counts, unsigned long long* deg_sum,
-                                                      uint32_t* vcount) {
+                                                      uint32_t* head) {
   __shared__ uint32_t sh[kNumBins];
   __shared__ unsigned long long sh_deg;
-  __shared__ uint32_t sh_cnt;
+  __shared__ uint32_t sh_cnt, sh_max;
   if (threadIdx.x < kNumBins) sh[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     sh_deg = 0;
     sh_cnt = 0;
+    sh_max = 0;
   }
   __syncthreads();
   uint32_t local[kNumBins];
 #pragma unroll
   for (int b = 0; b < kNumBins; ++b) local[b] = 0;
   unsigned long long deg_acc = 0;
-  uint32_t cnt = 0;
+  uint32_t cnt = 0, mx = 0;
   for (uint64_t v = uint64_t(blockIdx.x) * 256 + threadIdx.x; v < n; v += uint64_t(gridDim.x) * 256) {
     if (!pred(static_cast<uint32_t>(v))) continue;
     const uint64_t d = off[v + 1] - off[v];
@@ -308,6 +318,7 @@ __global__ void __launch_bounds__(256) BinCountKernel(uint32_t n, const uint64_t
 #pragma unroll
     for (int q = 0; q < kNumBins; ++q) local[q] += (q == b);
     deg_acc += d;
+    mx = max(mx, static_cast<uint32_t>(d));
     cnt++;
   }
 #pragma unroll
@@ -315,11 +326,13 @@ __global__ void __launch_bounds__(256) BinCountKernel(uint32_t n, const uint64_t
     if (local[q]) atomicAdd(&sh[q], local[q]);
   if (deg_acc) atomicAdd(&sh_deg, deg_acc);
   if (cnt) atomicAdd(&sh_cnt, cnt);
+  if (mx) atomicMax(&sh_max, mx);
   __syncthreads();
-  if (threadIdx.x < kNumBins && sh[threadIdx.x]) atomicAdd(&counts[threadIdx.x], sh[threadIdx.x]);
+  if (threadIdx.x < kNumBins && sh[threadIdx.x]) atomicAdd(&head[threadIdx.x], sh[threadIdx.x]);
   if (threadIdx.x == 0) {
-    if (deg_sum && sh_deg) atomicAdd(deg_sum, sh_deg);
-    if (vcount && sh_cnt) atomicAdd(vcount, sh_cnt);
+    if (sh_deg) atomicAdd(reinterpret_cast<unsigned long long*>(head + kBinDegSum), sh_deg);
+    if (sh_cnt) atomicAdd(head + kBinSize, sh_cnt);
+    if (sh_max) atomicMax(head + kBinMaxDegAt, sh_max);
   }
 }
 
@@ -357,13 +370,23 @@ __global__ void __launch_bounds__(256) CountDegreesKernel(uint32_t n, const uint
   }
 }
 
-// counts[0..B) -> starts[0..B] and cursors zeroed.
-__global__ void BinStartsKernel(const uint32_t* counts, uint32_t* starts, uint32_t* cursor);
-
+// Writes the binned vertices to the list; every block derives the starts from
+// the counts, block 0 stores them.
 template <class P>
 __global__ void __launch_bounds__(256) BinScatterKernel(uint32_t n, const uint64_t* __restrict__ off, P pred,
-                                                        const uint32_t* __restrict__ starts, uint32_t* cursor,
-                                                        uint32_t* list) {
+                                                        uint32_t* head, uint32_t* list) {
+  __shared__ uint32_t starts[kNumBins + 1];
+  if (threadIdx.x == 0) {
+    uint32_t acc = 0;
+    for (int b = 0; b < kNumBins; ++b) {
+      starts[b] = acc;
+      acc += head[b];
+    }
+    starts[kNumBins] = acc;
+  }
+  __syncthreads();
+  if (blockIdx.x == 0 && threadIdx.x <= kNumBins) head[kNumBins + threadIdx.x] = starts[threadIdx.x];
+  uint32_t* cursor = head + kBinCursors;
   const uint64_t stride = uint64_t(gridDim.x) * 256;
   const uint64_t limit = (uint64_t(n) + 31) & ~uint64_t(31);
   for (uint64_t v = uint64_t(blockIdx.x) * 256 + threadIdx.x; v < limit; v += stride) {
@@ -378,34 +401,19 @@ __global__ void __launch_bounds__(256) BinScatterKernel(uint32_t n, const uint64
   }
 }
 
-// Bins the vertices of [0, n) that satisfy pred into b (list must hold n
-// entries, counts 3 * kNumBins + 1).  deg_sum / vcount (device, nullable)
-// accumulate the sum of degrees and the number of binned vertices.
+// Bins the vertices of [0, n) that satisfy pred into b.
 template <class P>
-Status BinVertices(Context* ctx, uint32_t n, const uint64_t* off, P pred, BinSet* b,
-                   unsigned long long* deg_sum, uint32_t* vcount) {
-  uint32_t* counts = b->counts.p;
-  uint32_t* starts = counts + kNumBins;
-  uint32_t* cursor = starts + kNumBins + 1;
-  PCC_CUDA(cudaMemsetAsync(counts, 0, sizeof(uint32_t) * kNumBins, ctx->stream));
+Status BinVertices(Context* ctx, uint32_t n, const uint64_t* off, P pred, BinSet* b) {
+  PCC_RETURN_IF_ERROR(b->list.Reserve(ctx, std::max<uint64_t>(n, 1)));
+  PCC_RETURN_IF_ERROR(b->counts.Reserve(ctx, kBinWords));
+  PCC_CUDA(cudaMemsetAsync(b->counts.p, 0, sizeof(uint32_t) * kBinWords, ctx->stream));
   const unsigned grid = Blocks(n, 256, unsigned(ctx->num_sms) * 16);
   if (n) {
-    BinCountKernel<P><<<grid, 256, 0, ctx->stream>>>(n, off, pred, counts, deg_sum, vcount);
-    PCC_COUNT(1);
-  }
-  BinStartsKernel<<<1, 1, 0, ctx->stream>>>(counts, starts, cursor);
-  PCC_COUNT(1);
-  if (n) {
-    BinScatterKernel<P><<<grid, 256, 0, ctx->stream>>>(n, off, pred, starts, cursor, b->list.p);
-    PCC_COUNT(1);
+    BinCountKernel<P><<<grid, 256, 0, ctx->stream>>>(n, off, pred, b->counts.p);
+    BinScatterKernel<P><<<grid, 256, 0, ctx->stream>>>(n, off, pred, b->counts.p, b->list.p);
+    PCC_COUNT(2);
   }
   return LaunchCheck();
-}
-
-inline Status AllocBins(Context* ctx, uint32_t n, BinSet* b) {
-  PCC_RETURN_IF_ERROR(b->list.Reserve(ctx, std::max<uint64_t>(n, 1)));
-  PCC_RETURN_IF_ERROR(b->counts.Reserve(ctx, 3 * kNumBins + 1));
-  return Status::Ok();
 }
 
 }  // namespace pcc

@@ -55,12 +55,26 @@ __global__ void FillF64Kernel(uint64_t n, double v, double* out) {
     out[i] = v;
 }
 
-// Singletons: C = i, s = 1, K = k (SetClustering with an empty clustering).
-__global__ void SingletonsKernel(uint32_t n, const double* __restrict__ k, uint32_t* C, uint32_t* s, double* K) {
+// A level's state in one pass: node weights (src, or 1) and their FP32 images;
+// singletons (C = i, s = 1, K = k, SetClustering with an empty clustering), or
+// the given labels with empty clusters.
+__global__ void LevelInitKernel(uint32_t n, const double* __restrict__ src, const uint32_t* __restrict__ labels,
+                                double* k, float* kf, uint32_t* C, uint32_t* s, double* K, float* Kf) {
   for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
-    C[i] = static_cast<uint32_t>(i);
-    s[i] = 1u;
-    K[i] = k[i];
+    const double x = src ? src[i] : 1.0;
+    const float f = FilterF32(x);
+    k[i] = x;
+    kf[i] = f;
+    if (labels) {
+      C[i] = labels[i];
+      s[i] = 0u;
+      K[i] = 0.0;
+    } else {
+      C[i] = static_cast<uint32_t>(i);
+      s[i] = 1u;
+      K[i] = x;
+      Kf[i] = f;
+    }
   }
 }
 
@@ -101,7 +115,7 @@ __global__ void RefreshKfKernel(uint32_t n, const double* __restrict__ K, float*
 }
 
 // kf = FilterF32(k): node weights for the FP32 pre-filter and certified
-// decisions.
+// decisions (replay).
 __global__ void NodeKfKernel(uint32_t n, const double* __restrict__ k, float* kf) {
   for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
     kf[i] = FilterF32(k[i]);
@@ -754,21 +768,15 @@ class Engine {
     PCC_RETURN_IF_ERROR(L->Kf.Alloc(ctx_, nn));
     PCC_RETURN_IF_ERROR(L->kf.Alloc(ctx_, nn));
     if (n) {
-      if (k_is_ones || !d_k) {
-        FillF64Kernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, 1.0, L->k.p); PCC_COUNT(1);
-      } else {
-        PCC_CUDA(cudaMemcpyAsync(L->k.p, d_k, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx_->stream));
-      }
+      const double* ks = k_is_ones ? nullptr : d_k;
+      LevelInitKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, ks, d_labels, L->k.p, L->kf.p, L->C.p, L->s.p,
+                                                                 L->K.p, L->Kf.p);
+      PCC_COUNT(1);
       if (d_labels) {
-        PCC_CUDA(cudaMemcpyAsync(L->C.p, d_labels, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, ctx_->stream));
-        PCC_RETURN_IF_ERROR(L->s.Zero());
-        PCC_RETURN_IF_ERROR(L->K.Zero());
-        AccumulateClustersKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, L->C.p, L->k.p, L->s.p, L->K.p); PCC_COUNT(1);
-      } else {
-        SingletonsKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, L->k.p, L->C.p, L->s.p, L->K.p); PCC_COUNT(1);
+        AccumulateClustersKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, L->C.p, L->k.p, L->s.p, L->K.p);
+        RefreshKfKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, L->K.p, L->Kf.p, nullptr, 0, nullptr);
+        PCC_COUNT(2);
       }
-      RefreshKfKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, L->K.p, L->Kf.p, nullptr, 0, nullptr); PCC_COUNT(1);
-      NodeKfKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, L->k.p, L->kf.p); PCC_COUNT(1);
       PCC_RETURN_IF_ERROR(LaunchCheck());
     }
     L->mode = SumModeFor(*g, cfg_.edge_weight_offset);
@@ -1236,16 +1244,12 @@ class Engine {
   // most kLoopMaxEntries entries with exact sums.
   Status IterateLoop(Level* L, int64_t num_inner, bool* moved_out) {
     const DevGraph& g = *L->g;
-    RoundState h{};
-    h.front_all = 1;
-    h.front_edges = g.m;
-    h.front_size = g.n;
-    h.visited = L->bins->size;
-    h.stamp = stamp_;  // the first round's stamp is the next one
-    PCC_RETURN_IF_ERROR(rs_.FromHost(&h, 1));
-    PCC_CUDA(cudaMemsetAsync(&ctr_.p->level_moved, 0, sizeof(uint32_t) * 2, ctx_->stream));  // level_moved, rounds
-    PCC_CUDA(cudaMemsetAsync(&ctr_.p->edge_visits, 0, sizeof(unsigned long long) * 2, ctx_->stream));
-    PCC_CUDA(cudaMemsetAsync(&ctr_.p->sync_moves, 0, sizeof(unsigned long long) * 2, ctx_->stream));
+    LoopHead h{};
+    h.rs.front_all = 1;
+    h.rs.front_edges = g.m;
+    h.rs.front_size = g.n;
+    h.rs.visited = L->bins->size;
+    h.rs.stamp = stamp_;  // the first round's stamp is the next one
     if (!loop_state_.p) {
       PCC_RETURN_IF_ERROR(loop_state_.Alloc(ctx_, 1));
       PCC_RETURN_IF_ERROR(old_cluster_.Alloc(ctx_, std::max<uint64_t>(n_max_, 1)));
@@ -1269,23 +1273,16 @@ class Engine {
     l.zero_ids = zero_ids_.p;
     l.new_list = new_list_.p;
     l.Kf_mut = L->Kf.p;
-    l.rs = rs_.p;
     l.st = loop_state_.p;
     SetLoopHubs(&l, *g.hub_plan, hub_state_);
-    PCC_RETURN_IF_ERROR(LaunchRoundLoop(ctx_, l, L->mode, L->bins->host_counts, g.max_deg));
-    DevCounters hc;
-    RoundState hr;
-    PCC_RETURN_IF_ERROR(ctr_.ToHost(&hc, 1));
-    PCC_RETURN_IF_ERROR(rs_.ToHost(&hr, 1));
-    PCC_RETURN_IF_ERROR(Sync(ctx_));
-    if (hc.error) return MakeError(PCC_INTERNAL, "device error flag " + std::to_string(hc.error));
-    stamp_ = hr.stamp;
-    res_.rounds += static_cast<int32_t>(hc.rounds);
-    res_.edge_visits += hc.edge_visits;
-    res_.vertex_visits += hc.vertex_visits;
-    res_.algo_bytes += (g.w.p ? 12ull : 8ull) * hc.edge_visits + 40ull * hc.visited;
-    res_.moves += hc.sync_moves;
-    *moved_out = hc.level_moved != 0;
+    PCC_RETURN_IF_ERROR(RunRoundLoop(ctx_, l, L->mode, L->bins->host_counts, g.max_deg, &h));
+    stamp_ = h.rs.stamp;
+    res_.rounds += static_cast<int32_t>(h.rounds);
+    res_.edge_visits += h.edge_visits;
+    res_.vertex_visits += h.vertex_visits;
+    res_.algo_bytes += (g.w.p ? 12ull : 8ull) * h.edge_visits + 40ull * h.visited;
+    res_.moves += h.moves;
+    *moved_out = h.level_moved != 0;
     return Status::Ok();
   }
 

@@ -93,16 +93,28 @@ __global__ void __launch_bounds__(1024) ScanTileSumsKernel(uint64_t tiles, T* ti
   if (threadIdx.x == 1023 && total) *total = part[1023];
 }
 
+// raw: tile_sums holds the tiles' own sums, and every tile adds up the ones
+// before it (up to kScanRawTiles of them: 16 loads a thread) instead of a
+// kernel of its own between the two passes; the last one writes *total.
+constexpr uint64_t kScanRawTiles = 4096;
 template <class T, class F, class W>
-__global__ void __launch_bounds__(kScanThreads) ScanTileApplyKernel(uint64_t n, F f, const T* tile_sums, W w) {
+__global__ void __launch_bounds__(kScanThreads) ScanTileApplyKernel(uint64_t n, F f, const T* tile_sums, W w, int raw,
+                                                                   T* total_out) {
   __shared__ T vals[kScanTile];
   const uint64_t base = uint64_t(blockIdx.x) * kScanTile;
+  T before = 0;
+  if (raw) {
+    for (unsigned i = threadIdx.x; i < blockIdx.x; i += kScanThreads) before += tile_sums[i];
+  } else if (threadIdx.x == 0) {
+    before = tile_sums[blockIdx.x];
+  }
 #pragma unroll
   for (int j = 0; j < kScanItems; ++j) {
     const uint64_t i = base + uint64_t(j) * kScanThreads + threadIdx.x;
     vals[j * kScanThreads + threadIdx.x] = i < n ? f(i) : T(0);
   }
-  __syncthreads();
+  __shared__ T first;
+  BlockExclusiveScan<T>(before, &first);  // its barriers also complete vals
   T local[kScanItems];
   T acc = 0;
 #pragma unroll
@@ -111,7 +123,8 @@ __global__ void __launch_bounds__(kScanThreads) ScanTileApplyKernel(uint64_t n, 
     acc += local[j];
   }
   __shared__ T total;
-  T pre = BlockExclusiveScan<T>(acc, &total) + tile_sums[blockIdx.x];
+  T pre = BlockExclusiveScan<T>(acc, &total) + first;
+  if (raw && total_out && blockIdx.x + 1 == gridDim.x && threadIdx.x == 0) *total_out = first + total;
 #pragma unroll
   for (int j = 0; j < kScanItems; ++j) {
     const uint64_t i = base + uint64_t(threadIdx.x) * kScanItems + j;
@@ -120,7 +133,43 @@ __global__ void __launch_bounds__(kScanThreads) ScanTileApplyKernel(uint64_t n, 
   }
 }
 
+// A short scan (a few tiles) by one CTA.
+constexpr uint64_t kScanOneCta = 4 * kScanTile;
+template <class T, class F, class W>
+__global__ void __launch_bounds__(kScanThreads) ScanOneKernel(uint64_t n, F f, W w, T* total_out) {
+  __shared__ T vals[kScanTile];
+  __shared__ T total;
+  T run = 0;
+  for (uint64_t base = 0; base < n; base += kScanTile) {
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+      const uint64_t i = base + uint64_t(j) * kScanThreads + threadIdx.x;
+      vals[j * kScanThreads + threadIdx.x] = i < n ? f(i) : T(0);
+    }
+    __syncthreads();
+    T local[kScanItems];
+    T acc = 0;
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+      local[j] = vals[threadIdx.x * kScanItems + j];
+      acc += local[j];
+    }
+    T pre = BlockExclusiveScan<T>(acc, &total) + run;  // ends with a barrier
+    run += total;
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+      const uint64_t i = base + uint64_t(threadIdx.x) * kScanItems + j;
+      if (i < n) w(i, pre, local[j]);
+      pre += local[j];
+    }
+    __syncthreads();
+  }
+  if (total_out && threadIdx.x == 0) *total_out = run;
+}
+
 // Scratch for scans: tile sums.  `total` (device) receives the grand total.
+// One kernel up to 8,192 items, two up to 8.4M, else three: the short scans of
+// a small level cost their launches.
 template <class T, class F, class W>
 Status ScanApply(Context* ctx, uint64_t n, F f, W w, DBuf<T>& tile_buf, T* d_total) {
   const uint64_t tiles = (n + kScanTile - 1) / kScanTile;
@@ -128,10 +177,18 @@ Status ScanApply(Context* ctx, uint64_t n, F f, W w, DBuf<T>& tile_buf, T* d_tot
     if (d_total) PCC_CUDA(cudaMemsetAsync(d_total, 0, sizeof(T), ctx->stream));
     return Status::Ok();
   }
+  if (n <= kScanOneCta) {
+    ScanOneKernel<T, F, W><<<1, kScanThreads, 0, ctx->stream>>>(n, f, w, d_total); PCC_COUNT(1);
+    return LaunchCheck();
+  }
   PCC_RETURN_IF_ERROR(tile_buf.Reserve(ctx, tiles));
+  const int raw = tiles <= kScanRawTiles ? 1 : 0;
   ScanTileReduceKernel<T, F><<<unsigned(tiles), kScanThreads, 0, ctx->stream>>>(n, f, tile_buf.p); PCC_COUNT(1);
-  ScanTileSumsKernel<T><<<1, 1024, 0, ctx->stream>>>(tiles, tile_buf.p, d_total); PCC_COUNT(1);
-  ScanTileApplyKernel<T, F, W><<<unsigned(tiles), kScanThreads, 0, ctx->stream>>>(n, f, tile_buf.p, w); PCC_COUNT(1);
+  if (!raw) {
+    ScanTileSumsKernel<T><<<1, 1024, 0, ctx->stream>>>(tiles, tile_buf.p, d_total); PCC_COUNT(1);
+  }
+  ScanTileApplyKernel<T, F, W><<<unsigned(tiles), kScanThreads, 0, ctx->stream>>>(n, f, tile_buf.p, w, raw, d_total);
+  PCC_COUNT(1);
   return LaunchCheck();
 }
 
@@ -328,19 +385,25 @@ struct SortScratch {
   DBuf<uint32_t> tile_sums;
 };
 
-// Sorts keys[0..n) (with vals) by the low `bits` bits of the key; the
-// result is left in keys/vals.  n < 2^32.
-static inline Status RadixSortPairs(Context* ctx, uint64_t* keys, uint32_t* vals, uint64_t n, int bits,
-                             SortScratch& sc) {
+// The other buffers of a sort: n keys and values, SortHistWords(n) counters.
+struct SortBuffers {
+  uint64_t* keys;
+  uint32_t* vals;
+  uint32_t* hist;
+};
+inline uint64_t SortHistWords(uint64_t n) { return ((n + kSortTile - 1) / kSortTile) * 256; }
+
+// Sorts (*keys)[0..n) (with vals) by the low `bits` bits of the key, from one
+// buffer to the other pass by pass; *keys and *vals then point to the result.
+// n < 2^32.
+static inline Status RadixSortInto(Context* ctx, uint64_t** keys, uint32_t** vals, uint64_t n, int bits,
+                                   const SortBuffers& b, DBuf<uint32_t>& tile_sums) {
   if (n <= 1 || bits <= 0) return Status::Ok();
   const uint32_t tiles = uint32_t((n + kSortTile - 1) / kSortTile);
-  PCC_RETURN_IF_ERROR(sc.keys.Reserve(ctx, n));
-  PCC_RETURN_IF_ERROR(sc.vals.Reserve(ctx, n));
-  PCC_RETURN_IF_ERROR(sc.hist.Reserve(ctx, uint64_t(tiles) * 256));
-  uint64_t* kin = keys;
-  uint32_t* vin = vals;
-  uint64_t* kout = sc.keys.p;
-  uint32_t* vout = sc.vals.p;
+  uint64_t* kin = *keys;
+  uint32_t* vin = *vals;
+  uint64_t* kout = b.keys;
+  uint32_t* vout = b.vals;
   const int passes = (bits + 7) / 8;
   {
     static std::once_flag once;
@@ -353,18 +416,33 @@ static inline Status RadixSortPairs(Context* ctx, uint64_t* keys, uint32_t* vals
   }
   for (int p = 0; p < passes; ++p) {
     const int shift = p * 8;
-    RadixHistKernel<<<tiles, kSortThreads, 0, ctx->stream>>>(kin, n, shift, sc.hist.p, tiles); PCC_COUNT(1);
-    PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx, uint64_t(tiles) * 256, HistInput{sc.hist.p},
-                                            StorePrefix<uint32_t>{sc.hist.p}, sc.tile_sums,
+    RadixHistKernel<<<tiles, kSortThreads, 0, ctx->stream>>>(kin, n, shift, b.hist, tiles); PCC_COUNT(1);
+    PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx, uint64_t(tiles) * 256, HistInput{b.hist},
+                                            StorePrefix<uint32_t>{b.hist}, tile_sums,
                                             static_cast<uint32_t*>(nullptr)));
     RadixScatterKernel<<<tiles, kSortThreads, kSortScatterSmem, ctx->stream>>>(kin, vin, kout, vout, n, shift,
-                                                                               sc.hist.p, tiles); PCC_COUNT(1);
+                                                                               b.hist, tiles); PCC_COUNT(1);
     std::swap(kin, kout);
     std::swap(vin, vout);
   }
-  if (kin != keys) {
-    PCC_CUDA(cudaMemcpyAsync(keys, kin, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, ctx->stream));
-    PCC_CUDA(cudaMemcpyAsync(vals, vin, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, ctx->stream));
+  *keys = kin;
+  *vals = vin;
+  return LaunchCheck();
+}
+
+// The same with the result left in keys / vals.
+static inline Status RadixSortPairs(Context* ctx, uint64_t* keys, uint32_t* vals, uint64_t n, int bits,
+                             SortScratch& sc) {
+  if (n <= 1 || bits <= 0) return Status::Ok();
+  PCC_RETURN_IF_ERROR(sc.keys.Reserve(ctx, n));
+  PCC_RETURN_IF_ERROR(sc.vals.Reserve(ctx, n));
+  PCC_RETURN_IF_ERROR(sc.hist.Reserve(ctx, SortHistWords(n)));
+  uint64_t* k = keys;
+  uint32_t* v = vals;
+  PCC_RETURN_IF_ERROR(RadixSortInto(ctx, &k, &v, n, bits, SortBuffers{sc.keys.p, sc.vals.p, sc.hist.p}, sc.tile_sums));
+  if (k != keys) {
+    PCC_CUDA(cudaMemcpyAsync(keys, k, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, ctx->stream));
+    PCC_CUDA(cudaMemcpyAsync(vals, v, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, ctx->stream));
   }
   return LaunchCheck();
 }

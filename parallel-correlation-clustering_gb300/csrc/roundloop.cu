@@ -24,6 +24,8 @@
 // with an iteration limit after which the kernel reports kErrBarrier and
 // returns.
 #include <algorithm>
+#include <cstddef>
+#include <cstring>
 
 #include "certmoves.cuh"
 #include "hubeval.cuh"
@@ -150,10 +152,11 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
   __syncthreads();
 
   RoundView rv;
-  rv.stamp = l.rs->stamp + 1;
-  rv.front_val = l.rs->front_val;
-  rv.all = l.rs->front_all != 0;
-  unsigned long long front_edges = l.rs->front_edges, front_size = l.rs->front_size, visited = l.rs->visited;
+  const RoundState rs = l.st->head.rs;
+  rv.stamp = rs.stamp + 1;
+  rv.front_val = rs.front_val;
+  rv.all = rs.front_all != 0;
+  unsigned long long front_edges = rs.front_edges, front_size = rs.front_size, visited = rs.visited;
   const uint32_t n = a.n;
   uint32_t* count = &l.st->barrier;
   uint32_t arrivals = 0;
@@ -685,14 +688,14 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
     const unsigned long long E = all_move ? l.m : ctr->pend_edges;
     const bool next = F > 0;
     if (blockIdx.x == 0 && tid == 0) {
-      DevCounters* dc = a.ctr;
-      dc->rounds += 1;
-      dc->edge_visits += front_edges;
-      dc->vertex_visits += front_size;
-      dc->visited += visited;
-      dc->sync_moves += M;
-      if (next) dc->level_moved = 1;
-      l.rs->stamp = rv.stamp;
+      LoopHead& h = l.st->head;
+      h.rounds += 1;
+      h.edge_visits += front_edges;
+      h.vertex_visits += front_size;
+      h.visited += visited;
+      h.moves += M;
+      if (next) h.level_moved = 1;
+      h.rs.stamp = rv.stamp;
     }
     rv.front_val = rv.stamp;
     rv.all = all_move;
@@ -703,7 +706,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
     if (!next) break;
   }
   __syncthreads();
-  if (tid == 0 && !sh.ok) atomicExch(&a.ctr->error, kErrBarrier);
+  if (tid == 0 && !sh.ok) l.st->head.error = kErrBarrier;
   if (tid < kNumFamilies && sh.fam_v[tid]) {
     atomicAdd(&a.ctr->fam_entries[tid], sh.fam_e[tid]);
     atomicAdd(&a.ctr->fam_vertices[tid], sh.fam_v[tid]);
@@ -784,16 +787,32 @@ void SetLoopHubs(RoundLoopArgs* l, const HubPlan& plan, const HubState& st) {
   l->gdone = st.gdone.p;
 }
 
-Status LaunchRoundLoop(Context* ctx, RoundLoopArgs l, const SumMode& mode, const uint32_t* host_counts,
-                       uint32_t max_deg) {
+Status RunRoundLoop(Context* ctx, RoundLoopArgs l, const SumMode& mode, const uint32_t* host_counts,
+                    uint32_t max_deg, LoopHead* head) {
   // Table slots of a CTA: 16 warps x 256 or four teams x 2048 (which also
   // holds 16 warps x 512 and a hub of degree 4096).
   bool wide = max_deg > kHubMinDegree;
   for (int b = kBinW256; b <= kBinW1000; ++b) wide = wide || host_counts[b] > 0;
   l.table_slots = wide ? 2 * kHubSmallMax : 4096;
-  PCC_CUDA(cudaMemsetAsync(l.st, 0, offsetof(LoopState, zeros), ctx->stream));
-  if (!mode.narrow) return LaunchLoop<long long, true>(ctx, l);
-  return mode.conv ? LaunchLoop<int, true>(ctx, l) : LaunchLoop<int, false>(ctx, l);
+  constexpr size_t kSent = offsetof(LoopState, zeros);
+  static_assert(Context::kPinLoop + kSent <= Context::kPinnedBytes, "staging");
+  unsigned char* stage;
+  PCC_RETURN_IF_ERROR(ctx->Pinned(Context::kPinLoop, &stage));
+  std::memset(stage, 0, kSent);
+  std::memcpy(stage, head, sizeof(LoopHead));
+  PCC_CUDA(cudaMemcpyAsync(l.st, stage, kSent, cudaMemcpyHostToDevice, ctx->stream));
+  if (!mode.narrow) {
+    PCC_RETURN_IF_ERROR((LaunchLoop<long long, true>(ctx, l)));
+  } else if (mode.conv) {
+    PCC_RETURN_IF_ERROR((LaunchLoop<int, true>(ctx, l)));
+  } else {
+    PCC_RETURN_IF_ERROR((LaunchLoop<int, false>(ctx, l)));
+  }
+  PCC_CUDA(cudaMemcpyAsync(stage, l.st, sizeof(LoopHead), cudaMemcpyDeviceToHost, ctx->stream));
+  PCC_RETURN_IF_ERROR(Sync(ctx));
+  std::memcpy(head, stage, sizeof(LoopHead));
+  if (head->error) return MakeError(PCC_INTERNAL, "device error flag " + std::to_string(head->error));
+  return Status::Ok();
 }
 
 }  // namespace pcc

@@ -20,7 +20,17 @@ struct LoopCounters {
 // Device state of the kernel: the counter sets, the grid barrier and each
 // CTA's counts of empty ids and new movers in its slice of the vertices.
 constexpr uint32_t kLoopMaxCtas = 1024;
+// Sent before and read after a run (with the counters, zero at its start).
+struct LoopHead {
+  RoundState rs;             // in: stamp and the round-0 frontier; out: the last stamp
+  uint32_t level_moved;      // some round's next frontier was not empty
+  uint32_t rounds;
+  uint32_t error;            // kErrBarrier
+  uint32_t pad;
+  unsigned long long edge_visits, vertex_visits, visited, moves;
+};
 struct LoopState {
+  LoopHead head;
   LoopCounters ctr[3];
   uint32_t barrier;
   uint32_t pad;
@@ -45,7 +55,6 @@ struct RoundLoopArgs {
   uint32_t* zero_ids;
   uint32_t* new_list;
   float* Kf_mut;
-  RoundState* rs;           // in: stamp and the round-0 frontier; out: the last stamp
   LoopState* st;
   uint32_t table_slots;     // shared-memory table slots of a CTA
   // Hubs (degree > 1000): HubPlan and HubState.
@@ -84,8 +93,9 @@ inline bool RoundLoopFits(const Context* ctx, const DevGraph& g, const SumMode& 
 // Fills the hub fields from the level's plan and state.
 void SetLoopHubs(RoundLoopArgs* l, const HubPlan& plan, const HubState& st);
 
-// Launches the rounds on the context stream.  bins: host counts of `list`.
-Status LaunchRoundLoop(Context* ctx, RoundLoopArgs l, const SumMode& mode, const uint32_t* host_counts,
-                       uint32_t max_deg);
+// Runs the rounds and waits for them.  bins: host counts of `list`; *head: in
+// the round state, out the run's results.
+Status RunRoundLoop(Context* ctx, RoundLoopArgs l, const SumMode& mode, const uint32_t* host_counts,
+                    uint32_t max_deg, LoopHead* head);
 
 }  // namespace pcc
