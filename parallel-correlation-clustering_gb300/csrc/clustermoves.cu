@@ -17,13 +17,16 @@
 //   * the best D has the largest value, ties to the lowest id, and must
 //     beat `change` (staying); the cluster moves when the value is > 0 and
 //     c < D (the reference's id rule for simultaneous moves).
-// GB300 shape: the entries with C(u) != C(v) are keyed (rank C(v), rank
-// C(u)) in CSR order and stably radix-sorted, so each (c, D) run holds its
-// entries in the reference's summation order.  A run's sum is a sequential
-// FP64 fold (real weights) or warp-combined FP64 atomics (integral values,
-// exact in any order).  Every run's value is computed in parallel; the
-// per-cluster best is an atomic max over order-preserving bits, then an
-// atomic min of the id over the runs at that max.
+// GB300 shape: integral values sum exactly in any order, so every entry with
+// C(u) != C(v) adds to its (c, D) sum in one hash table of 1.5 m + 64 slots, and
+// nothing is sorted, compacted or waited for on the host.  Real weights keep
+// the reference's summation order: the entries are keyed (rank C(v), rank
+// C(u)) in CSR order and stably radix-sorted, and a run's sum is a sequential
+// FP64 fold.  Every sum's value is computed in parallel; the per-cluster best
+// is an atomic max over order-preserving bits, then an atomic min of the id
+// over the sums at that max.  (120,001 vertices and 1.9M
+// entries with integer weights, 20 rounds: 17.9 ms sorted, with three host
+// waits a round; 7.6 by the table, in a device-side loop.)
 #include <functional>
 
 #include "graphops.cuh"
@@ -149,7 +152,8 @@ __global__ void CmWeightKernel(uint32_t n, const uint32_t* __restrict__ C, const
     atomicAdd(&W[C[i]], k[i]);
 }
 
-__device__ __forceinline__ double HalfSquare(double x) { return __ddiv_rn(Dmul(x, x), 2.0); }
+// x * x / 2 (the halving is exact, as a product as well as a quotient).
+__device__ __forceinline__ double HalfSquare(double x) { return Dmul(Dmul(x, x), 0.5); }
 
 // change of BestMoveFromStats for a cluster of weight w (K_c its cluster
 // weight): the class-2 and class-1-together terms, both empty sums.
@@ -678,8 +682,217 @@ Status AsyncSetMoves(Context* ctx, const SetMoveArgs& a, const std::function<Sta
   return Sync(ctx);  // scratch buffers go out of scope
 }
 
+namespace {
+
+// Every entry that leaves its cluster adds float(w - offset), an integer here,
+// to its (C(v), C(u)) sum.  Bound by the two atomics an entry, each a round
+// trip to the die that holds the slot: 1.9M entries take 160 us from a cold
+// L2.  Integer sums, because FP64 conversions and adds run at 1/64 rate.
+struct CmTableInsert {
+  const uint32_t* nbr;
+  const float* w;
+  const uint32_t* C;
+  double offset;
+  uint64_t cap;
+  unsigned long long* keys;
+  unsigned long long* sums;
+  int* error;
+  __device__ void operator()(const uint32_t (&v)[kEdgeBatch], const uint64_t (&j)[kEdgeBatch]) const {
+    uint32_t cv[kEdgeBatch], cu[kEdgeBatch];
+    float wj[kEdgeBatch];
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k) {
+      cu[k] = v[k] != kNone ? nbr[j[k]] : kNone;
+      wj[k] = v[k] != kNone && w ? w[j[k]] : 1.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k) {
+      cv[k] = v[k] != kNone ? C[v[k]] : kNone;
+      cu[k] = v[k] != kNone ? C[cu[k]] : kNone;
+    }
+    unsigned long long key[kEdgeBatch];
+    uint64_t s[kEdgeBatch];
+    long long x[kEdgeBatch];
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k) {
+      // ~0: nothing to add.
+      key[k] = cv[k] == cu[k] ? ~0ull : (static_cast<unsigned long long>(cv[k]) << 32) | cu[k];
+      // The value is an integer below 2^53; FP64 only where there is an offset.
+      const float f = offset == 0.0 ? wj[k] : __double2float_rn(Dsub(static_cast<double>(wj[k]), offset));
+      x[k] = fabsf(f) < 1073741824.0f ? static_cast<long long>(__float2int_rn(f)) : __float2ll_rn(f);
+      // Lanes that hold the same sum (a row in few clusters, or a graph of few
+      // clusters, has many) add once.  Where the sums are few enough to queue
+      // up, two lanes that are alike sit side by side in some pair.
+      const unsigned long long other = __shfl_xor_sync(kFull, key[k], 1);
+      if (__any_sync(kFull, other == key[k] && key[k] != ~0ull)) {
+        const unsigned peers = __match_any_sync(kFull, key[k]);
+        if (key[k] != ~0ull && (peers & (peers - 1))) {
+          long long tot = 0;
+          for (unsigned mm = peers; mm; mm &= mm - 1) tot += __shfl_sync(peers, x[k], __ffs(mm) - 1);
+          x[k] = tot;
+          if (int(LaneId()) != __ffs(peers) - 1) key[k] = ~0ull;
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k) {
+      // MurmurHash3's 64-bit finalizer; its high bits pick the slot.
+      unsigned long long h = key[k];
+      h ^= h >> 33;
+      h *= 0xFF51AFD7ED558CCDull;
+      h ^= h >> 33;
+      h *= 0xC4CEB9FE1A85EC53ull;
+      h ^= h >> 33;
+      s[k] = __umul64hi(h, cap);
+    }
+    // The slot of each key, claimed if it is new: a probe of all entries at a
+    // time, so that their round trips overlap, without a look before the CAS
+    // (a look and a CAS are two trips to the slot's home die: 1% of the
+    // clustering); the lanes meet again before they add.
+    uint32_t todo = 0;
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k) todo |= key[k] != ~0ull ? 1u << k : 0u;
+    for (uint64_t probe = 0; __any_sync(kFull, todo); ++probe) {
+      unsigned long long seen[kEdgeBatch];
+#pragma unroll
+      for (int k = 0; k < kEdgeBatch; ++k)
+        if (todo >> k & 1) seen[k] = atomicCAS(keys + s[k], ~0ull, key[k]);
+#pragma unroll
+      for (int k = 0; k < kEdgeBatch; ++k)
+        if (todo >> k & 1) {
+          if (seen[k] == ~0ull || seen[k] == key[k]) todo &= ~(1u << k);
+          else s[k] = s[k] + 1 == cap ? 0 : s[k] + 1;
+        }
+      if (probe > cap) {  // cannot happen: 1.5 m + 64 slots
+        atomicExch(error, kErrHashFull);
+        return;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k)
+      if (key[k] != ~0ull) atomicAdd(sums + s[k], static_cast<unsigned long long>(x[k]));
+  }
+};
+
+struct CmTableArgs {
+  uint64_t cap;
+  unsigned long long* keys;
+  unsigned long long* sums;  // then the values' order bits
+  const double* W;
+  const double* K;
+  double res;
+  const double* stay;
+  unsigned long long* best_bits;
+  uint32_t* best_id;
+};
+
+__global__ void CmStayKernel(uint32_t n, const double* __restrict__ W, const double* __restrict__ K, double res,
+                             double* __restrict__ stay) {
+  for (uint64_t c = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; c < n; c += uint64_t(gridDim.x) * blockDim.x)
+    stay[c] = StayValue(res, W[c], K[c]);
+}
+
+// Every sum becomes its value(D); the max per cluster.
+__global__ void CmTableValueKernel(CmTableArgs a) {
+  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < a.cap;
+       i += uint64_t(gridDim.x) * blockDim.x) {
+    const unsigned long long key = a.keys[i];
+    if (key == ~0ull) continue;
+    const uint32_t c = static_cast<uint32_t>(key >> 32), d = static_cast<uint32_t>(key);
+    const double val =
+        Dadd(a.stay[c], Dsub(static_cast<double>(static_cast<long long>(a.sums[i])),
+                             Dmul(a.res, Dmul(a.W[c], Dsub(a.K[d], 0.0)))));
+    const unsigned long long o = OrdBits(val);
+    a.sums[i] = o;
+    if (o > __ldcg(a.best_bits + c)) atomicMax(&a.best_bits[c], o);
+  }
+}
+
+// Ties at the max go to the lowest cluster id; the table is emptied.
+__global__ void CmTableTieKernel(CmTableArgs a) {
+  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < a.cap;
+       i += uint64_t(gridDim.x) * blockDim.x) {
+    const unsigned long long key = a.keys[i];
+    if (key == ~0ull) continue;
+    const uint32_t c = static_cast<uint32_t>(key >> 32);
+    if (a.sums[i] == a.best_bits[c]) atomicMin(&a.best_id[c], static_cast<uint32_t>(key));
+    a.keys[i] = ~0ull;
+    a.sums[i] = 0;
+  }
+}
+
+// CmDecideKernel with the staying values at hand; the per-cluster results are
+// reset for the next round.
+__global__ void CmTableDecideKernel(uint32_t n, uint32_t* __restrict__ best_id,
+                                    unsigned long long* __restrict__ best_bits, const double* __restrict__ stay,
+                                    uint32_t* __restrict__ cmove) {
+  for (uint64_t c = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; c < n; c += uint64_t(gridDim.x) * blockDim.x) {
+    const uint32_t d = best_id[c];
+    uint32_t move = kNone;
+    if (d != kNone) {
+      const double change = stay[c];
+      const double bv = FromOrd(best_bits[c]);
+      uint32_t target = n;
+      double val = change;
+      if (bv > change) {
+        target = d;
+        val = bv;
+      }
+      if (target < n && c >= target) val = 0.0;
+      if (val > 0) move = target;
+      best_id[c] = kNone;
+      best_bits[c] = 0;
+    }
+    cmove[c] = move;
+  }
+}
+
+}  // namespace
+
+Status AllocClusterMoveTable(Context* ctx, const DevGraph& g, ClusterMoveTable* t) {
+  // A device short of 24 bytes an entry has the sorted path.
+  const uint64_t cap = g.m + g.m / 2 + 64;
+  if (!t->keys.Alloc(ctx, cap).ok() || !t->sums.Alloc(ctx, cap).ok()) {
+    t->keys.Release();
+    t->sums.Release();
+    return Status::Ok();
+  }
+  t->cap = cap;
+  PCC_RETURN_IF_ERROR(t->best_bits.Alloc(ctx, g.n));
+  PCC_RETURN_IF_ERROR(t->best_id.Alloc(ctx, g.n));
+  PCC_RETURN_IF_ERROR(t->cmove.Alloc(ctx, g.n));
+  PCC_RETURN_IF_ERROR(t->W.Alloc(ctx, g.n));
+  PCC_RETURN_IF_ERROR(t->stay.Alloc(ctx, g.n));
+  PCC_RETURN_IF_ERROR(t->keys.Fill(0xFF));
+  PCC_RETURN_IF_ERROR(t->sums.Zero());
+  PCC_RETURN_IF_ERROR(t->best_bits.Zero());
+  return t->best_id.Fill(0xFF);
+}
+
+Status FindClusterMovesExact(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k, const double* K,
+                             double res, double offset, ClusterMoveTable* t, uint32_t* moves, uint32_t* movers,
+                             DevCounters* ctr) {
+  const uint32_t n = g.n;
+  cudaStream_t st = ctx->stream;
+  const unsigned grid_n = Blocks(n, 256, ctx->num_sms * 8);
+  PCC_RETURN_IF_ERROR(t->W.Zero());
+  CmWeightKernel<<<grid_n, 256, 0, st>>>(n, C, k, t->W.p);
+  CmStayKernel<<<grid_n, 256, 0, st>>>(n, t->W.p, K, res, t->stay.p);
+  PCC_COUNT(2);
+  LaunchEdgeBatch(ctx, g.bins, g.off.p,
+                  CmTableInsert{g.nbr.p, g.wp(), C, offset, t->cap, t->keys.p, t->sums.p, &ctr->error});
+  const CmTableArgs a{t->cap, t->keys.p, t->sums.p, t->W.p, K, res, t->stay.p, t->best_bits.p, t->best_id.p};
+  const unsigned grid_t = Blocks(t->cap, 256 * 4, ctx->num_sms * 8);
+  CmTableValueKernel<<<grid_t, 256, 0, st>>>(a);
+  CmTableTieKernel<<<grid_t, 256, 0, st>>>(a);
+  CmTableDecideKernel<<<grid_n, 256, 0, st>>>(n, t->best_id.p, t->best_bits.p, t->stay.p, t->cmove.p);
+  CmMoversKernel<<<grid_n, 256, 0, st>>>(n, C, t->cmove.p, moves, movers, ctr);
+  PCC_COUNT(4);
+  return LaunchCheck();
+}
+
 Status FindClusterMoves(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k, const double* K,
-                        double res, double offset, bool exact_sums, uint32_t* moves, uint32_t* movers,
+                        double res, double offset, uint32_t* moves, uint32_t* movers,
                         DevCounters* ctr) {
   const uint32_t n = g.n;
   if (n == 0 || g.m == 0) return Status::Ok();
@@ -732,11 +945,10 @@ Status FindClusterMoves(Context* ctx, const DevGraph& g, const uint32_t* C, cons
   }
 
   // Runs of equal (c, D) and their sums.
-  DBuf<uint32_t> run_start, run_of, counts;
+  DBuf<uint32_t> run_start, counts;
   PCC_RETURN_IF_ERROR(run_start.Alloc(ctx, uint64_t(M) + 1));
-  if (exact_sums) PCC_RETURN_IF_ERROR(run_of.Alloc(ctx, M));
   PCC_RETURN_IF_ERROR(counts.Alloc(ctx, 1));
-  PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx, M, CmRunHead{keys.p}, CmRunWriter{run_start.p, run_of.p}, scan_tiles,
+  PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx, M, CmRunHead{keys.p}, CmRunWriter{run_start.p, nullptr}, scan_tiles,
                                           counts.p));
   uint32_t nruns = 0;
   PCC_RETURN_IF_ERROR(counts.ToHost(&nruns, 1));
@@ -746,13 +958,7 @@ Status FindClusterMoves(Context* ctx, const DevGraph& g, const uint32_t* C, cons
   DBuf<double> run_sum;
   PCC_RETURN_IF_ERROR(run_sum.Alloc(ctx, nruns));
   const unsigned grid_runs = Blocks(nruns, 256, ctx->num_sms * 16);
-  if (exact_sums) {
-    PCC_RETURN_IF_ERROR(run_sum.Zero());
-    CmRunAtomicKernel<<<Blocks(M, 256, ctx->num_sms * 16), 256, 0, st>>>(M, run_of.p, vals.p, run_sum.p);
-    PCC_COUNT(1);
-  } else {
-    CmRunFoldKernel<<<grid_runs, 256, 0, st>>>(counts.p, run_start.p, vals.p, run_sum.p); PCC_COUNT(1);
-  }
+  CmRunFoldKernel<<<grid_runs, 256, 0, st>>>(counts.p, run_start.p, vals.p, run_sum.p); PCC_COUNT(1);
 
   // Cluster weights, run values, and the decisions.
   DBuf<double> W, run_val;

@@ -201,7 +201,7 @@ struct DevCounters {
   uint32_t frontier;        // vertices in the frontier being built
   uint32_t movers;          // real movers of this round
   uint32_t new_movers;      // movers to a new cluster
-  uint32_t marked;          // vertices marked for the next frontier
+  uint32_t marked;          // the vertex movers of a round with whole-cluster moves
   uint32_t level_moved;     // OR over rounds of "next frontier non-empty"
   uint32_t rounds;          // best-move rounds executed
   uint32_t present;         // generic count used by compaction steps
@@ -332,6 +332,17 @@ inline void SetSumMode(BMArgs* a, const SumMode& m) {
   }
   a->res32 = FilterF32(a->res * static_cast<double>(a->wscale));
 }
+
+// Whole-cluster moves with exact sums (FindClusterMovesExact, clustermoves.cu):
+// the table of (c, D) sums and per-cluster results, clean between rounds.
+struct ClusterMoveTable {
+  uint64_t cap = 0;
+  DBuf<unsigned long long> keys;       // c << 32 | D, all ones: empty
+  DBuf<unsigned long long> sums;       // integers, in two's complement
+  DBuf<unsigned long long> best_bits;  // per cluster id
+  DBuf<uint32_t> best_id, cmove;
+  DBuf<double> W, stay;
+};
 
 // Asynchronous whole-cluster moves (AsyncSetMoves, clustermoves.cu).
 struct SetMoveArgs {

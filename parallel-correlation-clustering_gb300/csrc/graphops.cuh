@@ -153,14 +153,145 @@ inline void LaunchEdgeIter(Context* ctx, const uint32_t* list, const uint32_t* c
 }
 
 // ---------------------------------------------------------------------------
+// The same walk with kEdgeBatch entries of a lane at a time: f(v, j) gets
+// arrays of kEdgeBatch rows and entries (rows kNone where there is none) with
+// every lane of the warp converged, so that it can issue all its loads before
+// it stores and can combine over the warp.
+// ---------------------------------------------------------------------------
+constexpr int kEdgeBatch = 4;
+
+template <class F, class R>
+__global__ void __launch_bounds__(kIterThreads) EdgeBatchSmallKernel(const uint32_t* __restrict__ list,
+                                                                    const uint32_t* __restrict__ starts,
+                                                                    const uint64_t* __restrict__ off, F f, R row) {
+  __shared__ uint32_t incl[kIterThreads / 32][32];
+  __shared__ uint64_t begin[kIterThreads / 32][32];
+  __shared__ uint32_t vert[kIterThreads / 32][32];
+  const uint32_t s0 = starts[kBinG4];
+  const uint32_t count = starts[kBinW128] - s0;  // bins G4..G32 are contiguous
+  const unsigned lane = LaneId(), warp = threadIdx.x >> 5;
+  for (uint64_t i0 = (uint64_t(blockIdx.x) * (kIterThreads / 32) + warp) * 32; i0 < count;
+       i0 += uint64_t(gridDim.x) * kIterThreads) {
+    const uint64_t i = i0 + lane;
+    uint32_t d = 0, vl = 0;
+    uint64_t b = 0;
+    if (i < count) {
+      vl = list[s0 + i];
+      if (row(vl)) {
+        b = off[vl];
+        d = static_cast<uint32_t>(off[vl + 1] - b);
+      }
+    }
+    const uint32_t inc = WarpInclusiveScan<uint32_t>(d);
+    incl[warp][lane] = inc;
+    begin[warp][lane] = b - (inc - d);  // of the entry e of the 32 rows: begin + e
+    vert[warp][lane] = vl;
+    const uint32_t total = __shfl_sync(kFull, inc, 31);
+    __syncwarp();
+    for (uint32_t e0 = 0; e0 < total; e0 += 32 * kEdgeBatch) {
+      uint32_t v[kEdgeBatch];
+      uint64_t j[kEdgeBatch];
+#pragma unroll
+      for (int k = 0; k < kEdgeBatch; ++k) {
+        const uint32_t e = e0 + 32 * k + lane;
+        int r = 0;
+#pragma unroll
+        for (int step = 16; step; step >>= 1)
+          if (incl[warp][r + step - 1] <= e) r += step;
+        v[k] = e < total ? vert[warp][r & 31] : kNone;
+        j[k] = begin[warp][r & 31] + e;
+      }
+      f(v, j);
+    }
+    __syncwarp();
+  }
+}
+
+template <class F, class R>
+__global__ void __launch_bounds__(kIterThreads) EdgeBatchMidKernel(const uint32_t* __restrict__ list,
+                                                                  const uint32_t* __restrict__ starts,
+                                                                  const uint64_t* __restrict__ off, F f, R row) {
+  const uint32_t s0 = starts[kBinW128];
+  const uint32_t count = starts[kBinCta] - s0;  // bins W128..W1000
+  const unsigned lane = LaneId(), warp = threadIdx.x >> 5;
+  for (uint64_t i = uint64_t(blockIdx.x) * (kIterThreads / 32) + warp; i < count;
+       i += uint64_t(gridDim.x) * (kIterThreads / 32)) {
+    const uint32_t vr = list[s0 + i];
+    if (!row(vr)) continue;
+    const uint64_t b = off[vr], e = off[vr + 1];
+    for (uint64_t j0 = b; j0 < e; j0 += 32 * kEdgeBatch) {
+      uint32_t v[kEdgeBatch];
+      uint64_t j[kEdgeBatch];
+#pragma unroll
+      for (int k = 0; k < kEdgeBatch; ++k) {
+        j[k] = j0 + 32 * k + lane;
+        v[k] = j[k] < e ? vr : kNone;
+      }
+      f(v, j);
+    }
+  }
+}
+
+template <class F, class R>
+__global__ void __launch_bounds__(kIterBigThreads) EdgeBatchBigKernel(const uint32_t* __restrict__ list,
+                                                                     const uint32_t* __restrict__ starts,
+                                                                     const uint64_t* __restrict__ off, F f, R row) {
+  const uint32_t s0 = starts[kBinCta];
+  const uint32_t count = starts[kNumBins] - s0;  // bins Cta, Global
+  for (uint64_t i = blockIdx.x; i < count; i += gridDim.x) {
+    const uint32_t vr = list[s0 + i];
+    if (!row(vr)) continue;
+    const uint64_t b = off[vr], e = off[vr + 1];
+    for (uint64_t j0 = b; j0 < e; j0 += uint64_t(kIterBigThreads) * kEdgeBatch) {
+      uint32_t v[kEdgeBatch];
+      uint64_t j[kEdgeBatch];
+#pragma unroll
+      for (int k = 0; k < kEdgeBatch; ++k) {
+        j[k] = j0 + uint64_t(kIterBigThreads) * k + threadIdx.x;
+        v[k] = j[k] < e ? vr : kNone;
+      }
+      f(v, j);
+    }
+  }
+}
+
+template <class F, class R = RowAll>
+inline void LaunchEdgeBatch(Context* ctx, const BinSet& bins, const uint64_t* off, F f, R row = R()) {
+  auto any = [&](int b0, int b1) {
+    for (int b = b0; b < b1; ++b)
+      if (bins.host_counts[b]) return true;
+    return false;
+  };
+  const uint32_t *list = bins.list.p, *starts = bins.counts.p + kNumBins;
+  cudaStream_t st = ctx->stream;
+  if (any(kBinG4, kBinW128)) {
+    EdgeBatchSmallKernel<F, R><<<IterSmallGrid(ctx), kIterThreads, 0, st>>>(list, starts, off, f, row);
+    PCC_COUNT(1);
+  }
+  if (any(kBinW128, kBinCta)) {
+    EdgeBatchMidKernel<F, R><<<IterMidGrid(ctx), kIterThreads, 0, st>>>(list, starts, off, f, row);
+    PCC_COUNT(1);
+  }
+  if (any(kBinCta, kNumBins)) {
+    EdgeBatchBigKernel<F, R><<<IterBigGrid(ctx), kIterBigThreads, 0, st>>>(list, starts, off, f, row);
+    PCC_COUNT(1);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Frontier push (gbbs edgeMap with an always-true update): stamp[u] = value
 // for every neighbour u of a row passing `row`.  The mid and big shapes load
 // kPushBatch neighbour ids per thread before storing any stamp: through the
 // generic functor the compiler must assume a store may alias the next id and
-// keeps one load in flight.  Small rows use EdgeIterSmallKernel.  A stamp
+// keeps one load in flight.  Small rows use EdgeBatchSmallKernel.  A stamp
 // already equal to the value is not stored again: hub vertices are
 // neighbours of a large share of all rows, and same-address stores
-// serialise at their L2 slice while the loads are served by L1.
+// serialise at their L2 slice while the loads are served by L1.  Without hubs
+// (`blind`) small rows store without a look: the look at a line that other
+// SMs write makes it travel between the dies (120,001 vertices, 1.9M entries:
+// 43 us with it, 24 without).  The line is 4,096 entries a vertex, as many
+// stores as can queue at one address: an RMAT graph of scale 22 takes the same
+// time either way, and a star's leaves would all queue at its centre.
 // ---------------------------------------------------------------------------
 constexpr int kPushBatch = 8;
 
@@ -235,9 +366,17 @@ struct PushStampFn {
   const uint32_t* nbr;
   uint32_t* stamp;
   StampValue sv;
-  __device__ void operator()(uint32_t, uint64_t j, uint64_t) const {
-    const uint32_t u = nbr[j], value = StampIn(sv.rs, sv.stamp);
-    if (stamp[u] != value) stamp[u] = value;
+  bool blind;
+  __device__ void operator()(const uint32_t (&v)[kEdgeBatch], const uint64_t (&j)[kEdgeBatch]) const {
+    const uint32_t value = StampIn(sv.rs, sv.stamp);
+    uint32_t u[kEdgeBatch], cur[kEdgeBatch];
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k) u[k] = v[k] != kNone ? nbr[j[k]] : kNone;
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k) cur[k] = u[k] == kNone ? value : blind ? ~value : stamp[u[k]];
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k)
+      if (cur[k] != value) stamp[u[k]] = value;
   }
 };
 
@@ -246,7 +385,7 @@ struct PushStampFn {
 template <class R>
 inline void LaunchPush(Context* ctx, const uint32_t* list, const uint32_t* counts, const uint32_t* starts,
                        const uint32_t* host_counts, const uint64_t* off, const uint32_t* nbr, uint32_t* stamp,
-                       StampValue sv, R row) {
+                       StampValue sv, bool blind, R row) {
   auto any = [&](int b0, int b1) {
     if (!host_counts) return true;
     for (int b = b0; b < b1; ++b)
@@ -255,8 +394,8 @@ inline void LaunchPush(Context* ctx, const uint32_t* list, const uint32_t* count
   };
   cudaStream_t st = ctx->stream;
   if (any(kBinG4, kBinW128)) {
-    EdgeIterSmallKernel<PushStampFn, R><<<IterSmallGrid(ctx), kIterThreads, 0, st>>>(
-        list, counts, starts, off, PushStampFn{nbr, stamp, sv}, row);
+    EdgeBatchSmallKernel<PushStampFn, R><<<IterSmallGrid(ctx), kIterThreads, 0, st>>>(
+        list, starts, off, PushStampFn{nbr, stamp, sv, blind}, row);
     PCC_COUNT(1);
   }
   if (any(kBinW128, kBinCta)) {

@@ -27,8 +27,11 @@ namespace pcc {
 Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k,
                      std::unique_ptr<DevGraph>* out);
 Status FindClusterMoves(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k, const double* K,
-                        double res, double offset, bool exact_sums, uint32_t* moves, uint32_t* movers,
-                        DevCounters* ctr);
+                        double res, double offset, uint32_t* moves, uint32_t* movers, DevCounters* ctr);
+Status AllocClusterMoveTable(Context* ctx, const DevGraph& g, ClusterMoveTable* t);
+Status FindClusterMovesExact(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k, const double* K,
+                             double res, double offset, ClusterMoveTable* t, uint32_t* moves, uint32_t* movers,
+                             DevCounters* ctr);
 Status AsyncSetMoves(Context* ctx, const SetMoveArgs& a, const std::function<Status(uint32_t)>& vertex_moves);
 Status ComputeSubclustersDevice(Context* ctx, const DevGraph& g, const uint32_t* C, int method, double res,
                                 double offset, DBuf<uint32_t>* sub, DBuf<uint64_t>* next, uint32_t* num_clusters,
@@ -295,6 +298,14 @@ __global__ void __launch_bounds__(kT) ApplyJoinKernel(ApplyArgs a) {
     }
     if (in) a.C[v] = t;
   }
+}
+
+// The round's vertex movers are applied: their count goes to `marked`, and the
+// whole-cluster movers are counted from zero.
+__global__ void SpendMoversKernel(DevCounters* ctr) {
+  ctr->marked = ctr->movers;
+  ctr->movers = 0;
+  ctr->new_movers = 0;
 }
 
 // Gated inputs for the new-cluster compactions: nothing to do when no
@@ -591,7 +602,7 @@ __global__ void RoundEndKernel(RoundState* rs, DevCounters* ctr, cudaGraphCondit
   ctr->edge_visits += rs->front_edges;
   ctr->vertex_visits += rs->front_size;
   ctr->visited += rs->visited;
-  ctr->sync_moves += ctr->movers;
+  ctr->sync_moves += ctr->movers + ctr->marked;  // marked: before whole-cluster moves
   bool next;
   if (all_move) {
     next = n > 0;
@@ -902,7 +913,7 @@ class Engine {
         PCC_COUNT(1);
       }
       PCC_RETURN_IF_ERROR(LaunchCheck());
-      if (cfg_.clustering_moves_method == PCC_DEFAULT_CLUSTER_MOVES) PCC_RETURN_IF_ERROR(WholeClusterMoves(L));
+      if (cfg_.clustering_moves_method == PCC_DEFAULT_CLUSTER_MOVES) PCC_RETURN_IF_ERROR(WholeClusterMoves(L, rs));
     } else if (cfg_.clustering_moves_method == PCC_DEFAULT_CLUSTER_MOVES) {
       PCC_RETURN_IF_ERROR(AsyncWholeClusterMoves(L, a));
     }
@@ -915,10 +926,10 @@ class Engine {
     const StampValue sv{stamp_, rs};
     if (cfg_.move_method == PCC_NBHR_CLUSTER_MOVE) {
       LaunchPush(ctx_, g.bins.list.p, g.bins.counts.p, g.bins.counts.p + kNumBins, g.bins.host_counts, g.off.p,
-                 g.nbr.p, next_stamp_.p, sv, PredModifiedCluster{L->C.p, mod_stamp_.p, stamp_, rs});  // rows with d > 0
+                 g.nbr.p, next_stamp_.p, sv, g.max_deg <= 4096, PredModifiedCluster{L->C.p, mod_stamp_.p, stamp_, rs});  // rows with d > 0
     } else {
       LaunchPush(ctx_, g.bins.list.p, g.bins.counts.p, g.bins.counts.p + kNumBins, g.bins.host_counts, g.off.p,
-                 g.nbr.p, next_stamp_.p, sv, PredStamp{moved_stamp_.p, stamp_, rs});
+                 g.nbr.p, next_stamp_.p, sv, g.max_deg <= 4096, PredStamp{moved_stamp_.p, stamp_, rs});
     }
     if (n) {
       CountDegreesKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, g.off.p, PredStamp{next_stamp_.p, stamp_, rs},
@@ -988,41 +999,49 @@ class Engine {
     return st;
   }
 
+  // The table of whole-cluster moves for synchronous rounds over g, where
+  // integral entry values whose every partial sum stays below 2^53 sum exactly
+  // in any order.
+  Status PrepareClusterMoves(const Level& L) {
+    const DevGraph& g = *L.g;
+    if (cm_table_.keys.p || cfg_.async || g.n == 0 || g.m == 0 || !L.mode.exact || L.mode.conv) return Status::Ok();
+    const double most = static_cast<double>(g.m) * (g.max_abs_w + std::fabs(cfg_.edge_weight_offset));
+    return most < 9007199254740992.0 ? AllocClusterMoveTable(ctx_, g, &cm_table_) : Status::Ok();
+  }
+
   // Whole-cluster moves after the round's vertex moves (DEFAULT_CLUSTER_MOVES,
   // parallel-correlation-clusterer.cc:167-297): the moving clusters'
   // members go through the same apply as vertex movers, and the clusters it
   // modifies carry this round's stamp, so the NBHR_CLUSTER_MOVE frontier
-  // sees them (moved_clusters |= additional_moved_clusters).  Host-driven
-  // rounds only (the step reads sizes on the host).
-  Status WholeClusterMoves(Level* L) {
+  // sees them (moved_clusters |= additional_moved_clusters).  rs as in
+  // EnqueueRound: with the table (cm_table_) nothing is read on the host;
+  // without it only host-driven rounds come here.
+  Status WholeClusterMoves(Level* L, const RoundState* rs) {
     const DevGraph& g = *L->g;
     const uint32_t n = g.n;
-    DevCounters hc;
-    PCC_RETURN_IF_ERROR(ctr_.ToHost(&hc, 1));
-    PCC_RETURN_IF_ERROR(Sync(ctx_));
-    res_.moves += hc.movers;  // the vertex movers; the caller adds the cluster movers
-    PCC_CUDA(cudaMemsetAsync(&ctr_.p->movers, 0, sizeof(uint32_t), ctx_->stream));
-    PCC_CUDA(cudaMemsetAsync(&ctr_.p->new_movers, 0, sizeof(uint32_t), ctx_->stream));
+    // The vertex movers are kept in `marked` (the caller adds both counts).
+    SpendMoversKernel<<<1, 1, 0, ctx_->stream>>>(ctr_.p); PCC_COUNT(1);
     // The vertex movers' new-cluster marks of this round are spent (0 is no stamp).
     PCC_CUDA(cudaMemsetAsync(new_stamp_.p, 0, sizeof(uint32_t) * n, ctx_->stream));
-    // Integral entry values whose every partial sum stays below 2^53 sum
-    // exactly in any order.
-    const bool exact = L->mode.exact && !L->mode.conv && static_cast<double>(g.m) * (g.max_abs_w + std::fabs(cfg_.edge_weight_offset)) <
-                                          9007199254740992.0;
-    PCC_RETURN_IF_ERROR(FindClusterMoves(ctx_, g, L->C.p, L->k.p, L->K.p, cfg_.resolution, cfg_.edge_weight_offset,
-                                         exact, moves_.p, movers_.p, ctr_.p));
+    if (cm_table_.keys.p) {
+      PCC_RETURN_IF_ERROR(FindClusterMovesExact(ctx_, g, L->C.p, L->k.p, L->K.p, cfg_.resolution,
+                                                cfg_.edge_weight_offset, &cm_table_, moves_.p, movers_.p, ctr_.p));
+    } else {
+      PCC_RETURN_IF_ERROR(FindClusterMoves(ctx_, g, L->C.p, L->k.p, L->K.p, cfg_.resolution,
+                                           cfg_.edge_weight_offset, moves_.p, movers_.p, ctr_.p));
+    }
     ApplyArgs ap{n, L->C.p, L->s.p, L->k.p, L->K.p, moves_.p, movers_.p, mod_stamp_.p, new_stamp_.p, stamp_,
-                 ctr_.p, nullptr};
+                 ctr_.p, rs};
     const unsigned grid = GridFor(ctx_, n);
     ApplyLeaveKernel<<<grid, kT, 0, ctx_->stream>>>(ap); PCC_COUNT(1);
     ApplyJoinKernel<<<grid, kT, 0, ctx_->stream>>>(ap); PCC_COUNT(1);
     PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx_, n, ZeroSizeInput{L->s.p, ctr_.p}, StoreIndexIfSet{zero_ids_.p},
                                             scan_tiles_, static_cast<uint32_t*>(nullptr)));
-    PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx_, n, NewMoverInput{new_stamp_.p, stamp_, ctr_.p, nullptr},
+    PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx_, n, NewMoverInput{new_stamp_.p, stamp_, ctr_.p, rs},
                                             StoreIndexIfSet{new_list_.p}, scan_tiles_,
                                             static_cast<uint32_t*>(nullptr)));
     AssignNewKernel<<<grid, kT, 0, ctx_->stream>>>(ap, zero_ids_.p, new_list_.p); PCC_COUNT(1);
-    RefreshKfKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, L->K.p, L->Kf.p, mod_stamp_.p, stamp_, nullptr);
+    RefreshKfKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, L->K.p, L->Kf.p, mod_stamp_.p, stamp_, rs);
     PCC_COUNT(1);
     return LaunchCheck();
   }
@@ -1098,7 +1117,7 @@ class Engine {
       PCC_RETURN_IF_ERROR(gedges_.ToHost(h_gedges_.data(), un_->B));
     }
     PCC_RETURN_IF_ERROR(Sync(ctx_));
-    if (!cfg_.async) res_.moves += hc.movers;
+    if (!cfg_.async) res_.moves += hc.movers + hc.marked;  // marked: before whole-cluster moves
     if (cfg_.move_method == PCC_ALL_MOVE) {
       *next_nonempty = n > 0;
       *next_front_stamp = 0;
@@ -1294,8 +1313,10 @@ class Engine {
     if (!cfg_.async && !un_ && !ctx_->detailed_timing && !ctx_->tuned && ctx_->overlap_families && num_inner > 0 &&
         cfg_.clustering_moves_method == PCC_LOUVAIN && RoundLoopFits(ctx_, *L->g, L->mode))
       return IterateLoop(L, num_inner, moved_out);
+    if (cfg_.clustering_moves_method == PCC_DEFAULT_CLUSTER_MOVES) PCC_RETURN_IF_ERROR(PrepareClusterMoves(*L));
     if (!cfg_.async && !un_ && !ctx_->detailed_timing && !ctx_->graphs_failed &&
-        cfg_.clustering_moves_method == PCC_LOUVAIN && L->g->m >= ctx_->device_loop_min_entries)
+        (cfg_.clustering_moves_method == PCC_LOUVAIN || cm_table_.keys.p) &&
+        L->g->m >= ctx_->device_loop_min_entries)
       return IterateDevice(L, num_inner, moved_out);
     return IterateBestMoves(L, num_inner, moved_out);
   }
@@ -1800,6 +1821,7 @@ class Engine {
   uint32_t sm_val_ = 0;
   DBuf<uint32_t> scan_tiles_;
   HubState hub_state_;
+  ClusterMoveTable cm_table_;  // whole-cluster moves
   DBuf<LoopState> loop_state_;  // one-kernel round loop
   DBuf<uint32_t> old_cluster_;
   DBuf<DevCounters> ctr_;

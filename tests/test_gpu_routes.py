@@ -180,3 +180,32 @@ def test_one_kernel_rounds_given_labels(ctx):
             np.testing.assert_array_equal(lab, want)
             assert (st["rounds"], st["edge_visits"]) == (so["rounds"], so["edge_visits"])
         dg.free()
+
+
+@pytest.mark.parametrize("name", ["two", "cliques33", "clique1002", "hubby", "star9000", "rmat15"])
+@pytest.mark.parametrize("weights", ["unit", "integer"])
+def test_whole_cluster_moves_table(ctx, name, weights):
+    """Whole-cluster moves summed in the (cluster, cluster) table, rounds on
+    the device and driven by the host: singletons (every sum one entry), given
+    labels of few clusters (few sums, many entries), negative values."""
+    g = LOOP_GRAPHS[name]()
+    if weights == "integer":
+        g = _weighted(g, lambda a, b: (a * 7 + b * 13) % 5 + 1)
+    dg, og = ctx.upload(g), O.OracleGraph(g)
+    rng = np.random.default_rng(4)
+    for res, offset, move, groups in ((0.02, 0.0, P.NBHR_CLUSTER_MOVE, 0), (0.5, 2.0, P.NBHR_MOVE, 3),
+                                      (0.1, 0.0, P.ALL_MOVE, 40)):
+        init = rng.integers(0, min(groups, g.n), g.n).astype(np.uint32) if groups else None
+        cfg = P.make_config(resolution=res, edge_weight_offset=offset, move_method=move, num_iterations=6,
+                            clustering_moves_method=P.DEFAULT_CLUSTER_MOVES)
+        want, so = O.correlation_cluster(og, cfg, None, init)
+        for detailed in (False, True):
+            ctx.set_detailed_timing(detailed)
+            try:
+                lab, st = P.correlation_cluster(dg, cfg, None, init)
+            finally:
+                ctx.set_detailed_timing(False)
+            np.testing.assert_array_equal(lab, want)
+            for key in ("edge_visits", "rounds", "levels", "moves"):
+                assert st[key] == so[key], key
+    dg.free()
