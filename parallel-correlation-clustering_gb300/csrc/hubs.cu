@@ -10,6 +10,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "certmoves.cuh"
 #include "hubeval.cuh"
 
 namespace pcc {
@@ -108,6 +109,56 @@ __global__ void __launch_bounds__(kSmallThreads) HubSmallKernel(HubArgs h) {
     EvalTable<BT, kInt, kAsync, V>(a, x, a.kf[v], change, smax, skeys, svals, cap, sh, &bv, &bi);
     if (tid == 0) HubDecide<kAsync>(a, x, bv, bi, change, StampIn(a.rs, a.stamp), &a.ctr->movers);
     __syncthreads();
+  }
+  if (tid == 0 && fam_v) {
+    atomicAdd(&a.ctr->fam_entries[kFamHubSmall], fam_e);
+    atomicAdd(&a.ctr->fam_vertices[kFamHubSmall], fam_v);
+  }
+}
+
+// Small hubs with exact sums, synchronous moves: a CTA of TW warps takes a hub
+// the way the warp rows go (CtaStep, certmoves.cuh): certified FP32 decisions
+// over the used slots instead of HubSmallKernel's evaluation of every slot of
+// the table.  Two table sizes: HC = 4096 slots with 8 warps, 8192 with 16, so
+// that 48 warps of 32-bit sums fit an SM with either.  Bound by the gathers of
+// the neighbours' clusters and shared-memory atomics.  (All rounds of RMAT
+// scale 20: 34.9 ms by HubSmallKernel, 14.9; scale 22: 28.1, 22.0; 1M vertices
+// with real weights, 64-bit sums: 39.6, 20.6.)
+template <int HC, int TW, typename V>
+__host__ __device__ constexpr size_t HubCertSmem() {
+  return size_t(HC) * (sizeof(V) + sizeof(uint32_t)) + size_t(HC / 2) * sizeof(uint16_t);  // vals, keys, used
+}
+
+template <int HC, int TW, typename V, bool kConv>
+__global__ void __launch_bounds__(TW * 32) HubCertKernel(HubArgs h) {
+  constexpr int BT = TW * 32;
+  extern __shared__ __align__(16) unsigned char smem[];
+  V* vals = reinterpret_cast<V*>(smem);
+  uint32_t* keys = reinterpret_cast<uint32_t*>(smem + size_t(HC) * sizeof(V));
+  uint16_t* used = reinterpret_cast<uint16_t*>(smem + size_t(HC) * (sizeof(V) + sizeof(uint32_t)));
+  __shared__ CtaShared<V, TW> sh;
+  const BMArgs& a = h.a;
+  const unsigned tid = threadIdx.x;
+  unsigned long long fam_e = 0, fam_v = 0;  // entries and vertices evaluated (tid 0)
+  const bool replay = a.out_target != nullptr;
+  const RoundView rv = RoundOf(a);
+  for (uint32_t i = tid; i < HC; i += BT) {
+    keys[i] = kNone;
+    vals[i] = 0;
+  }
+  if (tid == 0) sh.nused = 0;
+  __syncthreads();
+  for (uint32_t item = h.small_lo + blockIdx.x; item < h.small_hi; item += gridDim.x) {
+    const uint32_t v = h.small_v[item];
+    if (!InFront(a, rv, v)) continue;  // uniform over the CTA
+    const VertexCtx x = LoadVertexAs<ConstLoads>(a, v);
+    if (tid == 0) {
+      fam_e += x.d;
+      fam_v += 1;
+    }
+    const bool append =
+        CtaStep<HC, V, kConv, ConstLoads, TW>(a, rv, x, vals, keys, used, sh, tid, 0, replay);
+    if (tid == 0 && append) a.movers[atomicAdd(&a.ctr->movers, 1u)] = v;
   }
   if (tid == 0 && fam_v) {
     atomicAdd(&a.ctr->fam_entries[kFamHubSmall], fam_e);
@@ -435,20 +486,45 @@ Status LaunchSmallClass(Context* ctx, const HubArgs& h, uint32_t lo, uint32_t hi
   return Status::Ok();
 }
 
+// The same for HubCertKernel.
+template <int HC, int TW, typename V>
+Status LaunchCertClass(Context* ctx, const HubArgs& h, uint32_t lo, uint32_t hi) {
+  if (hi <= lo) return Status::Ok();
+  constexpr size_t smem = HubCertSmem<HC, TW, V>();
+  auto k = HubCertKernel<HC, TW, V, true>;
+  if constexpr (sizeof(V) == 4) {
+    if (!h.a.conv) k = HubCertKernel<HC, TW, V, false>;
+  }
+  const int per_sm = PrepareOnce(k, TW * 32, smem);
+  if (per_sm <= 0) return MakeError(PCC_INTERNAL, "small-hub kernel cannot be configured");
+  HubArgs hc = h;
+  hc.small_lo = lo;
+  hc.small_hi = hi;
+  k<<<Blocks(hi - lo, 1, unsigned(ctx->num_sms) * unsigned(per_sm)), TW * 32, smem, ctx->stream>>>(hc);
+  PCC_COUNT(1);
+  return Status::Ok();
+}
+
 template <bool kInt, bool kAsync, typename V>
 Status LaunchHubT(Context* ctx, const HubArgs& h, uint32_t num_small, uint32_t num_wide, uint32_t num_mid,
                   int families) {
   const unsigned sms = unsigned(ctx->num_sms);
   if (num_small && (families & kLaunchSmallHubs)) {
-    // Three table sizes, each hub in the smallest that holds its 2d + 2
-    // slots (the classes are consecutive in small_v, widest first): smaller
-    // tables fit more CTAs per SM.
+    // Each hub in the smallest table that holds its 2d + 2 slots (the classes
+    // are consecutive in small_v, widest first): smaller tables fit more CTAs
+    // per SM.
     const uint32_t end_mid = num_wide + num_mid;
-    const int nl = (num_wide > 0) + (num_mid > 0) + (num_small > end_mid);
+    int nl = (num_wide > 0) + (num_mid > 0) + (num_small > end_mid);
     FamBegin(ctx, kFamHubSmall);
-    PCC_RETURN_IF_ERROR((LaunchSmallClass<kInt, kAsync, V, kSmallSlots>(ctx, h, 0, num_wide)));
-    PCC_RETURN_IF_ERROR((LaunchSmallClass<kInt, kAsync, V, kSmallMidSlots>(ctx, h, num_wide, end_mid)));
-    PCC_RETURN_IF_ERROR((LaunchSmallClass<kInt, kAsync, V, kSmallNarrowSlots>(ctx, h, end_mid, num_small)));
+    if constexpr (kInt && !kAsync) {
+      PCC_RETURN_IF_ERROR((LaunchCertClass<2 * kHubSmallMax, 16, V>(ctx, h, 0, end_mid)));
+      PCC_RETURN_IF_ERROR((LaunchCertClass<kHubSmallMax, 8, V>(ctx, h, end_mid, num_small)));
+      nl = (end_mid > 0) + (num_small > end_mid);
+    } else {
+      PCC_RETURN_IF_ERROR((LaunchSmallClass<kInt, kAsync, V, kSmallSlots>(ctx, h, 0, num_wide)));
+      PCC_RETURN_IF_ERROR((LaunchSmallClass<kInt, kAsync, V, kSmallMidSlots>(ctx, h, num_wide, end_mid)));
+      PCC_RETURN_IF_ERROR((LaunchSmallClass<kInt, kAsync, V, kSmallNarrowSlots>(ctx, h, end_mid, num_small)));
+    }
     FamEnd(ctx, kFamHubSmall, nl);
   }
   const bool glob = !kAsync && h.num_glob;
@@ -674,15 +750,18 @@ Status PrepareHubKernels() {
   auto big = [&](auto k, size_t slots, size_t vsize) {
     ok = ok && PrepareOnce(k, kBigThreads, slots * (vsize + sizeof(uint32_t))) > 0;
   };
-  small(HubSmallKernel<true, false, int, kSmallSlots>, kSmallSlots, sizeof(int));
-  small(HubSmallKernel<true, false, int, kSmallNarrowSlots>, kSmallNarrowSlots, sizeof(int));
-  small(HubSmallKernel<true, false, int, kSmallMidSlots>, kSmallMidSlots, sizeof(int));
-  small(HubSmallKernel<true, false, long long, kSmallMidSlots>, kSmallMidSlots, sizeof(long long));
   small(HubSmallKernel<false, false, double, kSmallMidSlots>, kSmallMidSlots, sizeof(double));
-  small(HubSmallKernel<true, false, long long, kSmallSlots>, kSmallSlots, sizeof(long long));
-  small(HubSmallKernel<true, false, long long, kSmallNarrowSlots>, kSmallNarrowSlots, sizeof(long long));
   small(HubSmallKernel<false, false, double, kSmallSlots>, kSmallSlots, sizeof(double));
   small(HubSmallKernel<false, false, double, kSmallNarrowSlots>, kSmallNarrowSlots, sizeof(double));
+  auto cert = [&](auto sum, auto conv) {
+    using V = decltype(sum);
+    constexpr bool kC = decltype(conv)::value;
+    ok = ok && PrepareOnce(HubCertKernel<2 * kHubSmallMax, 16, V, kC>, 512, HubCertSmem<2 * kHubSmallMax, 16, V>()) > 0 &&
+         PrepareOnce(HubCertKernel<kHubSmallMax, 8, V, kC>, 256, HubCertSmem<kHubSmallMax, 8, V>()) > 0;
+  };
+  cert(0, std::false_type{});
+  cert(0, std::true_type{});
+  cert(0ll, std::true_type{});
   big(HubBigKernel<true, false, int>, BigSlots<int>(), sizeof(int));
   big(HubBigKernel<true, false, long long>, BigSlots<long long>(), sizeof(long long));
   big(HubBigKernel<false, false, double>, BigSlots<double>(), sizeof(double));

@@ -209,3 +209,36 @@ def test_whole_cluster_moves_table(ctx, name, weights):
             for key in ("edge_visits", "rounds", "levels", "moves"):
                 assert st[key] == so[key], key
     dg.free()
+
+
+def _hub_degrees(degs, n=9000, seed=6):
+    """A block model with one hub of each given degree (its ids first)."""
+    g, _ = G.sbm(n, 30, 0.03, 0.001, seed)
+    src = np.repeat(np.arange(n), np.diff(g.offsets).astype(np.int64))
+    far = (src >= len(degs)) & (g.neighbors >= len(degs)) & (src < g.neighbors)
+    s, d = [src[far]], [g.neighbors[far].astype(np.int64)]
+    rng = np.random.default_rng(seed)
+    for hub, deg in enumerate(degs):
+        s.append(np.full(deg, hub)), d.append(len(degs) + rng.permutation(n - len(degs))[:deg])
+    return P.CsrGraph.from_edges(n, np.concatenate(s), np.concatenate(d))
+
+
+@pytest.mark.parametrize("kind", ["unit", "integer", "uniform", "wide"])
+@pytest.mark.parametrize("move", [P.NBHR_CLUSTER_MOVE, P.ALL_MOVE])
+def test_hubs_at_table_edges(ctx, kind, move):
+    """Hubs at the limits of the table sizes, the degree-binned kernels driven
+    by the host; their rows are pushed whole and in pieces."""
+    g = _hub_degrees((1000, 1001, 2047, 2048, 3071, 4096, 4097, 6144, 6145, 8500))
+    if kind == "integer":
+        g = _weighted(g, lambda a, b: (a * 7 + b * 13) % 5 + 1)
+    elif kind == "uniform":
+        g = _weighted(g, WEIGHTS["uniform"][0])
+    elif kind == "wide":
+        g = _weighted(g, lambda a, b: ((a * 7 + b * 13) % 5 + 1) * 1000003)
+    scale = float(np.abs(g.weights).mean()) if g.weights is not None else 1.0
+    ctx.set_detailed_timing(True)
+    try:
+        for res, modularity in ((0.02 * scale, False), (1.0, True)):
+            _same(ctx, g, P.make_config(resolution=res, refine=True, move_method=move), modularity)
+    finally:
+        ctx.set_detailed_timing(False)
