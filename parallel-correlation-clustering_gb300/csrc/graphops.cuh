@@ -14,6 +14,7 @@
 #pragma once
 
 #include "engine.cuh"
+#include "hubs.cuh"
 
 namespace pcc {
 
@@ -332,33 +333,66 @@ __global__ void __launch_bounds__(kIterThreads) PushMidKernel(const uint32_t* __
   }
 }
 
+// Rows of more than kHubSmallMax entries in pieces (HubPlan).
+struct PushChunks {
+  const uint32_t* big_v;
+  const uint32_t* chunk_hub;
+  const uint32_t* chunk_start;
+  uint32_t num;
+};
+
+// The pieces of the longest rows, then the rows of bin Cta, dealt to the CTAs.
+// Each thread first looks up one of the CTA's items (five dependent loads), so
+// that the chain is paid once for 256 items, and a row of any length is spread
+// over the GPU.  (RMAT scale 20, largest row 86k entries, a CTA of 512 threads
+// per row: 96 us a round; 11.)
 template <class R>
-__global__ void __launch_bounds__(kIterBigThreads) PushBigKernel(const uint32_t* __restrict__ list,
-                                                                const uint32_t* __restrict__ starts,
-                                                                const uint64_t* __restrict__ off,
-                                                                const uint32_t* __restrict__ nbr,
-                                                                uint32_t* __restrict__ stamp, StampValue sv, R row) {
+__global__ void __launch_bounds__(kIterThreads) PushBigKernel(const uint32_t* __restrict__ list,
+                                                             const uint32_t* __restrict__ starts,
+                                                             const uint64_t* __restrict__ off,
+                                                             const uint32_t* __restrict__ nbr,
+                                                             uint32_t* __restrict__ stamp, StampValue sv,
+                                                             PushChunks c, uint32_t chunk, R row) {
+  __shared__ uint64_t from[kIterThreads];
+  __shared__ uint32_t len[kIterThreads];
   const uint32_t s0 = starts[kBinCta];
-  const uint32_t count = starts[kNumBins] - s0;  // bins Cta, Global
+  const uint64_t items = uint64_t(c.num) + (starts[kBinGlobal] - s0);
   const uint32_t value = StampIn(sv.rs, sv.stamp);
-  for (uint64_t i = blockIdx.x; i < count; i += gridDim.x) {
-    const uint32_t v = list[s0 + i];
-    if (!row(v)) continue;
-    const uint64_t b = off[v], e = off[v + 1];
-    for (uint64_t j0 = b; j0 < e; j0 += uint64_t(kIterBigThreads) * kPushBatch) {
-      uint32_t u[kPushBatch];
-#pragma unroll
-      for (int k = 0; k < kPushBatch; ++k) {
-        const uint64_t j = j0 + uint64_t(kIterBigThreads) * k + threadIdx.x;
-        u[k] = j < e ? nbr[j] : kNone;
-      }
-      uint32_t cur[kPushBatch];
-#pragma unroll
-      for (int k = 0; k < kPushBatch; ++k) cur[k] = u[k] != kNone ? stamp[u[k]] : value;
-#pragma unroll
-      for (int k = 0; k < kPushBatch; ++k)
-        if (cur[k] != value) stamp[u[k]] = value;
+  const unsigned tid = threadIdx.x;
+  for (uint64_t base = blockIdx.x; base < items; base += uint64_t(gridDim.x) * kIterThreads) {
+    const uint64_t it = base + uint64_t(gridDim.x) * tid;
+    uint64_t b = 0;
+    uint32_t n = 0;
+    if (it < items) {
+      const bool piece = it < c.num;
+      const uint32_t v = piece ? c.big_v[c.chunk_hub[it]] : list[s0 + (it - c.num)];
+      const uint64_t o0 = off[v], o1 = off[v + 1];
+      b = o0 + (piece ? c.chunk_start[it] : 0u);
+      if (row(v)) n = static_cast<uint32_t>(piece ? min(o1 - b, uint64_t(chunk)) : o1 - b);
     }
+    from[tid] = b;
+    len[tid] = n;
+    __syncthreads();
+    const uint64_t left = (items - base + gridDim.x - 1) / gridDim.x;
+    const int count = left < kIterThreads ? int(left) : kIterThreads;
+    for (int q = 0; q < count; ++q) {
+      const uint64_t b0 = from[q];
+      const uint32_t l = len[q];
+      for (uint32_t j0 = 0; j0 < l; j0 += kIterThreads * kPushBatch) {
+        uint32_t u[kPushBatch], cur[kPushBatch];
+#pragma unroll
+        for (int k = 0; k < kPushBatch; ++k) {
+          const uint32_t j = j0 + kIterThreads * k + tid;
+          u[k] = j < l ? nbr[b0 + j] : kNone;
+        }
+#pragma unroll
+        for (int k = 0; k < kPushBatch; ++k) cur[k] = u[k] != kNone ? stamp[u[k]] : value;
+#pragma unroll
+        for (int k = 0; k < kPushBatch; ++k)
+          if (cur[k] != value) stamp[u[k]] = value;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -380,30 +414,30 @@ struct PushStampFn {
   }
 };
 
-// The push over a BinSet-layout list (starts on device; host_counts may be
-// null: every shape launched).
+// The push over a graph's static bins.
 template <class R>
-inline void LaunchPush(Context* ctx, const uint32_t* list, const uint32_t* counts, const uint32_t* starts,
-                       const uint32_t* host_counts, const uint64_t* off, const uint32_t* nbr, uint32_t* stamp,
-                       StampValue sv, bool blind, R row) {
+inline void LaunchPush(Context* ctx, const DevGraph& g, const PushChunks& hub_rows, uint32_t* stamp, StampValue sv,
+                       R row) {
+  const BinSet& bins = g.bins;
   auto any = [&](int b0, int b1) {
-    if (!host_counts) return true;
     for (int b = b0; b < b1; ++b)
-      if (host_counts[b]) return true;
+      if (bins.host_counts[b]) return true;
     return false;
   };
+  const uint32_t *list = bins.list.p, *starts = bins.counts.p + kNumBins;
   cudaStream_t st = ctx->stream;
   if (any(kBinG4, kBinW128)) {
     EdgeBatchSmallKernel<PushStampFn, R><<<IterSmallGrid(ctx), kIterThreads, 0, st>>>(
-        list, starts, off, PushStampFn{nbr, stamp, sv, blind}, row);
+        list, starts, g.off.p, PushStampFn{g.nbr.p, stamp, sv, g.max_deg <= kHubSmallMax}, row);
     PCC_COUNT(1);
   }
   if (any(kBinW128, kBinCta)) {
-    PushMidKernel<R><<<IterMidGrid(ctx), kIterThreads, 0, st>>>(list, starts, off, nbr, stamp, sv, row);
+    PushMidKernel<R><<<IterMidGrid(ctx), kIterThreads, 0, st>>>(list, starts, g.off.p, g.nbr.p, stamp, sv, row);
     PCC_COUNT(1);
   }
   if (any(kBinCta, kNumBins)) {
-    PushBigKernel<R><<<IterBigGrid(ctx), kIterBigThreads, 0, st>>>(list, starts, off, nbr, stamp, sv, row);
+    PushBigKernel<R><<<IterMidGrid(ctx), kIterThreads, 0, st>>>(list, starts, g.off.p, g.nbr.p, stamp, sv, hub_rows,
+                                                                kLoopChunk, row);
     PCC_COUNT(1);
   }
 }

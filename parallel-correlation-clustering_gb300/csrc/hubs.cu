@@ -583,7 +583,7 @@ Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan
   std::vector<uint32_t> small_v, big_v, parts, pbase, item_hub, item_part;
   std::vector<uint32_t> big_glob, glob_hub, glob_cap, glob_item, glob_item_start;
   std::vector<uint32_t> glob_nslices, glob_sbase, slice_hub, slice_start;
-  std::vector<uint32_t> loop_cap, loop_nslices, loop_sbase, loop_chunk_hub, loop_chunk_start, loop_slice_hub,
+  std::vector<uint32_t> loop_cap, loop_nslices, loop_sbase, chunk_hub, chunk_start, loop_slice_hub,
       loop_slice_start;
   std::vector<unsigned long long> glob_base, loop_base;
   uint64_t total = 0;
@@ -619,6 +619,10 @@ Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan
     } else {
       big_glob.push_back(kNone);
     }
+    for (uint32_t e = 0; e < hd[i]; e += kLoopChunk) {
+      chunk_hub.push_back(hb);
+      chunk_start.push_back(e);
+    }
     if (g.m <= kLoopMaxEntries) {
       const uint32_t cap = 2 * hd[i] + 2;
       loop_base.push_back(plan->loop_slots);
@@ -626,10 +630,6 @@ Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan
       loop_cap.push_back(cap);
       loop_nslices.push_back((cap + kLoopSlice - 1) / kLoopSlice);
       loop_sbase.push_back(static_cast<uint32_t>(loop_slice_hub.size()));
-      for (uint32_t e = 0; e < hd[i]; e += kLoopChunk) {
-        loop_chunk_hub.push_back(hb);
-        loop_chunk_start.push_back(e);
-      }
       for (uint32_t s0 = 0; s0 < cap; s0 += kLoopSlice) {
         loop_slice_hub.push_back(hb);
         loop_slice_start.push_back(s0);
@@ -678,13 +678,13 @@ Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan
   std::vector<unsigned long long> pack64 = glob_base;
   const size_t loop_base_at = pack64.size();
   pack64.insert(pack64.end(), loop_base.begin(), loop_base.end());
-  plan->num_loop_chunks = static_cast<uint32_t>(loop_chunk_hub.size());
+  plan->num_chunks = static_cast<uint32_t>(chunk_hub.size());
   plan->num_loop_slices = static_cast<uint32_t>(loop_slice_hub.size());
   add(&plan->loop_cap, loop_cap);
   add(&plan->loop_nslices, loop_nslices);
   add(&plan->loop_sbase, loop_sbase);
-  add(&plan->loop_chunk_hub, loop_chunk_hub);
-  add(&plan->loop_chunk_start, loop_chunk_start);
+  add(&plan->chunk_hub, chunk_hub);
+  add(&plan->chunk_start, chunk_start);
   add(&plan->loop_slice_hub, loop_slice_hub);
   add(&plan->loop_slice_start, loop_slice_start);
   PCC_RETURN_IF_ERROR(plan->pack.Alloc(ctx, std::max<size_t>(pack.size(), 1)));

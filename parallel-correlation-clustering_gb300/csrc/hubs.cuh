@@ -31,7 +31,7 @@ constexpr uint32_t kHubSmallMax = 4096;   // one-partition hubs
 constexpr uint32_t kHubBigKeys = 12288;   // expected distinct keys per big-hub partition
 constexpr uint32_t kHubGlobalParts = 4;    // big hubs with >= this many partitions take the global path
 constexpr uint32_t kHubGlobalSlice = 1024;   // table slots evaluated by one CTA
-constexpr uint32_t kLoopChunk = 2048;         // row entries per work item (roundloop.cu)
+constexpr uint32_t kLoopChunk = 2048;         // row entries per work item (roundloop.cu, the frontier push)
 constexpr uint32_t kLoopSlice = 2048;         // table slots per work item (roundloop.cu)
 
 // Static part (depends on the graph only).
@@ -72,18 +72,19 @@ struct HubPlan {
   const uint32_t* glob_sbase = nullptr;            // per global hub: first partial
   const uint32_t* slice_hub = nullptr;             // per slice: global hub index
   const uint32_t* slice_start = nullptr;           // per slice: first slot (within the hub's table)
-  // The same for every big hub, in rows of kLoopChunk entries and slices of
-  // kLoopSlice slots: the kernel that runs a whole level's rounds
-  // (roundloop.cu; graphs of at most kLoopMaxEntries entries).
-  uint32_t num_loop_chunks = 0;
+  // The rows of every big hub in pieces of kLoopChunk entries.
+  uint32_t num_chunks = 0;
+  const uint32_t* chunk_hub = nullptr;             // per chunk: big-hub index
+  const uint32_t* chunk_start = nullptr;           // per chunk: first entry
+  // Tables and slices of kLoopSlice slots for every big hub: the kernel that
+  // runs a whole level's rounds (roundloop.cu; graphs of at most
+  // kLoopMaxEntries entries).
   uint32_t num_loop_slices = 0;
   uint64_t loop_slots = 0;
   const unsigned long long* loop_base = nullptr;   // per big hub: first table slot
   const uint32_t* loop_cap = nullptr;              // per big hub: 2 * degree + 2
   const uint32_t* loop_nslices = nullptr;          // per big hub
   const uint32_t* loop_sbase = nullptr;            // per big hub: first partial
-  const uint32_t* loop_chunk_hub = nullptr;        // per chunk: big-hub index
-  const uint32_t* loop_chunk_start = nullptr;      // per chunk: first entry
   const uint32_t* loop_slice_hub = nullptr;        // per slice: big-hub index
   const uint32_t* loop_slice_start = nullptr;      // per slice: first slot
 };

@@ -308,27 +308,33 @@ __global__ void SpendMoversKernel(DevCounters* ctr) {
   ctr->new_movers = 0;
 }
 
-// Gated inputs for the new-cluster compactions: nothing to do when no
-// vertex moves to a new cluster.
-struct ZeroSizeInput {
+// The two lists that new clusters are made of in one scan: the empty cluster
+// ids (low words) and the vertices that open a cluster (high words), each
+// ascending; skipped in rounds that open none.  (RMAT scale 20, 138 rounds:
+// two scans took 28 us a round, read or not.)
+struct NewClusterInput {
   const uint32_t* s;
+  const uint32_t* st;
+  uint32_t stamp;
   const DevCounters* ctr;
-  __device__ uint32_t operator()(uint64_t i) const { return ctr->new_movers && s[i] == 0u ? 1u : 0u; }
+  const RoundState* rs;
+  __device__ bool Skip() const { return ctr->new_movers == 0; }
+  __device__ uint64_t operator()(uint64_t i) const {
+    return (s[i] == 0u ? 1ull : 0ull) | (st[i] == StampIn(rs, stamp) ? 1ull << 32 : 0ull);
+  }
+};
+struct StoreNewClusterLists {
+  uint32_t* zero_ids;
+  uint32_t* new_list;
+  __device__ void operator()(uint64_t i, uint64_t pre, uint64_t v) const {
+    if (static_cast<uint32_t>(v)) zero_ids[static_cast<uint32_t>(pre)] = static_cast<uint32_t>(i);
+    if (v >> 32) new_list[pre >> 32] = static_cast<uint32_t>(i);
+  }
 };
 struct EmptyClusterInput {
   const uint32_t* s;
   __device__ uint32_t operator()(uint64_t i) const { return s[i] == 0u ? 1u : 0u; }
 };
-struct NewMoverInput {
-  const uint32_t* st;
-  uint32_t stamp;
-  const DevCounters* ctr;
-  const RoundState* rs = nullptr;
-  __device__ uint32_t operator()(uint64_t i) const {
-    return ctr->new_movers && st[i] == StampIn(rs, stamp) ? 1u : 0u;
-  }
-};
-
 // New clusters take the ascending list of empty ids, in ascending node order.
 __global__ void __launch_bounds__(kT) AssignNewKernel(ApplyArgs a, const uint32_t* __restrict__ zero_ids,
                                                       const uint32_t* __restrict__ new_list) {
@@ -362,11 +368,11 @@ __device__ __forceinline__ uint32_t LowerBound(const uint32_t* __restrict__ a, u
 // rest of its vertices); an index outside graph j's range is reported as
 // kErrUnionRange and skipped.
 __global__ void __launch_bounds__(kT) AssignNewUnionKernel(ApplyArgs a, const uint32_t* __restrict__ zero_ids,
-                                                           const uint32_t* __restrict__ zcount,
+                                                           const uint64_t* __restrict__ zcount,
                                                            const uint32_t* __restrict__ new_list,
                                                            const uint32_t* __restrict__ vbase, uint32_t B) {
   const uint32_t count = a.ctr->new_movers;
-  const uint32_t zc = *zcount;
+  const uint32_t zc = static_cast<uint32_t>(*zcount);  // the low word: empty ids
   for (uint64_t i = uint64_t(blockIdx.x) * kT + threadIdx.x; i < count; i += uint64_t(gridDim.x) * kT) {
     const uint32_t v = new_list[i];
     const uint32_t j = GraphOf(vbase, B, v);
@@ -749,6 +755,7 @@ class Engine {
     PCC_RETURN_IF_ERROR(rs_.Alloc(ctx_, 1));
     // Scan scratch for every level (no allocation inside a captured round).
     PCC_RETURN_IF_ERROR(scan_tiles_.Reserve(ctx_, (nn + kScanTile - 1) / kScanTile + 1));
+    PCC_RETURN_IF_ERROR(new_tiles_.Reserve(ctx_, (nn + kScanTile - 1) / kScanTile + 1));
     (void)max_deg;
     return Status::Ok();
   }
@@ -896,12 +903,9 @@ class Engine {
                    ctr_.p, rs};
       const unsigned grid = GridFor(ctx_, rs ? uint64_t(n) : front_size);
       ApplyMoveKernel<<<grid, kT, 0, ctx_->stream>>>(ap); PCC_COUNT(1);
-      PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx_, n, ZeroSizeInput{L->s.p, ctr_.p},
-                                              StoreIndexIfSet{zero_ids_.p}, scan_tiles_,
-                                              un_ ? zcount_.p : static_cast<uint32_t*>(nullptr)));
-      PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx_, n, NewMoverInput{new_stamp_.p, stamp_, ctr_.p, rs},
-                                              StoreIndexIfSet{new_list_.p}, scan_tiles_,
-                                              static_cast<uint32_t*>(nullptr)));
+      PCC_RETURN_IF_ERROR(ScanApply<uint64_t>(ctx_, n, NewClusterInput{L->s.p, new_stamp_.p, stamp_, ctr_.p, rs},
+                                              StoreNewClusterLists{zero_ids_.p, new_list_.p}, new_tiles_,
+                                              un_ ? zcount_.p : static_cast<uint64_t*>(nullptr)));
       if (un_) {
         AssignNewUnionKernel<<<grid, kT, 0, ctx_->stream>>>(ap, zero_ids_.p, zcount_.p, new_list_.p,
                                                              un_->d_vbase.p, un_->B); PCC_COUNT(1);
@@ -924,12 +928,13 @@ class Engine {
     // degree bins with a marked-row predicate, then the next frontier's size.
     timer_.Begin(kPhaseFrontier);
     const StampValue sv{stamp_, rs};
+    const PushChunks hub_rows{g.hub_plan->big_v, g.hub_plan->chunk_hub, g.hub_plan->chunk_start,
+                              g.hub_plan->num_chunks};
     if (cfg_.move_method == PCC_NBHR_CLUSTER_MOVE) {
-      LaunchPush(ctx_, g.bins.list.p, g.bins.counts.p, g.bins.counts.p + kNumBins, g.bins.host_counts, g.off.p,
-                 g.nbr.p, next_stamp_.p, sv, g.max_deg <= 4096, PredModifiedCluster{L->C.p, mod_stamp_.p, stamp_, rs});  // rows with d > 0
+      LaunchPush(ctx_, g, hub_rows, next_stamp_.p, sv,
+                 PredModifiedCluster{L->C.p, mod_stamp_.p, stamp_, rs});  // rows with d > 0
     } else {
-      LaunchPush(ctx_, g.bins.list.p, g.bins.counts.p, g.bins.counts.p + kNumBins, g.bins.host_counts, g.off.p,
-                 g.nbr.p, next_stamp_.p, sv, g.max_deg <= 4096, PredStamp{moved_stamp_.p, stamp_, rs});
+      LaunchPush(ctx_, g, hub_rows, next_stamp_.p, sv, PredStamp{moved_stamp_.p, stamp_, rs});
     }
     if (n) {
       CountDegreesKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, g.off.p, PredStamp{next_stamp_.p, stamp_, rs},
@@ -1035,11 +1040,9 @@ class Engine {
     const unsigned grid = GridFor(ctx_, n);
     ApplyLeaveKernel<<<grid, kT, 0, ctx_->stream>>>(ap); PCC_COUNT(1);
     ApplyJoinKernel<<<grid, kT, 0, ctx_->stream>>>(ap); PCC_COUNT(1);
-    PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx_, n, ZeroSizeInput{L->s.p, ctr_.p}, StoreIndexIfSet{zero_ids_.p},
-                                            scan_tiles_, static_cast<uint32_t*>(nullptr)));
-    PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx_, n, NewMoverInput{new_stamp_.p, stamp_, ctr_.p, rs},
-                                            StoreIndexIfSet{new_list_.p}, scan_tiles_,
-                                            static_cast<uint32_t*>(nullptr)));
+    PCC_RETURN_IF_ERROR(ScanApply<uint64_t>(ctx_, n, NewClusterInput{L->s.p, new_stamp_.p, stamp_, ctr_.p, rs},
+                                            StoreNewClusterLists{zero_ids_.p, new_list_.p}, new_tiles_,
+                                            static_cast<uint64_t*>(nullptr)));
     AssignNewKernel<<<grid, kT, 0, ctx_->stream>>>(ap, zero_ids_.p, new_list_.p); PCC_COUNT(1);
     RefreshKfKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, L->K.p, L->Kf.p, mod_stamp_.p, stamp_, rs);
     PCC_COUNT(1);
@@ -1820,6 +1823,7 @@ class Engine {
   DBuf<uint32_t> sm_front_, sm_moved_, sm_dummy_;
   uint32_t sm_val_ = 0;
   DBuf<uint32_t> scan_tiles_;
+  DBuf<uint64_t> new_tiles_;
   HubState hub_state_;
   ClusterMoveTable cm_table_;  // whole-cluster moves
   DBuf<LoopState> loop_state_;  // one-kernel round loop
@@ -1832,7 +1836,8 @@ class Engine {
   // and degree sums of the round, round-0 masks, the empty-id count.
   DBuf<RoundState> rs_;  // device-side round loop state
   const UnionLayout* un_ = nullptr;
-  DBuf<uint32_t> gflags_, gmask_, zcount_;
+  DBuf<uint32_t> gflags_, gmask_;
+  DBuf<uint64_t> zcount_;
   DBuf<unsigned long long> gedges_;
   // Device-side union loop: in_loop[B] | moved[B], per-graph frontier
   // entries, edge visits and rounds.

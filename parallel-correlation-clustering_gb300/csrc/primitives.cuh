@@ -52,8 +52,20 @@ __device__ __forceinline__ T BlockExclusiveScan(T x, T* total) {
   return r;
 }
 
+// An input with a member Skip() that is true (on the device, for the whole
+// scan) is not read, and nothing is written.
+template <class F>
+__device__ __forceinline__ auto ScanSkip(const F& f, int) -> decltype(f.Skip()) {
+  return f.Skip();
+}
+template <class F>
+__device__ __forceinline__ bool ScanSkip(const F&, long) {
+  return false;
+}
+
 template <class T, class F>
 __global__ void __launch_bounds__(kScanThreads) ScanTileReduceKernel(uint64_t n, F f, T* tile_sums) {
+  if (ScanSkip(f, 0)) return;
   const uint64_t base = uint64_t(blockIdx.x) * kScanTile;
   T acc = 0;
 #pragma unroll
@@ -100,6 +112,7 @@ constexpr uint64_t kScanRawTiles = 4096;
 template <class T, class F, class W>
 __global__ void __launch_bounds__(kScanThreads) ScanTileApplyKernel(uint64_t n, F f, const T* tile_sums, W w, int raw,
                                                                    T* total_out) {
+  if (ScanSkip(f, 0)) return;
   __shared__ T vals[kScanTile];
   const uint64_t base = uint64_t(blockIdx.x) * kScanTile;
   T before = 0;
@@ -137,6 +150,7 @@ __global__ void __launch_bounds__(kScanThreads) ScanTileApplyKernel(uint64_t n, 
 constexpr uint64_t kScanOneCta = 4 * kScanTile;
 template <class T, class F, class W>
 __global__ void __launch_bounds__(kScanThreads) ScanOneKernel(uint64_t n, F f, W w, T* total_out) {
+  if (ScanSkip(f, 0)) return;
   __shared__ T vals[kScanTile];
   __shared__ T total;
   T run = 0;

@@ -773,9 +773,9 @@ void SetLoopHubs(RoundLoopArgs* l, const HubPlan& plan, const HubState& st) {
   l->big_cap = plan.loop_cap;
   l->big_nslices = plan.loop_nslices;
   l->big_sbase = plan.loop_sbase;
-  l->chunk_hub = plan.loop_chunk_hub;
-  l->chunk_start = plan.loop_chunk_start;
-  l->num_chunks = plan.num_loop_chunks;
+  l->chunk_hub = plan.chunk_hub;
+  l->chunk_start = plan.chunk_start;
+  l->num_chunks = plan.num_chunks;
   l->slice_hub = plan.loop_slice_hub;
   l->slice_start = plan.loop_slice_start;
   l->num_slices = plan.num_loop_slices;
