@@ -604,7 +604,65 @@ struct CtaShared {
   V ls[TW], ts[TW];
   unsigned long long lk[TW], tk[TW];
   uint32_t li[TW], ti[TW];
+  uint32_t exact;  // the vertex goes to TeamExact, with:
+  int cres;
+  uint32_t cmove;
+  double change;
+  double bv[TW];
+  uint32_t bi[TW];
 };
+
+// WarpExact by a whole team: FP64 values of the contenders on the used list,
+// cleared as they are read.  (One warp over the 12,288 slots that a hub can
+// use took longer than the rest of its CTA's work.)
+template <typename V, int TW>
+__device__ __noinline__ bool TeamExact(const BMArgs& a, const VertexCtx& x, V* vals, uint32_t* keys,
+                                       const uint16_t* used, uint32_t nused, CtaShared<V, TW>& sh, unsigned tid,
+                                       unsigned bar, bool replay, uint32_t stamp) {
+  const double change = sh.change;
+  double best = -CUDART_INF;
+  uint32_t bid = kNone;
+  for (uint32_t i = tid; i < nused; i += TW * 32) {
+    const uint32_t slot = used[i];
+    if (slot == 0xFFFFu) continue;
+    const uint32_t key = keys[slot];
+    const double val = ValOf(a, x, change, UnitsToDouble<V>(a, vals[slot]), a.K[key]);
+    keys[slot] = kNone;
+    vals[slot] = 0;
+    if (Better(val, key, best, bid)) {
+      best = val;
+      bid = key;
+    }
+  }
+  if (__any_sync(kFull, bid != kNone)) {
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      const double ov = __shfl_xor_sync(kFull, best, o);
+      const uint32_t oid = __shfl_xor_sync(kFull, bid, o);
+      if (Better(ov, oid, best, bid)) {
+        best = ov;
+        bid = oid;
+      }
+    }
+  }
+  if ((tid & 31) == 0) {
+    sh.bv[tid >> 5] = best;
+    sh.bi[tid >> 5] = bid;
+  }
+  TeamSync<TW * 32>(bar);
+  bool append = false;
+  if (tid == 0) {
+    for (int w = 1; w < TW; ++w)
+      if (Better(sh.bv[w], sh.bi[w], best, bid)) {
+        best = sh.bv[w];
+        bid = sh.bi[w];
+      }
+    append = Decide<false>(a, x, best, bid, change, stamp);
+    if (replay && sh.cres != kUncertain && a.out_moves && a.out_moves[x.v] != sh.cmove)
+      atomicExch(&a.ctr->error, kErrCertMismatch);
+  }
+  return append;
+}
 
 // A team of TW warps (its thread index tid) on one vertex x of degree
 // <= HC / 2, with the team's table (clean before and after, as sh.nused) and
@@ -753,22 +811,32 @@ __device__ __forceinline__ bool CtaStep(const BMArgs& a, const RoundView& rv, co
       cres = CertifyDecision<V>(ca, Res32Of(a, x.v), k32, top.id != kNone, top.S, KfA, top.id, a.n, &ctarget);
     }
     const uint32_t cmove = cres == kUncertain ? kNone : CertifiedMove(a, x, ctarget, cres == kCertMove);
+    if (lane == 0) sh.exact = 0;
     if (TW > kCtaWarps && nused == 0) {
       // A hub whose entries are all self-loops: the reduce identity (0, 0.0).
       if (lane == 0) append = Decide<false>(a, x, 0.0, 0, ChangeOf(a, x, 0.0), rv.stamp);
     } else if (replay || !single) {
-      append = WarpExact<HC, V>(a, x, T, keys, vals, used, nused, replay, cres, cmove, rv.stamp);
+      if (lane == 0) {
+        sh.exact = 1;
+        sh.cres = cres;
+        sh.cmove = cmove;
+        sh.change = ChangeOf(a, x, UnitsToDouble<V>(a, T));
+      }
     } else if (lane == 0) {
       append = cres == kUncertain ? DecideClass<V, L>(a, x.v, top.id, T, top.S, rv.stamp)
                                   : ApplyCertified(a, x, cmove, rv.stamp);
     }
   }
-  TeamSync<BT>(bar);  // the table is read by WarpExact up to here
-  for (uint32_t i = tid; i < nused; i += BT) {
-    const uint32_t slot = used[i];
-    if (slot != 0xFFFFu) {
-      keys[slot] = kNone;
-      vals[slot] = 0;
+  TeamSync<BT>(bar);
+  if (sh.exact) {
+    append = TeamExact<V, TW>(a, x, vals, keys, used, nused, sh, tid, bar, replay, rv.stamp);
+  } else {
+    for (uint32_t i = tid; i < nused; i += BT) {
+      const uint32_t slot = used[i];
+      if (slot != 0xFFFFu) {
+        keys[slot] = kNone;
+        vals[slot] = 0;
+      }
     }
   }
   if (tid == 0) sh.nused = 0;

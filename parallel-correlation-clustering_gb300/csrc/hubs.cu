@@ -124,9 +124,12 @@ __global__ void __launch_bounds__(kSmallThreads) HubSmallKernel(HubArgs h) {
 // the neighbours' clusters and shared-memory atomics.  (All rounds of RMAT
 // scale 20: 34.9 ms by HubSmallKernel, 14.9; scale 22: 28.1, 22.0; 1M vertices
 // with real weights, 64-bit sums: 39.6, 20.6.)
+// Degrees 4,097 to 12,288 go the same way with 16,384 slots and 32 warps
+// (up to three quarters full).
 template <int HC, int TW, typename V>
 __host__ __device__ constexpr size_t HubCertSmem() {
-  return size_t(HC) * (sizeof(V) + sizeof(uint32_t)) + size_t(HC / 2) * sizeof(uint16_t);  // vals, keys, used
+  return size_t(HC) * (sizeof(V) + sizeof(uint32_t)) +
+         size_t(TW == 32 ? kHubBigKeys : HC / 2) * sizeof(uint16_t);  // vals, keys, used
 }
 
 template <int HC, int TW, typename V, bool kConv>
@@ -161,8 +164,9 @@ __global__ void __launch_bounds__(TW * 32) HubCertKernel(HubArgs h) {
     if (tid == 0 && append) a.movers[atomicAdd(&a.ctr->movers, 1u)] = v;
   }
   if (tid == 0 && fam_v) {
-    atomicAdd(&a.ctr->fam_entries[kFamHubSmall], fam_e);
-    atomicAdd(&a.ctr->fam_vertices[kFamHubSmall], fam_v);
+    constexpr int fam = TW == 32 ? kFamHubBig : kFamHubSmall;
+    atomicAdd(&a.ctr->fam_entries[fam], fam_e);
+    atomicAdd(&a.ctr->fam_vertices[fam], fam_v);
   }
 }
 
@@ -506,8 +510,9 @@ Status LaunchCertClass(Context* ctx, const HubArgs& h, uint32_t lo, uint32_t hi)
 }
 
 template <bool kInt, bool kAsync, typename V>
-Status LaunchHubT(Context* ctx, const HubArgs& h, uint32_t num_small, uint32_t num_wide, uint32_t num_mid,
-                  int families) {
+Status LaunchHubT(Context* ctx, const HubArgs& h, const HubPlan& plan, int families) {
+  const uint32_t num_small = plan.num_small, num_wide = plan.num_small_wide, num_mid = plan.num_small_mid;
+  const uint32_t num_big = plan.num_big, num_multi = plan.num_multi, num_multi_items = plan.num_multi_items;
   const unsigned sms = unsigned(ctx->num_sms);
   if (num_small && (families & kLaunchSmallHubs)) {
     // Each hub in the smallest table that holds its 2d + 2 slots (the classes
@@ -536,15 +541,28 @@ Status LaunchHubT(Context* ctx, const HubArgs& h, uint32_t num_small, uint32_t n
       PCC_COUNT(1);
     }
     FamEnd(ctx, kFamHubBig, glob ? 1 : 0);
-    constexpr size_t smem = size_t(BigSlots<V>()) * (sizeof(V) + sizeof(uint32_t));
-    auto k = HubBigKernel<kInt, kAsync, V>;
-    const int per_sm = PrepareOnce(k, kBigThreads, smem);
-    if (per_sm <= 0) return MakeError(PCC_INTERNAL, "big-hub kernel cannot be configured");
-    const unsigned grid = Blocks(h.num_items, 1, sms * unsigned(std::max(per_sm, 1)));
-    FamBegin(ctx, kFamHubBig);
-    k<<<grid, kBigThreads, smem, ctx->stream>>>(h);
-    FamEnd(ctx, kFamHubBig, 1);
-    PCC_COUNT(1);
+    HubArgs hm = h;
+    if constexpr (kInt && !kAsync) {
+      hm.num_items = num_multi_items;
+      if (num_big > num_multi) {
+        HubArgs hs = h;
+        hs.small_v = h.big_v;
+        FamBegin(ctx, kFamHubBig);
+        PCC_RETURN_IF_ERROR((LaunchCertClass<16384, 32, V>(ctx, hs, num_multi, num_big)));
+        FamEnd(ctx, kFamHubBig, 1);
+      }
+    }
+    if (hm.num_items) {
+      constexpr size_t smem = size_t(BigSlots<V>()) * (sizeof(V) + sizeof(uint32_t));
+      auto k = HubBigKernel<kInt, kAsync, V>;
+      const int per_sm = PrepareOnce(k, kBigThreads, smem);
+      if (per_sm <= 0) return MakeError(PCC_INTERNAL, "big-hub kernel cannot be configured");
+      const unsigned grid = Blocks(hm.num_items, 1, sms * unsigned(std::max(per_sm, 1)));
+      FamBegin(ctx, kFamHubBig);
+      k<<<grid, kBigThreads, smem, ctx->stream>>>(hm);
+      FamEnd(ctx, kFamHubBig, 1);
+      PCC_COUNT(1);
+    }
     if (glob) {
       FamBegin(ctx, kFamHubBig);
       HubGlobalEvalKernel<kInt, V><<<std::min<unsigned>(h.num_glob_slices, 8 * sms), kGlobThreads, 0,
@@ -638,6 +656,10 @@ Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan
     parts.push_back(P);
     pbase.push_back(static_cast<uint32_t>(total));
     total += P;
+    if (P > 1) {
+      plan->num_multi = hb + 1;
+      plan->num_multi_items = static_cast<uint32_t>(total);
+    }
     for (uint32_t p = 0; p < P; ++p) {
       item_hub.push_back(hb);
       item_part.push_back(p);
@@ -757,7 +779,8 @@ Status PrepareHubKernels() {
     using V = decltype(sum);
     constexpr bool kC = decltype(conv)::value;
     ok = ok && PrepareOnce(HubCertKernel<2 * kHubSmallMax, 16, V, kC>, 512, HubCertSmem<2 * kHubSmallMax, 16, V>()) > 0 &&
-         PrepareOnce(HubCertKernel<kHubSmallMax, 8, V, kC>, 256, HubCertSmem<kHubSmallMax, 8, V>()) > 0;
+         PrepareOnce(HubCertKernel<kHubSmallMax, 8, V, kC>, 256, HubCertSmem<kHubSmallMax, 8, V>()) > 0 &&
+         PrepareOnce(HubCertKernel<16384, 32, V, kC>, 1024, HubCertSmem<16384, 32, V>()) > 0;
   };
   cert(0, std::false_type{});
   cert(0, std::true_type{});
@@ -809,17 +832,13 @@ Status LaunchHubBestMoves(Context* ctx, const BMArgs& a, const HubPlan& plan, Hu
   h.gpart_id = st.gpart_id.p;
   h.gdone = st.gdone.p;
   if (a.async) {
-    if (!int_mode)
-      return LaunchHubT<false, true, double>(ctx, h, plan.num_small, plan.num_small_wide, plan.num_small_mid, families);
-    return narrow ? LaunchHubT<true, true, int>(ctx, h, plan.num_small, plan.num_small_wide, plan.num_small_mid, families)
-                  : LaunchHubT<true, true, long long>(ctx, h, plan.num_small, plan.num_small_wide, plan.num_small_mid,
-                                                      families);
+    if (!int_mode) return LaunchHubT<false, true, double>(ctx, h, plan, families);
+    return narrow ? LaunchHubT<true, true, int>(ctx, h, plan, families)
+                  : LaunchHubT<true, true, long long>(ctx, h, plan, families);
   }
-  if (!int_mode)
-    return LaunchHubT<false, false, double>(ctx, h, plan.num_small, plan.num_small_wide, plan.num_small_mid, families);
-  return narrow ? LaunchHubT<true, false, int>(ctx, h, plan.num_small, plan.num_small_wide, plan.num_small_mid, families)
-                : LaunchHubT<true, false, long long>(ctx, h, plan.num_small, plan.num_small_wide, plan.num_small_mid,
-                                                     families);
+  if (!int_mode) return LaunchHubT<false, false, double>(ctx, h, plan, families);
+  return narrow ? LaunchHubT<true, false, int>(ctx, h, plan, families)
+                : LaunchHubT<true, false, long long>(ctx, h, plan, families);
 }
 
 }  // namespace pcc

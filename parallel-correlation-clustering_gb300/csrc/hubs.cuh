@@ -42,6 +42,8 @@ struct HubPlan {
   uint32_t num_small_mid = 0;  // then those with 4096 < 2 * degree + 2 <= 6144
   uint32_t num_big = 0;
   uint32_t num_items = 0;      // big-hub work items (hub, partition)
+  uint32_t num_multi = 0;      // big hubs of more than one partition (the first ones)
+  uint32_t num_multi_items = 0;
   uint64_t num_partials = 0;   // one per big-hub item
   // The lists below lie in one device buffer each (one upload per plan).
   DBuf<uint32_t> pack;

@@ -242,3 +242,17 @@ def test_hubs_at_table_edges(ctx, kind, move):
             _same(ctx, g, P.make_config(resolution=res, refine=True, move_method=move), modularity)
     finally:
         ctx.set_detailed_timing(False)
+
+
+@pytest.mark.parametrize("kind", ["unit", "uniform"])
+def test_one_partition_hubs(ctx, kind):
+    """Hubs of one table of 16,384 slots, up to its last degree and beyond."""
+    g = _hub_degrees((4097, 8191, 8192, 12287, 12288, 12289, 24576, 24577), n=26000)
+    if kind == "uniform":
+        g = _weighted(g, WEIGHTS["uniform"][0])
+    ctx.set_detailed_timing(True)
+    try:
+        for res, modularity in ((0.005, False), (1.0, True)):
+            _same(ctx, g, P.make_config(resolution=res, refine=True, move_method=P.NBHR_CLUSTER_MOVE), modularity)
+    finally:
+        ctx.set_detailed_timing(False)
