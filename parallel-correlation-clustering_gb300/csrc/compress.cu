@@ -86,9 +86,12 @@ struct RankWriter {
 
 // Vertex sort keys: the dense rank of the vertex's cluster.
 __global__ void VertexKeysKernel(uint32_t n, const uint32_t* __restrict__ C, const uint32_t* __restrict__ rank,
-                                 uint64_t* __restrict__ vkey, uint32_t* __restrict__ vval) {
+                                 uint32_t* __restrict__ vrank, uint64_t* __restrict__ vkey,
+                                 uint32_t* __restrict__ vval) {
   for (uint64_t u = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; u < n; u += uint64_t(gridDim.x) * blockDim.x) {
-    vkey[u] = rank[C[u]];
+    const uint32_t r = rank[C[u]];
+    vrank[u] = r;
+    vkey[u] = r;
     vval[u] = static_cast<uint32_t>(u);
   }
 }
@@ -119,24 +122,39 @@ struct RowStartWriter {
   }
 };
 
-// Moves every entry to its row's place in the cluster-ordered array.
+// Moves every entry to its row's place in the cluster-ordered array.  vrank:
+// the dense rank of each vertex's cluster.  Bound by the gathers of vrank, one
+// an entry, four of a lane in flight.
 struct MoveEntries {
   const uint64_t* off;
   const uint32_t* nbr;
   const float* w;
-  const uint32_t* C;
-  const uint32_t* rank;
+  const uint32_t* vrank;
   const uint64_t* dstart;
   uint32_t drop;
   uint32_t* akey;
   uint32_t* aval;
-  __device__ void operator()(uint32_t u, uint64_t j, uint64_t) const {
-    const uint32_t v = nbr[j];
-    const uint32_t cu = C[u], cv = C[v];
-    const bool keep = v <= u || cu != cv;
-    const uint64_t d = dstart[u] + (j - off[u]);
-    akey[d] = keep ? rank[cv] : drop;
-    aval[d] = __float_as_uint(w ? w[j] : 1.0f);
+  __device__ void operator()(const uint32_t (&u)[kEdgeBatch], const uint64_t (&j)[kEdgeBatch]) const {
+    uint32_t v[kEdgeBatch], cv[kEdgeBatch], cu[kEdgeBatch];
+    uint64_t d[kEdgeBatch];
+    float x[kEdgeBatch];
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k) {
+      if (u[k] == kNone) continue;
+      v[k] = nbr[j[k]];
+      x[k] = w ? w[j[k]] : 1.0f;
+      cu[k] = vrank[u[k]];
+      d[k] = dstart[u[k]] + (j[k] - off[u[k]]);
+    }
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k)
+      if (u[k] != kNone) cv[k] = vrank[v[k]];
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k) {
+      if (u[k] == kNone) continue;
+      akey[d[k]] = v[k] <= u[k] || cu[k] != cv[k] ? cv[k] : drop;
+      aval[d[k]] = __float_as_uint(x[k]);
+    }
   }
 };
 
@@ -752,6 +770,8 @@ int BitsFor(uint64_t count) {
   return b;
 }
 
+constexpr uint64_t kForkEntries = 1u << 20;  // the segment classes on streams of their own from here on
+
 // Temporary arrays of a contraction: pieces of one allocation for the small
 // levels (whose 25 allocations and frees cost as much as their kernels),
 // separate ones, freed as soon as they are spent, for large graphs and under
@@ -759,7 +779,7 @@ int BitsFor(uint64_t count) {
 class Scratch {
  public:
   Scratch(Context* ctx, uint64_t n, uint64_t m) : ctx_(ctx) {
-    if (!ctx->budget && n <= (1u << 20) && m <= (16u << 20)) bytes_ = 80 * n + 8 * m + (n / kSortTile + 1) * 1024 + 16384;
+    if (!ctx->budget && n <= (1u << 20) && m <= (16u << 20)) bytes_ = 84 * n + 8 * m + (n / kSortTile + 1) * 1024 + 16384;
   }
   template <class T>
   Status Take(T** p, uint64_t count) {
@@ -852,10 +872,13 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
     // where each row starts in the cluster-ordered entry array.
     uint64_t *vkey, *dstart;
     uint32_t* vval;
+    uint32_t* vrank;
     PCC_RETURN_IF_ERROR(sc.Take(&vkey, n));
     PCC_RETURN_IF_ERROR(sc.Take(&vval, n));
-    VertexKeysKernel<<<Blocks(n, 256, sms * 8), 256, 0, st>>>(n, C, rank, vkey, vval);
+    PCC_RETURN_IF_ERROR(sc.Take(&vrank, n));
+    VertexKeysKernel<<<Blocks(n, 256, sms * 8), 256, 0, st>>>(n, C, rank, vrank, vkey, vval);
     PCC_COUNT(1);
+    sc.Done(rank);
     {
       SortBuffers sb;
       uint64_t* keys2;
@@ -881,10 +904,10 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
     // Every row moved into its cluster's segment.
     PCC_RETURN_IF_ERROR(sc.Take(&akey, g.m));
     PCC_RETURN_IF_ERROR(sc.Take(&aval, g.m));
-    LaunchEdgeIter(ctx, g.bins.list.p, g.bins.counts.p, g.bins.counts.p + kNumBins, g.bins.host_counts, g.off.p,
-                   MoveEntries{g.off.p, g.nbr.p, g.wp(), C, rank, dstart, drop, akey, aval});
+    LaunchEdgeBatch(ctx, g, MoveEntries{g.off.p, g.nbr.p, g.wp(), vrank, dstart, drop, akey, aval});
     PCC_RETURN_IF_ERROR(LaunchCheck());
     sc.Done(dstart);
+    sc.Done(vrank);
     // Segment classes.
     PCC_RETURN_IF_ERROR(sc.Take(&lists, uint64_t(R) * 4));
     const uint32_t* wlist = lists;
@@ -911,18 +934,35 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
     // bounds of it (a class-c segment has more than the class's entries).
     const uint64_t max_mid = std::min<uint64_t>(R, g.m / (kSegWarpMax + 1));
     const uint64_t max_cta = std::min<uint64_t>(R, g.m / (kSegMidMax + 1));
-    SegWarpKernel<<<Blocks(R, 8, sms * 16), 256, 0, st>>>(wlist, head->counts, segbase, ids, drop, akey, aval, ucount,
-                                                          row_count);
-    PCC_COUNT(1);
-    if (max_mid) {
-      SegMidKernel<<<Blocks(max_mid, kSegMidWarps, sms * 12), kSegMidWarps * 32, kSegMidSmem, st>>>(
-          mlist, head->counts, segbase, ids, drop, passes, akey, aval, ucount, row_count);
-      PCC_COUNT(1);
+    // Each class ends in a tail of few segments, so the three run side by side
+    // where they are long enough to pay for the fork.
+    const bool fork = max_cta && g.m >= kForkEntries && ctx->overlap_families && !ctx->detailed_timing;
+    cudaStream_t warp_st = st, mid_st = st;
+    if (fork) {
+      PCC_RETURN_IF_ERROR(ctx->EnsureSideStreams());
+      PCC_CUDA(cudaEventRecord(ctx->fork_ev, st));
+      for (int i = 0; i < 2; ++i) PCC_CUDA(cudaStreamWaitEvent(ctx->side[i], ctx->fork_ev, 0));
+      warp_st = ctx->side[0];
+      mid_st = ctx->side[1];
     }
     if (max_cta) {
       SegCtaKernel<<<Blocks(max_cta, 1, sms * 3), kSegCtaThreads, kSegCtaSmem, st>>>(
           clist, head->counts, segbase, ids, drop, passes, akey, aval, ucount, row_count);
       PCC_COUNT(1);
+    }
+    if (max_mid) {
+      SegMidKernel<<<Blocks(max_mid, kSegMidWarps, sms * 12), kSegMidWarps * 32, kSegMidSmem, mid_st>>>(
+          mlist, head->counts, segbase, ids, drop, passes, akey, aval, ucount, row_count);
+      PCC_COUNT(1);
+    }
+    SegWarpKernel<<<Blocks(R, 8, sms * 16), 256, 0, warp_st>>>(wlist, head->counts, segbase, ids, drop, akey, aval,
+                                                               ucount, row_count);
+    PCC_COUNT(1);
+    if (fork) {
+      for (int i = 0; i < 2; ++i) {
+        PCC_CUDA(cudaEventRecord(ctx->join_ev[i], ctx->side[i]));
+        PCC_CUDA(cudaStreamWaitEvent(st, ctx->join_ev[i], 0));
+      }
     }
     PCC_RETURN_IF_ERROR(LaunchCheck());
     if (maybe_big) PCC_RETURN_IF_ERROR(Sync(ctx));

@@ -161,6 +161,52 @@ inline void LaunchEdgeIter(Context* ctx, const uint32_t* list, const uint32_t* c
 // ---------------------------------------------------------------------------
 constexpr int kEdgeBatch = 4;
 
+// Rows of more than kHubSmallMax entries in pieces of kLoopChunk (HubPlan);
+// without them (num 0) these rows are taken whole.
+struct RowPieces {
+  const uint32_t* big_v;
+  const uint32_t* chunk_hub;
+  const uint32_t* chunk_start;
+  uint32_t num;
+};
+inline RowPieces PiecesOf(const DevGraph& g) {
+  if (!g.hub_plan) return RowPieces{};
+  return RowPieces{g.hub_plan->big_v, g.hub_plan->chunk_hub, g.hub_plan->chunk_start, g.hub_plan->num_chunks};
+}
+
+// The items of one CTA (pieces of the longest rows, then the rows of bin Cta):
+// each thread looks up one of 256 (a chain of dependent loads, paid once), and
+// then the whole CTA walks them in turn: walk(row, first entry, entries).
+template <class R, class W>
+__device__ __forceinline__ void ForBigItems(const uint32_t* __restrict__ list, const uint32_t* __restrict__ starts,
+                                            const uint64_t* __restrict__ off, const RowPieces& c, R row, W walk) {
+  __shared__ uint64_t from[kIterThreads];
+  __shared__ uint32_t len[kIterThreads], vert[kIterThreads];
+  const uint32_t s0 = starts[kBinCta];
+  const uint64_t items = uint64_t(c.num) + (starts[c.num ? kBinGlobal : kNumBins] - s0);
+  const unsigned tid = threadIdx.x;
+  for (uint64_t base = blockIdx.x; base < items; base += uint64_t(gridDim.x) * kIterThreads) {
+    const uint64_t it = base + uint64_t(gridDim.x) * tid;
+    uint64_t b = 0;
+    uint32_t n = 0, v = 0;
+    if (it < items) {
+      const bool piece = it < c.num;
+      v = piece ? c.big_v[c.chunk_hub[it]] : list[s0 + (it - c.num)];
+      const uint64_t o0 = off[v], o1 = off[v + 1];
+      b = o0 + (piece ? c.chunk_start[it] : 0u);
+      if (row(v)) n = static_cast<uint32_t>(piece ? min(o1 - b, uint64_t(kLoopChunk)) : o1 - b);
+    }
+    from[tid] = b;
+    len[tid] = n;
+    vert[tid] = v;
+    __syncthreads();
+    const uint64_t left = (items - base + gridDim.x - 1) / gridDim.x;
+    const int count = left < kIterThreads ? int(left) : kIterThreads;
+    for (int q = 0; q < count; ++q) walk(vert[q], from[q], len[q]);
+    __syncthreads();
+  }
+}
+
 template <class F, class R>
 __global__ void __launch_bounds__(kIterThreads) EdgeBatchSmallKernel(const uint32_t* __restrict__ list,
                                                                     const uint32_t* __restrict__ starts,
@@ -234,30 +280,30 @@ __global__ void __launch_bounds__(kIterThreads) EdgeBatchMidKernel(const uint32_
 }
 
 template <class F, class R>
-__global__ void __launch_bounds__(kIterBigThreads) EdgeBatchBigKernel(const uint32_t* __restrict__ list,
-                                                                     const uint32_t* __restrict__ starts,
-                                                                     const uint64_t* __restrict__ off, F f, R row) {
-  const uint32_t s0 = starts[kBinCta];
-  const uint32_t count = starts[kNumBins] - s0;  // bins Cta, Global
-  for (uint64_t i = blockIdx.x; i < count; i += gridDim.x) {
-    const uint32_t vr = list[s0 + i];
-    if (!row(vr)) continue;
-    const uint64_t b = off[vr], e = off[vr + 1];
-    for (uint64_t j0 = b; j0 < e; j0 += uint64_t(kIterBigThreads) * kEdgeBatch) {
+__global__ void __launch_bounds__(kIterThreads) EdgeBatchBigKernel(const uint32_t* __restrict__ list,
+                                                                  const uint32_t* __restrict__ starts,
+                                                                  const uint64_t* __restrict__ off, RowPieces c, F f,
+                                                                  R row) {
+  const unsigned tid = threadIdx.x;
+  ForBigItems(list, starts, off, c, row, [&](uint32_t vr, uint64_t b, uint32_t len) {
+    for (uint32_t e0 = 0; e0 < len; e0 += kIterThreads * kEdgeBatch) {
       uint32_t v[kEdgeBatch];
       uint64_t j[kEdgeBatch];
 #pragma unroll
       for (int k = 0; k < kEdgeBatch; ++k) {
-        j[k] = j0 + uint64_t(kIterBigThreads) * k + threadIdx.x;
-        v[k] = j[k] < e ? vr : kNone;
+        const uint32_t e = e0 + kIterThreads * k + tid;
+        j[k] = b + e;
+        v[k] = e < len ? vr : kNone;
       }
       f(v, j);
     }
-  }
+  });
 }
 
 template <class F, class R = RowAll>
-inline void LaunchEdgeBatch(Context* ctx, const BinSet& bins, const uint64_t* off, F f, R row = R()) {
+inline void LaunchEdgeBatch(Context* ctx, const DevGraph& g, F f, R row = R()) {
+  const BinSet& bins = g.bins;
+  const uint64_t* off = g.off.p;
   auto any = [&](int b0, int b1) {
     for (int b = b0; b < b1; ++b)
       if (bins.host_counts[b]) return true;
@@ -274,7 +320,7 @@ inline void LaunchEdgeBatch(Context* ctx, const BinSet& bins, const uint64_t* of
     PCC_COUNT(1);
   }
   if (any(kBinCta, kNumBins)) {
-    EdgeBatchBigKernel<F, R><<<IterBigGrid(ctx), kIterBigThreads, 0, st>>>(list, starts, off, f, row);
+    EdgeBatchBigKernel<F, R><<<IterMidGrid(ctx), kIterThreads, 0, st>>>(list, starts, off, PiecesOf(g), f, row);
     PCC_COUNT(1);
   }
 }
@@ -333,67 +379,32 @@ __global__ void __launch_bounds__(kIterThreads) PushMidKernel(const uint32_t* __
   }
 }
 
-// Rows of more than kHubSmallMax entries in pieces (HubPlan).
-struct PushChunks {
-  const uint32_t* big_v;
-  const uint32_t* chunk_hub;
-  const uint32_t* chunk_start;
-  uint32_t num;
-};
-
-// The pieces of the longest rows, then the rows of bin Cta, dealt to the CTAs.
-// Each thread first looks up one of the CTA's items (five dependent loads), so
-// that the chain is paid once for 256 items, and a row of any length is spread
-// over the GPU.  (RMAT scale 20, largest row 86k entries, a CTA of 512 threads
-// per row: 96 us a round; 11.)
+// The longest rows, in pieces dealt to all CTAs.  (RMAT scale 20, largest row
+// 86k entries, a CTA of 512 threads per row: 96 us a round; 11.)
 template <class R>
 __global__ void __launch_bounds__(kIterThreads) PushBigKernel(const uint32_t* __restrict__ list,
                                                              const uint32_t* __restrict__ starts,
                                                              const uint64_t* __restrict__ off,
                                                              const uint32_t* __restrict__ nbr,
                                                              uint32_t* __restrict__ stamp, StampValue sv,
-                                                             PushChunks c, uint32_t chunk, R row) {
-  __shared__ uint64_t from[kIterThreads];
-  __shared__ uint32_t len[kIterThreads];
-  const uint32_t s0 = starts[kBinCta];
-  const uint64_t items = uint64_t(c.num) + (starts[kBinGlobal] - s0);
+                                                             RowPieces c, R row) {
   const uint32_t value = StampIn(sv.rs, sv.stamp);
   const unsigned tid = threadIdx.x;
-  for (uint64_t base = blockIdx.x; base < items; base += uint64_t(gridDim.x) * kIterThreads) {
-    const uint64_t it = base + uint64_t(gridDim.x) * tid;
-    uint64_t b = 0;
-    uint32_t n = 0;
-    if (it < items) {
-      const bool piece = it < c.num;
-      const uint32_t v = piece ? c.big_v[c.chunk_hub[it]] : list[s0 + (it - c.num)];
-      const uint64_t o0 = off[v], o1 = off[v + 1];
-      b = o0 + (piece ? c.chunk_start[it] : 0u);
-      if (row(v)) n = static_cast<uint32_t>(piece ? min(o1 - b, uint64_t(chunk)) : o1 - b);
-    }
-    from[tid] = b;
-    len[tid] = n;
-    __syncthreads();
-    const uint64_t left = (items - base + gridDim.x - 1) / gridDim.x;
-    const int count = left < kIterThreads ? int(left) : kIterThreads;
-    for (int q = 0; q < count; ++q) {
-      const uint64_t b0 = from[q];
-      const uint32_t l = len[q];
-      for (uint32_t j0 = 0; j0 < l; j0 += kIterThreads * kPushBatch) {
-        uint32_t u[kPushBatch], cur[kPushBatch];
+  ForBigItems(list, starts, off, c, row, [&](uint32_t, uint64_t b, uint32_t len) {
+    for (uint32_t e0 = 0; e0 < len; e0 += kIterThreads * kPushBatch) {
+      uint32_t u[kPushBatch], cur[kPushBatch];
 #pragma unroll
-        for (int k = 0; k < kPushBatch; ++k) {
-          const uint32_t j = j0 + kIterThreads * k + tid;
-          u[k] = j < l ? nbr[b0 + j] : kNone;
-        }
-#pragma unroll
-        for (int k = 0; k < kPushBatch; ++k) cur[k] = u[k] != kNone ? stamp[u[k]] : value;
-#pragma unroll
-        for (int k = 0; k < kPushBatch; ++k)
-          if (cur[k] != value) stamp[u[k]] = value;
+      for (int k = 0; k < kPushBatch; ++k) {
+        const uint32_t e = e0 + kIterThreads * k + tid;
+        u[k] = e < len ? nbr[b + e] : kNone;
       }
+#pragma unroll
+      for (int k = 0; k < kPushBatch; ++k) cur[k] = u[k] != kNone ? stamp[u[k]] : value;
+#pragma unroll
+      for (int k = 0; k < kPushBatch; ++k)
+        if (cur[k] != value) stamp[u[k]] = value;
     }
-    __syncthreads();
-  }
+  });
 }
 
 struct PushStampFn {
@@ -416,8 +427,7 @@ struct PushStampFn {
 
 // The push over a graph's static bins.
 template <class R>
-inline void LaunchPush(Context* ctx, const DevGraph& g, const PushChunks& hub_rows, uint32_t* stamp, StampValue sv,
-                       R row) {
+inline void LaunchPush(Context* ctx, const DevGraph& g, uint32_t* stamp, StampValue sv, R row) {
   const BinSet& bins = g.bins;
   auto any = [&](int b0, int b1) {
     for (int b = b0; b < b1; ++b)
@@ -436,8 +446,8 @@ inline void LaunchPush(Context* ctx, const DevGraph& g, const PushChunks& hub_ro
     PCC_COUNT(1);
   }
   if (any(kBinCta, kNumBins)) {
-    PushBigKernel<R><<<IterMidGrid(ctx), kIterThreads, 0, st>>>(list, starts, g.off.p, g.nbr.p, stamp, sv, hub_rows,
-                                                                kLoopChunk, row);
+    PushBigKernel<R><<<IterMidGrid(ctx), kIterThreads, 0, st>>>(list, starts, g.off.p, g.nbr.p, stamp, sv,
+                                                                PiecesOf(g), row);
     PCC_COUNT(1);
   }
 }

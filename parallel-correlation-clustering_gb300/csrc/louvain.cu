@@ -928,13 +928,11 @@ class Engine {
     // degree bins with a marked-row predicate, then the next frontier's size.
     timer_.Begin(kPhaseFrontier);
     const StampValue sv{stamp_, rs};
-    const PushChunks hub_rows{g.hub_plan->big_v, g.hub_plan->chunk_hub, g.hub_plan->chunk_start,
-                              g.hub_plan->num_chunks};
     if (cfg_.move_method == PCC_NBHR_CLUSTER_MOVE) {
-      LaunchPush(ctx_, g, hub_rows, next_stamp_.p, sv,
+      LaunchPush(ctx_, g, next_stamp_.p, sv,
                  PredModifiedCluster{L->C.p, mod_stamp_.p, stamp_, rs});  // rows with d > 0
     } else {
-      LaunchPush(ctx_, g, hub_rows, next_stamp_.p, sv, PredStamp{moved_stamp_.p, stamp_, rs});
+      LaunchPush(ctx_, g, next_stamp_.p, sv, PredStamp{moved_stamp_.p, stamp_, rs});
     }
     if (n) {
       CountDegreesKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, g.off.p, PredStamp{next_stamp_.p, stamp_, rs},
