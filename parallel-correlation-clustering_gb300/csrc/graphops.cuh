@@ -334,7 +334,7 @@ inline void LaunchEdgeBatch(Context* ctx, const DevGraph& g, F f, R row = R()) {
 // already equal to the value is not stored again: hub vertices are
 // neighbours of a large share of all rows, and same-address stores
 // serialise at their L2 slice while the loads are served by L1.  Without hubs
-// (`blind`) small rows store without a look: the look at a line that other
+// (`blind`) rows are stored without a look: the look at a line that other
 // SMs write makes it travel between the dies (120,001 vertices, 1.9M entries:
 // 43 us with it, 24 without).  The line is 4,096 entries a vertex, as many
 // stores as can queue at one address: an RMAT graph of scale 22 takes the same
@@ -347,34 +347,48 @@ struct StampValue {
   const RoundState* rs;  // non-null: the value comes from here
 };
 
+// Rows of the warp bins: each lane looks up one of the warp's next 32 rows (a
+// chain of dependent loads, paid once), then the warp walks the marked ones.
 template <class R>
 __global__ void __launch_bounds__(kIterThreads) PushMidKernel(const uint32_t* __restrict__ list,
                                                              const uint32_t* __restrict__ starts,
                                                              const uint64_t* __restrict__ off,
                                                              const uint32_t* __restrict__ nbr,
-                                                             uint32_t* __restrict__ stamp, StampValue sv, R row) {
+                                                             uint32_t* __restrict__ stamp, StampValue sv, bool blind,
+                                                             R row) {
   const uint32_t s0 = starts[kBinW128];
   const uint32_t count = starts[kBinCta] - s0;  // bins W128..W1000
   const unsigned lane = LaneId(), warp = threadIdx.x >> 5;
   const uint32_t value = StampIn(sv.rs, sv.stamp);
-  for (uint64_t i = uint64_t(blockIdx.x) * (kIterThreads / 32) + warp; i < count;
-       i += uint64_t(gridDim.x) * (kIterThreads / 32)) {
-    const uint32_t v = list[s0 + i];
-    if (!row(v)) continue;
-    const uint64_t b = off[v], e = off[v + 1];
-    for (uint64_t j0 = b; j0 < e; j0 += 32 * kPushBatch) {
-      uint32_t u[kPushBatch];
-#pragma unroll
-      for (int k = 0; k < kPushBatch; ++k) {
-        const uint64_t j = j0 + 32 * k + lane;
-        u[k] = j < e ? nbr[j] : kNone;
+  const uint64_t warps = uint64_t(gridDim.x) * (kIterThreads / 32);
+  for (uint64_t i0 = uint64_t(blockIdx.x) * (kIterThreads / 32) + warp; i0 < count; i0 += 32 * warps) {
+    const uint64_t i = i0 + warps * lane;
+    uint64_t b = 0;
+    uint32_t len = 0;
+    if (i < count) {
+      const uint32_t v = list[s0 + i];
+      if (row(v)) {
+        b = off[v];
+        len = static_cast<uint32_t>(off[v + 1] - b);
       }
-      uint32_t cur[kPushBatch];
+    }
+    for (unsigned left = __ballot_sync(kFull, len != 0); left; left &= left - 1) {
+      const int q = __ffs(left) - 1;
+      const uint64_t bq = __shfl_sync(kFull, b, q);
+      const uint32_t lq = __shfl_sync(kFull, len, q);
+      for (uint32_t e0 = 0; e0 < lq; e0 += 32 * kPushBatch) {
+        uint32_t u[kPushBatch], cur[kPushBatch];
 #pragma unroll
-      for (int k = 0; k < kPushBatch; ++k) cur[k] = u[k] != kNone ? stamp[u[k]] : value;
+        for (int k = 0; k < kPushBatch; ++k) {
+          const uint32_t e = e0 + 32 * k + lane;
+          u[k] = e < lq ? nbr[bq + e] : kNone;
+        }
 #pragma unroll
-      for (int k = 0; k < kPushBatch; ++k)
-        if (cur[k] != value) stamp[u[k]] = value;
+        for (int k = 0; k < kPushBatch; ++k) cur[k] = u[k] == kNone ? value : blind ? ~value : stamp[u[k]];
+#pragma unroll
+        for (int k = 0; k < kPushBatch; ++k)
+          if (cur[k] != value) stamp[u[k]] = value;
+      }
     }
   }
 }
@@ -434,15 +448,16 @@ inline void LaunchPush(Context* ctx, const DevGraph& g, uint32_t* stamp, StampVa
       if (bins.host_counts[b]) return true;
     return false;
   };
+  const bool blind = g.max_deg <= kHubSmallMax;
   const uint32_t *list = bins.list.p, *starts = bins.counts.p + kNumBins;
   cudaStream_t st = ctx->stream;
   if (any(kBinG4, kBinW128)) {
     EdgeBatchSmallKernel<PushStampFn, R><<<IterSmallGrid(ctx), kIterThreads, 0, st>>>(
-        list, starts, g.off.p, PushStampFn{g.nbr.p, stamp, sv, g.max_deg <= kHubSmallMax}, row);
+        list, starts, g.off.p, PushStampFn{g.nbr.p, stamp, sv, blind}, row);
     PCC_COUNT(1);
   }
   if (any(kBinW128, kBinCta)) {
-    PushMidKernel<R><<<IterMidGrid(ctx), kIterThreads, 0, st>>>(list, starts, g.off.p, g.nbr.p, stamp, sv, row);
+    PushMidKernel<R><<<IterMidGrid(ctx), kIterThreads, 0, st>>>(list, starts, g.off.p, g.nbr.p, stamp, sv, blind, row);
     PCC_COUNT(1);
   }
   if (any(kBinCta, kNumBins)) {

@@ -393,24 +393,62 @@ __global__ void __launch_bounds__(kT) AssignNewUnionKernel(ApplyArgs a, const ui
 }
 
 // Per graph: flags[j] = stamp when the frontier (st == stamp) holds a vertex
-// of graph j, and edges[j] += the degrees of those vertices.
+// of graph j, and edges[j] += the degrees of those vertices; and the whole
+// frontier's size and degree sum.  A warp takes a contiguous span, so that it
+// looks its graph up when it enters one, not per vertex.  (1.3M vertices, 128
+// graphs: a search and an atomic per vertex and 32 vertices 28 us, with a
+// second pass for the totals 36; 13.)
 __global__ void __launch_bounds__(kT) GraphFrontierKernel(uint32_t n, const uint64_t* __restrict__ off,
                                                           const uint32_t* __restrict__ st, uint32_t stamp_arg,
                                                           const RoundState* rs, const uint32_t* __restrict__ vbase,
-                                                          uint32_t B, uint32_t* flags, unsigned long long* edges) {
+                                                          uint32_t B, uint32_t* flags, unsigned long long* edges,
+                                                          DevCounters* ctr) {
+  __shared__ unsigned long long block_deg;
+  __shared__ uint32_t block_count;
   const uint32_t stamp = StampIn(rs, stamp_arg);
-  const uint64_t limit = (uint64_t(n) + 31) & ~uint64_t(31);
-  for (uint64_t v = uint64_t(blockIdx.x) * kT + threadIdx.x; v < limit; v += uint64_t(gridDim.x) * kT) {
-    const bool in = v < n && st[v] == stamp;
-    const uint32_t j = in ? GraphOf(vbase, B, static_cast<uint32_t>(v)) : kNone;
-    const unsigned long long d = in ? off[v + 1] - off[v] : 0ull;
-    const unsigned peers = __match_any_sync(kFull, j);
-    unsigned long long tot = 0;
-    for (unsigned mm = peers; mm; mm &= mm - 1) tot += __shfl_sync(peers, d, __ffs(mm) - 1);
-    if (in && int(LaneId()) == __ffs(peers) - 1) {
-      if (flags[j] != stamp) flags[j] = stamp;
-      if (tot) atomicAdd(&edges[j], tot);
+  const unsigned lane = LaneId();
+  if (threadIdx.x == 0) {
+    block_deg = 0;
+    block_count = 0;
+  }
+  __syncthreads();
+  const uint64_t warps = uint64_t(gridDim.x) * (kT / 32);
+  const uint64_t span = ((uint64_t(n) + warps - 1) / warps + 31) & ~uint64_t(31);
+  const uint64_t lo = (uint64_t(blockIdx.x) * (kT / 32) + (threadIdx.x >> 5)) * span;
+  const uint64_t hi = min(uint64_t(n), lo + span);
+  unsigned long long all_deg = 0;
+  uint32_t all_count = 0;
+  for (uint64_t at = lo; at < hi;) {
+    const uint32_t j = GraphOf(vbase, B, static_cast<uint32_t>(at));
+    const uint64_t end = min(hi, uint64_t(vbase[j + 1]));
+    unsigned long long deg = 0;
+    uint32_t count = 0;
+    for (uint64_t v = at + lane; v < end; v += 32) {
+      if (st[v] != stamp) continue;
+      deg += off[v + 1] - off[v];
+      count++;
     }
+    count = __reduce_add_sync(kFull, count);
+    if (count) {
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) deg += __shfl_xor_sync(kFull, deg, o);
+      if (lane == 0) {
+        flags[j] = stamp;
+        if (deg) atomicAdd(&edges[j], deg);
+      }
+      all_deg += deg;
+      all_count += count;
+    }
+    at = end;
+  }
+  if (lane == 0 && all_count) {
+    atomicAdd(&block_deg, all_deg);
+    atomicAdd(&block_count, all_count);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && block_count) {
+    atomicAdd(&ctr->pend_edges, block_deg);
+    atomicAdd(&ctr->frontier, block_count);
   }
 }
 
@@ -935,15 +973,16 @@ class Engine {
       LaunchPush(ctx_, g, next_stamp_.p, sv, PredStamp{moved_stamp_.p, stamp_, rs});
     }
     if (n) {
-      CountDegreesKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, g.off.p, PredStamp{next_stamp_.p, stamp_, rs},
-                                                                    &ctr_.p->pend_edges, &ctr_.p->frontier);
-      PCC_COUNT(1);
       if (un_) {
         PCC_RETURN_IF_ERROR(gedges_.Zero());
         GraphFrontierKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(n, g.off.p, next_stamp_.p, stamp_, rs,
-                                                                       un_->d_vbase.p, un_->B, gflags_.p,
-                                                                       gedges_.p); PCC_COUNT(1);
+                                                                       un_->d_vbase.p, un_->B, gflags_.p, gedges_.p,
+                                                                       ctr_.p);
+      } else {
+        CountDegreesKernel<<<GridFor(ctx_, n), kT, 0, ctx_->stream>>>(
+            n, g.off.p, PredStamp{next_stamp_.p, stamp_, rs}, &ctr_.p->pend_edges, &ctr_.p->frontier);
       }
+      PCC_COUNT(1);
     }
     PCC_RETURN_IF_ERROR(LaunchCheck());
     timer_.End(kPhaseFrontier);
