@@ -174,7 +174,7 @@ struct StampInput {
   __device__ uint32_t operator()(uint64_t i) const { return st[i] == stamp ? 1u : 0u; }
 };
 
-__global__ void GatherKernel(uint32_t n, const uint32_t* __restrict__ idx, const uint32_t* __restrict__ table,
+__global__ void GatherKernel(uint32_t n, const uint32_t* idx, const uint32_t* __restrict__ table,
                              uint32_t* out) {
   for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
     out[i] = table[idx[i]];
@@ -582,12 +582,24 @@ struct ArrayInputF64 {
   __device__ double operator()(uint64_t i) const { return a[i]; }
 };
 
+// Entries inside a cluster: one atomic per 128 entries, over kCountSlots
+// addresses.
+constexpr uint32_t kCountSlots = 1024;
 struct SameLabelCount {
   const uint32_t* nbr;
   const uint32_t* L;
   unsigned long long* acc;
-  __device__ void operator()(uint32_t u, uint64_t j, uint64_t slot) const {
-    if (L[u] == L[nbr[j]]) acc[slot] += 1ull;
+  __device__ void operator()(const uint32_t (&u)[kEdgeBatch], const uint64_t (&j)[kEdgeBatch]) const {
+    uint32_t v[kEdgeBatch];
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k) v[k] = u[k] != kNone ? nbr[j[k]] : kNone;
+    uint32_t same = 0;
+#pragma unroll
+    for (int k = 0; k < kEdgeBatch; ++k) same += u[k] != kNone && L[u[k]] == L[v[k]] ? 1u : 0u;
+    same = __reduce_add_sync(kFull, same);
+    if (LaneId() == 0 && same)
+      atomicAdd(&acc[(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) % kCountSlots],
+                static_cast<unsigned long long>(same));
   }
 };
 
@@ -1932,17 +1944,15 @@ Status ComputeModularityDevice(Context* ctx, const DevGraph& g, const uint32_t* 
     return Status::Ok();
   }
   DBuf<unsigned long long> cnt, deg;
-  const uint64_t slots = EdgeIterSlots(ctx);
-  PCC_RETURN_IF_ERROR(cnt.Alloc(ctx, slots));
+  PCC_RETURN_IF_ERROR(cnt.Alloc(ctx, kCountSlots));
   PCC_RETURN_IF_ERROR(cnt.Zero());
   PCC_RETURN_IF_ERROR(deg.Alloc(ctx, n));
   PCC_RETURN_IF_ERROR(deg.Zero());
-  LaunchEdgeIter(ctx, g.bins.list.p, g.bins.counts.p, g.bins.counts.p + kNumBins, g.bins.host_counts, g.off.p,
-                 SameLabelCount{g.nbr.p, L, cnt.p});
+  LaunchEdgeBatch(ctx, g, SameLabelCount{g.nbr.p, L, cnt.p});
   DegreeSumKernel<<<GridFor(ctx, n), kT, 0, ctx->stream>>>(n, g.off.p, L, deg.p); PCC_COUNT(1);
   DBuf<unsigned long long> part64, tot64;
   PCC_RETURN_IF_ERROR(tot64.Alloc(ctx, 1));
-  PCC_RETURN_IF_ERROR(Reduce<unsigned long long>(ctx, slots, U64Input{cnt.p}, OpAdd{}, 0ull, tot64.p, part64));
+  PCC_RETURN_IF_ERROR(Reduce<unsigned long long>(ctx, kCountSlots, U64Input{cnt.p}, OpAdd{}, 0ull, tot64.p, part64));
   const double total = static_cast<double>(g.m);
   DBuf<double> part, sum;
   PCC_RETURN_IF_ERROR(sum.Alloc(ctx, 1));
@@ -1954,6 +1964,20 @@ Status ComputeModularityDevice(Context* ctx, const DevGraph& g, const uint32_t* 
   PCC_RETURN_IF_ERROR(Sync(ctx));
   *out = (static_cast<double>(same) - sub) / total;
   return Status::Ok();
+}
+
+// labels[i] = rank of labels[i] among the labels in use.  (500,009 labels with
+// two random host passes: 0.7 ms; on the device 0.04.)
+Status DenseLabels(Context* ctx, uint32_t n, uint32_t* labels) {
+  DBuf<uint32_t> present, rank, tiles;
+  PCC_RETURN_IF_ERROR(present.Alloc(ctx, n));
+  PCC_RETURN_IF_ERROR(present.Zero());
+  PCC_RETURN_IF_ERROR(rank.Alloc(ctx, n));
+  MarkStampKernel<<<GridFor(ctx, n), kT, 0, ctx->stream>>>(n, labels, present.p, 1u); PCC_COUNT(1);
+  PCC_RETURN_IF_ERROR(ScanApply<uint32_t>(ctx, n, StampInput{present.p, 1u}, StorePrefix<uint32_t>{rank.p}, tiles,
+                                          static_cast<uint32_t*>(nullptr)));
+  GatherKernel<<<GridFor(ctx, n), kT, 0, ctx->stream>>>(n, labels, rank.p, labels); PCC_COUNT(1);
+  return LaunchCheck();
 }
 
 Status ValidateGraphArgs(pcc_context* ctx, const pcc_graph* graph, const pcc_config* cfg) {
@@ -1969,6 +1993,9 @@ Status ValidateGraphArgs(pcc_context* ctx, const pcc_graph* graph, const pcc_con
 
 Status CheckLabels(const uint32_t* labels, uint32_t n) {
   if (!labels) return Status::Ok();
+  uint32_t top = 0;  // (a loop without an exit, which the compiler vectorises)
+  for (uint32_t i = 0; i < n; ++i) top = std::max(top, labels[i]);
+  if (top < n) return Status::Ok();
   for (uint32_t i = 0; i < n; ++i)
     if (labels[i] >= n)
       return MakeError(PCC_INVALID_ARGUMENT, "label of node " + std::to_string(i) + " is " +
@@ -2402,18 +2429,10 @@ pcc_status pcc_modularity(pcc_context* pctx, const pcc_graph* graph, double reso
     Context* ctx = &pctx->c;
     const uint32_t n = graph->g.n;
     // ComputeModularity walks the clustering in id order; dense ranks give it.
-    std::vector<uint32_t> present(n, 0), dense(n);
-    for (uint32_t i = 0; i < n; ++i) present[labels[i]] = 1;
-    uint32_t acc = 0;
-    for (uint32_t i = 0; i < n; ++i) {
-      const uint32_t p = present[i];
-      present[i] = acc;
-      acc += p;
-    }
-    for (uint32_t i = 0; i < n; ++i) dense[i] = present[labels[i]];
     DBuf<uint32_t> dl;
     st = dl.Alloc(ctx, std::max<uint64_t>(n, 1));
-    if (st.ok()) st = dl.FromHost(dense.data(), n);
+    if (st.ok()) st = dl.FromHost(labels, n);
+    if (st.ok() && n) st = DenseLabels(ctx, n, dl.p);
     if (st.ok()) st = ComputeModularityDevice(ctx, graph->g, dl.p, resolution, out_modularity);
   }
   return Finish(pctx, st);
