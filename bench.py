@@ -367,7 +367,7 @@ def lfr_leg(args, P, G, ctx, dist_steps: int = 2):
     score_ms = (time.perf_counter() - t) * 1000.0
     out = {
         "workload": "lfr_like_real_weights_correlation_refine_nbhr_cluster_sync",
-        "n": g.n, "m_entries": g.m, "dtype": "f64 (real weights: FP64 best moves)",
+        "n": g.n, "m_entries": g.m, "dtype": "f64 (real weights: exact 64-bit fixed-point sums, FP64 where the FP32 bounds do not decide)",
         "value": ev / (ms / 1000.0), "unit": UNIT, "ms_per_step": ms / dist_steps,
         "objective": st["objective"], "num_clusters": st["num_clusters"], "levels": st["levels"],
         "rounds": st["rounds"], "mean_degree": g.m / g.n,

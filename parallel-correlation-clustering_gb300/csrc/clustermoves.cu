@@ -879,7 +879,7 @@ Status FindClusterMovesExact(Context* ctx, const DevGraph& g, const uint32_t* C,
   CmWeightKernel<<<grid_n, 256, 0, st>>>(n, C, k, t->W.p);
   CmStayKernel<<<grid_n, 256, 0, st>>>(n, t->W.p, K, res, t->stay.p);
   PCC_COUNT(2);
-  LaunchEdgeBatch(ctx, g,
+  LaunchEdgeBatch(ctx, g, PiecesOf(g),
                   CmTableInsert{g.nbr.p, g.wp(), C, offset, t->cap, t->keys.p, t->sums.p, &ctr->error});
   const CmTableArgs a{t->cap, t->keys.p, t->sums.p, t->W.p, K, res, t->stay.p, t->best_bits.p, t->best_id.p};
   const unsigned grid_t = Blocks(t->cap, 256 * 4, ctx->num_sms * 8);

@@ -811,14 +811,15 @@ class Scratch {
 }  // namespace
 
 // Contracts g by C (device uint32[n], ids < n); k = node weights (device, or
-// null for 1).  The new graph carries its node weights in node_w.
+// null for 1).  The new graph carries its node weights in node_w.  planned:
+// the caller has had EnsureHubPlan (long rows then move in pieces).
 //
 // Host waits: the number of clusters; the segment classes, when a segment may
 // be longer than a CTA holds (the shorter ones are sorted meanwhile); the new
 // graph's size and properties together (above 16M entries its size alone
 // before, so that its arrays are not allocated at the old size).  A level of
 // 4,686 entries takes 3 waits and 18 kernels, 0.40 -> 0.2 ms.
-Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k,
+Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k, bool planned,
                      std::unique_ptr<DevGraph>* out) {
   const uint32_t n = g.n;
   cudaStream_t st = ctx->stream;
@@ -904,7 +905,7 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
     // Every row moved into its cluster's segment.
     PCC_RETURN_IF_ERROR(sc.Take(&akey, g.m));
     PCC_RETURN_IF_ERROR(sc.Take(&aval, g.m));
-    LaunchEdgeBatch(ctx, g, MoveEntries{g.off.p, g.nbr.p, g.wp(), vrank, dstart, drop, akey, aval});
+    LaunchEdgeBatch(ctx, g, planned ? PiecesOf(g) : RowPieces{}, MoveEntries{g.off.p, g.nbr.p, g.wp(), vrank, dstart, drop, akey, aval});
     PCC_RETURN_IF_ERROR(LaunchCheck());
     sc.Done(dstart);
     sc.Done(vrank);

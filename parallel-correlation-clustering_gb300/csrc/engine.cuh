@@ -420,6 +420,8 @@ Status LaunchBestMoves(Context* ctx, const BMArgs& a, const uint32_t* list, cons
 // sums 6.6 -> 6.5 ms, 20M with 64-bit sums 10.2 -> 12.4 ms, 31.4M 11.9 ->
 // 12.7 ms: above it the tails and launches that the one kernel saves are
 // small, and the binned kernels' higher occupancy wins.
+// (With certified hubs and the push in pieces on the binned side too, a line at
+// 2M or 6M entries still costs RMAT scale 18 17.9 -> 19.6 ms.)
 constexpr uint64_t kLoopMaxEntries = 12ull << 20;
 
 // The hub plan of a graph (built on first use).

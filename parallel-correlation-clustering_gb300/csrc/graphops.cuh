@@ -169,8 +169,9 @@ struct RowPieces {
   const uint32_t* chunk_start;
   uint32_t num;
 };
+// (For callers that have had EnsureHubPlan; the others take RowPieces{}: another
+// thread may be building the plan.)
 inline RowPieces PiecesOf(const DevGraph& g) {
-  if (!g.hub_plan) return RowPieces{};
   return RowPieces{g.hub_plan->big_v, g.hub_plan->chunk_hub, g.hub_plan->chunk_start, g.hub_plan->num_chunks};
 }
 
@@ -301,7 +302,7 @@ __global__ void __launch_bounds__(kIterThreads) EdgeBatchBigKernel(const uint32_
 }
 
 template <class F, class R = RowAll>
-inline void LaunchEdgeBatch(Context* ctx, const DevGraph& g, F f, R row = R()) {
+inline void LaunchEdgeBatch(Context* ctx, const DevGraph& g, const RowPieces& pieces, F f, R row = R()) {
   const BinSet& bins = g.bins;
   const uint64_t* off = g.off.p;
   auto any = [&](int b0, int b1) {
@@ -320,7 +321,7 @@ inline void LaunchEdgeBatch(Context* ctx, const DevGraph& g, F f, R row = R()) {
     PCC_COUNT(1);
   }
   if (any(kBinCta, kNumBins)) {
-    EdgeBatchBigKernel<F, R><<<IterMidGrid(ctx), kIterThreads, 0, st>>>(list, starts, off, PiecesOf(g), f, row);
+    EdgeBatchBigKernel<F, R><<<IterMidGrid(ctx), kIterThreads, 0, st>>>(list, starts, off, pieces, f, row);
     PCC_COUNT(1);
   }
 }

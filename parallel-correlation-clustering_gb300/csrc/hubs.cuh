@@ -5,16 +5,19 @@
 // correlation-clusterer-internal.cc:516-582).  Here a hub's neighbour-cluster
 // sums live in shared memory only:
 //
-//   small hubs (1000 < degree <= kHubSmallMax): one 256-thread CTA per hub,
-//     a table of at least 2 * degree + 2 slots, so it never fills (4096
-//     slots up to degree 2047, else 8192);
+//   small hubs (1000 < degree <= kHubSmallMax): one CTA per hub with a table
+//     that never fills: 4096 slots up to degree 2047, else 8192.  Synchronous
+//     exact sums take the certified path over the used slots (HubCertKernel,
+//     8 or 16 warps); FP64 mode and async evaluate the table (HubSmallKernel,
+//     256 threads, 6144 slots in between);
 //   big hubs (degree > kHubSmallMax): one 1024-thread CTA per (hub,
 //     partition) with a ~192 KB table.  Hubs with more than kHubBigKeys
 //     distinct neighbour clusters are split into P hash partitions (P =
 //     ceil(degree / kHubBigKeys)), whose CTAs re-read the row from L2.  A
 //     partition whose keys overflow its table is split again by further hash
 //     bits and rescanned (sub-passes), so correctness does not depend on the
-//     hash distribution.
+//     hash distribution.  Hubs of one partition (degree <= kHubBigKeys) take
+//     HubCertKernel too (16,384 slots, 32 warps) where small hubs do.
 //
 // Each CTA evaluates its table (FP32 pre-filter, exact FP64 values of the
 // survivors, argmax by value desc / id asc); for big hubs the partitions'

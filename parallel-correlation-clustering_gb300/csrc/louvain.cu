@@ -24,7 +24,7 @@
 
 namespace pcc {
 
-Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k,
+Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k, bool planned,
                      std::unique_ptr<DevGraph>* out);
 Status FindClusterMoves(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k, const double* K,
                         double res, double offset, uint32_t* moves, uint32_t* movers, DevCounters* ctr);
@@ -1455,7 +1455,7 @@ class Engine {
       if (last) break;
       std::unique_ptr<DevGraph> next;
       timer_.Begin(kPhaseCompress);
-      PCC_RETURN_IF_ERROR(CompressGraph(ctx_, *helper->g, map, helper->k.p, &next));
+      PCC_RETURN_IF_ERROR(CompressGraph(ctx_, *helper->g, map, helper->k.p, true, &next));
       timer_.End(kPhaseCompress);
       res_.algo_bytes_compress += CompressBytes(*helper->g, *next);
       DevGraph* ng = next.get();
@@ -1747,7 +1747,7 @@ class Engine {
       }
       std::unique_ptr<DevGraph> next;
       timer_.Begin(kPhaseCompress);
-      PCC_RETURN_IF_ERROR(CompressGraph(ctx_, *helper->g, helper->C.p, helper->k.p, &next));
+      PCC_RETURN_IF_ERROR(CompressGraph(ctx_, *helper->g, helper->C.p, helper->k.p, true, &next));
       timer_.End(kPhaseCompress);
       res_.algo_bytes_compress += CompressBytes(*helper->g, *next);
       DevGraph* ng = next.get();
@@ -1948,7 +1948,7 @@ Status ComputeModularityDevice(Context* ctx, const DevGraph& g, const uint32_t* 
   PCC_RETURN_IF_ERROR(cnt.Zero());
   PCC_RETURN_IF_ERROR(deg.Alloc(ctx, n));
   PCC_RETURN_IF_ERROR(deg.Zero());
-  LaunchEdgeBatch(ctx, g, SameLabelCount{g.nbr.p, L, cnt.p});
+  LaunchEdgeBatch(ctx, g, RowPieces{}, SameLabelCount{g.nbr.p, L, cnt.p});
   DegreeSumKernel<<<GridFor(ctx, n), kT, 0, ctx->stream>>>(n, g.off.p, L, deg.p); PCC_COUNT(1);
   DBuf<unsigned long long> part64, tot64;
   PCC_RETURN_IF_ERROR(tot64.Alloc(ctx, 1));
@@ -2566,7 +2566,7 @@ pcc_status pcc_compress(pcc_context* pctx, const pcc_graph* graph, const uint32_
       if (st.ok()) st = dk.FromHost(node_weights, n);
     }
     std::unique_ptr<DevGraph> res;
-    if (st.ok()) st = CompressGraph(ctx, graph->g, dC.p, dk.p, &res);
+    if (st.ok()) st = CompressGraph(ctx, graph->g, dC.p, dk.p, false, &res);
     if (st.ok()) st = Sync(ctx);
     if (st.ok()) {
       auto* h = new pcc_graph;

@@ -256,3 +256,16 @@ def test_one_partition_hubs(ctx, kind):
             _same(ctx, g, P.make_config(resolution=res, refine=True, move_method=P.NBHR_CLUSTER_MOVE), modularity)
     finally:
         ctx.set_detailed_timing(False)
+
+
+@pytest.mark.parametrize("labels", ["one", "own", "sparse"])
+def test_modularity_of_given_labels(ctx, labels):
+    """Labels of any spacing: one cluster, singletons, ids far apart."""
+    g = _hub_degrees((1001, 4097, 8500))
+    dg, og = ctx.upload(g), O.OracleGraph(g)
+    rng = np.random.default_rng(1)
+    lab = {"one": np.full(g.n, g.n - 1), "own": np.arange(g.n)[::-1].copy(),
+           "sparse": rng.permutation(g.n)[:37][rng.integers(0, 37, g.n)]}[labels].astype(np.uint32)
+    dense = np.unique(lab, return_inverse=True)[1].astype(np.uint32)
+    assert P.modularity(dg, 0.7, lab) == pytest.approx(O.modularity(og, 0.7, dense), rel=1e-12, abs=1e-12)
+    dg.free()
