@@ -68,8 +68,13 @@ struct DevGraph {
   DBuf<float> w;          // empty => unit weights
   DBuf<double> node_w;    // node weights attached by compression
   BinSet bins;            // static degree bins of the vertices with degree > 0
-  mutable BinSet bins_all;  // all vertices (built on first use)
-  mutable std::shared_ptr<HubPlan> hub_plan;  // degree > 1000 (built on first use)
+  // Built on first use by EnsureAllBins / EnsureHubPlan, under the lock and
+  // complete on the device before they are set: the graph outlives the call
+  // that builds them, and other contexts (their own streams and threads) may
+  // be using the graph.
+  mutable BinSet bins_all;  // all vertices
+  mutable std::shared_ptr<HubPlan> hub_plan;  // degree > 1000
+  std::unique_ptr<std::mutex> lazy_mu = std::make_unique<std::mutex>();
   uint32_t max_deg = 0;
   // Of the weights that a best move reads: in compressed graphs the
   // self-loops are left out (a vertex's own entry is never a candidate).
@@ -424,8 +429,9 @@ Status LaunchBestMoves(Context* ctx, const BMArgs& a, const uint32_t* list, cons
 // 2M or 6M entries still costs RMAT scale 18 17.9 -> 19.6 ms.)
 constexpr uint64_t kLoopMaxEntries = 12ull << 20;
 
-// The hub plan of a graph (built on first use).
-Status EnsureHubPlan(Context* ctx, const DevGraph* g);
+// The hub plan of a graph (built on first use).  shared: other contexts may
+// use the graph (a caller's; not the level graphs of one call).
+Status EnsureHubPlan(Context* ctx, const DevGraph* g, bool shared = true);
 
 }  // namespace pcc
 

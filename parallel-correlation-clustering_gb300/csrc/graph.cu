@@ -60,17 +60,23 @@ Status BuildBins(Context* ctx, const DevGraph* g, BinSet* b, bool include_isolat
 
 }  // namespace
 
-Status EnsureHubPlan(Context* ctx, const DevGraph* g) {
+Status EnsureHubPlan(Context* ctx, const DevGraph* g, bool shared) {
+  std::lock_guard<std::mutex> lk(*g->lazy_mu);
   if (g->hub_plan) return Status::Ok();
   auto plan = std::make_shared<HubPlan>();
   PCC_RETURN_IF_ERROR(BuildHubPlan(ctx, *g, g->bins, plan.get()));
+  if (shared && plan->num_hubs) PCC_RETURN_IF_ERROR(Sync(ctx));
   g->hub_plan = std::move(plan);
   return Status::Ok();
 }
 
 Status EnsureAllBins(Context* ctx, const DevGraph* g) {
+  std::lock_guard<std::mutex> lk(*g->lazy_mu);
   if (g->bins_all.list.p) return Status::Ok();
-  return BuildBins(ctx, g, &g->bins_all, true);
+  BinSet bins;
+  PCC_RETURN_IF_ERROR(BuildBins(ctx, g, &bins, true));  // (waits for the stream)
+  g->bins_all = std::move(bins);
+  return Status::Ok();
 }
 
 Status ComputeGraphProperties(Context* ctx, DevGraph* g, const WeightStats* d_stats, const uint64_t* d_m) {

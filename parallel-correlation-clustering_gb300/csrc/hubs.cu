@@ -718,7 +718,7 @@ Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan
     plan->glob_base = plan->pack64.p;
     plan->loop_base = plan->pack64.p + loop_base_at;
   }
-  return Status::Ok();  // (a copy from pageable memory has left it when the call returns)
+  return Status::Ok();  // (the host lists are spent; EnsureHubPlan waits for the device where it must)
 }
 
 Status AllocHubState(Context* ctx, const HubPlan& plan, HubState* st) {

@@ -863,7 +863,7 @@ class Engine {
     } else {
       L->bins = &g->bins;
     }
-    PCC_RETURN_IF_ERROR(EnsureHubPlan(ctx_, g));
+    PCC_RETURN_IF_ERROR(EnsureHubPlan(ctx_, g, L->own == nullptr));
     PCC_RETURN_IF_ERROR(AllocHubState(ctx_, *g->hub_plan, &hub_state_));
     *out = std::move(L);
     return Status::Ok();

@@ -3,6 +3,8 @@ edges of the rules that choose between the integer and the FP64 sums and
 between launch shapes, against the oracle (bit for bit: every sum here is
 exact in any order)."""
 
+from concurrent.futures import ThreadPoolExecutor
+
 import numpy as np
 import pytest
 
@@ -269,3 +271,30 @@ def test_modularity_of_given_labels(ctx, labels):
     dense = np.unique(lab, return_inverse=True)[1].astype(np.uint32)
     assert P.modularity(dg, 0.7, lab) == pytest.approx(O.modularity(og, 0.7, dense), rel=1e-12, abs=1e-12)
     dg.free()
+
+
+def test_graph_shared_by_contexts(ctx):
+    """One resident graph clustered by two contexts at once, from two threads:
+    whichever call builds the graph's hub plan and the bins of its isolated
+    vertices, the other finds them complete."""
+    degs = (1500, 4097, 9000, 13000, 40000)
+    g = _hub_degrees(degs, n=45000)
+    g = P.CsrGraph(np.concatenate([g.offsets, np.full(70, g.offsets[-1])]), g.neighbors)  # isolated vertices
+    init = np.random.default_rng(5).integers(0, 300, g.n).astype(np.uint32)
+    cfg = P.make_config(resolution=0.01, refine=True)
+    want = O.correlation_cluster(O.OracleGraph(g), cfg, None, init)[0]
+    other = P.Context(0)
+    try:
+        for _ in range(6):
+            dg = ctx.upload(g)
+            view = P.DeviceGraph(other, dg.handle)
+            try:
+                with ThreadPoolExecutor(2) as pool:
+                    got = list(pool.map(lambda v: P.correlation_cluster(v, cfg, None, init)[0], (dg, view)))
+            finally:
+                view._h = None  # the graph is dg's to free
+            dg.free()
+            for lab in got:
+                np.testing.assert_array_equal(lab, want)
+    finally:
+        other.close()
