@@ -60,7 +60,7 @@ def _run(cmd):
 def build_cuda(force: bool = False, jobs: int = 0, extra_flags=None) -> str:
     os.makedirs(os.path.join(BUILD, "obj"), exist_ok=True)
     sources = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
-    headers = sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + [os.path.join(INCLUDE, "pcc_gb300.h")]
+    headers = sorted(glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h"))) + [os.path.join(INCLUDE, "pcc_gb300.h")]
     nvcc = _nvcc()
     flags = ARCH + ["-O3", "-lineinfo", "-std=c++17", "--fmad=false", "-Xcompiler", "-fPIC",
                     "-Xcompiler", "-ffp-contract=off", "-I" + INCLUDE, "-I" + CSRC]

@@ -27,6 +27,7 @@
 #include <cstddef>
 #include <cstring>
 
+#include "barrier.h"
 #include "certmoves.cuh"
 #include "hubeval.cuh"
 #include "roundloop.cuh"
@@ -56,7 +57,7 @@ struct LoopShared {
   uint32_t ok;
 };
 
-// Grid-wide barrier number `target / gridDim.x` (target: arrivals so far).
+// Grid-wide barrier: waits until `target` arrivals are counted (modulo 2^32).
 // Release and acquire at GPU scope: the writes before it are visible after it,
 // and the L1 lines read before it are dropped.
 __device__ __forceinline__ bool GridSync(LoopShared& sh, uint32_t* count, uint32_t target) {
@@ -69,7 +70,7 @@ __device__ __forceinline__ bool GridSync(LoopShared& sh, uint32_t* count, uint32
       ok = 0;
       for (uint32_t t = 0; t < kSpinLimit; ++t) {
         asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
-        if (c >= target) {
+        if (BarrierReached(c, target)) {
           ok = 1;
           break;
         }
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
   unsigned long long front_edges = rs.front_edges, front_size = rs.front_size, visited = rs.visited;
   const uint32_t n = a.n;
   uint32_t* count = &l.st->barrier;
-  uint32_t arrivals = 0;
+  uint32_t arrivals = kBarrierStart;
   const bool all_move = l.move_method == PCC_ALL_MOVE;
   WarpMoverBuffer mb{sh.mover_buf[warp]};
   // Degree bins of the teams: 257-1000, with 64-bit sums (two table words
@@ -800,6 +801,7 @@ Status RunRoundLoop(Context* ctx, RoundLoopArgs l, const SumMode& mode, const ui
   PCC_RETURN_IF_ERROR(ctx->Pinned(Context::kPinLoop, &stage));
   std::memset(stage, 0, kSent);
   std::memcpy(stage, head, sizeof(LoopHead));
+  std::memcpy(stage + offsetof(LoopState, barrier), &kBarrierStart, sizeof(kBarrierStart));
   PCC_CUDA(cudaMemcpyAsync(l.st, stage, kSent, cudaMemcpyHostToDevice, ctx->stream));
   if (!mode.narrow) {
     PCC_RETURN_IF_ERROR((LaunchLoop<long long, true>(ctx, l)));

@@ -20,7 +20,8 @@ struct LoopCounters {
 // Device state of the kernel: the counter sets, the grid barrier and each
 // CTA's counts of empty ids and new movers in its slice of the vertices.
 constexpr uint32_t kLoopMaxCtas = 1024;
-// Sent before and read after a run (with the counters, zero at its start).
+// Sent before and read after a run (with the counters, zero at its start, and
+// the barrier's count).
 struct LoopHead {
   RoundState rs;             // in: stamp and the round-0 frontier; out: the last stamp
   uint32_t level_moved;      // some round's next frontier was not empty
