@@ -118,6 +118,9 @@ struct Context {
   cudaEvent_t fork_ev = nullptr;
   cudaEvent_t join_ev[kSideStreams] = {nullptr, nullptr, nullptr};
   bool overlap_families = true;  // off: every family on `stream` in turn
+  // Polls of the round kernel's grid barrier before it gives up (about two
+  // seconds; roundloop.cu).
+  uint32_t barrier_polls = 1u << 22;
   // Best-move launch shape set by pcc_set_launch_tuning (tuned false: the
   // compiled-in table by graph size).
   bool tuned = false;

@@ -330,6 +330,9 @@ pcc_status pcc_create(pcc_context** out, int device, uint64_t hbm_budget_bytes) 
   // other on the context stream instead of as parallel branches (same
   // results; for comparisons).
   if (const char* e = std::getenv("PCC_SERIAL_FAMILIES")) c.overlap_families = std::strcmp(e, "1") != 0;
+  // PCC_BARRIER_POLLS: the round kernel's limit, for tests of what happens when
+  // a barrier gives up (0: every CTA does, at its first one).
+  if (const char* e = std::getenv("PCC_BARRIER_POLLS")) c.barrier_polls = uint32_t(std::strtoul(e, nullptr, 10));
   if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete h;
     return PCC_UNAVAILABLE;

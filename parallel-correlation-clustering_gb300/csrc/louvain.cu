@@ -1337,6 +1337,7 @@ class Engine {
     l.binned = L->bins->size;
     l.num_inner = static_cast<uint32_t>(std::min<int64_t>(num_inner, 0xFFFFFFFF));
     l.move_method = cfg_.move_method;
+    l.polls = ctx_->barrier_polls;
     l.mod_stamp = mod_stamp_.p;
     l.new_stamp = new_stamp_.p;
     l.next_stamp = next_stamp_.p;

@@ -40,7 +40,6 @@ constexpr int kLW = kLT / 32;      // warps
 constexpr int kTeams = kLW / kCtaWarps;
 constexpr int kLoopUnroll = 4;
 constexpr int kMaskWords = 4;      // ids per thread of the empty-id scan, / 32
-constexpr uint32_t kSpinLimit = 1u << 22;  // polls of a barrier (about two seconds)
 
 struct LoopShared {
   union {
@@ -59,8 +58,10 @@ struct LoopShared {
 
 // Grid-wide barrier: waits until `target` arrivals are counted (modulo 2^32).
 // Release and acquire at GPU scope: the writes before it are visible after it,
-// and the L1 lines read before it are dropped.
-__device__ __forceinline__ bool GridSync(LoopShared& sh, uint32_t* count, uint32_t target) {
+// and the L1 lines read before it are dropped.  False: given up after `polls`
+// looks.  The CTA then leaves without arriving again, so no other one passes
+// the next barrier: what runs meanwhile reads only what was complete here.
+__device__ __forceinline__ bool GridSync(LoopShared& sh, uint32_t* count, uint32_t target, uint32_t polls) {
   __syncthreads();
   if (threadIdx.x == 0) {
     uint32_t ok = 1;
@@ -68,7 +69,7 @@ __device__ __forceinline__ bool GridSync(LoopShared& sh, uint32_t* count, uint32
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
       uint32_t c = 0;
       ok = 0;
-      for (uint32_t t = 0; t < kSpinLimit; ++t) {
+      for (uint32_t t = 0; t < polls; ++t) {
         asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
         if (BarrierReached(c, target)) {
           ok = 1;
@@ -411,7 +412,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
       atomicAdd(&sh.fam_e[kFamGroup], fam_e);
       atomicAdd(&sh.fam_v[kFamGroup], fam_v);
     }
-    if (!GridSync(sh, count, arrivals += G)) break;
+    if (!GridSync(sh, count, arrivals += G, l.polls)) break;
 
     // ---- Rows above degree 4096: their tables, slice by slice --------------
     if (l.num_slices) {
@@ -457,7 +458,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
         }
         __syncthreads();
       }
-      if (!GridSync(sh, count, arrivals += G)) break;
+      if (!GridSync(sh, count, arrivals += G, l.polls)) break;
     }
 
     // ---- Moves: every mover leaves its cluster and joins its target --------
@@ -495,7 +496,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
         }
         if (join) a.C_mut[v] = t;
       }
-      if (!GridSync(sh, count, arrivals += G)) break;
+      if (!GridSync(sh, count, arrivals += G, l.polls)) break;
 
       // New clusters take the ascending list of empty ids, in ascending
       // vertex order: each CTA counts both in its slice of the ids, then
@@ -544,7 +545,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
           l.st->zeros[blockIdx.x] = uint32_t(total);
           l.st->news[blockIdx.x] = uint32_t(total >> 32);
         }
-        if (!GridSync(sh, count, arrivals += G)) break;
+        if (!GridSync(sh, count, arrivals += G, l.polls)) break;
         uint32_t zb = 0, wb = 0;
         for (uint32_t i = tid; i < blockIdx.x; i += kLT) {
           zb += l.st->zeros[i];
@@ -557,7 +558,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
           for (uint32_t mk = zm[q]; mk && zb < N; mk &= mk - 1) l.zero_ids[zb++] = uint32_t(lo + 32 * q + __ffs(mk) - 1);
           for (uint32_t mk = wm[q]; mk; mk &= mk - 1) l.new_list[wb++] = uint32_t(lo + 32 * q + __ffs(mk) - 1);
         }
-        if (!GridSync(sh, count, arrivals += G)) break;
+        if (!GridSync(sh, count, arrivals += G, l.polls)) break;
         for (uint32_t i = blockIdx.x * kLT + tid; i < N; i += G * kLT) {
           const uint32_t v = l.new_list[i];
           const uint32_t cid = l.zero_ids[i];
@@ -566,7 +567,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
           a.K_mut[cid] = a.k[v];
           l.mod_stamp[cid] = rv.stamp;
         }
-        if (!GridSync(sh, count, arrivals += G)) break;
+        if (!GridSync(sh, count, arrivals += G, l.polls)) break;
       }
       // FP32 images of the modified clusters' weights.
       for (uint32_t i = blockIdx.x * kLT + tid; i < M; i += G * kLT) {
@@ -682,7 +683,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
         }
       }
     }
-    if (!GridSync(sh, count, arrivals += G)) break;
+    if (!GridSync(sh, count, arrivals += G, l.polls)) break;
 
     // ---- End of the round ----------------------------------------------------
     const uint32_t F = all_move ? n : ctr->frontier;

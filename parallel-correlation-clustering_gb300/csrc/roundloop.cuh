@@ -49,6 +49,7 @@ struct RoundLoopArgs {
   uint64_t binned;          // vertices on `list`
   uint32_t num_inner;       // rounds at most
   int32_t move_method;      // PCC_*_MOVE
+  uint32_t polls;           // of a barrier, then it gives up (Context::barrier_polls)
   uint32_t* mod_stamp;
   uint32_t* new_stamp;
   uint32_t* next_stamp;

@@ -298,3 +298,30 @@ def test_graph_shared_by_contexts(ctx):
                 np.testing.assert_array_equal(lab, want)
     finally:
         other.close()
+
+
+@pytest.mark.parametrize("name", ["hubby", "rmat15", "cliques130"])
+def test_round_kernel_gives_up(ctx, monkeypatch, name):
+    """A grid barrier whose bounded wait runs out (a limit of no polls: every
+    CTA leaves at its first barrier): the call answers INTERNAL, calls that
+    need no barrier go on working on that context, and other contexts give
+    the oracle's labels afterwards."""
+    monkeypatch.setenv("PCC_BARRIER_POLLS", "0")
+    short = P.Context(0)
+    monkeypatch.delenv("PCC_BARRIER_POLLS")
+    g = LOOP_GRAPHS[name]()
+    cfg = P.make_config(resolution=0.05, refine=True)
+    try:
+        dg = short.upload(g)
+        for _ in range(2):
+            with pytest.raises(P.PccError) as e:
+                P.correlation_cluster(dg, cfg)
+            assert e.value.code == 13 and "error flag 5" in str(e.value)
+        short.set_detailed_timing(True)  # rounds without the round kernel
+        np.testing.assert_array_equal(P.correlation_cluster(dg, cfg)[0], O.correlation_cluster(O.OracleGraph(g), cfg)[0])
+        short.set_detailed_timing(False)
+        _same(short, P.CsrGraph.from_edges(2, [0], [1]), cfg)  # one CTA: no barrier to wait at
+        dg.free()
+    finally:
+        short.close()
+    _same(ctx, g, cfg)
