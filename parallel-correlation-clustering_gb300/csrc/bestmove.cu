@@ -457,26 +457,10 @@ __global__ void __launch_bounds__(kCtaWarps * 32) CertCtaKernel(BMArgs a, const 
   }
 }
 
-// Sets the kernel's dynamic shared-memory limit and queries its resident
-// CTAs per SM once per process (the runtime calls take a lock that
-// serialises concurrent contexts).  Each kernel is launched with one fixed
-// shared-memory size.
+// (Each kernel is launched with one fixed shared-memory size.)
 template <class K>
 Status SetSmem(K kernel, size_t bytes, int threads, int* per_sm) {
-  static std::mutex mu;
-  static std::unordered_map<const void*, int> occ;
-  std::lock_guard<std::mutex> lk(mu);
-  auto it = occ.find(reinterpret_cast<const void*>(kernel));
-  if (it != occ.end()) {
-    *per_sm = it->second;
-    return Status::Ok();
-  }
-  PCC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-  int n = 0;
-  PCC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, bytes));
-  occ[reinterpret_cast<const void*>(kernel)] = n;
-  *per_sm = n;
-  return Status::Ok();
+  return PrepareKernel(kernel, threads, bytes, bytes, per_sm);
 }
 
 template <bool kInt, bool kAsync>
@@ -630,10 +614,6 @@ Status Prep(K kernel, size_t smem, int threads) {
 }  // namespace
 
 Status PrepareBestMoveKernels() {
-  static std::mutex mu;
-  static bool done = false;
-  std::lock_guard<std::mutex> lk(mu);
-  if (done) return Status::Ok();
   PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<4, int>, 0, 256));
   PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<8, int>, 0, 256));
   PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<16, int>, 0, 256));
@@ -672,7 +652,6 @@ Status PrepareBestMoveKernels() {
   PCC_RETURN_IF_ERROR(Prep(BestMoveWarpKernel<512, false, false>, WarpKernelSmem<512>(), kW));
   PCC_RETURN_IF_ERROR(Prep(BestMoveWarpKernel<1024, false, false>, WarpKernelSmem<1024>(), kW));
   PCC_RETURN_IF_ERROR(Prep(BestMoveWarpKernel<2048, false, false>, WarpKernelSmem<2048>(), kW));
-  done = true;
   return Status::Ok();
 }
 

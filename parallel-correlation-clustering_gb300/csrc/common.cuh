@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "pcc_gb300.h"
+#include "per_device.h"
 
 namespace pcc {
 
@@ -268,6 +269,24 @@ struct OnSideStream {
 inline Status Sync(Context* c) {
   PCC_CUDA(cudaStreamSynchronize(c->stream));
   PCC_CUDA(cudaGetLastError());
+  return Status::Ok();
+}
+
+// Sets a kernel's dynamic shared-memory limit (at least `smem`) on the current
+// device and gives its resident CTAs per SM at `smem` bytes.
+template <class K>
+inline Status PrepareKernel(K kernel, int threads, size_t smem, size_t limit, int* per_sm) {
+  static PerDevice cache;
+  int device = 0;
+  PCC_CUDA(cudaGetDevice(&device));
+  cudaError_t e = cudaSuccess;
+  cache.Get(device, reinterpret_cast<const void*>(kernel), smem, per_sm, [&](int* n) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(limit));
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kernel, threads, smem);
+    return e == cudaSuccess;
+  });
+  if (e != cudaSuccess) cudaGetLastError();
+  PCC_CUDA(e);
   return Status::Ok();
 }
 

@@ -922,14 +922,9 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
     const bool maybe_big = g.m > kSegCtaMax;
     if (maybe_big)
       PCC_CUDA(cudaMemcpyAsync(hh, head, offsetof(CompressHead, m2), cudaMemcpyDeviceToHost, st));
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-      attr = cudaFuncSetAttribute(SegMidKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSegMidSmem));
-      if (attr == cudaSuccess)
-        attr = cudaFuncSetAttribute(SegCtaKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSegCtaSmem));
-    });
-    PCC_CUDA(attr);
+    int per_sm;
+    PCC_RETURN_IF_ERROR(PrepareKernel(SegMidKernel, kSegMidWarps * 32, kSegMidSmem, kSegMidSmem, &per_sm));
+    PCC_RETURN_IF_ERROR(PrepareKernel(SegCtaKernel, kSegCtaThreads, kSegCtaSmem, kSegCtaSmem, &per_sm));
     const int passes = (kbits + 7) / 8;
     // The kernels read their class's length on the device; the grids follow
     // bounds of it (a class-c segment has more than the class's entries).

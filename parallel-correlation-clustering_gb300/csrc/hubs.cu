@@ -5,9 +5,7 @@
 // float after the offset, the argmax by (value desc, id asc), and "no
 // entries" giving the reduce identity (0, 0.0) unless change >= 0.
 #include <algorithm>
-#include <mutex>
 #include <numeric>
-#include <unordered_map>
 #include <vector>
 
 #include "certmoves.cuh"
@@ -454,24 +452,11 @@ __global__ void HubDegreesKernel(const uint32_t* list, uint32_t count, const uin
     deg[i] = static_cast<uint32_t>(off[list[i] + 1] - off[list[i]]);
 }
 
-// Dynamic shared-memory limit and resident CTAs per SM of a kernel, set up
-// and queried once per process (the runtime calls take a lock that
-// serialises concurrent contexts).  Returns 0 on failure.
+// Resident CTAs per SM of a kernel at `smem` bytes; 0 when it cannot be set up.
 template <class K>
 int PrepareOnce(K kernel, int threads, size_t smem) {
-  static std::mutex mu;
-  static std::unordered_map<const void*, int> per_sm_of;
-  std::lock_guard<std::mutex> lk(mu);
-  auto it = per_sm_of.find(reinterpret_cast<const void*>(kernel));
-  if (it != per_sm_of.end()) return it->second;
   int per_sm = 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  per_sm_of[reinterpret_cast<const void*>(kernel)] = per_sm;
-  return per_sm;
+  return PrepareKernel(kernel, threads, smem, smem, &per_sm).ok() ? per_sm : 0;
 }
 
 // One small-hub table class over small_v[lo, hi).
@@ -761,10 +746,6 @@ Status AllocHubState(Context* ctx, const HubPlan& plan, HubState* st) {
 }
 
 Status PrepareHubKernels() {
-  static std::mutex mu;
-  static bool done = false;
-  std::lock_guard<std::mutex> lk(mu);
-  if (done) return Status::Ok();
   bool ok = true;
   auto small = [&](auto k, size_t slots, size_t vsize) {
     ok = ok && PrepareOnce(k, kSmallThreads, slots * (vsize + sizeof(uint32_t))) > 0;
@@ -788,9 +769,7 @@ Status PrepareHubKernels() {
   big(HubBigKernel<true, false, int>, BigSlots<int>(), sizeof(int));
   big(HubBigKernel<true, false, long long>, BigSlots<long long>(), sizeof(long long));
   big(HubBigKernel<false, false, double>, BigSlots<double>(), sizeof(double));
-  if (!ok) return MakeError(PCC_INTERNAL, "hub kernels cannot be configured");
-  done = true;
-  return Status::Ok();
+  return ok ? Status::Ok() : MakeError(PCC_INTERNAL, "hub kernels cannot be configured");
 }
 
 Status LaunchHubBestMoves(Context* ctx, const BMArgs& a, const HubPlan& plan, HubState& st, bool int_mode,

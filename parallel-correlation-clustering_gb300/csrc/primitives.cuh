@@ -4,8 +4,6 @@
 // calls (parallel/parallel-sequence-ops.h:38-232).
 #pragma once
 
-#include <mutex>
-
 #include "common.cuh"
 
 namespace pcc {
@@ -442,15 +440,8 @@ static inline Status RadixSortInto(Context* ctx, uint64_t** keys, uint32_t** val
   uint64_t* kout = b.keys;
   uint32_t* vout = b.vals;
   const int passes = (bits + 7) / 8;
-  {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-      attr = cudaFuncSetAttribute(RadixScatterKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(kSortScatterSmem));
-    });
-    PCC_CUDA(attr);
-  }
+  int per_sm;
+  PCC_RETURN_IF_ERROR(PrepareKernel(RadixScatterKernel, kSortThreads, kSortScatterSmem, kSortScatterSmem, &per_sm));
   for (int p = 0; p < passes; ++p) {
     const int shift = p * 8;
     RadixHistKernel<<<tiles, kSortThreads, 0, ctx->stream>>>(kin, n, shift, b.hist, tiles); PCC_COUNT(1);

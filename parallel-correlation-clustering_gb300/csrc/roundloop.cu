@@ -717,37 +717,13 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
 
 static_assert(kLoopIdsPerCta == uint64_t(kLT) * kMaskWords * 32, "ids of a CTA");
 
-// Shared-memory limit and resident CTAs per SM of a kernel at a table size,
-// configured and queried once per process.
-template <class K>
-Status PrepareLoop(K kernel, size_t smem, size_t smem_max, int* per_sm) {
-  static std::mutex mu;
-  static std::unordered_map<uint64_t, int> occ;
-  static std::unordered_map<const void*, bool> set;
-  std::lock_guard<std::mutex> lk(mu);
-  const void* f = reinterpret_cast<const void*>(kernel);
-  if (!set[f]) {
-    PCC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_max)));
-    set[f] = true;
-  }
-  const uint64_t key = reinterpret_cast<uint64_t>(f) * 31 + smem;
-  auto it = occ.find(key);
-  if (it == occ.end()) {
-    int b = 0;
-    PCC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kLT, smem));
-    it = occ.emplace(key, b).first;
-  }
-  *per_sm = it->second;
-  return Status::Ok();
-}
-
 template <typename V, bool kConv>
 Status LaunchLoop(Context* ctx, RoundLoopArgs& l) {
   auto kernel = RoundLoopKernel<V, kConv>;
   constexpr size_t kSlotBytes = 4 + sizeof(V) + 1;
   int per_sm = 0;
   const size_t smem = size_t(l.table_slots) * kSlotBytes;
-  PCC_RETURN_IF_ERROR(PrepareLoop(kernel, smem, size_t(2 * kHubSmallMax) * kSlotBytes, &per_sm));
+  PCC_RETURN_IF_ERROR(PrepareKernel(kernel, kLT, smem, size_t(2 * kHubSmallMax) * kSlotBytes, &per_sm));
   if (per_sm <= 0) return MakeError(PCC_INTERNAL, "round kernel cannot be configured");
   // One CTA per 1024 entries (two steps of each of its warps) or per 16,384
   // vertices (the empty-id scan), at most every resident CTA: a barrier's cost

@@ -41,3 +41,40 @@ int main() {
 }
 """)
     assert out.strip() == "0"
+
+
+def test_kernel_setup_is_per_device(tmp_path):
+    """A second device, kernel or size is set up for itself, each once however
+    many threads ask; a set-up that failed is tried again."""
+    out = _run(tmp_path, r"""
+#include <atomic>
+#include <cstdio>
+#include <thread>
+#include <vector>
+#include "per_device.h"
+int main() {
+  static pcc::PerDevice cache;
+  static int kernels[2];
+  std::atomic<int> made{0}, wrong{0};
+  int v = 7;
+  wrong += cache.Get(0, &kernels[0], 64, &v, [&](int*) { return false; });
+  std::vector<std::thread> all;
+  for (int t = 0; t < 16; ++t)
+    all.emplace_back([&] {
+      for (int device = 0; device < 3; ++device)
+        for (int k = 0; k < 2; ++k)
+          for (int size : std::vector<int>{64, 96}) {
+            int got = 0;
+            wrong += !cache.Get(device, &kernels[k], size, &got, [&](int* n) {
+              ++made;
+              *n = device * 1000 + k * 100 + size;
+              return true;
+            });
+            wrong += got != device * 1000 + k * 100 + size;
+          }
+    });
+  for (auto& t : all) t.join();
+  std::printf("%d %d\n", made.load(), wrong.load());
+}
+""")
+    assert out.split() == ["12", "0"]
