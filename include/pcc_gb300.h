@@ -105,9 +105,10 @@ typedef struct pcc_stats {
                                      visit (8 when the graph has no weights) */
   /* Best-move kernel families: [0] lane groups (degree <= 32), [1] warps
      (degree <= 1000), [2] small hubs (<= 4096), [3] big hubs.  Device time
-     (CUDA events around the family's launches), launches, and the entries
-     and vertices evaluated (a big hub counts once however many partitions
-     it is split into). */
+     (CUDA events around the family's launches), launches (the round kernel's
+     one launch runs every family and counts for none), and the entries and
+     vertices evaluated, whichever kernel did it (a big hub counts once
+     however many partitions it is split into). */
   double family_ms[4];
   uint64_t family_launches[4];
   uint64_t family_entries[4];
@@ -144,16 +145,31 @@ uint64_t pcc_device_bytes_in_use(const pcc_context* ctx);
 uint64_t pcc_device_peak_bytes(pcc_context* ctx, int32_t reset);
 /*
  * Detailed timing (no reference counterpart).  Off (the default):
- * synchronous best-move rounds run as a device-side loop, one round captured
- * into a CUDA graph WHILE node, with one host read per level; pcc_stats
- * then carries the compress time but no per-phase or per-family kernel
- * times.  On: the host drives every round and CUDA events time each phase
- * and best-move kernel family.  Results are identical either way.
+ * synchronous best-move rounds run in a device-side loop with one host read
+ * per level: all rounds of a level of at most 12M entries in one kernel (see
+ * pcc_set_round_kernel), larger levels as one round captured into a CUDA graph
+ * WHILE node; pcc_stats then carries the compress time but no per-phase or
+ * per-family kernel times.  On: the host drives every round on the
+ * degree-binned kernels and CUDA events time each phase and best-move kernel
+ * family; on levels that the round kernel would take, the times are those of
+ * other and slower kernels than the default's.  Results are identical either
+ * way.
  */
 void pcc_set_detailed_timing(pcc_context* ctx, int32_t on);
 
 /*
- * Best-move launch shape (no reference counterpart).  Lane-group bins (degree
+ * The round kernel (no reference counterpart).  On (the default): the
+ * synchronous LOUVAIN rounds of a level of at most 12M entries whose sums are
+ * exact in integers run in one cooperative kernel.  Off: every level runs on the
+ * degree-binned kernels, as levels above 12M entries, FP64 levels, unions and
+ * calls with detailed timing do (for comparisons and for tune_launch.py).
+ * Results are identical either way.
+ */
+void pcc_set_round_kernel(pcc_context* ctx, int32_t on);
+
+/*
+ * Launch shape of the degree-binned best-move kernels (no reference
+ * counterpart); the round kernel has none.  Lane-group bins (degree
  * <= 4, 8, 16, 32) above group_max_degree (4, 8, 16 or 32) run on the warp
  * kernel; certified (INT-mode, synchronous) warp bins (degree <= 128, 256,
  * 512, 1000) above cta_min_degree (64, 128, 256, 512, or 1000 for none) run

@@ -119,6 +119,9 @@ struct Context {
   cudaEvent_t fork_ev = nullptr;
   cudaEvent_t join_ev[kSideStreams] = {nullptr, nullptr, nullptr};
   bool overlap_families = true;  // off: every family on `stream` in turn
+  // Levels that fit run all their rounds in one kernel (roundloop.cu); off:
+  // every level on the degree-binned kernels.
+  bool round_kernel = true;
   // Polls of the round kernel's grid barrier before it gives up (about two
   // seconds; roundloop.cu).
   uint32_t barrier_polls = 1u << 22;

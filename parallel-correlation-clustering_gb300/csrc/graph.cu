@@ -363,6 +363,10 @@ void pcc_set_detailed_timing(pcc_context* ctx, int32_t on) {
   if (ctx) ctx->c.detailed_timing = on != 0;
 }
 
+void pcc_set_round_kernel(pcc_context* ctx, int32_t on) {
+  if (ctx) ctx->c.round_kernel = on != 0;
+}
+
 pcc_status pcc_set_launch_tuning(pcc_context* ctx, uint32_t group_max_degree, uint32_t cta_min_degree,
                                  float grid_waves) {
   if (!ctx) return PCC_INVALID_ARGUMENT;

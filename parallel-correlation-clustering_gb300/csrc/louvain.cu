@@ -1359,11 +1359,11 @@ class Engine {
   }
 
   // The round loop of one level: on the device when it can be (synchronous
-  // moves, one graph, no detailed timing), else driven from the host.  The
-  // one-kernel loop takes the shapes it was built for: with launch shapes set
-  // by the caller, or serial families, the degree-binned kernels run.
+  // moves, one graph, no detailed timing), else driven from the host.  (The
+  // round kernel has no families to run serially: with PCC_SERIAL_FAMILIES the
+  // degree-binned kernels run.)
   Status Iterate(Level* L, int64_t num_inner, bool* moved_out) {
-    if (!cfg_.async && !un_ && !ctx_->detailed_timing && !ctx_->tuned && ctx_->overlap_families && num_inner > 0 &&
+    if (!cfg_.async && !un_ && !ctx_->detailed_timing && ctx_->round_kernel && ctx_->overlap_families && num_inner > 0 &&
         cfg_.clustering_moves_method == PCC_LOUVAIN && RoundLoopFits(ctx_, *L->g, L->mode))
       return IterateLoop(L, num_inner, moved_out);
     if (cfg_.clustering_moves_method == PCC_DEFAULT_CLUSTER_MOVES) PCC_RETURN_IF_ERROR(PrepareClusterMoves(*L));

@@ -227,6 +227,8 @@ def load_library(path: str = LIB_PATH) -> ctypes.CDLL:
     lib.pcc_cluster_batch.restype = ctypes.c_int
     lib.pcc_set_detailed_timing.argtypes = [vp, ctypes.c_int32]
     lib.pcc_set_detailed_timing.restype = None
+    lib.pcc_set_round_kernel.argtypes = [vp, ctypes.c_int32]
+    lib.pcc_set_round_kernel.restype = None
     lib.pcc_set_launch_tuning.argtypes = [vp, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_float]
     lib.pcc_set_launch_tuning.restype = ctypes.c_int32
     lib.pcc_cluster_union.argtypes = [vp, ctypes.c_uint32, vp, vp, ctypes.c_uint32, vp, ctypes.c_uint64, vp, vp,
@@ -351,8 +353,14 @@ class Context:
         self.lib.pcc_set_detailed_timing(self._h, 1 if on else 0)
         self.detailed_timing = bool(on)
 
+    def set_round_kernel(self, on: bool):
+        """pcc_set_round_kernel: levels of at most 12M entries with exact sums
+        in one kernel (on, the default), or every level on the degree-binned
+        kernels (off)."""
+        self.lib.pcc_set_round_kernel(self._h, 1 if on else 0)
+
     def set_launch_tuning(self, group_max_degree: int = 0, cta_min_degree: int = 0, grid_waves: float = 0.0):
-        """pcc_set_launch_tuning: lane-group bins above group_max_degree on
+        """pcc_set_launch_tuning (degree-binned kernels): lane-group bins above group_max_degree on
         the warp kernel, certified warp bins above cta_min_degree on one CTA
         per vertex, grid_waves waves of resident CTAs per best-move launch;
         (0, 0, 0) returns to the compiled-in table."""

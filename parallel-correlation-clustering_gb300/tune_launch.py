@@ -7,7 +7,10 @@ grid_waves {0.5, 1, 2}, set through pcc_set_launch_tuning) and keeps the fastest
 (stats.ms_total).  The winners are written as csrc/tuning_table.cuh (or
 --out), which the library compiles in; the full timing table is printed as
 markdown and JSON.  Every shape must give the same labels: the tuner checks
-that too, so a table it writes never changes a result.
+that too, so a table it writes never changes a result.  The round kernel is off
+meanwhile: the table serves the degree-binned kernels, which run levels above
+12M entries, FP64 levels and unions (levels of at most 12M entries of one graph
+take the round kernel, which has no such shapes).
 
 Classes (by vertices of the level graph, the key the library looks up):
   n <= 65,536       RMAT scale 15 (modularity, headline config) and an SBM
@@ -80,6 +83,7 @@ def pick_best(per_workload):
 
 def tune(reps: int, quick: bool):
     ctx = P.Context()
+    ctx.set_round_kernel(False)  # it has no launch shapes to choose
     results = {}
     table = []
     for cls in CLASSES:

@@ -325,3 +325,47 @@ def test_round_kernel_gives_up(ctx, monkeypatch, name):
     finally:
         short.close()
     _same(ctx, g, cfg)
+
+
+def test_tuned_context_keeps_round_kernel(ctx):
+    """A launch shape set on the context is for the degree-binned kernels: a
+    level that fits the round kernel takes it all the same (with the same few
+    launches), and switching it off takes none of the results."""
+    g, _ = G.sbm(3000, 30, 0.04, 0.001, 42)
+    dg = ctx.upload(g)
+    cfg = P.make_config(resolution=0.05, refine=True)
+    lab, st = P.correlation_cluster(dg, cfg)
+    try:
+        ctx.set_launch_tuning(16, 256, 0.5)
+        tuned, tuned_st = P.correlation_cluster(dg, cfg)
+        ctx.set_round_kernel(False)
+        binned, binned_st = P.correlation_cluster(dg, cfg)
+    finally:
+        ctx.set_round_kernel(True)
+        ctx.set_launch_tuning(0, 0, 0.0)
+    for other in (tuned, binned):
+        np.testing.assert_array_equal(lab, other)
+    assert tuned_st["kernel_launches"] == st["kernel_launches"]
+    assert binned_st["kernel_launches"] > 2 * st["kernel_launches"]
+    for key in ("rounds", "edge_visits", "vertex_visits", "moves", "objective"):
+        assert st[key] == tuned_st[key] == binned_st[key], key
+    # (The shape moves degrees 17-32 to the warp family of the binned kernels.)
+    assert st["family_entries"] == tuned_st["family_entries"]
+    assert sum(st["family_entries"]) == sum(binned_st["family_entries"])
+    dg.free()
+
+
+@pytest.mark.parametrize("name", ["hubby", "rmat15"])
+@pytest.mark.parametrize("shape", [(4, 1000, 1.0), (8, 512, 0.5), (16, 256, 2.0), (32, 128, 0.125), (32, 64, 4.0)])
+def test_launch_shapes_without_round_kernel(ctx, name, shape):
+    """The accepted launch shapes on the degree-binned kernels in the graph
+    loop, 32-bit and 64-bit sums."""
+    g = LOOP_GRAPHS[name]()
+    try:
+        ctx.set_round_kernel(False)
+        ctx.set_launch_tuning(*shape)
+        for gw, res in ((g, 0.02), (_weighted(g, WEIGHTS["uniform"][0]), 0.02)):
+            _same(ctx, gw, P.make_config(resolution=res, refine=True, move_method=P.NBHR_MOVE))
+    finally:
+        ctx.set_round_kernel(True)
+        ctx.set_launch_tuning(0, 0, 0.0)
