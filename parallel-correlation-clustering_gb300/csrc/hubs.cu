@@ -706,43 +706,65 @@ Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan
   return Status::Ok();  // (the host lists are spent; EnsureHubPlan waits for the device where it must)
 }
 
-Status AllocHubState(Context* ctx, const HubPlan& plan, HubState* st) {
+namespace {
+
+Status AllocTables(Context* ctx, uint64_t slots, uint32_t hubs, uint32_t slices, HubState* st, bool reset) {
+  if (!slots) return Status::Ok();
+  if (st->gkeys.count < slots || st->gt_int.count < hubs || st->gpart_val.count < slices) {
+    auto grow = [&]() -> Status {
+      if (st->gkeys.count < slots) {
+        PCC_RETURN_IF_ERROR(st->gkeys.Alloc(ctx, slots));
+        PCC_RETURN_IF_ERROR(st->gvals.Alloc(ctx, slots));
+      }
+      if (st->gt_int.count < hubs) {
+        PCC_RETURN_IF_ERROR(st->gt_int.Alloc(ctx, hubs));
+        PCC_RETURN_IF_ERROR(st->gt_dbl.Alloc(ctx, hubs));
+        PCC_RETURN_IF_ERROR(st->gsmax.Alloc(ctx, hubs));
+        PCC_RETURN_IF_ERROR(st->gdone.Alloc(ctx, hubs));
+      }
+      if (st->gpart_val.count < slices) {
+        PCC_RETURN_IF_ERROR(st->gpart_val.Alloc(ctx, slices));
+        PCC_RETURN_IF_ERROR(st->gpart_id.Alloc(ctx, slices));
+      }
+      return Status::Ok();
+    };
+    const Status got = grow();
+    if (!got.ok()) {
+      st->ReleaseTables();
+      return got;
+    }
+    reset = true;
+  }
+  if (!reset) return Status::Ok();
+  // The rounds leave the tables clean; they are cleared at every new level all
+  // the same, so that a run cut short cannot leave keys behind.
+  PCC_CUDA(cudaMemsetAsync(st->gkeys.p, 0xFF, slots * sizeof(uint32_t), ctx->stream));  // kNone
+  PCC_CUDA(cudaMemsetAsync(st->gvals.p, 0, slots * sizeof(unsigned long long), ctx->stream));
+  GlobalStateInitKernel<<<Blocks(hubs, 256, 1024), 256, 0, ctx->stream>>>(hubs, st->gt_int.p, st->gt_dbl.p,
+                                                                          st->gsmax.p, st->gdone.p);
+  PCC_COUNT(1);
+  return LaunchCheck();
+}
+
+}  // namespace
+
+Status AllocHubState(Context* ctx, const HubPlan& plan, HubState* st, bool reset) {
   const uint64_t np = std::max<uint64_t>(plan.num_partials, 1);
   if (st->part_val.count < np) {
     PCC_RETURN_IF_ERROR(st->part_val.Alloc(ctx, np));
     PCC_RETURN_IF_ERROR(st->part_id.Alloc(ctx, np));
   }
   const uint64_t nh = std::max<uint32_t>(plan.num_big, 1);
-  if (st->done.count < nh) PCC_RETURN_IF_ERROR(st->done.Alloc(ctx, nh));
-  // Tables and accumulators of the global path or of the whole-level kernel
-  // (one of the two runs a level).
-  const uint64_t slots = std::max(plan.glob_slots, plan.loop_slots);
-  const uint32_t hubs = plan.loop_slots ? plan.num_big : plan.num_glob;
-  const uint32_t slices = std::max(plan.num_glob_slices, plan.num_loop_slices);
-  if (slots) {
-    // The rounds leave the tables clean; they are reset here all the same,
-    // at every level, so that a run cut short cannot leave keys behind.
-    if (st->gkeys.count < slots) {
-      PCC_RETURN_IF_ERROR(st->gkeys.Alloc(ctx, slots));
-      PCC_RETURN_IF_ERROR(st->gvals.Alloc(ctx, slots));
-    }
-    if (st->gt_int.count < hubs) {
-      PCC_RETURN_IF_ERROR(st->gt_int.Alloc(ctx, hubs));
-      PCC_RETURN_IF_ERROR(st->gt_dbl.Alloc(ctx, hubs));
-      PCC_RETURN_IF_ERROR(st->gsmax.Alloc(ctx, hubs));
-      PCC_RETURN_IF_ERROR(st->gdone.Alloc(ctx, hubs));
-    }
-    if (st->gpart_val.count < slices) {
-      PCC_RETURN_IF_ERROR(st->gpart_val.Alloc(ctx, slices));
-      PCC_RETURN_IF_ERROR(st->gpart_id.Alloc(ctx, slices));
-    }
-    PCC_CUDA(cudaMemsetAsync(st->gkeys.p, 0xFF, slots * sizeof(uint32_t), ctx->stream));  // kNone
-    PCC_CUDA(cudaMemsetAsync(st->gvals.p, 0, slots * sizeof(unsigned long long), ctx->stream));
-    GlobalStateInitKernel<<<Blocks(hubs, 256, 1024), 256, 0, ctx->stream>>>(hubs, st->gt_int.p, st->gt_dbl.p,
-                                                                            st->gsmax.p, st->gdone.p);
-    PCC_COUNT(1);
+  if (st->done.count < nh) {
+    PCC_RETURN_IF_ERROR(st->done.Alloc(ctx, nh));
+    reset = true;
   }
-  return st->done.Zero();
+  PCC_RETURN_IF_ERROR(AllocTables(ctx, plan.glob_slots, plan.num_glob, plan.num_glob_slices, st, reset));
+  return reset ? st->done.Zero() : Status::Ok();
+}
+
+Status AllocLoopTables(Context* ctx, const HubPlan& plan, HubState* st, bool reset) {
+  return AllocTables(ctx, plan.loop_slots, plan.num_big, plan.num_loop_slices, st, reset);
 }
 
 Status PrepareHubKernels() {

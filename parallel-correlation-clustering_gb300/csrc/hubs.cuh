@@ -109,13 +109,24 @@ struct HubState {
   DBuf<double> gpart_val;                // per slice: best (value, id)
   DBuf<uint32_t> gpart_id;
   DBuf<uint32_t> gdone;                  // per global hub: slices evaluated (0 between rounds)
+  void ReleaseTables() {
+    gkeys.Release(), gvals.Release();
+    gt_int.Release(), gt_dbl.Release(), gsmax.Release(), gdone.Release();
+    gpart_val.Release(), gpart_id.Release();
+  }
 };
 
 Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan* plan);
 // Configures every synchronous hub kernel once per process (for launches
 // captured into a graph).
 Status PrepareHubKernels();
-Status AllocHubState(Context* ctx, const HubPlan& plan, HubState* st);
+// Buffers of the hub kernels over the plan (the global path's tables among
+// them), or the tables of the round kernel (24 bytes per entry of every big
+// hub: for the levels that enter it only).  Both use the same buffers, which
+// grow; reset: cleared even when they were large enough.  The tables are all
+// there or, when one cannot be had, all released.
+Status AllocHubState(Context* ctx, const HubPlan& plan, HubState* st, bool reset = true);
+Status AllocLoopTables(Context* ctx, const HubPlan& plan, HubState* st, bool reset);
 // narrow: INT mode with every neighbour-cluster sum below 2^31 in
 // magnitude, so the tables hold 32-bit sums.  families: kLaunchSmallHubs
 // (degree <= 4096, one CTA per hub) and/or kLaunchBigHubs (the partitioned

@@ -727,6 +727,7 @@ struct Level {
   // Integer sums in synchronous rounds; asynchronous ones take them for
   // integer weights only (no SumMode::conv).
   SumMode mode;
+  bool loop_tables = false;  // the round kernel's hub tables were cleared for this level
   // Subclustering: the vertex of the next level every vertex became (its
   // subcluster id); empty when the level was compressed by cluster id.
   DBuf<uint32_t> sub;
@@ -864,7 +865,7 @@ class Engine {
       L->bins = &g->bins;
     }
     PCC_RETURN_IF_ERROR(EnsureHubPlan(ctx_, g, L->own == nullptr));
-    PCC_RETURN_IF_ERROR(AllocHubState(ctx_, *g->hub_plan, &hub_state_));
+    if (!TakesRoundKernel(*L)) PCC_RETURN_IF_ERROR(AllocHubState(ctx_, *g->hub_plan, &hub_state_));
     *out = std::move(L);
     return Status::Ok();
   }
@@ -1311,20 +1312,46 @@ class Engine {
     return Status::Ok();
   }
 
-  // IterateBestMoves in one cooperative kernel (roundloop.cu): levels of at
-  // most kLoopMaxEntries entries with exact sums.
-  Status IterateLoop(Level* L, int64_t num_inner, bool* moved_out) {
+  // Whether a level's rounds go to the round kernel: synchronous Louvain moves
+  // of one graph with exact sums on at most kLoopMaxEntries entries.  (It has
+  // no families to run serially: with PCC_SERIAL_FAMILIES the degree-binned
+  // kernels run.)
+  bool TakesRoundKernel(const Level& L) const {
+    return !cfg_.async && !un_ && !ctx_->detailed_timing && ctx_->round_kernel && ctx_->overlap_families &&
+           cfg_.clustering_moves_method == PCC_LOUVAIN && RoundLoopFits(ctx_, *L.g, L.mode);
+  }
+
+  void ReleaseLoop() {
+    hub_state_.ReleaseTables();
+    loop_state_.Release();
+    old_cluster_.Release();
+  }
+
+  // The device memory that the round kernel takes beside the level's own.
+  Status AllocLoop(Level* L) {
+    PCC_RETURN_IF_ERROR(AllocLoopTables(ctx_, *L->g->hub_plan, &hub_state_, !L->loop_tables));
+    L->loop_tables = true;
+    PCC_RETURN_IF_ERROR(loop_state_.Reserve(ctx_, 1));
+    return old_cluster_.Reserve(ctx_, std::max<uint64_t>(n_max_, 1));
+  }
+
+  // IterateBestMoves in one cooperative kernel (roundloop.cu).  *ran: false when
+  // its memory cannot be had (an HBM budget that the degree-binned kernels fit);
+  // nothing has run then.
+  Status IterateLoop(Level* L, int64_t num_inner, bool* moved_out, bool* ran) {
     const DevGraph& g = *L->g;
+    const Status got = AllocLoop(L);
+    *ran = got.ok();
+    if (!got.ok()) {
+      ReleaseLoop();
+      return got.code == PCC_RESOURCE_EXHAUSTED ? Status::Ok() : got;
+    }
     LoopHead h{};
     h.rs.front_all = 1;
     h.rs.front_edges = g.m;
     h.rs.front_size = g.n;
     h.rs.visited = L->bins->size;
     h.rs.stamp = stamp_;  // the first round's stamp is the next one
-    if (!loop_state_.p) {
-      PCC_RETURN_IF_ERROR(loop_state_.Alloc(ctx_, 1));
-      PCC_RETURN_IF_ERROR(old_cluster_.Alloc(ctx_, std::max<uint64_t>(n_max_, 1)));
-    }
     RoundLoopArgs l{};
     l.a = LevelArgs(*L);
     l.a.front_stamp = next_stamp_.p;
@@ -1355,17 +1382,19 @@ class Engine {
     res_.algo_bytes += (g.w.p ? 12ull : 8ull) * h.edge_visits + 40ull * h.visited;
     res_.moves += h.moves;
     *moved_out = h.level_moved != 0;
+    if (ctx_->budget) ReleaseLoop();  // the contraction has its room as without the round kernel
     return Status::Ok();
   }
 
   // The round loop of one level: on the device when it can be (synchronous
-  // moves, one graph, no detailed timing), else driven from the host.  (The
-  // round kernel has no families to run serially: with PCC_SERIAL_FAMILIES the
-  // degree-binned kernels run.)
+  // moves, one graph, no detailed timing), else driven from the host.
   Status Iterate(Level* L, int64_t num_inner, bool* moved_out) {
-    if (!cfg_.async && !un_ && !ctx_->detailed_timing && ctx_->round_kernel && ctx_->overlap_families && num_inner > 0 &&
-        cfg_.clustering_moves_method == PCC_LOUVAIN && RoundLoopFits(ctx_, *L->g, L->mode))
-      return IterateLoop(L, num_inner, moved_out);
+    if (TakesRoundKernel(*L) && num_inner > 0) {
+      bool ran = false;
+      PCC_RETURN_IF_ERROR(IterateLoop(L, num_inner, moved_out, &ran));
+      if (ran) return Status::Ok();
+    }
+    PCC_RETURN_IF_ERROR(AllocHubState(ctx_, *L->g->hub_plan, &hub_state_, false));
     if (cfg_.clustering_moves_method == PCC_DEFAULT_CLUSTER_MOVES) PCC_RETURN_IF_ERROR(PrepareClusterMoves(*L));
     if (!cfg_.async && !un_ && !ctx_->detailed_timing && !ctx_->graphs_failed &&
         (cfg_.clustering_moves_method == PCC_LOUVAIN || cm_table_.keys.p) &&

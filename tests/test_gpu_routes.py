@@ -369,3 +369,59 @@ def test_launch_shapes_without_round_kernel(ctx, name, shape):
     finally:
         ctx.set_round_kernel(True)
         ctx.set_launch_tuning(0, 0, 0.0)
+
+
+def _peak(c, run):
+    """Device bytes that run() took beyond what the context held."""
+    held = c.bytes_in_use()
+    c.lib.pcc_device_peak_bytes(c.handle, 1)
+    out = run()
+    return c.lib.pcc_device_peak_bytes(c.handle, 0) - held, out
+
+
+def test_no_round_kernel_tables_elsewhere(ctx):
+    """A call that cannot enter the round kernel takes none of its hub tables
+    (24 bytes an entry of every row above 4096 entries): a best-move pass holds
+    some arrays of up to 8 bytes a vertex, 128 bytes in all, and small lists."""
+    g = _hub_degrees((8000,) * 60)
+    dg = ctx.upload(g)
+    C = np.arange(g.n, dtype=np.uint32)
+    one = np.ones(g.n)
+    cfg = P.make_config(resolution=0.1)
+    peak, _ = _peak(ctx, lambda: P.best_moves(dg, cfg, C, C * 0 + 1, one, one))
+    assert peak <= 128 * g.n + (2 << 20) < 24 * 60 * 8000
+    dg.free()
+
+
+BUDGET_GRAPHS = {
+    "hubs": lambda: _hub_degrees((8000,) * 60),
+    "rmat15": LOOP_GRAPHS["rmat15"],
+    "real": lambda: _weighted(_hubby(seed=4), WEIGHTS["uniform"][0]),
+}
+
+
+@pytest.mark.parametrize("name", list(BUDGET_GRAPHS))
+@pytest.mark.parametrize("modularity", [False, True])
+def test_round_kernel_within_a_budget(ctx, name, modularity):
+    """A budget that the degree-binned kernels just fit is enough with the round
+    kernel on: levels that it has no memory for run without it."""
+    g = BUDGET_GRAPHS[name]()
+    cfg = P.make_config(resolution=1.0 if modularity else 0.02, refine=True)
+
+    def call(budget, kernel=True):
+        c = P.Context(0, budget)
+        try:
+            c.set_round_kernel(kernel)
+            return _peak(c, lambda: P.cluster_host_csr(c, g, cfg, objective=int(modularity)))
+        finally:
+            c.close()
+
+    binned, (want, _) = call(1 << 38, False)
+    free, (lab, _) = call(1 << 38)
+    np.testing.assert_array_equal(lab, want)
+    for budget in np.linspace(binned, max(free, binned), 5).astype(int).tolist():
+        _, (lab, _) = call(budget)
+        np.testing.assert_array_equal(lab, want)
+    with pytest.raises(P.PccError) as e:
+        call(binned // 2)
+    assert e.value.code == 8
