@@ -890,9 +890,13 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
       sb.keys = keys2;
       sb.vals = vals2;
       sb.hist = hist;
+      // The result lies in one of the two buffers (by the number of passes);
+      // the other one is spent.
+      uint64_t* const keys1 = vkey;
+      uint32_t* const vals1 = vval;
       PCC_RETURN_IF_ERROR(RadixSortInto(ctx, &vkey, &vval, n, bits, sb, scan_tiles));
-      sc.Done(vkey == keys2 ? nullptr : keys2);
-      sc.Done(vval == vals2 ? nullptr : vals2);
+      sc.Done(vkey == keys2 ? keys1 : keys2);
+      sc.Done(vval == vals2 ? vals1 : vals2);
       sc.Done(hist);
     }
     PCC_RETURN_IF_ERROR(sc.Take(&dstart, n));

@@ -425,3 +425,31 @@ def test_round_kernel_within_a_budget(ctx, name, modularity):
     with pytest.raises(P.PccError) as e:
         call(binned // 2)
     assert e.value.code == 8
+
+
+@pytest.mark.parametrize("clusters", [200, 60000, 300000])  # 1, 2 and 3 passes of the vertex sort
+def test_contraction_frees_what_is_spent(built, clusters):
+    """Peak of a contraction under a budget, where arrays are freed as they are
+    spent: the vertex sort's spare buffers (12 bytes a vertex) are not held
+    beyond the sort, whichever of the two the result lies in."""
+    n = 300000
+    ring = np.arange(n)
+    g = P.CsrGraph.from_edges(n, ring, (ring + 1) % n)
+    C = (ring % clusters).astype(np.uint32)
+    c = P.Context(0, 1 << 38)
+    try:
+        dg = c.upload(g)
+        peak, out = _peak(c, lambda: P.compress(dg, C, np.ones(n)))
+        m2 = out.info()[1]
+        # Per vertex: 12 labels and node weights, 4 ids of the clusters, then
+        # 4 ranks, 12 sorted vertices, 12 spare, 8 row starts; per new vertex 12
+        # offset and count; per cluster 8 segment start, 20 class lists and count;
+        # per entry 8 moved; per new entry 8.
+        rows, r = (12 + 4) * n + 12 * clusters, clusters
+        held = max(rows + (4 + 12 + 12) * n, rows + (4 + 12 + 8) * n + 8 * r, rows + (4 + 8) * n + 8 * r + 8 * g.m,
+                   rows + 28 * r + 8 * g.m + 8 * m2)
+        assert peak <= held + (1 << 20)
+        out.free()
+        dg.free()
+    finally:
+        c.close()
