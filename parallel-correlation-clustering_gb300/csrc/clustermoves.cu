@@ -850,19 +850,16 @@ __global__ void CmTableDecideKernel(uint32_t n, uint32_t* __restrict__ best_id,
 }  // namespace
 
 Status AllocClusterMoveTable(Context* ctx, const DevGraph& g, ClusterMoveTable* t) {
-  // A device short of 24 bytes an entry has the sorted path.
+  // A device (or budget) short of 24 bytes an entry and 32 a vertex has the
+  // sorted path.
   const uint64_t cap = g.m + g.m / 2 + 64;
-  if (!t->keys.Alloc(ctx, cap).ok() || !t->sums.Alloc(ctx, cap).ok()) {
-    t->keys.Release();
-    t->sums.Release();
+  if (!t->keys.Alloc(ctx, cap).ok() || !t->sums.Alloc(ctx, cap).ok() || !t->best_bits.Alloc(ctx, g.n).ok() ||
+      !t->best_id.Alloc(ctx, g.n).ok() || !t->cmove.Alloc(ctx, g.n).ok() || !t->W.Alloc(ctx, g.n).ok() ||
+      !t->stay.Alloc(ctx, g.n).ok()) {
+    *t = ClusterMoveTable{};
     return Status::Ok();
   }
   t->cap = cap;
-  PCC_RETURN_IF_ERROR(t->best_bits.Alloc(ctx, g.n));
-  PCC_RETURN_IF_ERROR(t->best_id.Alloc(ctx, g.n));
-  PCC_RETURN_IF_ERROR(t->cmove.Alloc(ctx, g.n));
-  PCC_RETURN_IF_ERROR(t->W.Alloc(ctx, g.n));
-  PCC_RETURN_IF_ERROR(t->stay.Alloc(ctx, g.n));
   PCC_RETURN_IF_ERROR(t->keys.Fill(0xFF));
   PCC_RETURN_IF_ERROR(t->sums.Zero());
   PCC_RETURN_IF_ERROR(t->best_bits.Zero());

@@ -1399,8 +1399,11 @@ class Engine {
     if (!cfg_.async && !un_ && !ctx_->detailed_timing && !ctx_->graphs_failed &&
         (cfg_.clustering_moves_method == PCC_LOUVAIN || cm_table_.keys.p) &&
         L->g->m >= ctx_->device_loop_min_entries)
-      return IterateDevice(L, num_inner, moved_out);
-    return IterateBestMoves(L, num_inner, moved_out);
+      PCC_RETURN_IF_ERROR(IterateDevice(L, num_inner, moved_out));
+    else
+      PCC_RETURN_IF_ERROR(IterateBestMoves(L, num_inner, moved_out));
+    if (ctx_->budget) cm_table_ = ClusterMoveTable{};  // what follows has its room as after sorted rounds
+    return Status::Ok();
   }
 
   // IterateBestMoves (parallel-correlation-clusterer.cc:340-365).

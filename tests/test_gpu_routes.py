@@ -453,3 +453,34 @@ def test_contraction_frees_what_is_spent(built, clusters):
         dg.free()
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("name", ["sbm", "hubby"])
+def test_cluster_move_table_within_a_budget(built, name):
+    """Whole-cluster moves take their table when all of it fits, and give it
+    back before the scores are computed: a budget that the sorted path needs
+    (the same graph with weights that are no integers) is enough,
+    and a call that succeeds under a budget does under every larger one."""
+    g = G.sbm(20000, 40, 0.02, 0.0004, 4)[0] if name == "sbm" else _hubby()
+    gw = _weighted(g, lambda a, b: 1.5 + 0 * a)
+    cfg = P.make_config(resolution=0.1, clustering_moves_method=P.DEFAULT_CLUSTER_MOVES)
+    want = O.correlation_cluster(O.OracleGraph(g), cfg)[0]
+
+    def call(budget, graph=g):
+        c = P.Context(0, budget)
+        try:
+            peak, (lab, _) = _peak(c, lambda: P.cluster_host_csr(c, graph, cfg))
+        except P.PccError as e:
+            assert e.code == 8
+            return None
+        finally:
+            c.close()
+        if graph is g:
+            np.testing.assert_array_equal(lab, want)
+        return peak
+
+    sorted_path = call(1 << 38, gw) - 4 * g.m  # (weights are 4 bytes an entry)
+    assert call(sorted_path) is not None
+    full = call(1 << 38)
+    fits = [call(b) is not None for b in np.linspace(full - 24 * g.m - 32 * g.n, full, 60).astype(int).tolist()]
+    assert fits[-1] and fits == sorted(fits)
