@@ -75,6 +75,14 @@ struct Context {
   size_t smem_optin = 0;
   cudaStream_t stream = nullptr;
   uint64_t budget = 0;             // 0 = device capacity
+  // Calls were let in by an estimate of their device memory (a pool with an HBM
+  // budget, serve.cu), so large ones keep to what a budget would make them use:
+  // arrays of their exact size, freed as they are spent.  Calls of at most
+  // kAdmittedSmall entries need not: they differ by at most 12 MB, inside the
+  // estimate's fixed 64.
+  bool admitted = false;
+  static constexpr uint64_t kAdmittedSmall = 1u << 20;
+  bool Frugal(uint64_t entries) const { return budget || (admitted && entries > kAdmittedSmall); }
   // Synchronous rounds run as a device-side graph loop (one host read per
   // level) unless detailed timing (CUDA events around every phase and kernel
   // family, host-driven rounds) is on, or graphs are unavailable.

@@ -774,12 +774,12 @@ constexpr uint64_t kForkEntries = 1u << 20;  // the segment classes on streams o
 
 // Temporary arrays of a contraction: pieces of one allocation for the small
 // levels (whose 25 allocations and frees cost as much as their kernels),
-// separate ones, freed as soon as they are spent, for large graphs and under
-// an HBM budget.
+// separate ones, freed as soon as they are spent, for large graphs and where
+// memory is counted (Context::Frugal).
 class Scratch {
  public:
   Scratch(Context* ctx, uint64_t n, uint64_t m) : ctx_(ctx) {
-    if (!ctx->budget && n <= (1u << 20) && m <= (16u << 20)) bytes_ = 84 * n + 8 * m + (n / kSortTile + 1) * 1024 + 16384;
+    if (!ctx->Frugal(m) && n <= (1u << 20) && m <= (16u << 20)) bytes_ = 84 * n + 8 * m + (n / kSortTile + 1) * 1024 + 16384;
   }
   template <class T>
   Status Take(T** p, uint64_t count) {
@@ -816,8 +816,9 @@ class Scratch {
 //
 // Host waits: the number of clusters; the segment classes, when a segment may
 // be longer than a CTA holds (the shorter ones are sorted meanwhile); the new
-// graph's size and properties together (above 16M entries its size alone
-// before, so that its arrays are not allocated at the old size).  A level of
+// graph's size and properties together (above 16M entries, or where memory is
+// counted, its size alone before, so that its arrays are not allocated at the
+// old size).  A level of
 // 4,686 entries takes 3 waits and 18 kernels, 0.40 -> 0.2 ms.
 Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const double* k, bool planned,
                      std::unique_ptr<DevGraph>* out) {
@@ -1031,7 +1032,7 @@ Status CompressGraph(Context* ctx, const DevGraph& g, const uint32_t* C, const d
   PCC_RETURN_IF_ERROR(ScanApply<uint64_t>(ctx, uint64_t(n2) + 1, CountInput{row_count, n2},
                                           StorePrefix<uint64_t>{res->off.p}, scan64, m2));
   uint64_t entries = g.m;  // at most
-  const bool wait = ctx->budget || g.m > (16u << 20);
+  const bool wait = ctx->Frugal(g.m) || g.m > (16u << 20);
   if (wait) {
     PCC_CUDA(cudaMemcpyAsync(&hh->m2, m2, sizeof(hh->m2), cudaMemcpyDeviceToHost, st));
     PCC_RETURN_IF_ERROR(Sync(ctx));

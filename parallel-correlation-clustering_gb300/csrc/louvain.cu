@@ -1382,7 +1382,7 @@ class Engine {
     res_.algo_bytes += (g.w.p ? 12ull : 8ull) * h.edge_visits + 40ull * h.visited;
     res_.moves += h.moves;
     *moved_out = h.level_moved != 0;
-    if (ctx_->budget) ReleaseLoop();  // the contraction has its room as without the round kernel
+    if (ctx_->Frugal(g.m)) ReleaseLoop();  // the contraction has its room as without the round kernel
     return Status::Ok();
   }
 
@@ -1402,7 +1402,7 @@ class Engine {
       PCC_RETURN_IF_ERROR(IterateDevice(L, num_inner, moved_out));
     else
       PCC_RETURN_IF_ERROR(IterateBestMoves(L, num_inner, moved_out));
-    if (ctx_->budget) cm_table_ = ClusterMoveTable{};  // what follows has its room as after sorted rounds
+    if (ctx_->Frugal(L->g->m)) cm_table_ = ClusterMoveTable{};  // what follows has its room as after sorted rounds
     return Status::Ok();
   }
 

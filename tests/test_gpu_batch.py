@@ -283,3 +283,33 @@ def test_request_estimate_bounds_peak(built, kind):
     finally:
         c.close()
     assert 0 < peak <= P.request_bytes_estimate(g.n, g.m, g.weights is not None)
+
+
+def _pool_used():
+    """(current, highest) bytes used of the device's memory pool; the highest
+    is reset."""
+    import ctypes
+    rt = ctypes.CDLL("libcudart.so.13")
+    pool, used, high, zero = ctypes.c_void_p(), ctypes.c_uint64(), ctypes.c_uint64(), ctypes.c_uint64(0)
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    assert rt.cudaMemPoolGetAttribute(pool, 7, ctypes.byref(used)) == 0  # cudaMemPoolAttrUsedMemCurrent
+    assert rt.cudaMemPoolGetAttribute(pool, 8, ctypes.byref(high)) == 0  # cudaMemPoolAttrUsedMemHigh
+    assert rt.cudaMemPoolSetAttribute(pool, 8, ctypes.byref(zero)) == 0
+    return used.value, high.value
+
+
+@pytest.mark.parametrize("iterations,res", [(4, 0.5), (9, 0.5), (10, 0.1)])
+def test_request_estimate_bounds_served_peak(built, iterations, res):
+    """The memory of a request in a pool with a budget stays within the estimate
+    that let it in, also where many levels that hardly shrink are kept for
+    refinement."""
+    g, _ = G.lfr(150000, mean_degree=20, dmax=2000, seed=6)
+    est = P.request_bytes_estimate(g.n, g.m, True)
+    srv = P.Server(slots=1, hbm_budget=est)
+    try:
+        held, _ = _pool_used()
+        srv.wait(srv.submit(g, P.make_config(resolution=res, refine=True, louvain_num_iterations=iterations), 0))
+        _, high = _pool_used()
+        assert held < high <= held + est
+    finally:
+        srv.close()
