@@ -484,3 +484,152 @@ def test_cluster_move_table_within_a_budget(built, name):
     full = call(1 << 38)
     fits = [call(b) is not None for b in np.linspace(full - 24 * g.m - 32 * g.n, full, 60).astype(int).tolist()]
     assert fits[-1] and fits == sorted(fits)
+
+
+def _split_hubs():
+    """Hubs of every kind: one CTA, one, two and four partitions."""
+    return _hub_degrees((1500, 4097, 9000, 13000, 40000), n=45000)
+
+
+FP64_CALLS = {  # graph, weights, resolution, offset: no fixed point holds these sums
+    "spread_sbm": (lambda: G.sbm(3000, 20, 0.05, 0.002, 3)[0], "spread", 0.1, 0.0),
+    "spread_lfr": (lambda: G.lfr(20000, mean_degree=20, dmax=900, seed=9)[0], "spread", 0.1, 0.0),
+    "offset_lfr": (lambda: G.lfr(20000, mean_degree=20, dmax=900, seed=9)[0], "uniform", 0.1, 0.3),
+    "offset_unit": (lambda: G.sbm(3000, 20, 0.05, 0.002, 3)[0], None, 0.02, 0.25),
+    "spread_hubs": (_split_hubs, "spread", 0.01, 0.0),
+    "offset_hubs": (_split_hubs, "uniform", 0.01, 0.3),
+}
+
+
+@pytest.mark.parametrize("name", list(FP64_CALLS))
+@pytest.mark.parametrize("move", [P.NBHR_CLUSTER_MOVE, P.NBHR_MOVE])
+def test_fp64_clusterings(ctx, name, move):
+    """Whole synchronous clusterings on the FP64 kernels, in the graph loop and
+    driven by the host.  On the block models every row of every level is short,
+    its sums have the reference's order and every label is the oracle's; rows
+    above 1000 entries add in any order, as the reference's do, so there the
+    labels agree to 99.9% and the objective to 1e-9."""
+    make, kind, res, off = FP64_CALLS[name]
+    g = make()
+    if kind:
+        g = _weighted(g, WEIGHTS[kind][0])
+    scale = float(np.abs(g.weights).mean()) if kind else 1.0
+    cfg = P.make_config(resolution=res * scale, edge_weight_offset=off, refine=True, move_method=move)
+    dg, og = ctx.upload(g), O.OracleGraph(g)
+    want, so = O.correlation_cluster(og, cfg)
+    for detailed in (False, True):
+        ctx.set_detailed_timing(detailed)
+        try:
+            lab, st = P.correlation_cluster(dg, cfg)
+        finally:
+            ctx.set_detailed_timing(False)
+        assert st["objective"] == pytest.approx(so["objective"], rel=1e-9)
+        if not name.endswith(("sbm", "unit")):
+            assert np.mean(lab == want) >= 0.999
+        else:
+            np.testing.assert_array_equal(lab, want)
+            assert (st["rounds"], st["edge_visits"], st["levels"]) == (so["rounds"], so["edge_visits"], so["levels"])
+    dg.free()
+
+
+@pytest.mark.parametrize("name", ["hubby", "rmat15", "split_hubs", "clique1002"])
+@pytest.mark.parametrize("kind", ["unit", "uniform"])
+@pytest.mark.parametrize("move", [P.NBHR_CLUSTER_MOVE, P.NBHR_MOVE, P.ALL_MOVE])
+def test_graph_loop_without_round_kernel(ctx, name, kind, move):
+    """The degree-binned kernels in the graph loop, families on branches and one
+    after another, on levels that the round kernel takes by default: labels
+    and counters equal the round kernel's."""
+    g = _split_hubs() if name == "split_hubs" else LOOP_GRAPHS[name]()
+    if kind != "unit":
+        g = _weighted(g, WEIGHTS[kind][0])
+    cfg = P.make_config(resolution=0.02, refine=True, move_method=move, louvain_num_iterations=6,
+                        louvain_num_inner_iterations=5)
+    with pytest.MonkeyPatch.context() as mp:
+        mp.setenv("PCC_SERIAL_FAMILIES", "1")
+        serial = P.Context(0)
+    out = []
+    try:
+        for c, kernel in ((ctx, True), (ctx, False), (serial, True)):
+            c.set_round_kernel(kernel)
+            dg = c.upload(g)
+            out.append(P.correlation_cluster(dg, cfg))
+            dg.free()
+    finally:
+        ctx.set_round_kernel(True)
+        serial.close()
+    for lab, st in out[1:]:
+        np.testing.assert_array_equal(lab, out[0][0])
+        assert st["kernel_launches"] > out[0][1]["kernel_launches"]
+        for key in ("objective", "num_clusters", "levels", "rounds", "refine_passes", "edge_visits", "vertex_visits",
+                    "moves", "family_entries", "family_vertices"):
+            assert st[key] == out[0][1][key], key
+
+
+def _clique_moves(ctx, size, w_of, res):
+    """A best-move pass and a clustering of one clique with the given weights
+    (and a few isolated vertices), against the oracle's bits."""
+    g = _weighted(_ring_of_cliques(1, size, extra=9), w_of)
+    dg, og = ctx.upload(g), O.OracleGraph(g)
+    rng = np.random.default_rng(size)
+    one = np.ones(g.n)
+    for clusters in (1, 2, 7, g.n):
+        C = rng.integers(0, clusters, g.n).astype(np.uint32)
+        s, K = np.bincount(C, minlength=g.n).astype(np.uint32), np.bincount(C, minlength=g.n).astype(np.float64)
+        cfg = P.make_config(resolution=res)
+        for got, exp in zip(P.best_moves(dg, cfg, C, s, one, K), O.best_moves(og, cfg, C, s, one, K)):
+            np.testing.assert_array_equal(got.view(np.uint64 if got.dtype == np.float64 else got.dtype),
+                                          exp.view(np.uint64 if exp.dtype == np.float64 else exp.dtype))
+    dg.free()
+    _same(ctx, g, P.make_config(resolution=res, refine=True))
+
+
+@pytest.mark.parametrize("size,weight", [
+    (256, 2.0 ** 22), (257, 2.0 ** 22),                          # integers: rows of 2^30 - 2^22 and 2^30
+    (128, 2.0 ** 22 + 0.5), (129, 2.0 ** 22 + 0.5),              # halves: just below and above 2^30 units
+    (256, 2.0 ** 44), (257, 2.0 ** 44),                          # beside weights of 1: below and at 2^52
+    (256, 2.0 ** 14), (257, 2.0 ** 14)])                         # beside weights of 2^-30: below and at 2^52 units
+@pytest.mark.parametrize("sign", [1, -1, 0])
+def test_sums_at_the_limits(ctx, size, weight, sign):
+    """Rows whose sums lie right below and above the lines between 32-bit and
+    64-bit sums and between those and FP64; both signs, and mixed ones."""
+    small = {2.0 ** 44: 1.0, 2.0 ** 14: 2.0 ** -30}.get(weight)
+
+    def w_of(a, b):
+        w = np.full(a.shape, weight)
+        if small:
+            w[(a * 31 + b * 17) % 11 == 0] = small
+        return w * (sign if sign else np.where((a + b) % 2, 1.0, -1.0))
+
+    _clique_moves(ctx, size, w_of, 0.3 * weight)
+
+
+@pytest.mark.parametrize("kind", ["subnormal", "zero", "least", "negative_zero"])
+def test_tiny_weights(ctx, kind):
+    """Subnormal weights, the smallest one among ones, and zeros of both signs."""
+    w_of = {"subnormal": lambda a, b: np.ldexp(1.0 + (a * 7 + b * 13) % 5, -149),
+            "least": lambda a, b: np.where((a + b) % 9 == 0, np.ldexp(1.0, -149), 1.0),
+            "zero": lambda a, b: 0.0 * a,
+            "negative_zero": lambda a, b: np.where((a + b) % 3 == 0, -0.0, 2.0)}[kind]
+    _clique_moves(ctx, 70, w_of, {"subnormal": 1e-45, "least": 0.4, "zero": 0.4, "negative_zero": 0.4}[kind])
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_rows_beside_infinite_and_nan_weights(ctx, value):
+    """One edge of infinite or undefined weight decides nothing for the rows that
+    do not hold it."""
+    g = _hubby()
+    far = g.neighbors[g.offsets[20]]
+    g = _weighted(g, lambda a, b: np.where((np.minimum(20, far) == a) & (np.maximum(20, far) == b), value,
+                                           1.0 + (a + b) % 4))
+    rows = np.repeat(np.arange(g.n), np.diff(g.offsets).astype(np.int64))
+    odd = np.unique(rows[~np.isfinite(g.weights)])
+    assert odd.size == 2
+    low = (np.diff(g.offsets) <= 1000) & ~np.isin(np.arange(g.n), odd)
+    dg, og = ctx.upload(g), O.OracleGraph(g)
+    C = np.random.default_rng(1).integers(0, 40, g.n).astype(np.uint32)
+    one = np.ones(g.n)
+    s, K = np.bincount(C, minlength=g.n).astype(np.uint32), np.bincount(C, minlength=g.n).astype(np.float64)
+    cfg = P.make_config(resolution=0.02)
+    for got, exp in zip(P.best_moves(dg, cfg, C, s, one, K), O.best_moves(og, cfg, C, s, one, K)):
+        np.testing.assert_array_equal(got[low], exp[low])
+    dg.free()
