@@ -51,9 +51,7 @@ __device__ __forceinline__ V WarpMaxV(V x) {
   if constexpr (sizeof(V) == 4) {
     return __reduce_max_sync(kFull, x);
   } else {
-    const int hi = __reduce_max_sync(kFull, int(x >> 32));
-    const unsigned lo = __reduce_max_sync(kFull, int(x >> 32) == hi ? unsigned(x) : 0u);
-    return static_cast<V>((static_cast<unsigned long long>(static_cast<unsigned>(hi)) << 32) | lo);
+    return WarpMaxLL(x);
   }
 }
 
@@ -664,9 +662,11 @@ __device__ __noinline__ bool TeamExact(const BMArgs& a, const VertexCtx& x, V* v
   return append;
 }
 
-// A team of TW warps (its thread index tid) on one vertex x of degree
-// <= HC / 2, with the team's table (clean before and after, as sh.nused) and
-// hardware barrier.  Returns (on thread 0) whether the vertex must be
+// A team of TW warps (its thread index tid) on one vertex x of degree below
+// HC (the table must not fill: up to HC / 2 for the teams and small hubs, 3/4 HC
+// for the hubs of one partition), with the team's table (clean before and after,
+// as sh.nused), a `used` list of at least degree entries, and its hardware
+// barrier.  Returns (on thread 0) whether the vertex must be
 // appended to the movers list.
 template <int HC, typename V, bool kConv, class L, int TW = kCtaWarps>
 __device__ __forceinline__ bool CtaStep(const BMArgs& a, const RoundView& rv, const VertexCtx& x, V* vals,

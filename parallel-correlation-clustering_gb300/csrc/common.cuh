@@ -416,6 +416,14 @@ __device__ __forceinline__ double Dmul(double a, double b) { return __dmul_rn(a,
 __device__ __forceinline__ double Dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double Dsub(double a, double b) { return __dsub_rn(a, b); }
 
+// Sum of x over the lanes of `peers` (the caller's match group), in lane
+// order; every lane of the group gets the result.
+__device__ __forceinline__ double GroupSum(unsigned peers, double x) {
+  double tot = 0.0;
+  for (unsigned mm = peers; mm; mm &= mm - 1) tot += __shfl_sync(peers, x, __ffs(mm) - 1);
+  return tot;
+}
+
 }  // namespace pcc
 
 // The opaque C-ABI types.

@@ -43,7 +43,7 @@ constexpr int kSegCtaItems = kSegCtaMax / kSegCtaThreads;
 constexpr int kSegCtaWarps = kSegCtaThreads / 32;
 
 // Counters of one contraction, read back together where they are needed.
-struct CompressHead {  // (at most 256 bytes: Context::kPinCompress)
+struct CompressHead {  // (copied to Context::kPinCompress)
   uint32_t max_c;               // largest cluster id
   uint32_t R;                   // clusters in use
   uint32_t counts[4];           // segments per class
@@ -51,6 +51,7 @@ struct CompressHead {  // (at most 256 bytes: Context::kPinCompress)
   unsigned long long m2;        // entries of the new graph
   WeightStats stats;            // of its weights
 };
+static_assert(sizeof(CompressHead) <= Context::kPinBins - Context::kPinCompress, "staging");
 
 // pres[c] = 1 for every cluster id in use (< n), and the largest one.
 __global__ void __launch_bounds__(256) MarkPresentKernel(uint32_t n, const uint32_t* __restrict__ C,

@@ -376,7 +376,7 @@ struct SetMoveArgs {
 };
 
 // Configures (shared-memory limit, occupancy) every synchronous best-move
-// kernel once per process, so that launches captured into a graph make no
+// kernel, once per device, so that launches captured into a graph make no
 // runtime configuration calls.
 Status PrepareBestMoveKernels();
 
@@ -420,13 +420,20 @@ Status LaunchBestMoves(Context* ctx, const BMArgs& a, const uint32_t* list, cons
                        uint32_t max_deg, int families = kLaunchGroups | kLaunchWarps);
 
 // Level graphs of at most this many entries run their rounds in one kernel
-// (roundloop.cu).  Ten rounds, degree-binned kernels in a graph loop against
-// one kernel: 5.7M entries 4.3 -> 2.8 ms, 9.7M 6.5 -> 5.1 ms, 13.3M with 64-bit
-// sums 6.6 -> 6.5 ms, 20M with 64-bit sums 10.2 -> 12.4 ms, 31.4M 11.9 ->
-// 12.7 ms: above it the tails and launches that the one kernel saves are
-// small, and the binned kernels' higher occupancy wins.
-// (With certified hubs and the push in pieces on the binned side too, a line at
-// 2M or 6M entries still costs RMAT scale 18 17.9 -> 19.6 ms.)
+// (roundloop.cu): below, the launches and tails that it saves are most of a
+// round; above, they are small and the degree-binned kernels' higher occupancy
+// wins.  Ten rounds of one level, degree-binned kernels in a graph loop, then
+// the one kernel, ms (32-bit sums by unit weights, 64-bit sums by real ones):
+//   entries          1.0-1.8M      4M           6M           8M           12M
+//   RMAT, 32 bits    2.12 1.39   2.56 2.00   2.91 2.51   3.55 3.35   4.52 4.71
+//   RMAT, 64 bits    2.70 1.61   3.39 2.59   3.70 3.46   4.62 4.86   5.69 6.94
+//   LFR, 32 bits     1.49 1.09   2.26 2.13   2.61 2.65   3.08 3.31   4.12 4.61
+//   LFR, 64 bits     1.62 1.30   2.64 2.71   3.28 3.66   3.88 4.66   5.36 6.66
+// and with 32 bits 8.96 11.37 (RMAT, 31M), 6.20 7.43 (LFR, 20M).  The line was
+// drawn at 12M when the degree-binned kernels had no certified hubs and no push
+// in pieces (then 9.7M entries took 6.5 against 5.1 ms, 13.3M with 64-bit sums
+// 6.6 against 6.5).  By these figures the sides are now even near 10M (RMAT) and
+// 5.5M (LFR) entries with 32-bit sums and near 7M and 4M with 64-bit ones.
 constexpr uint64_t kLoopMaxEntries = 12ull << 20;
 
 // The hub plan of a graph (built on first use).  shared: other contexts may

@@ -38,6 +38,8 @@ struct PredNonZeroDegree {
   __device__ bool operator()(uint32_t v) const { return off[v + 1] > off[v]; }
 };
 
+static_assert(kBinWords * sizeof(uint32_t) <= Context::kPinStats - Context::kPinBins, "staging");
+
 // Bins the vertices; waits for the stream (with whatever was queued before).
 Status BuildBins(Context* ctx, const DevGraph* g, BinSet* b, bool include_isolated, uint32_t* max_deg = nullptr) {
   if (include_isolated) {
@@ -84,6 +86,7 @@ Status ComputeGraphProperties(Context* ctx, DevGraph* g, const WeightStats* d_st
     uint64_t m;
     WeightStats ws;
   };
+  static_assert(sizeof(Read) <= Context::kPinLoop - Context::kPinStats, "staging");
   Read* h;
   PCC_RETURN_IF_ERROR(ctx->Pinned(Context::kPinStats, &h));
   h->m = g->m;

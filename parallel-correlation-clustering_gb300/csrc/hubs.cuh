@@ -117,7 +117,7 @@ struct HubState {
 };
 
 Status BuildHubPlan(Context* ctx, const DevGraph& g, const BinSet& bins, HubPlan* plan);
-// Configures every synchronous hub kernel once per process (for launches
+// Configures every synchronous hub kernel, once per device (for launches
 // captured into a graph).
 Status PrepareHubKernels();
 // Buffers of the hub kernels over the plan (the global path's tables among

@@ -198,19 +198,6 @@ struct ApplyArgs {
   const RoundState* rs;  // non-null: the stamp comes from here
 };
 
-// Sum of x over the lanes of `peers` (the caller's match group), in lane
-// order; every lane of the group gets the result.
-__device__ __forceinline__ double GroupSum(unsigned peers, double x) {
-  double tot = 0.0;
-  unsigned mm = peers;
-  while (mm) {
-    const int j = __ffs(mm) - 1;
-    tot += __shfl_sync(peers, x, j);
-    mm &= mm - 1;
-  }
-  return tot;
-}
-
 // Leave: every mover leaves its cluster (sizes and weights), marks it
 // modified; movers to a new cluster are flagged for ranking.  Equal
 // clusters inside a warp are combined first (one atomic per cluster and

@@ -7,11 +7,12 @@
 // but took 12-33 kernel nodes of a device-side graph loop, 3-4 us each with
 // their launch and drain, and a level's degree bins ran as separate kernels
 // whose tails and serial chains left most of the GPU idle.  Here a round costs
-// its work plus three to six grid barriers of 1-2 us.  Per round, before and
-// after: 576 entries 45 -> 34 us, 4,686 entries 49 -> 27 us, 1M entries 147 ->
-// 77 us, 5.6M entries with a 147,524-entry row 430 -> 270 us.  Every kind of
-// work item goes through one queue, largest items first, so a CTA that runs
-// out of one kind goes on with the next:
+// its work plus grid barriers of 1-2 us: two when no vertex moves, three when
+// some do, three more when clusters are opened, and one more on levels with rows
+// above 4096.  Per round, before and after: 576 entries 45 -> 34 us, 4,686
+// entries 49 -> 27 us, 1M entries 147 -> 77 us, 5.6M entries with a 147,524-entry
+// row 430 -> 270 us.  Every kind of work item goes through one queue, largest
+// items first, so a CTA that runs out of one kind goes on with the next:
 //   stage 0  CTA items: chunks of the rows above degree 4096 (summed into
 //            per-hub tables in HBM), then hubs of degree 1001-4096 (one CTA,
 //            table in shared memory)
@@ -93,13 +94,6 @@ __device__ __forceinline__ uint32_t BlockSum32(uint32_t x, uint32_t* red) {
   for (int w = 0; w < kLW; ++w) r += red[w];
   __syncthreads();
   return r;
-}
-
-// Sum over the lanes of `peers` (the caller's match group).
-__device__ __forceinline__ double PeerSum(unsigned peers, double x) {
-  double tot = 0.0;
-  for (unsigned mm = peers; mm; mm &= mm - 1) tot += __shfl_sync(peers, x, __ffs(mm) - 1);
-  return tot;
 }
 
 // The next frontier: u is stamped; the thread that stamps it first counts it.
@@ -475,7 +469,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
         if (in) l.old_cluster[i] = c;
         {
           const unsigned peers = __match_any_sync(kFull, c);
-          const double tot = PeerSum(peers, kv);
+          const double tot = GroupSum(peers, kv);
           if (in && int(lane) == __ffs(peers) - 1) {
             atomicSub(&a.s_mut[c], uint32_t(__popc(peers)));
             atomicAdd(&a.K_mut[c], -tot);
@@ -488,7 +482,7 @@ __global__ void __launch_bounds__(kLT, 2) RoundLoopKernel(const __grid_constant_
         if (nb && lane == 0) atomicAdd(&ctr->new_movers, uint32_t(__popc(nb)));
         const bool join = in && t != n;
         const unsigned peers = __match_any_sync(kFull, join ? t : kNone);
-        const double tot = PeerSum(peers, join ? kv : 0.0);
+        const double tot = GroupSum(peers, join ? kv : 0.0);
         if (join && int(lane) == __ffs(peers) - 1) {
           atomicAdd(&a.s_mut[t], uint32_t(__popc(peers)));
           atomicAdd(&a.K_mut[t], tot);
