@@ -611,9 +611,7 @@ Status Prep(K kernel, size_t smem, int threads) {
   return SetSmem(kernel, smem, threads, &per_sm);
 }
 
-}  // namespace
-
-Status PrepareBestMoveKernels() {
+Status PrepareAll() {
   PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<4, int>, 0, 256));
   PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<8, int>, 0, 256));
   PCC_RETURN_IF_ERROR(Prep(CertGroupKernel<16, int>, 0, 256));
@@ -653,6 +651,13 @@ Status PrepareBestMoveKernels() {
   PCC_RETURN_IF_ERROR(Prep(BestMoveWarpKernel<1024, false, false>, WarpKernelSmem<1024>(), kW));
   PCC_RETURN_IF_ERROR(Prep(BestMoveWarpKernel<2048, false, false>, WarpKernelSmem<2048>(), kW));
   return Status::Ok();
+}
+
+}  // namespace
+
+Status PrepareBestMoveKernels() {
+  static PerDevice done;
+  return OncePerDevice(done, PrepareAll);
 }
 
 Status LaunchBestMoves(Context* ctx, const BMArgs& a, const uint32_t* list, const uint32_t* bin_counts,

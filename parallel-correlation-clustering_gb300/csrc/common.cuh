@@ -301,6 +301,19 @@ inline Status PrepareKernel(K kernel, int threads, size_t smem, size_t limit, in
   return Status::Ok();
 }
 
+// prepare() -> Status, once per device (`done` is the caller's own).
+template <class F>
+inline Status OncePerDevice(PerDevice& done, F prepare) {
+  int device = 0, unused;
+  PCC_CUDA(cudaGetDevice(&device));
+  Status st;
+  done.Get(device, nullptr, 0, &unused, [&](int*) {
+    st = prepare();
+    return st.ok();
+  });
+  return st;
+}
+
 inline Status LaunchCheck() {
   PCC_CUDA(cudaGetLastError());
   return Status::Ok();

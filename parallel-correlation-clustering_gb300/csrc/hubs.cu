@@ -767,7 +767,9 @@ Status AllocLoopTables(Context* ctx, const HubPlan& plan, HubState* st, bool res
   return AllocTables(ctx, plan.loop_slots, plan.num_big, plan.num_loop_slices, st, reset);
 }
 
-Status PrepareHubKernels() {
+namespace {
+
+Status PrepareAllHubKernels() {
   bool ok = true;
   auto small = [&](auto k, size_t slots, size_t vsize) {
     ok = ok && PrepareOnce(k, kSmallThreads, slots * (vsize + sizeof(uint32_t))) > 0;
@@ -792,6 +794,13 @@ Status PrepareHubKernels() {
   big(HubBigKernel<true, false, long long>, BigSlots<long long>(), sizeof(long long));
   big(HubBigKernel<false, false, double>, BigSlots<double>(), sizeof(double));
   return ok ? Status::Ok() : MakeError(PCC_INTERNAL, "hub kernels cannot be configured");
+}
+
+}  // namespace
+
+Status PrepareHubKernels() {
+  static PerDevice done;
+  return OncePerDevice(done, PrepareAllHubKernels);
 }
 
 Status LaunchHubBestMoves(Context* ctx, const BMArgs& a, const HubPlan& plan, HubState& st, bool int_mode,
