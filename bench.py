@@ -59,7 +59,7 @@ UNIT = "edge-visits/s"
 # frontier; cold L2); the summary and command are in profiles/.  Traffic
 # scales with the entries evaluated, so the per-launch figure at the bench's
 # size is this times the entries of a launch.
-TRAFFIC_BYTES_PER_ENTRY = {"groups": 51.9, "warps": 8.82, "small_hubs": 6.22, "big_hubs": 9.92}
+TRAFFIC_BYTES_PER_ENTRY = {"groups": 37.2, "warps": 8.82, "small_hubs": 6.23, "big_hubs": 12.3}
 
 
 def parse_args():
@@ -469,7 +469,7 @@ def serving_leg(args, P, G, ctx):
             "sbm": {"requests": len(sbm_idx), "capacity": cap_sbm, "per_graph_calls": plain_sbm,
                     "speedup_vs_per_graph_calls": cap_sbm / plain_sbm},
             "rmat20": {"requests": len(rmat_idx), "capacity": cap_rmat,
-                       "note": "RMAT scale 20 requests take 30-220 ms each alone (NBHR_CLUSTER_MOVE); "
+                       "note": "RMAT scale 20 requests take 15-106 ms each alone (NBHR_CLUSTER_MOVE); "
                                "they bound the mix's closed-loop capacity"},
         },
         "loads": loads,
