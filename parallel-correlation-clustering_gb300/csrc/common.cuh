@@ -78,8 +78,8 @@ struct Context {
   // Calls were let in by an estimate of their device memory (a pool with an HBM
   // budget, serve.cu), so large ones keep to what a budget would make them use:
   // arrays of their exact size, freed as they are spent.  Calls of at most
-  // kAdmittedSmall entries need not: they differ by at most 12 MB, inside the
-  // estimate's fixed 64.
+  // kAdmittedSmall entries need not: theirs take up to 36 bytes a vertex (of at
+  // most 1M) and 8 an entry more, which the estimate's fixed 64 MB cover.
   bool admitted = false;
   static constexpr uint64_t kAdmittedSmall = 1u << 20;
   bool Frugal(uint64_t entries) const { return budget || (admitted && entries > kAdmittedSmall); }

@@ -278,8 +278,9 @@ extern "C" {
 // state, the engine's per-round arrays, and the contraction of level 0
 // (sort keys and values with their double buffers) -- the peak -- plus a
 // fixed allowance for pools and small tables.  Levels kept for refinement are
-// not counted one by one: ten that hardly shrink can exceed it by some percent
-// (LFR, 150,000 vertices with weights, resolution 0.5: 294 MB for 277).
+// not counted one by one: ten that hardly shrink exceed it, by some percent
+// (LFR, 150,000 vertices with weights, resolution 0.5: 294 MB for 277) or, on
+// sparse graphs, twice (1M vertices and 1M entries: 648 MB for 311).
 uint64_t pcc_request_bytes_estimate(uint32_t n, uint64_t m, int32_t has_weights) {
   const uint64_t per_entry = 52 + (has_weights ? 8 : 0);
   return per_entry * m + 192ull * n + (64ull << 20);

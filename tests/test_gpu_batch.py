@@ -298,13 +298,22 @@ def _pool_used():
     return used.value, high.value
 
 
-@pytest.mark.parametrize("iterations,res", [(4, 0.5), (9, 0.5), (10, 0.1)])
-def test_request_estimate_bounds_served_peak(built, iterations, res):
+@pytest.mark.parametrize("kind,iterations,res", [("lfr", 4, 0.5), ("lfr", 9, 0.5), ("lfr", 10, 0.1),
+                                                 ("sparse", 2, 0.1), ("sbm", 10, 0.5)])
+def test_request_estimate_bounds_served_peak(built, kind, iterations, res):
     """The memory of a request in a pool with a budget stays within the estimate
     that let it in, also where many levels that hardly shrink are kept for
-    refinement."""
-    g, _ = G.lfr(150000, mean_degree=20, dmax=2000, seed=6)
-    est = P.request_bytes_estimate(g.n, g.m, True)
+    refinement, and where the graph is just small enough for the arrays of a
+    context without a budget."""
+    if kind == "lfr":
+        g, _ = G.lfr(150000, mean_degree=20, dmax=2000, seed=6)
+    elif kind == "sbm":
+        g, _ = G.sbm(50000, 100, 0.018, 0.0002, 3)
+    else:
+        ends = np.random.default_rng(2).integers(0, 1000000, (2, 500000))
+        g = P.CsrGraph.from_edges(1000000, ends[0], ends[1], drop_self_loops=True)
+    est = P.request_bytes_estimate(g.n, g.m, g.weights is not None)
+    assert kind == "lfr" or g.m <= 1 << 20
     srv = P.Server(slots=1, hbm_budget=est)
     try:
         held, _ = _pool_used()
